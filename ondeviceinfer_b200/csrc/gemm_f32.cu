@@ -1,71 +1,121 @@
 // True 32-bit matrix product for the float32 path: C[M,N] = A[M,K] * W[N,K]^T (+ bias[N]) (+ R).
 //
-// Plain FMA on the CUDA cores: no tensor cores, no TF32, no split of the K loop.  Each
-// output element is accumulated over k = 0..K-1 in that order whatever M is, so a row's
-// result does not depend on how many other rows are in the batch.
+// Plain FMA on the CUDA cores: no tensor cores, no TF32.  Each output element is two running sums, one over the even
+// and one over the odd k, each in rising k, added at the end: whatever M, N and the tile, so a row's result does not
+// depend on how many other rows are in the batch.
 //
-// 64x64 output tile per block of 256 threads, 4x4 outputs per thread, K in slices of 16
-// staged through shared memory (stored k-major so the inner loop reads float4s).
-// Any M, N, K >= 1; rows of A and W are read with float4 when K, lda, ldw are multiples
-// of 4 and the bases 16-byte aligned, else element by element.
+// What bounds it: with many rows the FMA pipes (128 multiply-adds per clock and multiprocessor, 74 TFLOP/s at
+// 1,965 MHz), with a few rows the weights' bytes.  The two sums are the halves of a packed fma.rn.f32x2 whose operands are
+// neighbouring k of a row, as shared memory holds them: no operand is moved or doubled, and a thread's tile of RM x RN
+// outputs takes RM + RN 8-byte reads per RM RN packed operations.  128 threads as 8 x 16; a thread owns rows
+// ty + 8 i and columns tx + 16 j, so that the lanes of a warp read neighbouring rows of the stage (4 rows of A,
+// 8 of W): at a row pitch of 36 words no two of them meet in a bank.  Stages of 32 k arrive by asynchronous copies.
+// Any M, N, K >= 1; 16-byte copies when K, lda, ldw are multiples of 4 and the bases 16-byte aligned, else 4-byte ones.
 #include "common.cuh"
 
-#define TM 64
-#define TN 64
-#define TK 16
+#define KS 32                 // k per stage
+#define PITCH (KS + 4)        // floats per staged row
+#define NTH 128
 
-template <bool VEC>
-__global__ void __launch_bounds__(256)
-gemm_f32_kernel(const float* __restrict__ A, const float* __restrict__ W, float* C,
-                const float* R, const float* __restrict__ bias, int M, int N, int K, int lda, int ldw, int ldc, int ldr) {
-  pdl_launch_dependents();
-  pdl_wait();
-  __shared__ __align__(16) float As[TK][TM + 4];
-  __shared__ __align__(16) float Ws[TK][TN + 4];
-  const int tid = threadIdx.x;
-  const int m0 = blockIdx.y * TM, n0 = blockIdx.x * TN;
-  const int tx = tid & 15, ty = tid >> 4;  // 16 x 16 threads; thread owns rows ty*4.., cols tx*4..
-  const int lr = tid >> 2, lk = (tid & 3) * 4;  // loader: row lr of the tile, k offset lk
-  float acc[4][4] = {};
+__device__ __forceinline__ void cp_async16(uint32_t dst, const float* src, bool ok) {      // zeros where !ok
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(ok ? 16 : 0) : "memory");
+}
+__device__ __forceinline__ void cp_async4(uint32_t dst, const float* src, bool ok) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst), "l"(src), "r"(ok ? 4 : 0) : "memory");
+}
+__device__ __forceinline__ void fma_pair(unsigned long long& acc, unsigned long long a, unsigned long long w) {
+  asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(a), "l"(w));
+}
 
-  for (int k0 = 0; k0 < K; k0 += TK) {
-    float a[4] = {0.f, 0.f, 0.f, 0.f}, w[4] = {0.f, 0.f, 0.f, 0.f};
-    const int gm = m0 + lr, gn = n0 + lr, gk = k0 + lk;
-    if (VEC) {
-      if (gm < M && gk < K) { float4 v = *(const float4*)(A + (size_t)gm * lda + gk); a[0] = v.x; a[1] = v.y; a[2] = v.z; a[3] = v.w; }
-      if (gn < N && gk < K) { float4 v = *(const float4*)(W + (size_t)gn * ldw + gk); w[0] = v.x; w[1] = v.y; w[2] = v.z; w[3] = v.w; }
-    } else {
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        if (gm < M && gk + i < K) a[i] = A[(size_t)gm * lda + gk + i];
-        if (gn < N && gk + i < K) w[i] = W[(size_t)gn * ldw + gk + i];
-      }
+// ROWS rows of X [limit, K] from row r0 on, k0 .. k0 + KS - 1, into dst (pitch PITCH); zeros beyond either end
+template <int ROWS, bool VEC>
+__device__ __forceinline__ void stage_rows(uint32_t dst, const float* __restrict__ X, int r0, int limit, int k0, int K, int ld) {
+  if (VEC) {
+    for (int i = threadIdx.x; i < ROWS * (KS / 4); i += NTH) {
+      const int r = i / (KS / 4), k = (i % (KS / 4)) * 4;
+      const bool ok = r0 + r < limit && k0 + k < K;
+      cp_async16(dst + (r * PITCH + k) * 4, ok ? X + (size_t)(r0 + r) * ld + k0 + k : X, ok);
     }
-    __syncthreads();
-#pragma unroll
-    for (int i = 0; i < 4; ++i) { As[lk + i][lr] = a[i]; Ws[lk + i][lr] = w[i]; }
-    __syncthreads();
-#pragma unroll
-    for (int k = 0; k < TK; ++k) {
-      const float4 av = *(const float4*)&As[k][ty * 4];
-      const float4 wv = *(const float4*)&Ws[k][tx * 4];
-      const float ar[4] = {av.x, av.y, av.z, av.w};
-      const float wr[4] = {wv.x, wv.y, wv.z, wv.w};
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(ar[i], wr[j], acc[i][j]);
+  } else {
+    for (int i = threadIdx.x; i < ROWS * KS; i += NTH) {
+      const int r = i / KS, k = i % KS;
+      const bool ok = r0 + r < limit && k0 + k < K;
+      cp_async4(dst + (r * PITCH + k) * 4, ok ? X + (size_t)(r0 + r) * ld + k0 + k : X, ok);
     }
   }
+}
+
+template <int RM, int RN, int STAGES, bool VEC>
+__global__ void __launch_bounds__(NTH)
+gemm_f32_kernel(const float* __restrict__ A, const float* __restrict__ W, float* C,
+                const float* R, const float* __restrict__ bias, int M, int N, int K, int lda, int ldw, int ldc, int ldr) {
+  constexpr int BM = 8 * RM, BN = 16 * RN, STAGE = (BM + BN) * PITCH;
+  extern __shared__ __align__(16) float smem[];
+  pdl_wait();
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int ty = (warp & 1) * 4 + (lane >> 3), tx = (warp >> 1) * 8 + (lane & 7);
+  const int row_tiles = (M + BM - 1) / BM;      // those of a column tile run side by side: they share its weights in L2
+  const int m0 = blockIdx.x % row_tiles * BM, n0 = blockIdx.x / row_tiles * BN;
+  const uint32_t base = (uint32_t)__cvta_generic_to_shared(smem);
+  const int n_stages = (K + KS - 1) / KS;
+  auto issue = [&](int s) {
+    if (s < n_stages) {
+      const uint32_t dst = base + (s % STAGES) * STAGE * 4;
+      stage_rows<BM, VEC>(dst, A, m0, M, s * KS, K, lda);
+      stage_rows<BN, VEC>(dst + BM * PITCH * 4, W, n0, N, s * KS, K, ldw);
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  unsigned long long acc[RM][RN];
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const int m = m0 + ty * 4 + i;
+  for (int i = 0; i < RM; ++i)
+#pragma unroll
+    for (int j = 0; j < RN; ++j) acc[i][j] = 0ull;
+
+  // operands of two k at a time in two sets of registers: the next two are read while these are multiplied
+  unsigned long long a[2][RM], w[2][RN];
+  auto read = [&](int set, int s, int k) {
+    const float* as = smem + (s % STAGES) * STAGE + ty * PITCH + k;
+    const float* ws = smem + (s % STAGES) * STAGE + (BM + tx) * PITCH + k;
+#pragma unroll
+    for (int i = 0; i < RM; ++i) a[set][i] = *(const unsigned long long*)(as + 8 * i * PITCH);
+#pragma unroll
+    for (int j = 0; j < RN; ++j) w[set][j] = *(const unsigned long long*)(ws + 16 * j * PITCH);
+  };
+
+#pragma unroll
+  for (int s = 0; s < STAGES; ++s) issue(s);
+  asm volatile("cp.async.wait_group %0;" ::"n"(STAGES - 1) : "memory");
+  __syncthreads();
+  read(0, 0, 0);
+  for (int s = 0; s < n_stages; ++s) {
+#pragma unroll
+    for (int k = 0; k < KS; k += 2) {
+      const int set = (k >> 1) & 1;
+      if (k + 2 < KS) {
+        read(set ^ 1, s, k + 2);
+      } else {
+        asm volatile("cp.async.wait_group %0;" ::"n"(STAGES - 2) : "memory");
+        __syncthreads();      // stage s + 1 has arrived; everybody has read the last of stage s, whose place the next copies take
+        if (s + 1 < n_stages) read(set ^ 1, s + 1, 0);
+        issue(s + STAGES);
+      }
+#pragma unroll
+      for (int i = 0; i < RM; ++i)
+#pragma unroll
+        for (int j = 0; j < RN; ++j) fma_pair(acc[i][j], a[set][i], w[set][j]);
+    }
+  }
+  pdl_launch_dependents();      // not earlier: blocks of the next kernel would take the places of this one's
+#pragma unroll
+  for (int i = 0; i < RM; ++i) {
+    const int m = m0 + ty + 8 * i;
     if (m >= M) continue;
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const int n = n0 + tx * 4 + j;
+    for (int j = 0; j < RN; ++j) {
+      const int n = n0 + tx + 16 * j;
       if (n >= N) continue;
-      float v = acc[i][j];
+      float v = __uint_as_float((unsigned)acc[i][j]) + __uint_as_float((unsigned)(acc[i][j] >> 32));
       if (bias != nullptr) v += bias[n];
       if (R != nullptr) v += R[(size_t)m * ldr + n];
       C[(size_t)m * ldc + n] = v;
@@ -73,17 +123,70 @@ gemm_f32_kernel(const float* __restrict__ A, const float* __restrict__ W, float*
   }
 }
 
+template <int RM, int RN, int STAGES, bool VEC>
+static int launch_form(const float* A, const float* W, float* C, const float* R, const float* bias, int M, int N, int K,
+                       int lda, int ldw, int ldc, int ldr, cudaStream_t stream) {
+  constexpr size_t smem = sizeof(float) * STAGES * (8 * RM + 16 * RN) * PITCH;
+  const long tiles = (long)((M + 8 * RM - 1) / (8 * RM)) * ((N + 16 * RN - 1) / (16 * RN));
+  if (tiles > 0x7fffffffL) return ODI_ERR_UNSUPPORTED;
+  const dim3 grid((unsigned)tiles);
+  if (smem > 48 * 1024) {
+    const cudaError_t e = cudaFuncSetAttribute(gemm_f32_kernel<RM, RN, STAGES, VEC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return (int)e;
+  }
+  odi_rc = launch_pdl((gemm_f32_kernel<RM, RN, STAGES, VEC>), grid, dim3(NTH), smem, stream, A, W, C, R, bias, M, N, K, lda, ldw, ldc, ldr);
+  return launch_status();
+}
+
+// The tile of a product: the one with the least time by what the forms measured.  c tiles side by side on a multiprocessor take
+// first + (c - 1) more (us at K = 4,096, all in proportion to K: below), `slots` of them fit; the last wave counts with the tiles
+// that its busiest multiprocessor gets, which has a second one before all 148 have one (from about 133 tiles on, tall tiles from
+// about 110).  Measured, best form by the rule against the 64 x 64 tile of 4 x 4 outputs a thread that served every size before
+// (us): 185 x 24,576 x 4,096 871 and 1,170; 185 x 4,096 x 12,288 682 and 1,210; 185 x 151,936 x 4,096 5,253 (43.8 TFLOP/s) and 6,824;
+// 1,024 x 24,576 x 4,096 4,427 and 5,877; 3 x 4,096 x 4,096 51 and 210.  Norm of the error against 64 bits, K = 4,096: 8.1e-7, 1.15e-6
+// before (one chain of sums).  At 64 x 128 the FMA pipes are busy 62 % of the time: beside them the reads of shared memory want 45 %.
+// `force` picks a form for sweeps and tests (-1: by the rule).
+struct F32Form { int rows, cols, slots; double first, more; };
+static const F32Form forms[] = {{8, 32, 4, 51, 18}, {8, 64, 3, 83, 24}, {16, 32, 4, 60, 22.5}, {16, 64, 3, 94, 35}, {32, 32, 4, 93, 32},
+                                {32, 64, 4, 122, 58.5}, {48, 64, 3, 145, 85}, {64, 64, 4, 170, 106}, {64, 128, 2, 253, 181}};
+#define F32_FORMS 9
+static int pick_form(int M, int N) {
+  int best = 0;
+  double least = 1e300;
+  for (int f = 0; f < F32_FORMS; ++f) {
+    const F32Form& x = forms[f];
+    const long tiles = (long)((M + x.rows - 1) / x.rows) * ((N + x.cols - 1) / x.cols), wave = 148L * x.slots, rest = tiles % wave;
+    double cost = (double)(tiles / wave) * (x.first + (x.slots - 1) * x.more);
+    if (rest > 0) cost += x.first + (double)min(x.slots - 1L, (rest - 1) / (x.rows < 64 ? 133 : 110)) * x.more;
+    if (cost < least) { least = cost; best = f; }
+  }
+  return best;
+}
+
 // R may be null (no residual) or alias C (in-place add: each element is read and then
 // written by the same thread).  bias may be null; it is added to the product before the residual.
 extern "C" int odi_gemm_f32(const float* A, const float* W, float* C, const float* R, const float* bias, int M, int N,
-                            int K, int lda, int ldw, int ldc, int ldr, cudaStream_t stream) {
+                            int K, int lda, int ldw, int ldc, int ldr, int force, cudaStream_t stream) {
   if (M <= 0 || N <= 0) return 0;
   if (K <= 0) return ODI_ERR_ARGUMENT;
-  dim3 grid((N + TN - 1) / TN, (M + TM - 1) / TM);
-  if (grid.y > 65535) return ODI_ERR_UNSUPPORTED;
+  if ((M - 1) / 64 >= 65535) return ODI_ERR_UNSUPPORTED;
   const bool vec = (K % 4 == 0) && (lda % 4 == 0) && (ldw % 4 == 0) &&
                    ((uintptr_t)A % 16 == 0) && ((uintptr_t)W % 16 == 0);
-  if (vec) odi_rc = launch_pdl((gemm_f32_kernel<true>), dim3(grid), dim3(256), 0, stream, A, W, C, R, bias, M, N, K, lda, ldw, ldc, ldr);
-  else odi_rc = launch_pdl((gemm_f32_kernel<false>), dim3(grid), dim3(256), 0, stream, A, W, C, R, bias, M, N, K, lda, ldw, ldc, ldr);
-  return launch_status();
+  const int form = force >= 0 && force < F32_FORMS ? force : pick_form(M, N);
+#define ODI_F32(RM, RN, STAGES) launch_form<RM, RN, STAGES, true>(A, W, C, R, bias, M, N, K, lda, ldw, ldc, ldr, stream)
+#define ODI_F32_SCALAR(RM, RN) launch_form<RM, RN, 3, false>(A, W, C, R, bias, M, N, K, lda, ldw, ldc, ldr, stream)
+  if (!vec) return form < 4 ? ODI_F32_SCALAR(2, 4) : (form < 6 ? ODI_F32_SCALAR(4, 4) : ODI_F32_SCALAR(8, 8));
+  switch (form) {
+    case 0: return ODI_F32(1, 2, 8);
+    case 1: return ODI_F32(1, 4, 6);
+    case 2: return ODI_F32(2, 2, 8);
+    case 3: return ODI_F32(2, 4, 6);
+    case 4: return ODI_F32(4, 2, 6);
+    case 5: return ODI_F32(4, 4, 4);
+    case 6: return ODI_F32(6, 4, 4);
+    case 7: return ODI_F32(8, 4, 3);
+    default: return ODI_F32(8, 8, 3);
+  }
+#undef ODI_F32
+#undef ODI_F32_SCALAR
 }

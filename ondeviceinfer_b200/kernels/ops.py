@@ -261,8 +261,9 @@ def _require_bias(bias: Optional[torch.Tensor], rows: int) -> None:
 
 
 def gemm_f32(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, residual: Optional[torch.Tensor] = None,
-             bias: Optional[torch.Tensor] = None) -> None:
-    """out[M,N] = a[M,K] w[N,K]^T (+ bias[N]) (+ residual) in true fp32; residual may be ``out`` itself."""
+             bias: Optional[torch.Tensor] = None, form: int = -1) -> None:
+    """out[M,N] = a[M,K] w[N,K]^T (+ bias[N]) (+ residual) in true fp32; residual may be ``out`` itself.  ``form`` names a
+    tile of the kernel (sweeps and tests; all give the same bits), -1: by its rule."""
     _require(a, "a", torch.float32, 2)
     _require(w, "w", torch.float32, 2)
     _require(out, "out", torch.float32, 2)
@@ -277,7 +278,7 @@ def gemm_f32(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, residual: Opti
     _require_bias(bias, N)
     lib = load_library("gemm_f32")
     _check(lib.odi_gemm_f32(_ptr(a), _ptr(w), _ptr(out), _ptr(residual), _ptr(bias), c_int(M), c_int(N), c_int(K),
-                            c_int(K), c_int(K), c_int(N), c_int(N), _stream()), "gemm_f32")
+                            c_int(K), c_int(K), c_int(N), c_int(N), c_int(form), _stream()), "gemm_f32")
 
 
 EPI_STORE_BF16, EPI_STORE_F32, EPI_RESIDUAL, EPI_SWIGLU, EPI_HEAD_PREP, EPI_GELU, EPI_GEGLU, EPI_RELU2 = 0, 1, 2, 3, 4, 5, 6, 7

@@ -333,6 +333,21 @@ def test_gemm_f32_is_true_fp32_and_row_independent(M, N, K):
     assert torch.equal(r.cpu(), (out.cpu() + bias) + res)
 
 
+@pytest.mark.parametrize("form", range(9))
+def test_gemm_f32_tiles_give_the_same_bits(form):
+    # every tile at sizes around its edges, K around a stage of 32 and off its multiples of 4 (4-byte copies)
+    torch.manual_seed(9)
+    for M, N, K in [(1, 1, 1), (9, 65, 31), (47, 113, 36), (65, 129, 64), (131, 225, 33), (193, 97, 260)]:
+        a, w = torch.randn(M, K, device=DEV), torch.randn(N, K, device=DEV)
+        out, one = torch.full((M, N), math.nan, device=DEV), torch.empty(1, N, device=DEV)
+        ops.gemm_f32(a, w, out, form=form)
+        # at most K / 2 + 1 roundings of 2^-24 each of sums below sum |a||w|
+        bound = (K / 2 + 1) * 2.0 ** -24 * (a.double().abs() @ w.double().abs().t())
+        assert bool(((out.double() - a.double() @ w.double().t()).abs() <= bound).all())
+        ops.gemm_f32(a[M - 1:].contiguous(), w, one)
+        assert torch.equal(one[0], out[M - 1])
+
+
 def test_sample_greedy_ties_and_temperature_against_plain():
     torch.manual_seed(8)
     V = 1237
