@@ -18,7 +18,7 @@
 //              q, k, g, v and beta are staged through shared memory 16 (8 for wide heads) tokens at a time, the next
 //              chunk being requested into registers while the current one is worked through;
 //  out_norm    per (token, head): o / rms(o) (eps inside the root) * weight * sigmoid(gate), rounded to T.
-#include "common.cuh"
+#include "delta_chunk.cuh"
 
 #ifndef ODI_DELTA_DIM
 #error "compile with -DODI_DELTA_DIM=<key size of a head>"
@@ -53,6 +53,7 @@ struct DeltaArgs {
   float* beta;            // [n_tokens, heads]
   float* state;           // [slots, heads, d, dv]
   float* o;               // [n_tokens, heads * dv]
+  float* chunks;          // scratch of the run in chunks (delta_chunk.cuh): slots * heads * (DC_WORDS(D) + 2 DC dv); null: token by token
   const float* norm_w;    // [dv]
   void* out;              // [n_tokens, heads * dv] in T
   const int* cu_q;
@@ -244,34 +245,141 @@ __global__ void delta_values_kernel(DeltaArgs a) {
   for (int i = threadIdx.x; i < n; i += blockDim.x) a.o[(size_t)t * n + i] = to_f<T>(v[i]);
 }
 
+// One warp per (token, head).
 template <typename T>
 __global__ void __launch_bounds__(128)
 delta_out_norm_kernel(DeltaArgs a) {
   pdl_launch_dependents();
   pdl_wait();
-  __shared__ float scratch[33];
-  const int t = blockIdx.x, h = blockIdx.y;
-  const float* o = a.o + (size_t)t * a.heads * a.dv + h * a.dv;
-  const float* gate = a.decay_in + (size_t)t * a.ld_decay + a.heads * D + h * a.dv;
+  const int lane = threadIdx.x & 31;
+  const long item = (long)blockIdx.x * 4 + (threadIdx.x >> 5);
+  if (item >= (long)a.n_tokens * a.heads) return;
+  const size_t t = item / a.heads;
+  const int h = (int)(item % a.heads);
+  const float* o = a.o + item * a.dv;
+  const float* gate = a.decay_in + t * a.ld_decay + a.heads * D + (size_t)h * a.dv;
   float ss = 0.f;
-  for (int i = threadIdx.x; i < a.dv; i += blockDim.x) ss += o[i] * o[i];
-  ss = block_sum(ss, scratch);
+  for (int i = lane; i < a.dv; i += 32) ss = fmaf(o[i], o[i], ss);
+  ss = warp_sum(ss);
   const float inv = 1.0f / sqrtf(ss / (float)a.dv + a.eps);
-  T* out = (T*)a.out + (size_t)t * a.heads * a.dv + h * a.dv;
-  for (int i = threadIdx.x; i < a.dv; i += blockDim.x)
-    out[i] = from_f<T>(o[i] * inv * a.norm_w[i] / (1.f + expf(-gate[i])));
+  T* out = (T*)a.out + item * a.dv;
+  for (int i = lane; i < a.dv; i += 32) out[i] = from_f<T>(o[i] * inv * a.norm_w[i] / (1.f + expf(-gate[i])));
 }
+
+#if D % 64 == 0 && D <= 128
+#define ODI_DELTA_CHUNKS 1
+// The parts of a chunk straight from the projections: convolutions (rounded to T as the conv kernel does), unit vectors,
+// decays, step sizes, then dc_parts.
+template <typename T>
+__global__ void __launch_bounds__(2 * D)
+delta_parts_kernel(DeltaArgs a, DeltaChunkArgs c) {
+  pdl_launch_dependents();
+  pdl_wait();
+  __shared__ DeltaChunkShared<D> sh;
+  const int h = blockIdx.y, src = h / (a.heads / a.kv_heads);
+  int seq, first, nt;
+  if (!run_chunk<DC>(a.cu_q, a.n_seqs, blockIdx.x, sh.found, seq, first, nt)) return;
+  const int q_begin = a.cu_q[seq], slot = a.slots[seq], keep = a.taps_n - 1;
+  const size_t tok = (size_t)q_begin + first;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  // a channel's 16 tokens behind its convolution, side by side
+  auto convolved = [&](int ch, float (&y)[DC]) {
+#pragma unroll
+    for (int t = 0; t < DC; ++t) y[t] = 0.f;
+    if (a.taps_n == 4 && first >= 3 && nt == DC) {      // every input once
+      const T* in = (const T*)a.proj + (tok - 3) * a.ld_proj + ch;
+      float x[DC + 3], w[4];
+#pragma unroll
+      for (int t = 0; t < DC + 3; ++t) x[t] = to_f<T>(in[(size_t)t * a.ld_proj]);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) w[j] = a.taps[(size_t)ch * 4 + j];
+#pragma unroll
+      for (int t = 0; t < DC; ++t)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) y[t] = fmaf(w[j], x[t + j], y[t]);
+    } else {
+      for (int j = 0; j < a.taps_n; ++j) {
+        const float w = a.taps[(size_t)ch * a.taps_n + j];
+#pragma unroll
+        for (int t = 0; t < DC; ++t)
+          if (t < nt) y[t] = fmaf(w, conv_input<T>(a, q_begin, slot, first + t - keep + j, ch), y[t]);
+      }
+    }
+#pragma unroll
+    for (int t = 0; t < DC; ++t) y[t] = t < nt ? round_to<T>(y[t] / (1.f + expf(-y[t]))) : 0.f;
+  };
+  {
+    float y[DC];
+    const int i = threadIdx.x % D;
+    const bool is_k = threadIdx.x >= D;
+    convolved((is_k ? a.kv_heads * D : 0) + src * D + i, y);
+#pragma unroll
+    for (int t = 0; t < DC; ++t) (is_k ? sh.k : sh.q)[t][i] = y[t];
+  }
+  const float rate = expf(a.a_log[h]);
+  for (int x = threadIdx.x; x < DC * D; x += blockDim.x) {
+    const int t = x / D, i = x % D;
+    float g = 1.f;
+    if (t < nt) g = expf(-rate * softplus_f(a.decay_in[(tok + t) * a.ld_decay + h * D + i] + a.dt_bias[h * D + i]));
+    sh.g[t][i] = g;
+  }
+  if (threadIdx.x < DC) {
+    const int t = threadIdx.x;
+    sh.beta[t] = t < nt ? 1.f / (1.f + expf(-to_f<T>(((const T*)a.proj)[(tok + t) * a.ld_proj + a.C + h]))) : 0.f;
+  }
+  __syncthreads();
+  for (int r = warp; r < 2 * DC; r += 2 * D / 32) {
+    float* row = r < DC ? sh.q[r] : sh.k[r - DC];
+    float ss = 0.f;
+#pragma unroll
+    for (int e = 0; e < D; e += 32) ss = fmaf(row[lane + e], row[lane + e], ss);
+    ss = warp_sum(ss);
+    const float scale = 1.0f / sqrtf(ss + a.unit_eps) * (r < DC ? 1.0f / sqrtf((float)D) : 1.f);
+#pragma unroll
+    for (int e = 0; e < D; e += 32) row[lane + e] *= scale;
+  }
+  __syncthreads();
+  // the values of this thread's columns: all its tokens at once when it comes to a new column
+  float v[DC];
+  dc_parts<D>(sh, c, blockIdx.x, h, [&](int t, int col) {
+    if (t == 0) convolved(2 * a.kv_heads * D + h * a.dv + col, v);
+    return v[t];
+  });
+}
+
+template <typename T>
+static int launch_chunks(const DeltaArgs& a, const DeltaChunkArgs& c, cudaStream_t stream) {
+  odi_rc = launch_pdl((delta_parts_kernel<T>), dim3((unsigned)run_chunk_slots(a.n_tokens, a.n_seqs, DC), a.heads), dim3(2 * D), 0, stream, a, c);
+  if (odi_rc == 0 && a.taps_n > 1)
+    odi_rc = launch_pdl((delta_conv_state_kernel<T>), dim3(a.n_seqs, (a.C + 255) / 256), dim3(256), 0, stream, a);
+  if (odi_rc == 0) odi_rc = dc_launch<D>(c, stream);
+  if (odi_rc == 0)
+    odi_rc = launch_pdl((delta_out_norm_kernel<T>), dim3((unsigned)(((long)a.n_tokens * a.heads + 3) / 4)), dim3(128), 0, stream, a);
+  return launch_status();
+}
+#endif
 
 extern "C" int odi_delta_dim() { return D; }
 
 // The whole mixer between its input products and its output product: convolutions (and their state), the
-// recurrence's inputs, the recurrence, the gated output norm.  Six launches.
+// recurrence's inputs, the recurrence, the gated output norm.  Six launches token by token, four in chunks (one fewer
+// without a convolution state).
 extern "C" int odi_delta_rule(const DeltaArgs* args, int dtype, cudaStream_t stream) {
   const DeltaArgs a = *args;
   if (a.n_tokens <= 0 || a.n_seqs <= 0) return 0;
   if (a.taps_n < 1 || a.taps_n > MAX_TAPS || a.heads % a.kv_heads != 0 || a.C != 2 * a.kv_heads * D + a.heads * a.dv)
     return ODI_ERR_ARGUMENT;
   if (a.n_seqs > 65535 || a.heads > 65535) return ODI_ERR_UNSUPPORTED;
+  if (a.chunks != nullptr) {
+#ifdef ODI_DELTA_CHUNKS
+    if (a.dv % 4 != 0 || (uintptr_t)a.chunks % 16 != 0) return ODI_ERR_UNSUPPORTED;
+    const size_t slots = run_chunk_slots(a.n_tokens, a.n_seqs, DC);
+    const DeltaChunkArgs c = {a.chunks, a.chunks + slots * a.heads * DC_WORDS(D), a.state, a.o, a.cu_q, a.slots, a.n_seqs, a.heads, a.dv};
+    return dtype == 0 ? launch_chunks<float>(a, c, stream) : launch_chunks<bf16>(a, c, stream);
+#else
+    return ODI_ERR_UNSUPPORTED;
+#endif
+  }
   const dim3 cgrid(a.n_tokens, (a.C + 255) / 256), sgrid(a.n_seqs, (a.C + 255) / 256), hgrid(a.n_tokens, a.heads);
   const dim3 rgrid((a.dv + CB - 1) / CB, a.heads, a.n_seqs);
   if (dtype == 0) {
@@ -286,7 +394,8 @@ extern "C" int odi_delta_rule(const DeltaArgs* args, int dtype, cudaStream_t str
     odi_rc = launch_pdl((delta_values_kernel<bf16>), dim3(a.n_tokens), dim3(128), 0, stream, a);
   }
   odi_rc = launch_pdl(delta_rule_kernel, rgrid, dim3(CB * RS), 0, stream, a);
-  if (dtype == 0) odi_rc = launch_pdl((delta_out_norm_kernel<float>), hgrid, dim3(128), 0, stream, a);
-  else odi_rc = launch_pdl((delta_out_norm_kernel<bf16>), hgrid, dim3(128), 0, stream, a);
+  const dim3 ngrid((unsigned)(((long)a.n_tokens * a.heads + 3) / 4));
+  if (dtype == 0) odi_rc = launch_pdl((delta_out_norm_kernel<float>), ngrid, dim3(128), 0, stream, a);
+  else odi_rc = launch_pdl((delta_out_norm_kernel<bf16>), ngrid, dim3(128), 0, stream, a);
   return launch_status();
 }

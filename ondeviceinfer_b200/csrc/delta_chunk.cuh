@@ -1,0 +1,271 @@
+// The gated delta rule over runs of tokens, 16 tokens at a time.
+//
+// Per sequence and head, with S [D, dv] the state before the chunk, g_t [D] the decays of token t, G_t = g_0 .. g_t and
+// D_ts = g_(s+1) .. g_t (products lane by lane; nothing is divided, so no decay is too small), the recurrence
+//     S <- diag(g) S;   u = beta (v - S^T k);   S <- S + k u^T;   o = S^T q
+// unrolls over the chunk to
+//     u_t = beta_t (v_t - (G_t k_t)^T S - sum_(s<t) A_ts u_s),      A_ts = k_t . (D_ts k_s)
+//     o_t = (G_t q_t)^T S + sum_(s<=t) B_ts u_s,                    B_ts = q_t . (D_ts k_s)
+//     S  <- diag(G_15) S + sum_s (D_15,s k_s) u_s^T.
+// The triangular system is linear in S: u_t = wv_t - wk_t^T S with wv and wk its solutions for v and for G k.  So
+//  parts  (every chunk and head at once) leaves wk, q' = G q - B wk, k^ = D_15 k, G_15, wv and B wv;
+//  scan   (a block per sequence, head and COLS value columns) goes through a sequence's chunks in order:
+//             u = wv - wk S;   o = B wv + q' S;   S <- diag(G_15) S + k^T u
+//         the 32 sums of a column over D rows lie on 16 lanes and are halved side by side, so that a chunk costs one
+//         chain of shuffles where token by token costs 32.
+// Everything is fp32, as token by token.  A last chunk of fewer tokens is filled with tokens that do nothing (k, q, v
+// and beta 0, g 1).
+//
+// What bounds it: the scan's chain of latencies (1.25 us a chunk of one sequence, a quarter of which is instruction issue);
+// with many sequences its reads of shared memory.  The scratch has a slot per chunk (run_chunks.cuh).
+#pragma once
+#include "run_chunks.cuh"
+
+#define DC 16                                      // tokens of a chunk
+#define DC_WORDS(D) ((3 * DC + 1) * (D))           // floats per slot and head: wk, q', k^ [16][D] each, G_15 [D]
+
+struct DeltaChunkArgs {
+  float* wq;              // [slots, heads, DC_WORDS(D)]
+  float* vo;              // [slots, heads, 2, DC, dv]: wv, B wv
+  float* state;           // [cache slots, heads, D, dv]
+  float* o;               // [n_tokens, heads, dv]: the read-outs
+  const int* cu_q;
+  const int* slots;
+  int n_seqs, heads, dv;
+};
+
+template <int D>
+struct DeltaChunkShared {
+  float q[DC][D], k[DC][D], g[DC][D];
+  __align__(16) float A[DC][DC];
+  __align__(16) float B[DC][DC];
+  float beta[DC];
+  int found[3];
+};
+
+// The parts of a chunk from its unit vectors, decays and step sizes in shared memory (written before a barrier) and
+// its values; by all threads of a block of whole warps, D + dv columns in turn.
+template <int D, typename Value>
+__device__ __forceinline__ void dc_parts(DeltaChunkShared<D>& sh, const DeltaChunkArgs& a, int b, int h, Value value) {
+  static_assert(D % 32 == 0, "lanes own whole channels");
+  constexpr int NI = D / 32;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, n_warps = blockDim.x >> 5;
+  // A and B: a warp takes a token s, its lanes carry D_ts k_s on over the tokens behind it; the 32 sums over the lanes (A's and
+  // B's column s) are halved side by side
+  for (int s = warp; s < DC; s += n_warps) {
+    float w[NI], r[2 * DC];
+#pragma unroll
+    for (int e = 0; e < NI; ++e) w[e] = sh.k[s][lane + 32 * e];
+#pragma unroll
+    for (int t = 0; t < DC; ++t) {
+      r[t] = r[DC + t] = 0.f;
+      if (t >= s) {
+#pragma unroll
+        for (int e = 0; e < NI; ++e) {
+          if (t > s) w[e] *= sh.g[t][lane + 32 * e];
+          r[t] = fmaf(w[e], sh.k[t][lane + 32 * e], r[t]);
+          r[DC + t] = fmaf(w[e], sh.q[t][lane + 32 * e], r[DC + t]);
+        }
+      }
+    }
+#pragma unroll
+    for (int m = 16; m > 0; m >>= 1) {
+      const bool up = lane & m;
+#pragma unroll
+      for (int i = 0; i < m; ++i) {
+        const float keep = up ? r[m + i] : r[i], give = up ? r[i] : r[m + i];
+        r[i] = keep + __shfl_xor_sync(0xffffffffu, give, m);
+      }
+    }
+    (lane < DC ? sh.A : sh.B)[lane & (DC - 1)][s] = r[0];      // column s; A's diagonal and what lies above are not read
+  }
+  __syncthreads();
+  const size_t item = (size_t)b * a.heads + h;
+  float* wk = a.wq + item * DC_WORDS(D);
+  float* vo = a.vo + item * 2 * DC * a.dv;
+  for (int c = threadIdx.x; c < D + a.dv; c += blockDim.x) {
+    const bool is_k = c < D;
+    float w[DC], decay = 1.f;
+#pragma unroll
+    for (int t = 0; t < DC; ++t) {
+      if (is_k) decay *= sh.g[t][c];
+      float x = is_k ? sh.k[t][c] * decay : value(t, c - D);
+#pragma unroll
+      for (int s = 0; s < t; ++s) x = fmaf(-sh.A[t][s], w[s], x);
+      w[t] = sh.beta[t] * x;
+    }
+    float run = 1.f, tail = 1.f;
+#pragma unroll
+    for (int t = 0; t < DC; ++t) {
+      float x = 0.f;
+#pragma unroll
+      for (int s = 0; s <= t; ++s) x = fmaf(sh.B[t][s], w[s], x);
+      if (is_k) {
+        run *= sh.g[t][c];
+        wk[t * D + c] = w[t];
+        wk[(DC + t) * D + c] = fmaf(sh.q[t][c], run, -x);
+      } else {
+        vo[t * a.dv + c - D] = w[t];
+        vo[(DC + t) * a.dv + c - D] = x;
+      }
+    }
+    if (is_k) {
+#pragma unroll
+      for (int t = DC - 1; t >= 0; --t) {
+        wk[(2 * DC + t) * D + c] = sh.k[t][c] * tail;
+        tail *= sh.g[t][c];
+      }
+      wk[3 * DC * D + c] = decay;
+    }
+  }
+}
+
+__device__ __forceinline__ void dc_cp16(uint32_t dst, const float* src, bool ok) {      // zeros where !ok
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(ok ? 16 : 0) : "memory");
+}
+
+#define DC_STAGES 3
+#define DC_STAGE(D, COLS) (DC_WORDS(D) + 2 * DC * (COLS))      // floats of a chunk in shared memory
+
+// COLS columns of one head's state: CPT of them per group of 16 lanes, a lane holding rows 4 (lane + 16 j) .. + 3.  dv a
+// multiple of 4 (16-byte copies of COLS columns).
+template <int D, int COLS, int CPT>
+__global__ void __launch_bounds__(COLS / CPT * 16)
+dc_scan_kernel(DeltaChunkArgs a) {
+  pdl_wait();
+  constexpr int NTH = COLS / CPT * 16, NJ = D / 64, R = D / 16;
+  constexpr size_t STAGE = DC_STAGE(D, COLS);
+  static_assert(D % 64 == 0 && COLS % 4 == 0 && COLS % CPT == 0 && NTH % 32 == 0, "sizes of a block");
+  extern __shared__ __align__(16) float dc_smem[];
+  const int seq = blockIdx.z, h = blockIdx.y, c0 = blockIdx.x * COLS;
+  const int tid = threadIdx.x, rl = tid & 15, col = (tid >> 4) * CPT;
+  const int q_begin = a.cu_q[seq], q_len = a.cu_q[seq + 1] - q_begin;
+  if (q_len <= 0) return;
+  const int dv = a.dv, chunks = (q_len + DC - 1) / DC;
+  const size_t slot0 = (size_t)(q_begin / DC) + seq;
+  float* S_g = a.state + ((size_t)a.slots[seq] * a.heads + h) * D * dv;
+  float* xs = dc_smem + DC_STAGES * STAGE + col * DC;
+  const uint32_t base = (uint32_t)__cvta_generic_to_shared(dc_smem);
+
+  auto issue = [&](int c) {
+    if (c < chunks) {
+      const size_t item = (slot0 + c) * a.heads + h;
+      const uint32_t dst = base + (uint32_t)((c % DC_STAGES) * STAGE * 4);
+      const float* src = a.wq + item * DC_WORDS(D);
+      for (int i = tid * 4; i < DC_WORDS(D); i += NTH * 4) dc_cp16(dst + i * 4, src + i, true);
+      const float* vo = a.vo + item * 2 * DC * dv + c0;
+      for (int i = tid; i < 2 * DC * (COLS / 4); i += NTH) {
+        const int t = i / (COLS / 4), e = (i % (COLS / 4)) * 4;
+        const bool ok = c0 + e < dv;
+        dc_cp16(dst + (DC_WORDS(D) + t * COLS + e) * 4, ok ? vo + (size_t)t * dv + e : vo, ok);
+      }
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+#pragma unroll
+  for (int c = 0; c < DC_STAGES - 1; ++c) issue(c);
+
+  float S[CPT][R];
+#pragma unroll
+  for (int cc = 0; cc < CPT; ++cc)
+#pragma unroll
+    for (int r = 0; r < R; ++r)
+      S[cc][r] = c0 + col + cc < dv ? S_g[(size_t)(4 * (rl + 16 * (r >> 2)) + (r & 3)) * dv + c0 + col + cc] : 0.f;
+
+  for (int c = 0; c < chunks; ++c) {
+    asm volatile("cp.async.wait_group %0;" ::"n"(DC_STAGES - 2) : "memory");
+    __syncthreads();      // chunk c has arrived; everybody has left chunk c - 1, whose place the next copies take
+    issue(c + DC_STAGES - 1);
+    const float* buf = dc_smem + (c % DC_STAGES) * STAGE;
+    const float* vs = buf + DC_WORDS(D);
+    float sum[CPT][2 * DC];      // wk S, then q' S
+#pragma unroll
+    for (int t = 0; t < 2 * DC; ++t) {
+#pragma unroll
+      for (int cc = 0; cc < CPT; ++cc) sum[cc][t] = 0.f;
+#pragma unroll
+      for (int j = 0; j < NJ; ++j) {
+        const float4 x = *(const float4*)(buf + t * D + 4 * (rl + 16 * j));
+#pragma unroll
+        for (int cc = 0; cc < CPT; ++cc)
+          sum[cc][t] = fmaf(x.x, S[cc][4 * j], fmaf(x.y, S[cc][4 * j + 1], fmaf(x.z, S[cc][4 * j + 2], fmaf(x.w, S[cc][4 * j + 3], sum[cc][t]))));
+      }
+    }
+    // over the 16 lanes: a lane keeps one half of its sums and hands the other on, down to two sums a lane, 2 rl and 2 rl + 1
+#pragma unroll
+    for (int cc = 0; cc < CPT; ++cc) {
+#pragma unroll
+      for (int m = 8; m > 0; m >>= 1) {
+        const bool up = rl & m;
+#pragma unroll
+        for (int i = 0; i < 2 * m; ++i) {
+          const float keep = up ? sum[cc][2 * m + i] : sum[cc][i], give = up ? sum[cc][i] : sum[cc][2 * m + i];
+          sum[cc][i] = keep + __shfl_xor_sync(0xffffffffu, give, m);
+        }
+      }
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        const int t = (2 * rl + i) & (DC - 1);
+        const float part = vs[(2 * rl + i) * COLS + col + cc];
+        if (rl < 8) xs[cc * DC + t] = part - sum[cc][i];
+        else if (c * DC + t < q_len && c0 + col + cc < dv)
+          a.o[((size_t)(q_begin + c * DC + t) * a.heads + h) * dv + c0 + col + cc] = part + sum[cc][i];
+      }
+    }
+    __syncwarp();
+    float u[CPT][DC];
+#pragma unroll
+    for (int cc = 0; cc < CPT; ++cc)
+#pragma unroll
+      for (int t = 0; t < DC; t += 4) {
+        const float4 x = *(const float4*)(xs + cc * DC + t);
+        u[cc][t] = x.x; u[cc][t + 1] = x.y; u[cc][t + 2] = x.z; u[cc][t + 3] = x.w;
+      }
+#pragma unroll
+    for (int j = 0; j < NJ; ++j) {
+      const float4 g = *(const float4*)(buf + 3 * DC * D + 4 * (rl + 16 * j));
+      // the chunk's writes are summed before they join the state: one rounding of the larger number instead of sixteen
+      float4 add[CPT];
+#pragma unroll
+      for (int cc = 0; cc < CPT; ++cc) add[cc] = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+      for (int t = 0; t < DC; ++t) {
+        const float4 x = *(const float4*)(buf + (2 * DC + t) * D + 4 * (rl + 16 * j));
+#pragma unroll
+        for (int cc = 0; cc < CPT; ++cc) {
+          add[cc].x = fmaf(x.x, u[cc][t], add[cc].x); add[cc].y = fmaf(x.y, u[cc][t], add[cc].y);
+          add[cc].z = fmaf(x.z, u[cc][t], add[cc].z); add[cc].w = fmaf(x.w, u[cc][t], add[cc].w);
+        }
+      }
+#pragma unroll
+      for (int cc = 0; cc < CPT; ++cc) {
+        S[cc][4 * j] = fmaf(S[cc][4 * j], g.x, add[cc].x); S[cc][4 * j + 1] = fmaf(S[cc][4 * j + 1], g.y, add[cc].y);
+        S[cc][4 * j + 2] = fmaf(S[cc][4 * j + 2], g.z, add[cc].z); S[cc][4 * j + 3] = fmaf(S[cc][4 * j + 3], g.w, add[cc].w);
+      }
+    }
+    __syncwarp();      // xs is written again in the next chunk
+  }
+  pdl_launch_dependents();
+#pragma unroll
+  for (int cc = 0; cc < CPT; ++cc)
+#pragma unroll
+    for (int r = 0; r < R; ++r)
+      if (c0 + col + cc < dv) S_g[(size_t)(4 * (rl + 16 * (r >> 2)) + (r & 3)) * dv + c0 + col + cc] = S[cc][r];
+}
+
+// Columns a block and a thread.  More columns a thread read the chunk's rows from shared memory fewer times, more blocks spread
+// one sequence over the chip.  Measured, whole mixer, 16 heads, us for (columns a block, a thread): heads of 64, 2,048 tokens of
+// one sequence (8, 1) 239, (8, 2) 243, (16, 2) 274, (16, 4) 326; 8 x 1,000 tokens 591, 494, 492, 462; heads of 128, one sequence
+// (8, 1) 440, (8, 2) 354, (16, 2) 343, (16, 4) 640; 8 x 1,000 1,497, 1,199, 1,155, 1,290.
+template <int D>
+static int dc_launch(const DeltaChunkArgs& a, cudaStream_t stream) {
+  constexpr int COLS = D == 64 ? 8 : 16, CPT = 2;
+  constexpr size_t smem = sizeof(float) * (DC_STAGES * DC_STAGE(D, COLS) + COLS * DC);
+  auto kernel = dc_scan_kernel<D, COLS, CPT>;
+  const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e != cudaSuccess) return (int)e;
+  // an ordinary launch: started early, while the kernel before still holds multiprocessors, the few long blocks of a
+  // single sequence would be packed several to one and stay there
+  kernel<<<dim3((a.dv + COLS - 1) / COLS, a.heads, a.n_seqs), dim3(COLS / CPT * 16), smem, stream>>>(a);
+  return (int)cudaPeekAtLastError();
+}

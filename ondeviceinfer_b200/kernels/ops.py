@@ -1580,11 +1580,25 @@ def gated_row_add(acc: torch.Tensor, y: torch.Tensor, x: torch.Tensor, gate: tor
 class _DeltaArgs(Structure):
     _fields_ = [("proj", c_void_p), ("taps", c_void_p), ("conv_state", c_void_p), ("conv_out", c_void_p),
                 ("decay_in", c_void_p), ("a_log", c_void_p), ("dt_bias", c_void_p), ("qkg", c_void_p), ("beta", c_void_p),
-                ("state", c_void_p), ("o", c_void_p), ("norm_w", c_void_p), ("out", c_void_p), ("cu_q", c_void_p),
+                ("state", c_void_p), ("o", c_void_p), ("chunks", c_void_p), ("norm_w", c_void_p), ("out", c_void_p), ("cu_q", c_void_p),
                 ("tok_seq", c_void_p), ("slots", c_void_p),
                 ("n_tokens", c_int), ("n_seqs", c_int), ("ld_proj", c_int), ("ld_decay", c_int), ("heads", c_int),
                 ("kv_heads", c_int), ("dv", c_int), ("taps_n", c_int), ("C", c_int), ("eps", c_float),
                 ("unit_eps", c_float)]
+
+
+# Delta rules over runs of tokens go 16 tokens at a time (csrc/delta_chunk.cuh) when a sequence brings this many on average
+# (24 tokens: 37 us in chunks, 35 token by token; 8 x 24: 56 and 42; 64: 46 and 62).
+DELTA_CHUNK, DELTA_CHUNK_MIN_RUN, DELTA_CHUNK_MAX_SCRATCH = 16, 40, 1 << 30
+
+
+def delta_chunk_floats(n_tokens: int, n_seqs: int, heads: int, d: int, dv: int) -> int:
+    """Floats of scratch for a delta rule's run in chunks; 0 where it goes token by token: short runs, sizes that the
+    chunk kernels do not take, more scratch than DELTA_CHUNK_MAX_SCRATCH bytes."""
+    if n_tokens < DELTA_CHUNK_MIN_RUN * n_seqs or d not in (64, 128) or dv % 4 != 0:
+        return 0
+    floats = (n_tokens // DELTA_CHUNK + n_seqs) * heads * ((3 * DELTA_CHUNK + 1) * d + 2 * DELTA_CHUNK * dv)
+    return floats if 4 * floats <= DELTA_CHUNK_MAX_SCRATCH else 0
 
 
 DELTA_MAX_DIM = 480     # the recurrence stages 8 tokens of q, k and decay in 48 KB of shared memory
@@ -1619,16 +1633,21 @@ def delta_rule(proj: torch.Tensor, decay_in: torch.Tensor, taps: torch.Tensor, a
         if tuple(conv_state.shape[1:]) != (K - 1, C):
             raise KernelError("the convolution state does not fit the taps")
     dev = proj.device
-    conv_out = torch.empty((n, C), dtype=proj.dtype, device=dev)
-    qkg = torch.empty((n, heads, 3, d), dtype=torch.float32, device=dev)
-    beta = torch.empty((n, heads), dtype=torch.float32, device=dev)
+    conv_out = qkg = beta = chunks = None
+    scratch = delta_chunk_floats(n, n_seqs, heads, d, dv)
+    if scratch:
+        chunks = torch.empty(scratch, dtype=torch.float32, device=dev)
+    else:
+        conv_out = torch.empty((n, C), dtype=proj.dtype, device=dev)
+        qkg = torch.empty((n, heads, 3, d), dtype=torch.float32, device=dev)
+        beta = torch.empty((n, heads), dtype=torch.float32, device=dev)
     o = torch.empty((n, heads * dv), dtype=torch.float32, device=dev)
     args = _DeltaArgs(_ptr(proj), _ptr(taps), _ptr(conv_state), _ptr(conv_out), _ptr(decay_in), _ptr(a_log),
-                      _ptr(dt_bias), _ptr(qkg), _ptr(beta), _ptr(state), _ptr(o), _ptr(norm_w), _ptr(out), _ptr(cu_q),
+                      _ptr(dt_bias), _ptr(qkg), _ptr(beta), _ptr(state), _ptr(o), _ptr(chunks), _ptr(norm_w), _ptr(out), _ptr(cu_q),
                       _ptr(tok_seq), _ptr(slots), n, n_seqs, proj.shape[1], decay_in.shape[1], heads, kv_heads, dv, K, C,
                       eps, unit_eps)
     lib = load_library("delta", {"ODI_DELTA_DIM": d})
-    _check(lib.odi_delta_rule(byref(args), c_int(dtype_code(proj.dtype)), _stream()), "delta_rule", 6 if K > 1 else 5)
+    _check(lib.odi_delta_rule(byref(args), c_int(dtype_code(proj.dtype)), _stream()), "delta_rule", (3 if scratch else 5) + (K > 1))
 
 
 class _HeadDeltaArgs(Structure):

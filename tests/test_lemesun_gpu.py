@@ -79,6 +79,79 @@ def routed(case):
 # ----------------------------------------------------------------------------- kernels against plain functions
 
 
+def delta_by_token(proj, inner, w, m, eps):
+    """The mixer between its products, token by token in 64 bits: (out [T, heads dv], final state [heads, d, dv])."""
+    H, G, d, dv = m["heads"], m["kv_heads"], m["dim"], m["vdim"]
+    T, C = proj.shape[0], 2 * G * d + H * dv
+    y = plain.causal_conv_silu(proj[:, :C], w["taps"])
+    unit = lambda x: x / torch.sqrt((x * x).sum(-1, keepdim=True) + 1e-6)
+    q = (unit(y[:, :G * d].view(T, G, d)) * d ** -0.5).repeat_interleave(H // G, 1)
+    k = unit(y[:, G * d:2 * G * d].view(T, G, d)).repeat_interleave(H // G, 1)
+    v, beta = y[:, 2 * G * d:].view(T, H, dv), torch.sigmoid(proj[:, C:])
+    decay = torch.exp(-torch.exp(w["A_log"])[None, :, None]
+                      * torch.nn.functional.softplus((inner[:, :H * d] + w["dt_bias"]).view(T, H, d)))
+    S, out = torch.zeros(H, d, dv, dtype=proj.dtype), torch.zeros(T, H, dv, dtype=proj.dtype)
+    for t in range(T):
+        S = decay[t, :, :, None] * S
+        u = beta[t, :, None] * (v[t] - torch.einsum("hdv,hd->hv", S, k[t]))
+        S = S + k[t, :, :, None] * u[:, None]
+        out[t] = torch.einsum("hdv,hd->hv", S, q[t])
+    out = plain.rms(out, eps) * w["norm"] * torch.sigmoid(inner[:, H * d:].view(T, H, dv))
+    return out.reshape(T, H * dv), S
+
+
+@pytest.mark.parametrize("d,dv,heads,kv_heads,taps", [(64, 64, 3, 3, 4), (64, 20, 4, 2, 1), (128, 100, 2, 1, 3), (128, 128, 2, 2, 4)])
+def test_delta_rule_in_chunks_of_tokens(d, dv, heads, kv_heads, taps):
+    """Runs around the chunks' edges, one of a single token among them, continued by a second step, with decays from one
+    to those that wipe the state; against the recurrence token by token in 64 bits, and no further off than the token by
+    token kernel."""
+    gen = torch.Generator().manual_seed(d + dv + heads)
+    C, cuts, slots, eps = 2 * kv_heads * d + heads * dv, [[97, 16, 1, 60], [48, 33, 31, 80]], [3, 0, 4, 1], 1e-5
+    m = {"heads": heads, "kv_heads": kv_heads, "dim": d, "vdim": dv}
+    w = {"taps": torch.randn(C, taps, generator=gen) * 0.5, "A_log": torch.log(0.02 + 8 * torch.rand(heads, generator=gen)),
+         "dt_bias": torch.randn(heads * d, generator=gen) - 3, "norm": 1 + 0.1 * torch.randn(dv, generator=gen)}
+    lengths = [a + b for a, b in zip(*cuts)]
+    projs = [torch.randn(L, C + heads, generator=gen) for L in lengths]
+    inners = [torch.randn(L, heads * (d + dv), generator=gen) for L in lengths]
+    inners[0][20:22, :heads * d] = 400.0            # decays of zero inside a chunk
+    inners[1][:, :d // 2] = -60.0                   # half of a head's channels keep everything
+    wide = {n: t.double() for n, t in w.items()}
+    want = [delta_by_token(p.double(), i.double(), wide, m, eps) for p, i in zip(projs, inners)]
+    dev = {n: t.cuda() for n, t in w.items()}
+    ints = lambda *x: torch.tensor(x, dtype=torch.int32, device="cuda")
+
+    def run():
+        state = torch.zeros(6, heads, d, dv, device="cuda")
+        state[2] = 7.0                              # a slot of somebody else: must stay as it is
+        conv_state = torch.zeros(6, taps - 1, C, device="cuda") if taps > 1 else None
+        got, at = [[] for _ in lengths], [0] * len(lengths)
+        for lens in cuts:
+            cu = [0]
+            for n in lens:
+                cu.append(cu[-1] + n)
+            piece = lambda all_: torch.cat([x[o:o + n] for x, o, n in zip(all_, at, lens)]).cuda()
+            out = torch.empty(cu[-1], heads * dv, device="cuda")
+            ops.delta_rule(piece(projs), piece(inners), dev["taps"], dev["A_log"], dev["dt_bias"], dev["norm"], conv_state, state, out,
+                           ints(*cu), ints(*[s for s, n in enumerate(lens) for _ in range(n)]), ints(*slots), n_seqs=len(lens),
+                           heads=heads, kv_heads=kv_heads, d=d, dv=dv, eps=eps, unit_eps=1e-6)
+            for s, n in enumerate(lens):
+                got[s].append(out[cu[s]:cu[s + 1]].cpu())
+                at[s] += n
+        assert at == lengths and bool((state[2] == 7.0).all())
+        pieces = [(torch.cat(g).double(), state[slot].cpu().double()) for g, slot in zip(got, slots)]
+        return [float((a - b).norm() / b.norm()) for p, q in zip(pieces, want) for a, b in zip(p, q)]
+
+    assert ops.delta_chunk_floats(sum(cuts[0]), 4, heads, d, dv) > 0
+    chunked, least = run(), ops.DELTA_CHUNK_MIN_RUN
+    ops.DELTA_CHUNK_MIN_RUN = 1 << 30
+    try:
+        single = run()
+    finally:
+        ops.DELTA_CHUNK_MIN_RUN = least
+    assert max(chunked) < 5e-6 and max(single) < 5e-6      # sums of a hundred products of 2^-24 each
+    assert sum(chunked) <= 1.25 * sum(single)
+
+
 def test_offset_norm_scales_in_fp32():
     g = torch.Generator().manual_seed(0)
     x = torch.randn(7, 50, generator=g) * 3
