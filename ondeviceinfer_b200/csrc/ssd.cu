@@ -17,7 +17,7 @@
 //              root mean square, eps inside the root), times a weight per lane, rounded once to T.
 //
 // Everything but the projection's own output is fp32 in both compute dtypes.
-#include "common.cuh"
+#include "run_chunks.cuh"
 #include <type_traits>
 
 #define SSD_MAX_TAPS 16
@@ -36,6 +36,7 @@ struct SsdArgs {
   float* state;           // [slots, heads, N, P]
   float* xbc;             // [n_tokens, C] scratch
   float* y;               // [n_tokens, inner] scratch
+  float* chunks;          // scratch of the scan in chunks (ssd_chunk_floats in ops.py says how much); null: token by token
   void* out;              // [n_tokens, inner] in T
   const int* cu_q;        // [n_seqs + 1]
   const int* tok_seq;     // [n_tokens]
@@ -275,6 +276,265 @@ ssd_scan_kernel(SsdArgs a) {
   }
 }
 
+// The scan over runs of tokens, SSD_L tokens at a time.  With a_t = exp(-exp(A_log) dt_t), G_t = a_0 .. a_t and D_ts = a_(s+1)
+// .. a_t (products; nothing is divided, no difference of exponents is taken), S the state before the chunk:
+//     y_t = G_t C_t S + sum_(s<=t) (C_t . B_s) D_ts dt_s x_s + D x_t
+//     S  <- G_last S + sum_s B_s (D_last,s dt_s x_s)^T
+//  states   every chunk and head at once: E = sum_s B_s (D_last,s dt_s x_s)^T and G_last; in further blocks every chunk and
+//           group: the products C_t . B_s, which the heads of a group share;
+//  pass     per element of S: E of every chunk gives way to the state before it;
+//  outputs  every chunk and head at once: y.
+// All of it plain fp32 multiply-adds, as token by token, where a sequence's tokens were one chain of them.  The mixer between its
+// products, 32 heads of 128 x 64, us (in chunks, token by token): 2,048 tokens 187, 564; 2 x 1,024 183, 350; 8 x 1,000 715, 961;
+// 512 79, 152; 128 63, 60.  What bounds outputs (66 us of those 187) and states (54) is shared memory: three 16-byte reads per 32
+// multiply-adds of a thread.
+#define SSD_L 64
+
+// dt_t and a_t of the chunk's tokens into shared memory; tokens behind the run's end have dt 0, a 1
+template <typename T>
+__device__ __forceinline__ void ssd_chunk_steps(const SsdArgs& a, int h, size_t tok, int nt, float* dt_s, float* a_s) {
+  const int t = threadIdx.x;
+  if (t < SSD_L) {
+    float dt = 0.f, da = 1.f;
+    if (t < nt) {
+      const T* raw = (const T*)a.proj + (tok + t) * a.ld + 2 * (size_t)a.heads * a.P + 2 * (size_t)a.G * a.N + h;
+      dt = ssd_softplus(to_f<T>(*raw) + a.dt_bias[h]);
+      da = expf(-expf(a.a_log[h]) * dt);
+    }
+    dt_s[t] = dt;
+    a_s[t] = da;
+  }
+}
+
+struct SsdScratch {
+  float* E;               // [slots, heads, N, P]
+  float* cb;              // [slots, G, L (s), L (t)]: C_t . B_s
+  float* gamma;           // [slots, heads]
+};
+static __host__ __device__ __forceinline__ SsdScratch ssd_scratch(const SsdArgs& a) {
+  const size_t slots = (size_t)a.n_tokens / SSD_L + a.n_seqs;
+  SsdScratch s;
+  s.E = a.chunks;
+  s.cb = s.E + slots * a.heads * a.N * a.P;
+  s.gamma = s.cb + slots * a.G * SSD_L * SSD_L;
+  return s;
+}
+
+#define SSD_PAD (SSD_L + 4)
+
+// 32 rows of a product's reduction (CAUSAL: row k only into the outputs m >= k0 + k): acc[i][j] += sum_k A[k][m(i)] B[k][n(j)],
+// m = 4 mt + (0..3) and 32 + 4 mt + (0..3), n = 4 nt + (0..3); A rows of SSD_PAD, B rows of SSD_L words
+template <bool CAUSAL = false>
+__device__ __forceinline__ void ssd_mma32(float (&acc)[8][4], const float* A, const float* B, int mt, int nt, int k0 = 0) {
+#pragma unroll 1
+  for (int half = 0; half < 32; half += 16) {
+    float part[8][4] = {};      // sums of sixteen products, then of those: fewer roundings of large numbers than one chain
+#pragma unroll
+    for (int k = half; k < half + 16; ++k) {
+      const float4 a0 = *(const float4*)(A + k * SSD_PAD + 4 * mt), a1 = *(const float4*)(A + k * SSD_PAD + 32 + 4 * mt);
+      const float4 b = *(const float4*)(B + k * SSD_L + 4 * nt);
+      const float av[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w}, bv[4] = {b.x, b.y, b.z, b.w};
+#pragma unroll
+      for (int i = 0; i < 8; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+          if (!CAUSAL || (i & 4) * 8 + 4 * mt + (i & 3) >= k0 + k) part[i][j] = fmaf(av[i], bv[j], part[i][j]);
+    }
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) acc[i][j] += part[i][j];
+  }
+}
+
+// 64 tokens x 32 lanes of rows `src` (pitch ld; tokens from nt on are zero) times w[t], turned over: dst[lane][t]
+__device__ __forceinline__ void ssd_stage_turned(float* dst, int pitch, const float* src, size_t ld, int nt, const float* w) {
+  for (int i = threadIdx.x; i < SSD_L * 8; i += blockDim.x) {
+    const int t = i >> 3, k = (i & 7) * 4;
+    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (t < nt) v = *(const float4*)(src + (size_t)t * ld + k);
+    const float f = w != nullptr ? w[t] : 1.f;
+    dst[k * pitch + t] = v.x * f; dst[(k + 1) * pitch + t] = v.y * f;
+    dst[(k + 2) * pitch + t] = v.z * f; dst[(k + 3) * pitch + t] = v.w * f;
+  }
+}
+
+// Blocks y < heads * ceil(P / 64) * (N / 64): 64 rows x 64 columns of a head's E; those behind: C B^T of a group.
+template <typename T>
+__global__ void __launch_bounds__(128)
+ssd_states_kernel(SsdArgs a) {
+  pdl_launch_dependents();
+  pdl_wait();
+  __shared__ __align__(16) float As[32 * SSD_PAD], Bs[32 * SSD_L];
+  __shared__ float dt_s[SSD_L], a_s[SSD_L], w_s[SSD_L];
+  __shared__ int found[3];
+  int seq, first, nt;
+  if (!run_chunk<SSD_L>(a.cu_q, a.n_seqs, blockIdx.x, found, seq, first, nt)) return;
+  const SsdScratch out = ssd_scratch(a);
+  const int inner = a.heads * a.P, C = inner + 2 * a.G * a.N, tid = threadIdx.x;
+  const size_t tok = (size_t)a.cu_q[seq] + first;
+  const float* rows = a.xbc + tok * C;
+  const int mt = tid >> 4, nn = tid & 15;
+  const int p_tiles = (a.P + SSD_L - 1) / SSD_L, n_tiles = a.N / SSD_L, state_blocks = a.heads * p_tiles * n_tiles;
+  float acc[8][4] = {};
+  if ((int)blockIdx.y >= state_blocks) {          // rows s, columns t, over the lanes of B and C
+    const int g = blockIdx.y - state_blocks;
+    const float* Bg = rows + inner + (size_t)g * a.N;
+    for (int n0 = 0; n0 < a.N; n0 += 32) {
+      __syncthreads();
+      ssd_stage_turned(As, SSD_PAD, Bg + n0, C, nt, nullptr);
+      ssd_stage_turned(Bs, SSD_L, Bg + (size_t)a.G * a.N + n0, C, nt, nullptr);
+      __syncthreads();
+      ssd_mma32(acc, As, Bs, mt, nn);
+    }
+    float* cb = out.cb + ((size_t)blockIdx.x * a.G + g) * SSD_L * SSD_L;
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+      *(float4*)(cb + (size_t)((i & 4) * 8 + 4 * mt + (i & 3)) * SSD_L + 4 * nn) = make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
+    return;
+  }
+  const int h = blockIdx.y / (p_tiles * n_tiles), p0 = blockIdx.y / n_tiles % p_tiles * SSD_L, n0 = blockIdx.y % n_tiles * SSD_L;
+  ssd_chunk_steps<T>(a, h, tok, nt, dt_s, a_s);
+  __syncthreads();
+  if (tid == 0) {                                 // D_last,s dt_s, from the last token on
+    float tail = 1.f;
+#pragma unroll 16
+    for (int s = SSD_L - 1; s >= 0; --s) { w_s[s] = tail * dt_s[s]; tail *= a_s[s]; }
+    if (p0 == 0 && n0 == 0) out.gamma[(size_t)blockIdx.x * a.heads + h] = tail;
+  }
+  const float* Bg = rows + inner + (size_t)(h / (a.heads / a.G)) * a.N + n0;
+  const float* X = rows + (size_t)h * a.P + p0;
+  for (int s0 = 0; s0 < SSD_L; s0 += 32) {        // rows n, columns p, over the tokens
+    __syncthreads();
+    for (int i = tid; i < 32 * 16; i += 128) {
+      const int s = i >> 4, k = (i & 15) * 4;
+      float4 b = make_float4(0.f, 0.f, 0.f, 0.f), x = b;
+      if (s0 + s < nt) {
+        const float w = w_s[s0 + s];
+        b = *(const float4*)(Bg + (size_t)(s0 + s) * C + k);
+        if (p0 + k < a.P) x = *(const float4*)(X + (size_t)(s0 + s) * C + k);
+        x.x *= w; x.y *= w; x.z *= w; x.w *= w;
+      }
+      *(float4*)(As + s * SSD_PAD + k) = b;
+      *(float4*)(Bs + s * SSD_L + k) = x;
+    }
+    __syncthreads();
+    ssd_mma32(acc, As, Bs, mt, nn);
+  }
+  float* E = out.E + (((size_t)blockIdx.x * a.heads + h) * a.N + n0) * a.P + p0;
+  if (p0 + 4 * nn < a.P) {
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+      *(float4*)(E + (size_t)((i & 4) * 8 + 4 * mt + (i & 3)) * a.P + 4 * nn) = make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
+  }
+}
+
+// Four elements of a head's state per thread, chunk after chunk; the loads of the next chunks run ahead.
+__global__ void __launch_bounds__(128)
+ssd_pass_kernel(SsdArgs a) {
+  pdl_launch_dependents();
+  pdl_wait();
+  const int seq = blockIdx.z, h = blockIdx.y, e = (blockIdx.x * 128 + threadIdx.x) * 4;
+  const int q_begin = a.cu_q[seq], q_len = a.cu_q[seq + 1] - q_begin, size = a.N * a.P;
+  if (q_len <= 0 || e >= size) return;
+  const SsdScratch sc = ssd_scratch(a);
+  const int chunks = (q_len + SSD_L - 1) / SSD_L;
+  const size_t slot0 = (size_t)(q_begin / SSD_L) + seq, step = (size_t)a.heads * size;
+  float* E = sc.E + (slot0 * a.heads + h) * size + e;
+  const float* gamma = sc.gamma + slot0 * a.heads + h;
+  float4* S_g = (float4*)(a.state + ((size_t)a.slots[seq] * a.heads + h) * size + e);
+  float4 S = *S_g;
+  for (int c0 = 0; c0 < chunks; c0 += 8) {
+    float4 x[8];
+    float g[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+      if (c0 + i < chunks) { x[i] = *(const float4*)(E + (c0 + i) * step); g[i] = gamma[(size_t)(c0 + i) * a.heads]; }
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+      if (c0 + i < chunks) {
+        *(float4*)(E + (c0 + i) * step) = S;
+        S.x = fmaf(g[i], S.x, x[i].x); S.y = fmaf(g[i], S.y, x[i].y); S.z = fmaf(g[i], S.z, x[i].z); S.w = fmaf(g[i], S.w, x[i].w);
+      }
+  }
+  *S_g = S;
+}
+
+template <typename T>
+__global__ void __launch_bounds__(128)
+ssd_outputs_kernel(SsdArgs a) {
+  pdl_launch_dependents();
+  pdl_wait();
+  __shared__ __align__(16) float As[32 * SSD_PAD], Bs[32 * SSD_L];
+  __shared__ __align__(16) float Ds[SSD_L * SSD_PAD];      // [s][t]: D_ts dt_s, 0 for t < s
+  __shared__ float dt_s[SSD_L], a_s[SSD_L], g_s[SSD_L];
+  __shared__ int found[3];
+  int seq, first, nt;
+  if (!run_chunk<SSD_L>(a.cu_q, a.n_seqs, blockIdx.x, found, seq, first, nt)) return;
+  const SsdScratch sc = ssd_scratch(a);
+  const int inner = a.heads * a.P, C = inner + 2 * a.G * a.N, tid = threadIdx.x;
+  const int p_tiles = (a.P + SSD_L - 1) / SSD_L, h = blockIdx.y / p_tiles, p0 = blockIdx.y % p_tiles * SSD_L, g = h / (a.heads / a.G);
+  const size_t tok = (size_t)a.cu_q[seq] + first;
+  const float* rows = a.xbc + tok * C;
+  const float* X = rows + (size_t)h * a.P + p0;
+  ssd_chunk_steps<T>(a, h, tok, nt, dt_s, a_s);
+  __syncthreads();
+  if (tid < SSD_L) {                              // a thread a token s: its decays on the way to every later token
+    float d = dt_s[tid];
+#pragma unroll 16
+    for (int t = 0; t < SSD_L; ++t) {
+      if (t > tid) d *= a_s[t];
+      Ds[tid * SSD_PAD + t] = t < tid ? 0.f : d;
+    }
+  } else if (tid == SSD_L) {
+    float run = 1.f;
+#pragma unroll 16
+    for (int t = 0; t < SSD_L; ++t) { run *= a_s[t]; g_s[t] = run; }
+  }
+  const int mt = tid >> 4, nn = tid & 15;
+  float acc[8][4] = {};
+  const float* S = sc.E + ((size_t)blockIdx.x * a.heads + h) * a.N * a.P + p0;
+  const float* Cg = rows + inner + (size_t)a.G * a.N + (size_t)g * a.N;
+  for (int n0 = 0; n0 < a.N; n0 += 32) {          // rows t, columns p, over the lanes of the state
+    __syncthreads();
+    ssd_stage_turned(As, SSD_PAD, Cg + n0, C, nt, g_s);
+    for (int i = tid; i < 32 * 16; i += 128) {
+      const int n = i >> 4, k = (i & 15) * 4;
+      *(float4*)(Bs + n * SSD_L + k) = p0 + k < a.P ? *(const float4*)(S + (size_t)(n0 + n) * a.P + k) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    __syncthreads();
+    ssd_mma32(acc, As, Bs, mt, nn);
+  }
+  const float* cb = sc.cb + ((size_t)blockIdx.x * a.G + g) * SSD_L * SSD_L;
+  for (int s0 = 0; s0 < nt; s0 += 32) {           // over the chunk's tokens
+    __syncthreads();
+    bool odd = false;      // a value that is not finite: times the zeros of the earlier tokens' rows it would reach them
+    for (int i = tid; i < 32 * 16; i += 128) {
+      const int s = i >> 4, k = (i & 15) * 4;
+      const float4 c = *(const float4*)(cb + (size_t)(s0 + s) * SSD_L + k), d = *(const float4*)(Ds + (s0 + s) * SSD_PAD + k);
+      float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (s0 + s < nt && p0 + k < a.P) x = *(const float4*)(X + (size_t)(s0 + s) * C + k);
+      const float4 m = make_float4(c.x * d.x, c.y * d.y, c.z * d.z, c.w * d.w);
+      odd = odd || !isfinite(((m.x + m.y) + (m.z + m.w)) * 0.f + ((x.x + x.y) + (x.z + x.w)) * 0.f);
+      *(float4*)(As + s * SSD_PAD + k) = m;
+      *(float4*)(Bs + s * SSD_L + k) = x;
+    }
+    if (__syncthreads_or(odd)) ssd_mma32<true>(acc, As, Bs, mt, nn, s0);
+    else ssd_mma32(acc, As, Bs, mt, nn);
+  }
+  if (p0 + 4 * nn < a.P) {
+    const float skip = a.d_skip[h];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const int t = (i & 4) * 8 + 4 * mt + (i & 3);
+      if (t >= nt) continue;
+      const float4 x = *(const float4*)(X + (size_t)t * C + 4 * nn);
+      *(float4*)(a.y + (tok + t) * inner + (size_t)h * a.P + p0 + 4 * nn) =
+          make_float4(fmaf(skip, x.x, acc[i][0]), fmaf(skip, x.y, acc[i][1]), fmaf(skip, x.z, acc[i][2]), fmaf(skip, x.w, acc[i][3]));
+    }
+  }
+}
+
 template <typename T>
 __global__ void __launch_bounds__(256)
 ssd_gate_norm_kernel(SsdArgs a) {
@@ -306,6 +566,15 @@ static int ssd_launch(const SsdArgs& a, cudaStream_t stream) {
   odi_rc = launch_pdl((ssd_conv_kernel<T>), dim3(a.n_tokens, (C + 255) / 256), dim3(256), 0, stream, a);
   if (odi_rc == 0 && a.taps > 1)
     odi_rc = launch_pdl((ssd_conv_state_kernel<T>), dim3(a.n_seqs, (C + 255) / 256), dim3(256), 0, stream, a);
+  if (a.chunks != nullptr) {
+    const int p_tiles = (a.P + SSD_L - 1) / SSD_L;
+    const unsigned slots = (unsigned)run_chunk_slots(a.n_tokens, a.n_seqs, SSD_L);
+    if (odi_rc == 0) odi_rc = launch_pdl((ssd_states_kernel<T>), dim3(slots, a.heads * p_tiles * (a.N / SSD_L) + a.G), dim3(128), 0, stream, a);
+    if (odi_rc == 0) odi_rc = launch_pdl(ssd_pass_kernel, dim3((a.N * a.P + 511) / 512, a.heads, a.n_seqs), dim3(128), 0, stream, a);
+    if (odi_rc == 0) odi_rc = launch_pdl((ssd_outputs_kernel<T>), dim3(slots, a.heads * p_tiles), dim3(128), 0, stream, a);
+    if (odi_rc == 0) odi_rc = launch_pdl((ssd_gate_norm_kernel<T>), dim3(a.n_tokens, a.norm_groups), dim3(256), 0, stream, a);
+    return launch_status();
+  }
   // Two forms: 32 columns a block when that already gives two blocks per multiprocessor (many sequences); else 8
   // columns, four times the blocks, since a warp's time is the chain of its sequence's tokens and a step of one long
   // sequence has nothing else to run beside it.  (Measured at 32 heads of 64 columns, 128 rows, 2,048 tokens: 32
@@ -334,7 +603,7 @@ static int ssd_launch(const SsdArgs& a, cudaStream_t stream) {
   return launch_status();
 }
 
-// Kernels launched by one call: 3, or 4 with a convolution state.
+// Kernels launched by one call: 3 token by token, 5 in chunks; one more with a convolution state.
 extern "C" int odi_ssd(const SsdArgs* args, int dtype, cudaStream_t stream) {
   const SsdArgs a = *args;
   if (a.n_tokens <= 0 || a.n_seqs <= 0) return 0;
@@ -343,5 +612,8 @@ extern "C" int odi_ssd(const SsdArgs* args, int dtype, cudaStream_t stream) {
     return ODI_ERR_ARGUMENT;
   if (a.N > 256 || a.taps > SSD_MAX_TAPS || a.heads > 65535 || a.n_seqs > 65535 || a.norm_groups > 65535) return ODI_ERR_UNSUPPORTED;
   if (a.taps > 1 && a.conv_state == nullptr) return ODI_ERR_ARGUMENT;
+  if (a.chunks != nullptr && (a.N % SSD_L != 0 || a.P % 4 != 0 || ((uintptr_t)a.chunks | (uintptr_t)a.xbc | (uintptr_t)a.y | (uintptr_t)a.state) % 16 != 0 ||
+                              (long)a.heads * ((a.P + SSD_L - 1) / SSD_L) * (a.N / SSD_L) + a.G > 65535))
+    return ODI_ERR_UNSUPPORTED;
   return dtype == 0 ? ssd_launch<float>(a, stream) : ssd_launch<bf16>(a, stream);
 }

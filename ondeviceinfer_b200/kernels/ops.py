@@ -2034,12 +2034,25 @@ def gated_lookup(z: torch.Tensor, table: torch.Tensor, ids: torch.Tensor, out: t
 class _SsdArgs(Structure):
     _fields_ = [("proj", c_void_p), ("conv_w", c_void_p), ("conv_b", c_void_p), ("dt_bias", c_void_p), ("a_log", c_void_p),
                 ("d_skip", c_void_p), ("norm_w", c_void_p), ("conv_state", c_void_p), ("state", c_void_p), ("xbc", c_void_p),
-                ("y", c_void_p), ("out", c_void_p), ("cu_q", c_void_p), ("tok_seq", c_void_p), ("slots", c_void_p),
+                ("y", c_void_p), ("chunks", c_void_p), ("out", c_void_p), ("cu_q", c_void_p), ("tok_seq", c_void_p), ("slots", c_void_p),
                 ("n_tokens", c_int), ("n_seqs", c_int), ("ld", c_int), ("heads", c_int), ("P", c_int), ("N", c_int),
                 ("G", c_int), ("taps", c_int), ("norm_groups", c_int), ("eps", c_float)]
 
 
 SSD_MAX_STATE, SSD_MAX_TAPS = 256, 16
+# The scan of runs of tokens goes 64 tokens at a time when a sequence brings this many on average
+# (the mixer of 32 heads of 128 x 64, us in chunks and token by token: 64 tokens 57, 38; 128 63, 60; 8 x 100 99, 107; 512 79, 152).
+SSD_CHUNK, SSD_CHUNK_MIN_RUN, SSD_CHUNK_MAX_SCRATCH = 64, 128, 1 << 30
+
+
+def ssd_chunk_floats(n_tokens: int, n_seqs: int, heads: int, head_dim: int, state_dim: int, groups: int) -> int:
+    """Floats of scratch for a state-space scan in chunks (the chunks' states, products of B and C, decays); 0 where it goes
+    token by token: short runs, sizes that the chunk kernels do not take, more scratch than SSD_CHUNK_MAX_SCRATCH bytes."""
+    if (n_tokens < SSD_CHUNK_MIN_RUN * n_seqs or state_dim % SSD_CHUNK != 0 or head_dim % 4 != 0
+            or heads * -(-head_dim // SSD_CHUNK) * (state_dim // SSD_CHUNK) + groups > 65535):
+        return 0
+    floats = (n_tokens // SSD_CHUNK + n_seqs) * (heads * state_dim * head_dim + groups * SSD_CHUNK * SSD_CHUNK + heads)
+    return floats if 4 * floats <= SSD_CHUNK_MAX_SCRATCH else 0
 
 
 def ssd_mix(proj: torch.Tensor, conv_w: torch.Tensor, conv_b: torch.Tensor, dt_bias: torch.Tensor, a_log: torch.Tensor,
@@ -2069,12 +2082,14 @@ def ssd_mix(proj: torch.Tensor, conv_w: torch.Tensor, conv_b: torch.Tensor, dt_b
             raise KernelError("ssd_mix: the convolution state is [slots, taps - 1, channels]")
     xbc = torch.empty((n, C), dtype=torch.float32, device=proj.device)
     y = torch.empty((n, inner), dtype=torch.float32, device=proj.device)
+    scratch = ssd_chunk_floats(n, n_seqs, heads, head_dim, state_dim, groups)
+    chunks = torch.empty(scratch, dtype=torch.float32, device=proj.device) if scratch else None
     args = _SsdArgs(_ptr(proj), _ptr(conv_w), _ptr(conv_b), _ptr(dt_bias), _ptr(a_log), _ptr(d_skip), _ptr(norm_w),
-                    _ptr(conv_state if taps > 1 else None), _ptr(state), _ptr(xbc), _ptr(y), _ptr(out), _ptr(cu_q),
+                    _ptr(conv_state if taps > 1 else None), _ptr(state), _ptr(xbc), _ptr(y), _ptr(chunks), _ptr(out), _ptr(cu_q),
                     _ptr(tok_seq), _ptr(slots), n, n_seqs, proj.shape[1], heads, head_dim, state_dim, groups, taps,
                     norm_groups, eps)
     lib = load_library("ssd")
-    _check(lib.odi_ssd(byref(args), c_int(dtype_code(proj.dtype)), _stream()), "ssd_mix", 4 if taps > 1 else 3)
+    _check(lib.odi_ssd(byref(args), c_int(dtype_code(proj.dtype)), _stream()), "ssd_mix", (5 if scratch else 3) + (taps > 1))
 
 
 # ------------------------------------------------------------------------------ parallel residual streams

@@ -11,6 +11,7 @@ largest row error is bounded only for models without them."""
 import copy
 import json
 import math
+import math
 import subprocess
 import sys
 from pathlib import Path
@@ -278,6 +279,62 @@ def test_state_space_mixer_over_cut_sequences(dtype, heads, P, N, G, taps, parts
     for s in range(3):
         torch.testing.assert_close(torch.cat(got[s]).double(), want[s], **(dict(atol=2e-4, rtol=2e-4) if dtype == torch.float32
                                                                            else dict(atol=3e-2, rtol=3e-2)))
+
+
+@pytest.mark.parametrize("heads,P,N,G,taps,parts", [(4, 64, 128, 2, 4, 1), (3, 20, 64, 1, 1, 3), (2, 100, 192, 2, 2, 1)])
+def test_state_space_scan_in_chunks_of_tokens(heads, P, N, G, taps, parts):
+    """Runs around the chunks' edges, one of a single token among them, continued by a second step, with decays down to
+    those that wipe the state; against the recurrence over each whole sequence, and no further off than the token by token
+    kernel.  A token that is not a number reaches no token before it."""
+    gen = torch.Generator().manual_seed(heads * P + N)
+    inner, C = heads * P, heads * P + 2 * G * N
+    M, slots, cuts = inner + C + heads, [3, 0, 4, 1], [[380, 64, 1, 70], [63, 129, 250, 75]]
+    lengths = [a + b for a, b in zip(*cuts)]
+    projs = [torch.randn(L, M, generator=gen) for L in lengths]
+    projs[0][40:42, -heads:] = 300.0             # the state is wiped inside a chunk
+    w = {"in": torch.eye(M, dtype=torch.float64), "o": torch.eye(inner, dtype=torch.float64),
+         "conv": torch.randn(C, taps, generator=gen) * 0.5, "conv.b": torch.randn(C, generator=gen) * 0.1,
+         "dt_bias": torch.randn(heads, generator=gen) * 0.5 - 2, "A_log": torch.log(0.02 + 4 * torch.rand(heads, generator=gen)),
+         "D": 1 + 0.3 * torch.randn(heads, generator=gen), "norm": 1 + 0.1 * torch.randn(inner, generator=gen)}
+    m = {"heads": heads, "vdim": P, "state": N, "groups": G, "conv": taps, "norm_groups": parts}
+    want = [plain.state_space({k: v.double() for k, v in w.items()}, "", m, p.double(), 1e-5) for p in projs]
+    dev = {k: v.float().cuda() for k, v in w.items()}
+
+    def run(projs):
+        state = torch.zeros(6, heads, N, P, device="cuda")
+        conv_state = torch.zeros(6, taps - 1, C, device="cuda") if taps > 1 else None
+        state[2].fill_(7.0)          # a slot of somebody else: must stay as it is
+        got, at = [[] for _ in lengths], [0] * len(lengths)
+        for lens in cuts:
+            cu = [0]
+            for n in lens:
+                cu.append(cu[-1] + n)
+            out = torch.empty(cu[-1], inner, device="cuda")
+            ops.ssd_mix(torch.cat([x[o:o + n] for x, o, n in zip(projs, at, lens)]).cuda(), dev["conv"], dev["conv.b"], dev["dt_bias"],
+                        dev["A_log"], dev["D"], dev["norm"], conv_state, state, out, ints(*cu),
+                        ints(*[s for s, n in enumerate(lens) for _ in range(n)]), ints(*slots), n_seqs=len(lens), heads=heads, head_dim=P,
+                        state_dim=N, groups=G, norm_groups=parts, eps=1e-5)
+            for s, n in enumerate(lens):
+                got[s].append(out[cu[s]:cu[s + 1]].cpu().double())
+                at[s] += n
+        assert at == lengths and bool((state[2] == 7.0).all())
+        return [torch.cat(g) for g in got], state
+
+    off = lambda got: [float((a - b).norm() / b.norm()) for a, b in zip(got, want)]
+    assert ops.ssd_chunk_floats(sum(cuts[0]), 4, heads, P, N, G) > 0
+    (chunked, state), least = run(projs), ops.SSD_CHUNK_MIN_RUN
+    ops.SSD_CHUNK_MIN_RUN = 1 << 30
+    try:
+        single, state_single = run(projs)
+    finally:
+        ops.SSD_CHUNK_MIN_RUN = least
+    assert max(off(chunked)) < 5e-6 and max(off(single)) < 5e-6      # sums of a few hundred products of 2^-24 each
+    assert sum(off(chunked)) <= 1.25 * sum(off(single))
+    torch.testing.assert_close(state, state_single, atol=2e-5, rtol=2e-5)
+    broken = [p.clone() for p in projs]
+    broken[0][100, inner:] = math.nan      # in the middle of a chunk
+    got = run(broken)[0][0]
+    assert bool(torch.equal(got[:100], chunked[0][:100])) and not bool(torch.isfinite(got[100:]).any())
 
 
 # ----------------------------------------------------------------------------- attention with kept first positions
