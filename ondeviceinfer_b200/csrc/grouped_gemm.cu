@@ -17,9 +17,6 @@
 // TM = 64 (4 x 4 outputs a thread) or 16 (1 x 4), chosen by the caller from the rows a group has; for groups
 // of a few rows there is a form that streams the weights through registers only (grouped_gemv_kernel).
 #include "common.cuh"
-#include <algorithm>
-#include <cstring>
-#include <type_traits>
 
 #define TN 64
 
@@ -190,9 +187,10 @@ grouped_gemm_kernel(GroupedArgs a) {
 // the lanes at the end (a fixed tree: the result of a row does not depend on the other rows of the launch).
 // Needs what VEC needs.
 #define GV_ROWS 4
-template <typename T, bool GATED>
+template <bool GATED>
 __global__ void __launch_bounds__(256, 2)
 grouped_gemv_kernel(GroupedArgs a) {
+  typedef float T;
   pdl_launch_dependents();
   pdl_wait();
   extern __shared__ __align__(16) float xs[];       // [GV_ROWS][K]
@@ -291,170 +289,152 @@ grouped_gemv_kernel(GroupedArgs a) {
   }
 }
 
-// bf16 with the weights streamed through shared memory by cp.async: every lane keeps several requests of 16 bytes per
-// weight row in flight and later reads exactly the bytes it asked for, so the ring needs no barrier, and the stream
-// is decoupled from the arithmetic: far more bytes on their way per SM than the registers of the form above can hold.
-#define GS_CHUNK 256          // k per stage: 32 lanes x 8
-__device__ __forceinline__ void gs_cp_async16(void* dst, const void* src) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
+// bf16 on the tensor cores (mma.sync m16n8k16, fp32 sums): the weights are the 16-row operand, 8 NT input rows of a group the
+// 8-column ones, so a group's weights pass once over a tile of its rows (a table's larger tile: once per 8 NT rows of it).  What
+// bounds it is the stream of weights, so nothing stands between it and the tensor cores: a lane loads 16 bytes (8 neighbouring
+// k) of its weight rows straight into registers, and of its input rows likewise; the k of an mma may come in any order as long as
+// both operands agree, so those 8 are the lane's k of two mma.  A block owns 16 features (gated: and their 16 up rows) and all
+// k: its four warps take pieces of 128 k in turn, all of a piece's loads on their way at once (about 100 KB a multiprocessor), the
+// first weights before the input rows are looked up; the warps' sums meet in shared memory.  The tensor core cuts off what its
+// sums cannot hold, so 16 k are summed from zero there, eight such sums pairwise and then to the rest by rounded additions, in
+// an order that depends on neither the other rows nor NT.
+// Measured, bf16, four of 32 experts of 2,048 x 1,024 a token, L2 flushed, up / gated up / down in us, against the forms before (lists
+// of items walked by warps on the CUDA cores up to 4 rows an expert, else tiles of 16 rows there): 1 token 8 / 11 / 7 and 9 / 14 / 9, 8
+// tokens 20 / 34 / 18 and 34 / 54 / 34 (the weights alone 13 / 26 / 13), 32 tokens 26 / 50 / 27 and 79 / 122 / 124, 56 tokens 30 / 56 / 30
+// and 221 / 400 / 186, 250 tokens 70 / 123 / 72 and 467 / 810 / 434.  Tiles of 32 and 64 rows were no faster (250 tokens: 72 and 107).
+__device__ __forceinline__ void mma16(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+               : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
-__device__ __forceinline__ void gs_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N> __device__ __forceinline__ void gs_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
-__device__ __forceinline__ void gs_unpack8(const uint4& raw, float* out) {
-  const __nv_bfloat162* h = (const __nv_bfloat162*)&raw;
-#pragma unroll
-  for (int i = 0; i < 4; ++i) { const float2 f = __bfloat1622float2(h[i]); out[2 * i] = f.x; out[2 * i + 1] = f.y; }
-}
-
-// Blocks that stay: one block an SM, and every warp on its own walks a list of items (a tile of up to 4 input rows
-// x R weight rows), item after item through one ring of S stages, so that the requests for the next item's first
-// chunks are out before the current item ends and the ring stays full across items.  A stage holds one chunk
-// (256 k) of the R weight rows and of the tile's input rows (each lane asks for, and later reads, its own 16 bytes of
-// every row: no barrier anywhere).  The items of a warp are laid out 32 at a time by its lanes (group, rows and source
-// rows of the tile) in shared memory.  Sums per lane in the same order as the forms above, the same tree over lanes.
-template <bool GATED, int R, int S>
-__global__ void __launch_bounds__(256, 1)
-grouped_gemv_walk_kernel(GroupedArgs a, int row_tiles) {
+template <bool GATED, int NT>
+__global__ void __launch_bounds__(128, GATED ? (NT == 1 ? 4 : 3) : (NT == 1 ? 6 : 5))      // six blocks a multiprocessor: 80 registers (56 tokens: 28 us, with 147 35)
+grouped_mma_kernel(GroupedArgs a, int tm, int tiles) {
   pdl_launch_dependents();
   pdl_wait();
-  extern __shared__ __align__(16) uint8_t gs_smem[];
-  constexpr int STAGE = (R + GV_ROWS) * 512;
-  constexpr int FEATS = GATED ? R / 2 : R;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  uint8_t* ring = gs_smem + (size_t)warp * S * STAGE + lane * 16;
-  int* meta = (int*)(gs_smem + (size_t)8 * S * STAGE) + warp * 32 * 8;
+  constexpr int MT = GATED ? 2 : 1, ROWS = 8 * NT, PITCH = ROWS + 1, U = 4, PIECE = 32 * U;
+  __shared__ float red[4][MT * 16][PITCH];
+  __shared__ int arow[ROWS];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, gq = lane >> 2, tq = lane & 3;
   const bool table = a.tile_group != nullptr;
-  const int ncg = (a.N + FEATS - 1) / FEATS;
-  const long long n_items = (long long)(table ? a.n_tiles[0] : row_tiles * a.groups) * ncg;
-  const int nw = gridDim.x * 8, gw = warp * gridDim.x + blockIdx.x;       // neighbouring items on different SMs
-  if (gw >= n_items) return;
-  const int my_items = (int)((n_items - gw + nw - 1) / nw);
-  const int n_chunks = (a.K + GS_CHUNK - 1) / GS_CHUNK;
-  const int kl = lane * 8;
-  for (int base = 0; base < my_items; base += 32) {
-    const int cnt = min(32, my_items - base);
-    if (lane < cnt) {
-      const long long item = gw + (long long)(base + lane) * nw;
-      const int t = (int)(item / ncg);
-      int group, row0, rows;
-      if (table) { group = a.tile_group[t]; row0 = a.tile_row0[t]; rows = a.tile_rows[t]; }
-      else { group = t / row_tiles; row0 = (t % row_tiles) * GV_ROWS; rows = min(GV_ROWS, a.M - row0); }
-      int* m = meta + lane * 8;
-      m[0] = group; m[1] = row0; m[2] = rows; m[3] = (int)(item % ncg);
-#pragma unroll
-      for (int r = 0; r < GV_ROWS; ++r)
-        m[4 + r] = r < rows ? (a.row_index != nullptr ? a.row_index[row0 + r] / a.index_div : row0 + r) : -1;
-    }
-    __syncwarp();
-    // the requesting side: item and chunk of the next request, and the item's addresses
-    int is_it = 0, is_chunk = 0, is_stage = 0, is_n0 = 0;
-    const bf16* is_w = nullptr;
-    const bf16* is_x[GV_ROWS] = {};
-    auto issue = [&]() {
-      if (is_it < cnt) {
-        if (is_chunk == 0) {
-          const int* m = meta + is_it * 8;
-          const int group = m[0];
-          is_w = (const bf16*)a.W + (size_t)group * a.w_group_stride;
-          is_n0 = m[3] * FEATS;
-          const bf16* A = (const bf16*)a.A + (table ? 0 : (size_t)group * a.a_group_off);
-#pragma unroll
-          for (int r = 0; r < GV_ROWS; ++r) is_x[r] = m[4 + r] >= 0 ? A + (size_t)m[4 + r] * a.lda : nullptr;
-        }
-        const int k = is_chunk * GS_CHUNK + kl;
-        if (k < a.K) {
-          uint8_t* st = ring + (size_t)is_stage * STAGE;
-#pragma unroll
-          for (int j = 0; j < R; ++j) {
-            const int n = GATED ? is_n0 + (j >> 1) : is_n0 + j;
-            if (n < a.N) gs_cp_async16(st + j * 512, is_w + (size_t)((GATED && (j & 1)) ? a.N + n : n) * a.ldw + k);
-          }
-#pragma unroll
-          for (int r = 0; r < GV_ROWS; ++r)
-            if (is_x[r] != nullptr) gs_cp_async16(st + (R + r) * 512, is_x[r] + k);
-        }
-        if (++is_chunk == n_chunks) { is_chunk = 0; ++is_it; }
-      }
-      if (++is_stage == S) is_stage = 0;
-      gs_commit();                     // one group per request, empty or not: the count stays uniform
-    };
-#pragma unroll
-    for (int c = 0; c < S - 1; ++c) issue();
-    float acc[R][GV_ROWS];
-    int cp_it = 0, cp_chunk = 0, cp_stage = 0, rows = 0, n0 = 0;
-    const int total = cnt * n_chunks;
-    for (int i = 0; i < total; ++i) {
-      issue();
-      gs_wait<S - 1>();                // this lane's requests for step i have landed
-      if (cp_chunk == 0) {
-#pragma unroll
-        for (int j = 0; j < R; ++j)
-#pragma unroll
-          for (int r = 0; r < GV_ROWS; ++r) acc[j][r] = 0.f;
-        rows = meta[cp_it * 8 + 2];
-        n0 = meta[cp_it * 8 + 3] * FEATS;
-      }
-      if (cp_chunk * GS_CHUNK + kl < a.K) {
-        const uint8_t* st = ring + (size_t)cp_stage * STAGE;
-        auto step = [&](auto nr_tag) {
-          constexpr int NR = decltype(nr_tag)::value;
-          float x[NR][8];
-#pragma unroll
-          for (int r = 0; r < NR; ++r) gs_unpack8(*(const uint4*)(st + (R + r) * 512), x[r]);
-#pragma unroll
-          for (int j = 0; j < R; ++j) {
-            if ((GATED ? n0 + (j >> 1) : n0 + j) >= a.N) continue;
-            float w[8];
-            gs_unpack8(*(const uint4*)(st + j * 512), w);
-#pragma unroll
-            for (int r = 0; r < NR; ++r)
-#pragma unroll
-              for (int e = 0; e < 8; ++e) acc[j][r] = fmaf(w[e], x[r][e], acc[j][r]);
-          }
-        };
-        if (rows <= 1) step(std::integral_constant<int, 1>{});
-        else if (rows == 2) step(std::integral_constant<int, 2>{});
-        else if (rows == 3) step(std::integral_constant<int, 3>{});
-        else step(std::integral_constant<int, GV_ROWS>{});
-      }
-      if (++cp_stage == S) cp_stage = 0;
-      if (++cp_chunk == n_chunks) {
-#pragma unroll
-        for (int j = 0; j < R; ++j)
-#pragma unroll
-          for (int r = 0; r < GV_ROWS; ++r) acc[j][r] = warp_sum(acc[j][r]);
-        if (lane == 0) {
-          const int group = meta[cp_it * 8], row0 = meta[cp_it * 8 + 1];
-#pragma unroll
-          for (int r = 0; r < GV_ROWS; ++r) {
-            if (r >= rows) continue;
-            const size_t crow = (size_t)(row0 + r) * a.ldc + (table ? 0 : (size_t)group * a.c_group_off);
-            if (GATED) {
-#pragma unroll
-              for (int f = 0; f < R / 2; ++f) {
-                const int n = n0 + f;
-                if (n >= a.N) continue;
-                const float g = fminf(acc[2 * f][r], a.limit);
-                const float u = fminf(fmaxf(acc[2 * f + 1][r], -a.limit), a.limit);
-                ((bf16*)a.C)[crow + n] = from_f<bf16>(g / (1.f + expf(-a.alpha * g)) * (u + a.up_shift));
-              }
-            } else {
-#pragma unroll
-              for (int j = 0; j < R; ++j) {
-                const int n = n0 + j;
-                if (n >= a.N) continue;
-                if (a.epi == 1) ((float*)a.C)[crow + n] = acc[j][r];
-                else ((bf16*)a.C)[crow + n] = from_f<bf16>(grouped_act(acc[j][r], a.epi));
-              }
-            }
-          }
-        }
-        cp_chunk = 0; ++cp_it;
-      }
-    }
-    gs_wait<0>();
-    __syncwarp();                      // the next 32 items overwrite the list
+  int group, tile_row0, tile_rows;
+  if (table) {
+    const int t = blockIdx.x % tiles;
+    if (t >= a.n_tiles[0]) return;
+    group = a.tile_group[t]; tile_row0 = a.tile_row0[t]; tile_rows = a.tile_rows[t];
+  } else {
+    group = blockIdx.z; tile_row0 = blockIdx.x % tiles * tm; tile_rows = min(tm, a.M - tile_row0);
   }
+  const int n0 = blockIdx.x / tiles * 16;
+  const bf16* A = (const bf16*)a.A + (table ? 0 : (size_t)group * a.a_group_off) + 8 * tq;
+  const bf16* W = (const bf16*)a.W + (size_t)group * a.w_group_stride + 8 * tq;
+  const bf16* wrow[MT][2];
+#pragma unroll
+  for (int m = 0; m < MT; ++m)
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      const int n = n0 + 8 * i + gq;
+      wrow[m][i] = n < a.N ? W + (size_t)(m ? a.N + n : n) * a.ldw : nullptr;
+    }
+  const uint4 zero = make_uint4(0, 0, 0, 0);
+  uint4 w[U][MT][2];
+  auto load_w = [&](int kc) {
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int k = kc + 32 * u;
+      const bool in = k + 8 * tq < a.K;      // K is a multiple of 8: a lane's 8 are all inside or all outside
+#pragma unroll
+      for (int m = 0; m < MT; ++m)
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+          w[u][m][i] = zero;
+          if (in && wrow[m][i] != nullptr) {
+            uint4& r = w[u][m][i];
+            asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(r.x), "=r"(r.y), "=r"(r.z), "=r"(r.w) : "l"(wrow[m][i] + k));
+          }
+        }
+    }
+  };
+  for (int done = 0; done < tile_rows; done += ROWS) {
+    const int row0 = tile_row0 + done, rows = min(ROWS, tile_rows - done);
+    load_w(warp * PIECE);                    // on their way while the input rows are looked up
+    if (tid < ROWS) arow[tid] = tid < rows ? (a.row_index != nullptr ? a.row_index[row0 + tid] / a.index_div : row0 + tid) : -1;
+    __syncthreads();
+    const bf16* xrow[NT];
+#pragma unroll
+    for (int j = 0; j < NT; ++j) xrow[j] = arow[8 * j + gq] >= 0 ? A + (size_t)arow[8 * j + gq] * a.lda : nullptr;
+    float acc[MT][NT][4] = {};
+    for (int kc = warp * PIECE; kc < a.K; kc += 4 * PIECE) {
+      uint4 x[U][NT];
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+#pragma unroll
+        for (int j = 0; j < NT; ++j)
+          x[u][j] = xrow[j] != nullptr && kc + 32 * u + 8 * tq < a.K ? *(const uint4*)(xrow[j] + kc + 32 * u) : zero;
+#pragma unroll
+      for (int j = 0; j < NT; ++j)
+#pragma unroll
+        for (int m = 0; m < MT; ++m) {
+          if (GATED) {      // rounded to bf16 behind the gate: fewer registers before a last bit
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+              float lo[4] = {}, hi[4] = {};
+              mma16(lo, w[u][m][0].x, w[u][m][1].x, w[u][m][0].y, w[u][m][1].y, x[u][j].x, x[u][j].y);
+              mma16(hi, w[u][m][0].z, w[u][m][1].z, w[u][m][0].w, w[u][m][1].w, x[u][j].z, x[u][j].w);
+#pragma unroll
+              for (int e = 0; e < 4; ++e) acc[m][j][e] += lo[e] + hi[e];
+            }
+            continue;
+          }
+          float c[2 * U][4] = {};
+#pragma unroll
+          for (int u = 0; u < U; ++u) {
+            mma16(c[2 * u], w[u][m][0].x, w[u][m][1].x, w[u][m][0].y, w[u][m][1].y, x[u][j].x, x[u][j].y);
+            mma16(c[2 * u + 1], w[u][m][0].z, w[u][m][1].z, w[u][m][0].w, w[u][m][1].w, x[u][j].z, x[u][j].w);
+          }
+#pragma unroll
+          for (int e = 0; e < 4; ++e)
+            acc[m][j][e] += ((c[0][e] + c[1][e]) + (c[2][e] + c[3][e])) + ((c[4][e] + c[5][e]) + (c[6][e] + c[7][e]));
+        }
+      load_w(kc + 4 * PIECE);
+    }
+#pragma unroll
+    for (int m = 0; m < MT; ++m)
+#pragma unroll
+      for (int j = 0; j < NT; ++j)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) red[warp][16 * m + gq + 8 * (e >> 1)][8 * j + 2 * tq + (e & 1)] = acc[m][j][e];
+    __syncthreads();
+    const size_t c0 = table ? 0 : (size_t)group * a.c_group_off;
+    auto sum = [&](int f, int r) { return (red[0][f][r] + red[1][f][r]) + (red[2][f][r] + red[3][f][r]); };
+    for (int i = tid; i < 16 * rows; i += 128) {
+      const int f = i & 15, r = i >> 4;
+      if (n0 + f >= a.N) continue;
+      const size_t at = (size_t)(row0 + r) * a.ldc + c0 + n0 + f;
+      const float v = sum(f, r);
+      if (GATED) {
+        const float g = fminf(v, a.limit), up = fminf(fmaxf(sum(16 * (MT - 1) + f, r), -a.limit), a.limit);
+        ((bf16*)a.C)[at] = from_f<bf16>(g / (1.f + expf(-a.alpha * g)) * (up + a.up_shift));
+      } else if (a.epi == 1) {
+        ((float*)a.C)[at] = v;
+      } else {
+        ((bf16*)a.C)[at] = from_f<bf16>(grouped_act(v, a.epi));
+      }
+    }
+    __syncthreads();                         // the next rows' sums take the place of these
+  }
+}
+
+static int launch_mma(const GroupedArgs& a, int max_tiles, int tm, cudaStream_t stream) {
+  const bool table = a.tile_group != nullptr;
+  if (table ? max_tiles <= 0 : a.M <= 0) return 0;
+  const int tiles = table ? max_tiles : (a.M + tm - 1) / tm;
+  const long blocks = (long)tiles * ((a.N + 15) / 16);
+  if (blocks > 0x7fffffffL || (!table && a.groups > 65535)) return ODI_ERR_UNSUPPORTED;
+  const dim3 grid((unsigned)blocks, 1, table ? 1 : a.groups);
+  auto kernel = a.epi == 2 ? (tm <= 8 ? grouped_mma_kernel<true, 1> : grouped_mma_kernel<true, 2>)
+                           : (tm <= 8 ? grouped_mma_kernel<false, 1> : grouped_mma_kernel<false, 2>);
+  odi_rc = launch_pdl(kernel, grid, dim3(128), 0, stream, a, tm, tiles);
+  return launch_status();
 }
 
 // max_tiles: with a tile table, the most tiles the table can hold (the grid's width); tm: 16 or 64 (the
@@ -469,12 +449,16 @@ extern "C" int odi_grouped_gemm_takes_few_rows(const GroupedArgs* args) {
   return vector_loads(*args) && (size_t)GV_ROWS * args->K * sizeof(float) <= 200 * 1024;
 }
 
+extern "C" int odi_grouped_gemm_takes_tensor(const GroupedArgs* args) { return vector_loads(*args); }
+
 extern "C" int odi_grouped_gemm(const GroupedArgs* args, int max_tiles, int tm, int dtype, cudaStream_t stream) {
   const GroupedArgs a = *args;
   if (a.N <= 0 || a.groups <= 0) return 0;
-  if (a.K <= 0 || (tm != GV_ROWS && tm != 16 && tm != 64) || a.epi < 0 || a.epi > 5) return ODI_ERR_ARGUMENT;
+  if (a.K <= 0 || (tm != GV_ROWS && tm != 8 && tm != 16 && tm != 64) || a.epi < 0 || a.epi > 5) return ODI_ERR_ARGUMENT;
+  if (dtype == 1 && vector_loads(a)) return launch_mma(a, max_tiles, tm, stream);
+  if (tm == 8) return ODI_ERR_UNSUPPORTED;
   if (tm == GV_ROWS) {
-    if (!odi_grouped_gemm_takes_few_rows(args)) return ODI_ERR_UNSUPPORTED;
+    if (dtype != 0 || !odi_grouped_gemm_takes_few_rows(args)) return ODI_ERR_UNSUPPORTED;      // bf16 operands that allow it have left above
     dim3 grid;
     const int per_block = a.epi == 2 ? 32 : 64;
     if (a.tile_group != nullptr) {
@@ -486,47 +470,11 @@ extern "C" int odi_grouped_gemm(const GroupedArgs* args, int max_tiles, int tm, 
       if (grid.z > 65535) return ODI_ERR_UNSUPPORTED;
     }
     if (grid.y > 65535) return ODI_ERR_UNSUPPORTED;
-    const char* form = getenv("ODI_GROUPED_GEMV");
-    if (dtype == 1 && (form == nullptr || strcmp(form, "registers") != 0)) {
-      // bf16: the weights through a cp.async ring (ODI_GROUPED_GEMV=registers keeps the form above)
-      static int sms = 0;
-      if (sms == 0) {
-        int dev = 0;
-        if (cudaGetDevice(&dev) != cudaSuccess ||
-            cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0) {
-          sms = 0;
-          return ODI_ERR_UNSUPPORTED;
-        }
-      }
-      const int per_feat = a.epi == 2 ? 2 : 1;            // weight rows a feature takes
-      const int row_tiles = a.tile_group != nullptr ? 0 : (a.M + GV_ROWS - 1) / GV_ROWS;
-      const long long tiles = a.tile_group != nullptr ? max_tiles : (long long)row_tiles * a.groups;
-      if (tiles * ((a.N + 1) / 2 + 1) > (1ll << 40)) return ODI_ERR_UNSUPPORTED;
-      // items of 8 weight rows ask in larger pieces; items of 4 spread a short list more evenly over the warps
-      const long long items8 = tiles * ((a.N * per_feat + 7) / 8);
-      const bool wide = form != nullptr ? strcmp(form, "walk8") == 0 : items8 >= 10ll * 8 * sms;
-      const int feats = (wide ? 8 : 4) / per_feat;
-      const long long items = tiles * ((a.N + feats - 1) / feats);
-      const int blocks = (int)std::min<long long>(sms, (items + 7) / 8);
-      const size_t walk_smem = (size_t)8 * 6 * (4 + GV_ROWS) * 512 + 8 * 32 * 8 * sizeof(int);   // equal for both shapes
-#define ODI_GW(G, R, S) \
-      do { cudaError_t e = cudaFuncSetAttribute(grouped_gemv_walk_kernel<G, R, S>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)walk_smem); \
-           if (e != cudaSuccess) return (int)e; \
-           odi_rc = launch_pdl((grouped_gemv_walk_kernel<G, R, S>), dim3(blocks), dim3(256), walk_smem, stream, a, row_tiles); } while (0)
-      if (wide) { if (a.epi == 2) ODI_GW(true, 8, 4); else ODI_GW(false, 8, 4); }
-      else { if (a.epi == 2) ODI_GW(true, 4, 6); else ODI_GW(false, 4, 6); }
-#undef ODI_GW
-      return launch_status();
-    }
     const size_t smem = (size_t)GV_ROWS * a.K * sizeof(float);
-#define ODI_GV(T, G) \
-    do { cudaError_t e = cudaFuncSetAttribute(grouped_gemv_kernel<T, G>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
-         if (e != cudaSuccess) return (int)e; \
-         odi_rc = launch_pdl((grouped_gemv_kernel<T, G>), grid, dim3(256), smem, stream, a); } while (0)
-    const bool g = a.epi == 2;
-    if (dtype == 0) { if (g) ODI_GV(float, true); else ODI_GV(float, false); }
-    else { if (g) ODI_GV(bf16, true); else ODI_GV(bf16, false); }
-#undef ODI_GV
+    auto kernel = a.epi == 2 ? grouped_gemv_kernel<true> : grouped_gemv_kernel<false>;
+    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return (int)e;
+    odi_rc = launch_pdl(kernel, grid, dim3(256), smem, stream, a);
     return launch_status();
   }
   dim3 grid;
@@ -539,18 +487,15 @@ extern "C" int odi_grouped_gemm(const GroupedArgs* args, int max_tiles, int tm, 
     if (grid.z > 65535) return ODI_ERR_UNSUPPORTED;
   }
   if (grid.y > 65535) return ODI_ERR_UNSUPPORTED;
-  const bool vec = vector_loads(a);
-#define ODI_GG(T, TM, G) \
-  do { if (vec) odi_rc = launch_pdl((grouped_gemm_kernel<T, TM, G, true>), grid, dim3(256), 0, stream, a); \
-       else odi_rc = launch_pdl((grouped_gemm_kernel<T, TM, G, false>), grid, dim3(256), 0, stream, a); } while (0)
+#define ODI_GG(T, TM, G, VEC) odi_rc = launch_pdl((grouped_gemm_kernel<T, TM, G, VEC>), grid, dim3(256), 0, stream, a)
+#define ODI_GG_FORMS(T, VEC) \
+  do { if (tm == 64) { if (gated) ODI_GG(T, 64, true, VEC); else ODI_GG(T, 64, false, VEC); } \
+       else { if (gated) ODI_GG(T, 16, true, VEC); else ODI_GG(T, 16, false, VEC); } } while (0)
   const bool gated = a.epi == 2;
-  if (dtype == 0) {
-    if (tm == 64) { if (gated) ODI_GG(float, 64, true); else ODI_GG(float, 64, false); }
-    else { if (gated) ODI_GG(float, 16, true); else ODI_GG(float, 16, false); }
-  } else {
-    if (tm == 64) { if (gated) ODI_GG(bf16, 64, true); else ODI_GG(bf16, 64, false); }
-    else { if (gated) ODI_GG(bf16, 16, true); else ODI_GG(bf16, 16, false); }
-  }
+  if (dtype == 1) ODI_GG_FORMS(bf16, false);      // with aligned operands on the tensor cores, above
+  else if (vector_loads(a)) ODI_GG_FORMS(float, true);
+  else ODI_GG_FORMS(float, false);
+#undef ODI_GG_FORMS
 #undef ODI_GG
   return launch_status();
 }

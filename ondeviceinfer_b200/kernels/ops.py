@@ -1167,9 +1167,11 @@ GROUPED_STORE, GROUPED_STORE_F32, GROUPED_GATED_CLAMP, GROUPED_GELU_ERF, GROUPED
 FEW_ROWS = 4      # row tile of the grouped product's form for single-token steps (weights through registers only)
 
 
-def grouped_rows_tile(rows_per_group: float, few_rows_ok: bool = False) -> int:
-    """Row tile of the grouped product for groups of about this many rows: 4 (if the operands allow the form for
-    few rows), 16 or 64."""
+def grouped_rows_tile(rows_per_group: float, few_rows_ok: bool = False, tensor: bool = False) -> int:
+    """Row tile of the grouped product for groups of about this many rows: 8 or 16 on the tensor cores (``tensor``:
+    :func:`grouped_tensor_ok`), else 4 (if the operands allow the form for few rows), 16 or 64."""
+    if tensor:
+        return 8 if rows_per_group <= 8 else 16
     if few_rows_ok and rows_per_group <= FEW_ROWS:
         return FEW_ROWS
     return 64 if rows_per_group > 32 else 16
@@ -1179,6 +1181,11 @@ def grouped_few_rows_ok(K_values: Sequence[int], dtype: torch.dtype) -> bool:
     """Whether products over these inner sizes can take the form for few rows (multiples of 8, and four rows of
     floats within the shared memory of a block)."""
     return all(K % 8 == 0 and 4 * FEW_ROWS * K <= 200 * 1024 for K in K_values)
+
+
+def grouped_tensor_ok(K_values: Sequence[int], dtype: torch.dtype) -> bool:
+    """Whether products over these inner sizes run on the tensor cores (bf16, rows in pieces of 16 bytes)."""
+    return dtype == torch.bfloat16 and all(K % 8 == 0 for K in K_values)
 
 
 def grouped_gemm_heads(a: torch.Tensor, w: torch.Tensor, c: torch.Tensor, *, a_col: int, a_stride: int, c_col: int,
@@ -1200,7 +1207,8 @@ def grouped_gemm_heads(a: torch.Tensor, w: torch.Tensor, c: torch.Tensor, *, a_c
     # up to four rows: the form that streams the weights; five to eight rows too when the inner size is long (the
     # tile form would walk it in a few blocks per head), in two row tiles; else tiles of 16 or 64 rows
     few = M <= 2 * FEW_ROWS and (M <= FEW_ROWS or K >= 256) and bool(lib.odi_grouped_gemm_takes_few_rows(byref(args)))
-    tm = FEW_ROWS if few else grouped_rows_tile(M)
+    tensor = w.dtype == torch.bfloat16 and bool(lib.odi_grouped_gemm_takes_tensor(byref(args)))
+    tm = FEW_ROWS if few and not tensor else grouped_rows_tile(M, tensor=tensor)
     _check(lib.odi_grouped_gemm(byref(args), c_int(0), c_int(tm), c_int(dtype_code(w.dtype)), _stream()), "grouped_gemm")
 
 
@@ -1220,7 +1228,8 @@ def grouped_gemm_routed(a: torch.Tensor, w: torch.Tensor, c: torch.Tensor, table
                         _ptr(table.tile_row0), _ptr(table.tile_rows), _ptr(table.n_tiles), 0, w_rows * K, 0,
                         K, K, N, 0, N, K, experts, table.top if gather else 1, epi, limit, alpha, up_shift)
     lib = load_library("grouped_gemm")
-    _check(lib.odi_grouped_gemm(byref(args), c_int(table.max_tiles), c_int(table.tm), c_int(dtype_code(w.dtype)),
+    tiles = min(table.max_tiles, table.n_pairs)      # every tile holds a pair
+    _check(lib.odi_grouped_gemm(byref(args), c_int(tiles), c_int(table.tm), c_int(dtype_code(w.dtype)),
                                 _stream()), "grouped_gemm")
 
 
@@ -1262,9 +1271,10 @@ class RoutingTable:
     """The (token, choice) pairs of a step sorted by expert, made on the device by :func:`moe_group`: ``perm`` the
     sorted order, ``pos`` each pair's place in it, and the table of row tiles the grouped products walk."""
 
-    def __init__(self, n_tokens: int, top: int, n_experts: int, device, few_rows_ok: bool = False) -> None:
+    def __init__(self, n_tokens: int, top: int, n_experts: int, device, few_rows_ok: bool = False,
+                 tensor: bool = False) -> None:
         self.n_pairs, self.top, self.n_experts = n_tokens * top, top, n_experts
-        self.tm = grouped_rows_tile(self.n_pairs / max(n_experts, 1), few_rows_ok)
+        self.tm = grouped_rows_tile(self.n_pairs / max(n_experts, 1), few_rows_ok, tensor)
         self.max_tiles = -(-self.n_pairs // self.tm) + n_experts
         ints = torch.empty(3 * self.n_pairs + n_experts + 1 + 3 * self.max_tiles + 1, dtype=torch.int32, device=device)
         cuts = [self.n_pairs, self.n_pairs, self.n_pairs, n_experts + 1, self.max_tiles, self.max_tiles, self.max_tiles, 1]
