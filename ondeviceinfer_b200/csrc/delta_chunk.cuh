@@ -1,4 +1,5 @@
-// The gated delta rule over runs of tokens, 16 tokens at a time.
+// The gated delta rule over runs of tokens, 16 tokens at a time (delta.cu, with a decay per key channel; delta_head.cu, with one
+// per head, which is then every channel's).
 //
 // Per sequence and head, with S [D, dv] the state before the chunk, g_t [D] the decays of token t, G_t = g_0 .. g_t and
 // D_ts = g_(s+1) .. g_t (products lane by lane; nothing is divided, so no decay is too small), the recurrence
@@ -124,7 +125,7 @@ __device__ __forceinline__ void dc_cp16(uint32_t dst, const float* src, bool ok)
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(ok ? 16 : 0) : "memory");
 }
 
-#define DC_STAGES 3
+#define DC_STAGES(D) ((D) == 64 ? 3 : 2)      // heads of 128: two, so that four blocks share a multiprocessor
 #define DC_STAGE(D, COLS) (DC_WORDS(D) + 2 * DC * (COLS))      // floats of a chunk in shared memory
 
 // COLS columns of one head's state: CPT of them per group of 16 lanes, a lane holding rows 4 (lane + 16 j) .. + 3.  dv a
@@ -144,13 +145,13 @@ dc_scan_kernel(DeltaChunkArgs a) {
   const int dv = a.dv, chunks = (q_len + DC - 1) / DC;
   const size_t slot0 = (size_t)(q_begin / DC) + seq;
   float* S_g = a.state + ((size_t)a.slots[seq] * a.heads + h) * D * dv;
-  float* xs = dc_smem + DC_STAGES * STAGE + col * DC;
+  float* xs = dc_smem + DC_STAGES(D) * STAGE + col * DC;
   const uint32_t base = (uint32_t)__cvta_generic_to_shared(dc_smem);
 
   auto issue = [&](int c) {
     if (c < chunks) {
       const size_t item = (slot0 + c) * a.heads + h;
-      const uint32_t dst = base + (uint32_t)((c % DC_STAGES) * STAGE * 4);
+      const uint32_t dst = base + (uint32_t)((c % DC_STAGES(D)) * STAGE * 4);
       const float* src = a.wq + item * DC_WORDS(D);
       for (int i = tid * 4; i < DC_WORDS(D); i += NTH * 4) dc_cp16(dst + i * 4, src + i, true);
       const float* vo = a.vo + item * 2 * DC * dv + c0;
@@ -163,7 +164,7 @@ dc_scan_kernel(DeltaChunkArgs a) {
     asm volatile("cp.async.commit_group;" ::: "memory");
   };
 #pragma unroll
-  for (int c = 0; c < DC_STAGES - 1; ++c) issue(c);
+  for (int c = 0; c < DC_STAGES(D) - 1; ++c) issue(c);
 
   float S[CPT][R];
 #pragma unroll
@@ -173,10 +174,10 @@ dc_scan_kernel(DeltaChunkArgs a) {
       S[cc][r] = c0 + col + cc < dv ? S_g[(size_t)(4 * (rl + 16 * (r >> 2)) + (r & 3)) * dv + c0 + col + cc] : 0.f;
 
   for (int c = 0; c < chunks; ++c) {
-    asm volatile("cp.async.wait_group %0;" ::"n"(DC_STAGES - 2) : "memory");
+    asm volatile("cp.async.wait_group %0;" ::"n"(DC_STAGES(D) - 2) : "memory");
     __syncthreads();      // chunk c has arrived; everybody has left chunk c - 1, whose place the next copies take
-    issue(c + DC_STAGES - 1);
-    const float* buf = dc_smem + (c % DC_STAGES) * STAGE;
+    issue(c + DC_STAGES(D) - 1);
+    const float* buf = dc_smem + (c % DC_STAGES(D)) * STAGE;
     const float* vs = buf + DC_WORDS(D);
     float sum[CPT][2 * DC];      // wk S, then q' S
 #pragma unroll
@@ -260,7 +261,7 @@ dc_scan_kernel(DeltaChunkArgs a) {
 template <int D>
 static int dc_launch(const DeltaChunkArgs& a, cudaStream_t stream) {
   constexpr int COLS = D == 64 ? 8 : 16, CPT = 2;
-  constexpr size_t smem = sizeof(float) * (DC_STAGES * DC_STAGE(D, COLS) + COLS * DC);
+  constexpr size_t smem = sizeof(float) * (DC_STAGES(D) * DC_STAGE(D, COLS) + COLS * DC);
   auto kernel = dc_scan_kernel<D, COLS, CPT>;
   const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return (int)e;

@@ -26,7 +26,10 @@
 //             operations), two columns a thread; 16 tokens of q, k, v and the groups' numbers are staged in shared
 //             memory, the next 16 by asynchronous copies meanwhile;
 //  out_norm   per (token, head): o / rms(o) (eps inside the root) * weight * silu(gate), rounded once to T.
-#include "common.cuh"
+// A few long sequences of heads of 64 or 128 go in chunks of 16 tokens instead (delta_chunk.cuh): parts of every chunk, then a scan,
+// in the place of groups and rule (a prompt of 333 + 769 + 1,777 tokens, 16 heads of 128: 374 us of scan and 109 of parts against 522
+// and 13).
+#include "delta_chunk.cuh"
 
 #define HD_MAX_TAPS 16
 #define HD_CPT 2            // value columns per thread
@@ -45,6 +48,7 @@ struct HeadDeltaArgs {
   float* gb;              // [n_tokens, heads, 2] scratch: decay, step size
   float* coefs;           // [ceil(n_tokens / 4), heads, HD_COEFS] scratch: the groups' numbers
   float* o;               // [n_tokens, heads dv] scratch: v, then the read-outs in its place
+  float* chunks;          // scratch of the run in chunks (delta_chunk.cuh): slots * heads * (DC_WORDS(d) + 2 DC dv); null: four at a time
   void* out;              // [n_tokens, heads dv] in T
   const int* cu_q;
   const int* tok_seq;
@@ -639,6 +643,41 @@ static int launch_rule_form(const HeadDeltaArgs& a, cudaStream_t stream) {
   else return launch_rule<1, 16, 64, TCH>(a, stream);
 }
 
+// The parts of a chunk (delta_chunk.cuh) from what prep left; a block's scan puts the read-outs in the values' place afterwards.
+template <int D>
+__global__ void __launch_bounds__(2 * D, D == 64 ? 6 : 3)      // three resp. six blocks a multiprocessor
+hd_parts_kernel(HeadDeltaArgs a, DeltaChunkArgs c) {
+  pdl_launch_dependents();
+  pdl_wait();
+  __shared__ DeltaChunkShared<D> sh;
+  const int h = blockIdx.y, kvh = h / (a.heads / a.kv_heads);
+  int seq, first, nt;
+  if (!run_chunk<DC>(a.cu_q, a.n_seqs, blockIdx.x, sh.found, seq, first, nt)) return;
+  const size_t tok = (size_t)a.cu_q[seq] + first;
+  const float* qk = a.qk + (tok * a.kv_heads + kvh) * 2 * D;
+  for (int x = threadIdx.x; x < DC * D; x += blockDim.x) {
+    const int t = x / D, i = x % D;
+    const bool in = t < nt;
+    const float* row = qk + (size_t)t * a.kv_heads * 2 * D;
+    sh.q[t][i] = in ? row[i] : 0.f;
+    sh.k[t][i] = in ? row[D + i] : 0.f;
+    sh.g[t][i] = in ? a.gb[((tok + t) * a.heads + h) * 2] : 1.f;
+  }
+  if (threadIdx.x < DC) sh.beta[threadIdx.x] = (int)threadIdx.x < nt ? a.gb[((tok + threadIdx.x) * a.heads + h) * 2 + 1] : 0.f;
+  __syncthreads();
+  const float* v = a.o + (tok * a.heads + h) * a.dv;
+  const size_t step = (size_t)a.heads * a.dv;
+  dc_parts<D>(sh, c, blockIdx.x, h, [&](int t, int col) { return t < nt ? v[t * step + col] : 0.f; });
+}
+
+template <int D>
+static int launch_chunks(const HeadDeltaArgs& a, cudaStream_t stream) {
+  const size_t slots = run_chunk_slots(a.n_tokens, a.n_seqs, DC);
+  const DeltaChunkArgs c = {a.chunks, a.chunks + slots * a.heads * DC_WORDS(D), a.state, a.o, a.cu_q, a.slots, a.n_seqs, a.heads, a.dv};
+  const int rc = launch_pdl((hd_parts_kernel<D>), dim3((unsigned)slots, a.heads), dim3(2 * D), 0, stream, a, c);
+  return rc != 0 ? rc : dc_launch<D>(c, stream);
+}
+
 template <typename T>
 static int launch_head_delta(const HeadDeltaArgs& a, cudaStream_t stream) {
   const int C = 2 * a.kv_heads * a.d + a.heads * a.dv;
@@ -656,9 +695,10 @@ static int launch_head_delta(const HeadDeltaArgs& a, cudaStream_t stream) {
   odi_rc = launch_pdl(prep, dim3(a.n_tokens, parts), dim3(256), smem, stream, a);
   if (odi_rc == 0 && a.taps_n > 1 && a.max_q_len > 1)
     odi_rc = launch_pdl((hd_conv_state_kernel<T>), dim3(a.n_seqs, (C + 255) / 256), dim3(256), 0, stream, a);
-  if (odi_rc == 0 && a.max_q_len >= 4)
+  if (odi_rc == 0 && a.chunks != nullptr) odi_rc = a.d == 64 ? launch_chunks<64>(a, stream) : launch_chunks<128>(a, stream);
+  else if (odi_rc == 0 && a.max_q_len >= 4)
     odi_rc = launch_pdl(hd_groups_kernel, dim3((unsigned)(((long)a.n_tokens * a.kv_heads + 3) / 4)), dim3(128), 0, stream, a);
-  if (odi_rc == 0) {
+  if (odi_rc == 0 && a.chunks == nullptr) {
     if (a.d <= 16) odi_rc = launch_rule_form<16, 16>(a, stream);
     else if (a.d <= 32) odi_rc = launch_rule_form<32, 16>(a, stream);
     else if (a.d <= 64) odi_rc = launch_rule_form<64, 16>(a, stream);
@@ -672,12 +712,13 @@ static int launch_head_delta(const HeadDeltaArgs& a, cudaStream_t stream) {
 }
 
 // Kernels launched by one call: 3, one more with a convolution state to move on after a step of several tokens, one more
-// when a sequence brings four tokens or more.
+// when a sequence brings four tokens or more; in chunks 4, one more with a convolution state.
 extern "C" int odi_head_delta(const HeadDeltaArgs* args, int dtype, cudaStream_t stream) {
   const HeadDeltaArgs a = *args;
   if (a.n_tokens <= 0 || a.n_seqs <= 0) return 0;
   if (a.heads <= 0 || a.kv_heads <= 0 || a.heads % a.kv_heads != 0 || a.d <= 0 || a.dv <= 0 || a.taps_n < 1) return ODI_ERR_ARGUMENT;
   if (a.d > 512 || a.taps_n > HD_MAX_TAPS || a.heads > 65535 || a.n_seqs > 65535) return ODI_ERR_UNSUPPORTED;
   if (a.taps_n > 1 && a.conv_state == nullptr) return ODI_ERR_ARGUMENT;
+  if (a.chunks != nullptr && ((a.d != 64 && a.d != 128) || a.dv % 4 != 0 || (uintptr_t)a.chunks % 16 != 0)) return ODI_ERR_UNSUPPORTED;
   return dtype == 0 ? launch_head_delta<float>(a, stream) : launch_head_delta<bf16>(a, stream);
 }

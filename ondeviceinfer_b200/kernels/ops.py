@@ -1602,10 +1602,10 @@ class _DeltaArgs(Structure):
 DELTA_CHUNK, DELTA_CHUNK_MIN_RUN, DELTA_CHUNK_MAX_SCRATCH = 16, 40, 1 << 30
 
 
-def delta_chunk_floats(n_tokens: int, n_seqs: int, heads: int, d: int, dv: int) -> int:
+def delta_chunk_floats(n_tokens: int, n_seqs: int, heads: int, d: int, dv: int, least: Optional[int] = None) -> int:
     """Floats of scratch for a delta rule's run in chunks; 0 where it goes token by token: short runs, sizes that the
     chunk kernels do not take, more scratch than DELTA_CHUNK_MAX_SCRATCH bytes."""
-    if n_tokens < DELTA_CHUNK_MIN_RUN * n_seqs or d not in (64, 128) or dv % 4 != 0:
+    if n_tokens < (DELTA_CHUNK_MIN_RUN if least is None else least) * n_seqs or d not in (64, 128) or dv % 4 != 0:
         return 0
     floats = (n_tokens // DELTA_CHUNK + n_seqs) * heads * ((3 * DELTA_CHUNK + 1) * d + 2 * DELTA_CHUNK * dv)
     return floats if 4 * floats <= DELTA_CHUNK_MAX_SCRATCH else 0
@@ -1663,12 +1663,17 @@ def delta_rule(proj: torch.Tensor, decay_in: torch.Tensor, taps: torch.Tensor, a
 class _HeadDeltaArgs(Structure):
     _fields_ = [("proj", c_void_p), ("ab", c_void_p), ("taps", c_void_p), ("a_log", c_void_p), ("dt_bias", c_void_p),
                 ("norm_w", c_void_p), ("conv_state", c_void_p), ("state", c_void_p), ("qk", c_void_p), ("gb", c_void_p),
-                ("coefs", c_void_p), ("o", c_void_p), ("out", c_void_p), ("cu_q", c_void_p), ("tok_seq", c_void_p), ("slots", c_void_p),
+                ("coefs", c_void_p), ("o", c_void_p), ("chunks", c_void_p), ("out", c_void_p), ("cu_q", c_void_p), ("tok_seq", c_void_p), ("slots", c_void_p),
                 ("n_tokens", c_int), ("n_seqs", c_int), ("max_q_len", c_int), ("ld", c_int), ("heads", c_int),
                 ("kv_heads", c_int), ("d", c_int), ("dv", c_int), ("taps_n", c_int), ("eps", c_float), ("unit_eps", c_float)]
 
 
 HEAD_DELTA_MAX_DIM, HEAD_DELTA_MAX_TAPS = 512, 16
+# In chunks (csrc/delta_chunk.cuh) where a few long sequences leave the chip to chains of their tokens: at most this many heads in
+# all, at least so many tokens a sequence.  Measured against four tokens at a time, the mixer, us: 16 heads of 128 x 128, one
+# sequence of 2,048 tokens 334 and 432, 256 57 and 67, 128 42 and 42; 333 + 769 + 1,777 tokens 546 and 600; 8 x 512 544 and 430; heads
+# of 64 x 64: 2,048 256 and 383, 333 + 769 + 1,777 295 and 514, 8 x 512 288 and 264.
+HEAD_DELTA_CHUNK_MAX_HEADS, HEAD_DELTA_CHUNK_MIN_RUN = 64, 192
 
 
 def head_delta(proj: torch.Tensor, ab: torch.Tensor, taps: torch.Tensor, a_log: torch.Tensor, dt_bias: torch.Tensor,
@@ -1702,15 +1707,19 @@ def head_delta(proj: torch.Tensor, ab: torch.Tensor, taps: torch.Tensor, a_log: 
     dev = proj.device
     qk = torch.empty((n, kv_heads, 2, d), dtype=torch.float32, device=dev)
     gb = torch.empty((n, heads, 2), dtype=torch.float32, device=dev)
-    coefs = torch.empty(((n + 3) // 4 if max_q_len >= 4 else 0, heads, 32), dtype=torch.float32, device=dev)
+    scratch = 0
+    if heads * n_seqs <= HEAD_DELTA_CHUNK_MAX_HEADS:
+        scratch = delta_chunk_floats(n, n_seqs, heads, d, dv, HEAD_DELTA_CHUNK_MIN_RUN)
+    chunks = torch.empty(scratch, dtype=torch.float32, device=dev) if scratch else None
+    coefs = torch.empty(((n + 3) // 4 if max_q_len >= 4 and not scratch else 0, heads, 32), dtype=torch.float32, device=dev)
     o = torch.empty((n, heads * dv), dtype=torch.float32, device=dev)
     args = _HeadDeltaArgs(_ptr(proj), _ptr(ab), _ptr(taps), _ptr(a_log), _ptr(dt_bias), _ptr(norm_w),
-                          _ptr(conv_state if K > 1 else None), _ptr(state), _ptr(qk), _ptr(gb), _ptr(coefs), _ptr(o), _ptr(out), _ptr(cu_q),
+                          _ptr(conv_state if K > 1 else None), _ptr(state), _ptr(qk), _ptr(gb), _ptr(coefs), _ptr(o), _ptr(chunks), _ptr(out), _ptr(cu_q),
                           _ptr(tok_seq), _ptr(slots), n, n_seqs, max_q_len, proj.shape[1], heads, kv_heads, d, dv, K, eps,
                           unit_eps)
     lib = load_library("delta_head")
     _check(lib.odi_head_delta(byref(args), c_int(dtype_code(proj.dtype)), _stream()), "head_delta",
-           3 + (K > 1 and max_q_len > 1) + (max_q_len >= 4))
+           3 + (K > 1 and max_q_len > 1) + (max_q_len >= 4))      # the parts of chunks or the numbers of groups: one kernel each
 
 
 # ------------------------------------------------------------------------------ attention with mixed heads

@@ -391,6 +391,59 @@ def test_delta_rule_over_cut_sequences(dtype, heads, kv_heads, d, dv, taps):
                                                                            else dict(atol=4e-2, rtol=2e-2)))
 
 
+@pytest.mark.parametrize("heads,kv_heads,d,dv,taps", [(4, 2, 64, 64, 4), (3, 3, 64, 20, 1), (2, 1, 128, 100, 3), (2, 2, 128, 128, 4)])
+def test_delta_rule_in_chunks_of_tokens(heads, kv_heads, d, dv, taps):
+    """Runs around the chunks' edges, one of a single token among them, continued by a second step, with decays from one to
+    those that wipe the state; against the recurrence in 64 bits, and no further off than four tokens at a time."""
+    gen = torch.Generator().manual_seed(heads * d + dv)
+    v = heads * dv
+    C, cuts, slots = 2 * kv_heads * d + v, [[691, 16, 1, 80], [64, 97, 63, 545]], [3, 0, 4, 1]
+    lengths = [a + b for a, b in zip(*cuts)]
+    projs = [torch.randn(L, C + v, generator=gen) for L in lengths]
+    abs_ = [torch.randn(L, 2 * heads, generator=gen) for L in lengths]
+    abs_[0][20:22, 0] = 500.0                    # wiped inside a chunk
+    abs_[1][:, 0] = -80.0                        # no decay at all
+    w = {"taps": torch.randn(C, taps, generator=gen) * 0.5, "A_log": torch.log(0.03 + torch.rand(heads, generator=gen)),
+         "dt_bias": torch.randn(heads, generator=gen) * 0.5 - 1, "norm": 1 + 0.1 * torch.randn(dv, generator=gen)}
+    m = {"heads": heads, "kv_heads": kv_heads, "dim": d, "vdim": dv}
+    want = [plain.delta_core(m, p.double()[:, :C], ab.double()[:, heads:], ab.double()[:, :heads], p.double()[:, C:],
+                             w["taps"].double(), w["A_log"].double(), w["dt_bias"].double(), w["norm"].double(), 1e-5)
+            for p, ab in zip(projs, abs_)]
+    dev = {k: t.float().cuda() for k, t in w.items()}
+    dev["taps"] = dev["taps"].t().contiguous()
+
+    def run():
+        state = torch.zeros(6, heads, d, dv, device="cuda")
+        state[2].fill_(7.0)                      # a slot of somebody else: must stay as it is
+        conv_state = torch.zeros(6, taps - 1, C, device="cuda") if taps > 1 else None
+        got, at = [[] for _ in lengths], [0] * len(lengths)
+        for lens in cuts:
+            cu = [0]
+            for n in lens:
+                cu.append(cu[-1] + n)
+            piece = lambda all_: torch.cat([x[o:o + n] for x, o, n in zip(all_, at, lens)]).cuda()
+            out = torch.empty(cu[-1], v, device="cuda")
+            ops.head_delta(piece(projs), piece(abs_), dev["taps"], dev["A_log"], dev["dt_bias"], dev["norm"], conv_state, state, out,
+                           ints(*cu), ints(*[s for s, n in enumerate(lens) for _ in range(n)]), ints(*slots), n_seqs=len(lens),
+                           max_q_len=max(lens), heads=heads, kv_heads=kv_heads, d=d, dv=dv, eps=1e-5, unit_eps=1e-6)
+            for s, n in enumerate(lens):
+                got[s].append(out[cu[s]:cu[s + 1]].cpu().double())
+                at[s] += n
+        assert at == lengths and bool((state[2] == 7.0).all())
+        return [float((torch.cat(g) - x).norm() / x.norm()) for g, x in zip(got, want)], state
+
+    assert ops.delta_chunk_floats(sum(cuts[0]), 4, heads, d, dv, ops.HEAD_DELTA_CHUNK_MIN_RUN) > 0
+    (chunked, state), least = run(), ops.HEAD_DELTA_CHUNK_MIN_RUN
+    ops.HEAD_DELTA_CHUNK_MIN_RUN = 1 << 30
+    try:
+        fours, state_fours = run()
+    finally:
+        ops.HEAD_DELTA_CHUNK_MIN_RUN = least
+    assert max(chunked) < 5e-6 and max(fours) < 5e-6      # sums of a hundred products of 2^-24 each
+    assert sum(chunked) <= 1.25 * sum(fours)
+    torch.testing.assert_close(state, state_fours, atol=2e-5, rtol=2e-5)
+
+
 def test_delta_rule_with_decays_down_to_zero_and_no_decay_at_all():
     """Products of decays only, no quotients: a decay that underflows wipes the state, one of 1 keeps a far write."""
     heads, d, dv, L = 2, 16, 16, 90
