@@ -204,27 +204,31 @@ class SequenceCache:
 
     # ------------------------------------------------------------------ growth
 
-    def reserve(self, slots: Sequence[int], new_tokens: Sequence[int]) -> None:
-        """Make room for ``new_tokens[i]`` more positions in ``slots[i]``.  Either every
+    def reserve(self, slots: Sequence[int], new_tokens: Sequence[int]) -> bool:
+        """Make room for ``new_tokens[i]`` more positions in ``slots[i]``; whether any page was taken for it.  Either every
         sequence gets its pages or none does and :class:`CacheCapacityError` is raised."""
         if len(set(slots)) != len(slots):
             raise ValueError(f"a slot appears twice in the batch: {list(slots)}")
+        if self.kv_groups:
+            for slot, _ in zip(slots, new_tokens):
+                self._require_held(slot)
+        lengths, wanting = self.lengths, []
         for group in self.kv_groups:
             extra = 0
             for slot, t in zip(slots, new_tokens):
-                self._require_held(slot)
-                extra += group.pages_needed(self.lengths[slot] + t) - len(group.slot_pages[slot])
+                need = group.pages_needed(lengths[slot] + t) - len(group.slot_pages[slot])
+                extra += need
+                if need > 0:
+                    wanting.append((group, slot, need))
             if extra > group.pages.free_count:
                 total = sum(self.lengths[s] + t for s, t in zip(slots, new_tokens))
                 raise CacheCapacityError(
                     f"KV cache capacity exceeded: the batch needs {extra} more pages of {PAGE_SIZE} tokens "
                     f"({total} tokens in {len(slots)} sequences), {group.pages.free_count} of "
                     f"{group.pages.count} pages are free (capacity {self.max_tokens} tokens)")
-        for group in self.kv_groups:
-            for slot, t in zip(slots, new_tokens):
-                need = group.pages_needed(self.lengths[slot] + t) - len(group.slot_pages[slot])
-                if need > 0:
-                    group.slot_pages[slot].extend(group.pages.take_many(need))
+        for group, slot, need in wanting:
+            group.slot_pages[slot].extend(group.pages.take_many(need))
+        return bool(wanting)
 
     def advance(self, slots: Sequence[int], new_tokens: Sequence[int]) -> None:
         for slot, t in zip(slots, new_tokens):

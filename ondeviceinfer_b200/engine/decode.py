@@ -130,9 +130,10 @@ class _DecodeContext(StepDescription):
             per, splits = ops.plan_key_splits(self.kv_lens, block_rows)
             blocks = ops.key_split_list(self.kv_lens, per, entry[0].numel() - 2)
             if blocks != entry[1]:
-                # from pageable memory: the copy has left the host's list when the call returns, and is
-                # ordered on the stream before the replay that reads it
-                entry[0].copy_(torch.tensor(blocks, dtype=torch.int32))
+                # through pinned memory (torch hands the block out again only after the copy), ordered on the stream
+                # behind the replay that read the list before and ahead of the one that reads it next: nothing waits
+                host = torch.tensor(blocks, dtype=torch.int32, pin_memory=entry[0].is_cuda)
+                entry[0].copy_(host, non_blocking=True)
                 entry[1] = blocks
             needed.append(_power_of_two(splits))
             if fix_bounds:
@@ -158,6 +159,7 @@ class DecodeRunner:
         self._host_pages: List[np.ndarray] = []
         self._pinned_tokens: Optional[torch.Tensor] = None
         self._pinned_out: Optional[torch.Tensor] = None
+        self._tokens_view = self._out_view = None           # both as numpy arrays
 
     @property
     def cache(self):
@@ -222,11 +224,12 @@ class DecodeRunner:
 
     def _reserve_next(self, ahead: int = 1) -> None:
         """Pages for the next ``ahead`` positions of every live sequence; upload what changed."""
-        n = len(self.live_slots)
-        before = [[len(g.slot_pages[s]) for s in self.live_slots] for g in self.cache.kv_groups]
-        self.cache.reserve(self.live_slots, [ahead] * n)
-        for g, group in enumerate(self.cache.kv_groups):
-            for i, slot in enumerate(self.live_slots):
+        cache, slots = self.cache, self.live_slots
+        before = [[len(group.slot_pages[s]) for s in slots] for group in cache.kv_groups]
+        if not cache.reserve(slots, [ahead] * len(slots)):
+            return                             # 63 steps of 64
+        for g, group in enumerate(cache.kv_groups):
+            for i, slot in enumerate(slots):
                 pages = group.slot_pages[slot]
                 if len(pages) != before[g][i]:
                     self._host_pages[g][i, :len(pages)] = pages
@@ -334,14 +337,15 @@ class DecodeRunner:
     def step_device(self, n_steps: int = 1) -> None:
         """Replay ``n_steps`` decode steps back to back; tokens stay on the device."""
         self._reserve_next(n_steps)
-        lengths = [self.cache.lengths[s] for s in self.live_slots]
+        cache = self.cache
+        lengths = [cache.lengths[s] for s in self.live_slots]
         for i in range(n_steps):
             graph, launches, _ = self._graph_for(self.ctx.width, [n + i + 1 for n in lengths])
             with nvtx_range(f"decode_step[{self.ctx.width} rows]"):
                 graph.replay()
             ops.LAUNCHES["own"] += launches["own"]
             ops.LAUNCHES["library"] += launches["library"]
-        self.cache.advance(self.live_slots, [n_steps] * len(self.live_slots))
+        cache.advance(self.live_slots, [n_steps] * len(self.live_slots))
 
     def step(self, host_tokens: Optional[Sequence[int]] = None) -> List[int]:
         """One decode step; returns the sampled tokens of the live sequences.  With
@@ -350,19 +354,28 @@ class DecodeRunner:
         if host_tokens is not None:
             if self._pinned_tokens is None or self._pinned_tokens.numel() < n:
                 self._pinned_tokens = torch.empty(max(n, 64), dtype=torch.int32).pin_memory()
-            self._pinned_tokens[:n] = torch.as_tensor(host_tokens, dtype=torch.int32)
+                self._tokens_view = self._pinned_tokens.numpy()
+            if isinstance(host_tokens, (list, tuple)):      # without a tensor on the way: the GPU waits for this
+                self._tokens_view[:n] = host_tokens
+            else:
+                self._pinned_tokens[:n] = torch.as_tensor(host_tokens, dtype=torch.int32)
             self.ctx.token_ids[:n].copy_(self._pinned_tokens[:n], non_blocking=True)
         self.step_device(1)
         # the sampled tokens back through pinned memory, and with them the kernels' error word: two asynchronous
         # copies, one wait on the stream
         if self._pinned_out is None or self._pinned_out.numel() < n + 1:
             self._pinned_out = torch.empty(max(n, 64) + 1, dtype=torch.int32).pin_memory()
+            self._out_view = self._pinned_out.numpy()
         self._pinned_out[:n].copy_(self.ctx.token_ids[:n], non_blocking=True)
         self._pinned_out[n:n + 1].copy_(ops.kernel_status_word(self.model.device), non_blocking=True)
+        # while the GPU works: the list of key blocks of the step after this one (should another batch come first, its
+        # lengths differ and it is made again)
+        lengths = self.cache.lengths
+        self.ctx.plan_key_splits([lengths[s] + 1 for s in self.live_slots] + [1] * (self.ctx.width - n))
         torch.cuda.current_stream().synchronize()
-        if int(self._pinned_out[n]) != 0:
+        if self._out_view[n] != 0:
             ops.raise_on_kernel_fault()
-        return self._pinned_out[:n].tolist()
+        return self._out_view[:n].tolist()
 
     def last_logits(self) -> torch.Tensor:
         """fp32 logits ``[live sequences, vocab]`` of the step replayed last, on the device: a view of the

@@ -135,7 +135,7 @@ def compile_library(name: str, defines: Optional[Mapping[str, object]] = None, e
 
 def load_library(name: str, defines: Optional[Mapping[str, object]] = None) -> ctypes.CDLL:
     """The loaded library of ``csrc/<name>.cu`` (built on first use, then memoised)."""
-    memo = (name, tuple(sorted((defines or {}).items())))
+    memo = (name, tuple(sorted(defines.items())) if defines else ())
     lib = _loaded.get(memo)
     if lib is not None:
         return lib

@@ -577,11 +577,11 @@ def gemm_prefill_bf16(x: torch.Tensor, w: torch.Tensor, out: Optional[torch.Tens
     _require_bias(bias, w_rows)
     _, tickets, status = _gemm_buffers(w.device, 0)
     # the upper half of the ticket array serves as the tiles' flags (the few-token kernel counts tiles in the lower)
-    flags = tickets[tickets.numel() // 2:]
+    half = tickets.numel() // 2
     lib = load_library("gemm_prefill_tcgen05")
     _check(lib.odi_gemm_prefill_bf16(_ptr(x), _ptr(w), _ptr(out), c_int(tokens), c_int(n_out), c_int(K), c_int(w_rows),
                                      c_int(n_out), c_int(epi), byref(head_prep) if head_prep is not None else _ptr(None),
-                                     _ptr(bias), _ptr(status), _ptr(flags), c_int(flags.numel()),
+                                     _ptr(bias), _ptr(status), c_void_p(tickets.data_ptr() + 4 * half), c_int(tickets.numel() - half),
                                      c_int(PREFILL_BALANCE if balance is None else balance), _stream()),
            "gemm_prefill_tcgen05")
 
