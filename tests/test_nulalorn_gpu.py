@@ -335,6 +335,47 @@ def test_single_token_expert_products_that_walk_item_lists(tokens, experts, top,
         assert (out[i].double() - want).abs().max() < 1e-4
 
 
+@pytest.mark.parametrize("tokens,experts,top,K,F,tile", [(1, 2, 1, 8, 8, 8), (3, 5, 2, 136, 40, 8), (20, 6, 2, 520, 24, 8),      # a piece of k and a bit
+                                                         (40, 3, 1, 200, 72, 16), (33, 2, 2, 1032, 16, 16), (130, 2, 1, 64, 800, 16)])
+def test_expert_products_on_the_tensor_cores(tokens, experts, top, K, F, tile):
+    """bf16 products over tiles of 8 and 16 rows, whole and with rows left over, for every epilogue the experts use; a row's
+    result does not depend on the rows beside it."""
+    g = torch.Generator().manual_seed(K + F)
+    ids = torch.stack([torch.randperm(experts, generator=g)[:top] for _ in range(tokens)]).int().cuda()
+    x = torch.randn(tokens, K, generator=g).bfloat16().cuda()
+    w_up = (torch.randn(experts, 2 * F, K, generator=g) / K ** 0.5).bfloat16().cuda()
+    w_down = (torch.randn(experts, K, F, generator=g) / F ** 0.5).bfloat16().cuda()
+    assert ops.grouped_tensor_ok((K, F), torch.bfloat16) and not ops.grouped_tensor_ok((K, F), torch.float32)
+
+    def run(ids, x):
+        routing = ops.RoutingTable(ids.shape[0], top, experts, "cuda", tensor=True)
+        ops.moe_group(ids, torch.zeros(experts, dtype=torch.int32, device="cuda"), routing)
+        n = ids.numel()
+        gated, gelu = (torch.empty((n, F), dtype=torch.bfloat16, device="cuda") for _ in range(2))
+        ops.grouped_gemm_routed(x, w_up, gated, routing, gather=True, epi=ops.GROUPED_GATED_CLAMP, limit=0.8, alpha=1.702)
+        ops.grouped_gemm_routed(x, w_up[:, :F].contiguous(), gelu, routing, gather=True, epi=ops.GROUPED_GELU_ERF)
+        out = torch.empty((n, K), dtype=torch.float32, device="cuda")
+        ops.grouped_gemm_routed(gated, w_down, out, routing, gather=False, epi=ops.GROUPED_STORE_F32)
+        return routing.tm, routing.perm[:n].long(), gated, gelu, out
+
+    tm, perm, gated, gelu, out = run(ids, x)
+    assert tm == tile
+    e, t = ids.flatten()[perm].long(), perm // top
+    up = torch.einsum("rk,rnk->rn", x[t].double(), w_up[e].double())
+    gate, lin = up[:, :F].clamp(max=0.8), up[:, F:].clamp(-0.8, 0.8)
+    # one rounding to bf16 (2^-9, doubled for the product of two factors) of fp32 sums of K products (1e-5)
+    for got, want in ((gated, gate * torch.sigmoid(1.702 * gate) * (lin + 1.0)), (gelu, plain.gelu_erf(up[:, :F]))):
+        assert bool(((got.double() - want).abs() <= 1e-5 + 2.0 ** -8 * want.abs()).all())
+    want = torch.einsum("rk,rnk->rn", gated.double(), w_down[e].double())
+    bound = (F + 2) * 2.0 ** -24 * torch.einsum("rk,rnk->rn", gated.double().abs(), w_down[e].double().abs())
+    assert bool(((out.double() - want).abs() <= bound).all())
+    last = tokens - 1
+    _, perm1, gated1, _, out1 = run(ids[last:], x[last:].contiguous())
+    for i in range(top):
+        row = int((perm == last * top + int(perm1[i])).nonzero())
+        assert bool(torch.equal(gated1[i], gated[row])) and bool(torch.equal(out1[i], out[row]))
+
+
 # ----------------------------------------------------------------------------- whole models
 
 
