@@ -130,10 +130,9 @@ class _DecodeContext(StepDescription):
             per, splits = ops.plan_key_splits(self.kv_lens, block_rows)
             blocks = ops.key_split_list(self.kv_lens, per, entry[0].numel() - 2)
             if blocks != entry[1]:
-                # through pinned memory (torch hands the block out again only after the copy), ordered on the stream
-                # behind the replay that read the list before and ahead of the one that reads it next: nothing waits
-                host = torch.tensor(blocks, dtype=torch.int32, pin_memory=entry[0].is_cuda)
-                entry[0].copy_(host, non_blocking=True)
+                # from pageable memory: the copy has left the host's list when the call returns (nothing waits for the
+                # stream), ordered behind the replay that read the list before and ahead of the one that reads it next
+                entry[0].copy_(torch.tensor(blocks, dtype=torch.int32), non_blocking=True)
                 entry[1] = blocks
             needed.append(_power_of_two(splits))
             if fix_bounds:

@@ -122,12 +122,10 @@ class StepContext(StepDescription):
             np.cumsum([len(l) for l in lists], out=start[1:])
             pieces += [start, np.fromiter((p for l in lists for p in l), dtype=np.int64, count=int(start[-1]))]
         sizes = [len(p) for p in pieces]
-        # Through pinned memory, so that nothing waits: from pageable memory the upload would first wait for all that the
-        # stream still has to do, and the host could not describe a step while the GPU works on the one before.  (The
-        # pinned block goes back to torch's pool, which hands it out again only after the copy.)
-        packed = torch.empty(sum(sizes), dtype=torch.int32, pin_memory=torch.device(device).type == "cuda")
-        np.concatenate(pieces, out=packed.numpy(), casting="same_kind")
-        self._meta = packed.to(device, non_blocking=True)
+        # Not waited for: the driver has taken the host's block when the call returns and up to 64 KB need no wait for the
+        # stream, so that the host can describe a step while the GPU works on the one before.  (Not through pinned memory: a
+        # graph capture gives torch's unused pinned blocks back to the driver, and taking them again costs tens of milliseconds.)
+        self._meta = torch.from_numpy(np.concatenate(pieces).astype(np.int32)).to(device, non_blocking=True)
         views, offset = [], 0
         for size in sizes:
             views.append(self._meta[offset:offset + size])
