@@ -456,7 +456,7 @@ extern "C" int odi_grouped_gemm(const GroupedArgs* args, int max_tiles, int tm, 
   if (a.N <= 0 || a.groups <= 0) return 0;
   if (a.K <= 0 || (tm != GV_ROWS && tm != 8 && tm != 16 && tm != 64) || a.epi < 0 || a.epi > 5) return ODI_ERR_ARGUMENT;
   if (dtype == 1 && vector_loads(a)) return launch_mma(a, max_tiles, tm, stream);
-  if (tm == 8) return ODI_ERR_UNSUPPORTED;
+  if (tm == 8 && a.tile_group == nullptr) return ODI_ERR_UNSUPPORTED;      // a table's tiles of 8 rows fit the form for 16
   if (tm == GV_ROWS) {
     if (dtype != 0 || !odi_grouped_gemm_takes_few_rows(args)) return ODI_ERR_UNSUPPORTED;      // bf16 operands that allow it have left above
     dim3 grid;

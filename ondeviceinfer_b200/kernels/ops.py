@@ -2101,7 +2101,7 @@ def ssd_mix(proj: torch.Tensor, conv_w: torch.Tensor, conv_b: torch.Tensor, dt_b
             raise KernelError("ssd_mix: the convolution state is [slots, taps - 1, channels]")
     xbc = torch.empty((n, C), dtype=torch.float32, device=proj.device)
     y = torch.empty((n, inner), dtype=torch.float32, device=proj.device)
-    scratch = ssd_chunk_floats(n, n_seqs, heads, head_dim, state_dim, groups)
+    scratch = ssd_chunk_floats(n, n_seqs, heads, head_dim, state_dim, groups) if state.data_ptr() % 16 == 0 else 0
     chunks = torch.empty(scratch, dtype=torch.float32, device=proj.device) if scratch else None
     args = _SsdArgs(_ptr(proj), _ptr(conv_w), _ptr(conv_b), _ptr(dt_bias), _ptr(a_log), _ptr(d_skip), _ptr(norm_w),
                     _ptr(conv_state if taps > 1 else None), _ptr(state), _ptr(xbc), _ptr(y), _ptr(chunks), _ptr(out), _ptr(cu_q),

@@ -369,6 +369,13 @@ def test_expert_products_on_the_tensor_cores(tokens, experts, top, K, F, tile):
     want = torch.einsum("rk,rnk->rn", gated.double(), w_down[e].double())
     bound = (F + 2) * 2.0 ** -24 * torch.einsum("rk,rnk->rn", gated.double().abs(), w_down[e].double().abs())
     assert bool(((out.double() - want).abs() <= bound).all())
+    # operands off the 16-byte borders that the tensor-core form needs: the same table, the tiles of the CUDA cores
+    off = torch.empty(tokens * K + 1, dtype=torch.bfloat16, device="cuda")[1:].view(tokens, K)
+    off.copy_(x)
+    _, perm2, gated2, _, _ = run(ids, off)
+    back, back2 = torch.empty_like(perm).scatter_(0, perm, torch.arange(perm.numel(), device="cuda")), torch.empty_like(perm)
+    back2.scatter_(0, perm2, torch.arange(perm.numel(), device="cuda"))
+    assert bool(((gated2[back2].double() - gated[back].double()).abs() <= 1e-5 + 2.0 ** -7 * gated[back].double().abs()).all())
     last = tokens - 1
     _, perm1, gated1, _, out1 = run(ids[last:], x[last:].contiguous())
     for i in range(top):
