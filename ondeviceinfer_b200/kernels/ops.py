@@ -2059,15 +2059,16 @@ class _SsdArgs(Structure):
 
 
 SSD_MAX_STATE, SSD_MAX_TAPS = 256, 16
-# The scan of runs of tokens goes 64 tokens at a time when a sequence brings this many on average
-# (the mixer of 32 heads of 128 x 64, us in chunks and token by token: 64 tokens 57, 38; 128 63, 60; 8 x 100 99, 107; 512 79, 152).
-SSD_CHUNK, SSD_CHUNK_MIN_RUN, SSD_CHUNK_MAX_SCRATCH = 64, 128, 1 << 30
+# The scan of runs of tokens goes 64 tokens at a time when a sequence brings this many on average (the mixer of 32 heads of 128 x
+# 64, us in chunks and token by token: 64 tokens 57, 38; 128 63, 60; 8 x 100 99, 107; 512 79, 152), and a step so many in all: with fewer
+# the host's launches are the bound of the models that have it, and the chunks are two launches more.
+SSD_CHUNK, SSD_CHUNK_MIN_RUN, SSD_CHUNK_MIN_TOKENS, SSD_CHUNK_MAX_SCRATCH = 64, 128, 1024, 1 << 30
 
 
 def ssd_chunk_floats(n_tokens: int, n_seqs: int, heads: int, head_dim: int, state_dim: int, groups: int) -> int:
     """Floats of scratch for a state-space scan in chunks (the chunks' states, products of B and C, decays); 0 where it goes
     token by token: short runs, sizes that the chunk kernels do not take, more scratch than SSD_CHUNK_MAX_SCRATCH bytes."""
-    if (n_tokens < SSD_CHUNK_MIN_RUN * n_seqs or state_dim % SSD_CHUNK != 0 or head_dim % 4 != 0
+    if (n_tokens < max(SSD_CHUNK_MIN_RUN * n_seqs, SSD_CHUNK_MIN_TOKENS) or state_dim % SSD_CHUNK != 0 or head_dim % 4 != 0
             or heads * -(-head_dim // SSD_CHUNK) * (state_dim // SSD_CHUNK) + groups > 65535):
         return 0
     floats = (n_tokens // SSD_CHUNK + n_seqs) * (heads * state_dim * head_dim + groups * SSD_CHUNK * SSD_CHUNK + heads)

@@ -288,7 +288,7 @@ def test_state_space_scan_in_chunks_of_tokens(heads, P, N, G, taps, parts):
     kernel.  A token that is not a number reaches no token before it."""
     gen = torch.Generator().manual_seed(heads * P + N)
     inner, C = heads * P, heads * P + 2 * G * N
-    M, slots, cuts = inner + C + heads, [3, 0, 4, 1], [[380, 64, 1, 70], [63, 129, 250, 75]]
+    M, slots, cuts = inner + C + heads, [3, 0, 4, 1], [[890, 64, 1, 70], [63, 129, 800, 75]]
     lengths = [a + b for a, b in zip(*cuts)]
     projs = [torch.randn(L, M, generator=gen) for L in lengths]
     projs[0][40:42, -heads:] = 300.0             # the state is wiped inside a chunk
