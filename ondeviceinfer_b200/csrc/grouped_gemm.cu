@@ -296,15 +296,36 @@ grouped_gemv_kernel(GroupedArgs a) {
 // both operands agree, so those 8 are the lane's k of two mma.  A block owns 16 features (gated: and their 16 up rows) and all
 // k: its four warps take pieces of 128 k in turn, all of a piece's loads on their way at once (about 100 KB a multiprocessor), the
 // first weights before the input rows are looked up; the warps' sums meet in shared memory.  The tensor core cuts off what its
-// sums cannot hold, so 16 k are summed from zero there, eight such sums pairwise and then to the rest by rounded additions, in
-// an order that depends on neither the other rows nor NT.
+// sums cannot hold, so 16 k (gated: 8) are summed from zero there, the sums of a piece's 128 k pairwise and then to the rest by
+// rounded additions, in an order that depends on neither the other rows nor NT.  Norm of the error of a sum against 64 bits, K = 64 / 256 /
+// 1,024 / 4,096: 4.4e-8 / 5.7e-8 / 6.9e-8 / 8.5e-8; the CUDA cores' forms before: up to four rows a group 4.0e-8 / 5.5e-8 / 6.9e-8 / 9.5e-8, more
+// rows 5.2e-8 / 1.1e-7 / 2.5e-7 / 6.1e-7.
 // Measured, bf16, four of 32 experts of 2,048 x 1,024 a token, L2 flushed, up / gated up / down in us, against the forms before (lists
 // of items walked by warps on the CUDA cores up to 4 rows an expert, else tiles of 16 rows there): 1 token 8 / 11 / 7 and 9 / 14 / 9, 8
 // tokens 20 / 34 / 18 and 34 / 54 / 34 (the weights alone 13 / 26 / 13), 32 tokens 26 / 50 / 27 and 79 / 122 / 124, 56 tokens 30 / 56 / 30
 // and 221 / 400 / 186, 250 tokens 70 / 123 / 72 and 467 / 810 / 434.  Tiles of 32 and 64 rows were no faster (250 tokens: 72 and 107).
+// The gated form holds two accumulators, so eight sums of 16 k at once do not fit its registers; one after the other (32 k at a time)
+// they were 7.2e-8 off at K = 2,048, met pairwise from sums of 8 k 2.7e-8 (products that cancel, where the CUDA cores gave 4.1e-8),
+// and no slower (8 tokens 39 us against 42, 56 tokens 58 against 62, another run).
 __device__ __forceinline__ void mma16(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
   asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
                : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+// The same product over the 32 k that four lanes hold, 8 each: four sums of 8 k (m16n8k8), met pairwise; with few registers.
+__device__ __forceinline__ void mma_piece(float (&s)[4], const uint4& w0, const uint4& w1, const uint4& x) {
+  auto quarter = [](float (&c)[4], uint32_t a0, uint32_t a1, uint32_t b) {
+    asm volatile("mma.sync.aligned.m16n8k8.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5}, {%6}, {%7, %7, %7, %7};"
+                 : "=f"(c[0]), "=f"(c[1]), "=f"(c[2]), "=f"(c[3]) : "r"(a0), "r"(a1), "r"(b), "f"(0.f));
+  };
+  float p[4], q[4];
+  quarter(s, w0.x, w1.x, x.x);
+  quarter(p, w0.y, w1.y, x.y);
+#pragma unroll
+  for (int e = 0; e < 4; ++e) s[e] += p[e];
+  quarter(p, w0.z, w1.z, x.z);
+  quarter(q, w0.w, w1.w, x.w);
+#pragma unroll
+  for (int e = 0; e < 4; ++e) s[e] += p[e] + q[e];
 }
 template <bool GATED, int NT>
 __global__ void __launch_bounds__(128, GATED ? (NT == 1 ? 4 : 3) : (NT == 1 ? 6 : 5))      // six blocks a multiprocessor: 80 registers (56 tokens: 28 us, with 147 35)
@@ -374,15 +395,18 @@ grouped_mma_kernel(GroupedArgs a, int tm, int tiles) {
       for (int j = 0; j < NT; ++j)
 #pragma unroll
         for (int m = 0; m < MT; ++m) {
-          if (GATED) {      // rounded to bf16 behind the gate: fewer registers before a last bit
+          if (GATED) {
+            float s[2][4], t[4];
+            static_assert(U == 4, "two pairs of sums");
 #pragma unroll
-            for (int u = 0; u < U; ++u) {
-              float lo[4] = {}, hi[4] = {};
-              mma16(lo, w[u][m][0].x, w[u][m][1].x, w[u][m][0].y, w[u][m][1].y, x[u][j].x, x[u][j].y);
-              mma16(hi, w[u][m][0].z, w[u][m][1].z, w[u][m][0].w, w[u][m][1].w, x[u][j].z, x[u][j].w);
+            for (int h = 0; h < 2; ++h) {
+              mma_piece(s[h], w[2 * h][m][0], w[2 * h][m][1], x[2 * h][j]);
+              mma_piece(t, w[2 * h + 1][m][0], w[2 * h + 1][m][1], x[2 * h + 1][j]);
 #pragma unroll
-              for (int e = 0; e < 4; ++e) acc[m][j][e] += lo[e] + hi[e];
+              for (int e = 0; e < 4; ++e) s[h][e] += t[e];
             }
+#pragma unroll
+            for (int e = 0; e < 4; ++e) acc[m][j][e] += s[0][e] + s[1][e];
             continue;
           }
           float c[2 * U][4] = {};

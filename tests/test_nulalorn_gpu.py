@@ -383,6 +383,31 @@ def test_expert_products_on_the_tensor_cores(tokens, experts, top, K, F, tile):
         assert bool(torch.equal(gated1[i], gated[row])) and bool(torch.equal(out1[i], out[row]))
 
 
+@pytest.mark.parametrize("rows,K", [(1, 2048), (8, 2048), (40, 4096)])
+def test_gated_expert_products_sum_as_exactly_as_plain_ones(rows, K):
+    """The sums behind the gate, seen through products that cancel: the second half of k is minus the first, so that what
+    is left is the error of the sums, and the rounding to bf16 hardly adds to it.  The plain form leaves its sums in fp32."""
+    experts, F = 3, 256
+    g = torch.Generator().manual_seed(K + rows)
+    n, half = experts * rows, K // 2
+    ids = torch.arange(n).remainder(experts)[:, None].int().cuda()
+    x = torch.randn(n, K, generator=g).bfloat16()
+    x[:, 0] = 1.0
+    x[:, half:] = x[:, :half]
+    up = torch.randn(experts, F, K, generator=g).bfloat16()
+    up[:, :, half:] = -up[:, :, :half]
+    gate = torch.zeros(experts, F, K, dtype=torch.bfloat16)
+    gate[:, :, 0] = 1.0                                         # every gate is 1, and with alpha 0 its logistic 1/2
+    routing = ops.RoutingTable(n, 1, experts, "cuda", tensor=True)
+    ops.moe_group(ids, torch.zeros(experts, dtype=torch.int32, device="cuda"), routing)
+    gated, plain_sums = torch.empty((n, F), dtype=torch.bfloat16, device="cuda"), torch.empty((n, F), dtype=torch.float32, device="cuda")
+    ops.grouped_gemm_routed(x.cuda(), torch.cat([gate, up], 1).cuda(), gated, routing, gather=True, epi=ops.GROUPED_GATED_CLAMP,
+                            limit=1e30, alpha=0.0, up_shift=0.0)
+    ops.grouped_gemm_routed(x.cuda(), up.cuda(), plain_sums, routing, gather=True, epi=ops.GROUPED_STORE_F32)
+    # a tenth for the other grouping of the same products; sums that are not met pairwise are 2.6 times as far off
+    assert float(2.0 * gated.double().norm()) <= 1.1 * float(plain_sums.double().norm())
+
+
 # ----------------------------------------------------------------------------- whole models
 
 
