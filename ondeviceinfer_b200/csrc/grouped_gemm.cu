@@ -461,9 +461,10 @@ static int launch_mma(const GroupedArgs& a, int max_tiles, int tm, cudaStream_t 
   return launch_status();
 }
 
-// max_tiles: with a tile table, the most tiles the table can hold (the grid's width); tm: 16 or 64 (the
-// table must have been built for the same tm); tm = 4 asks for the form for few rows, which needs aligned
-// operands (odi_grouped_gemm_takes_few_rows says whether it can run).
+// max_tiles: with a tile table, the most tiles the table can hold (the grid's width).  tm: rows of a tile (a table must have been
+// built for the same).  bf16 with aligned operands: 4, 8 or 16 rows on the tensor cores, 64 on the CUDA cores (a product per head of
+// many rows and few k: grouped_heads_tile in ops.py says where).  Else 16 (8 with a table: the same form) or 64, or in float32 with
+// aligned operands 4, the form for few rows (odi_grouped_gemm_takes_few_rows says whether it can run).
 static bool vector_loads(const GroupedArgs& a) {
   return a.K % 8 == 0 && a.lda % 8 == 0 && a.ldw % 8 == 0 && a.a_group_off % 8 == 0 && a.w_group_stride % 8 == 0 &&
          (uintptr_t)a.A % 16 == 0 && (uintptr_t)a.W % 16 == 0;
@@ -479,7 +480,8 @@ extern "C" int odi_grouped_gemm(const GroupedArgs* args, int max_tiles, int tm, 
   const GroupedArgs a = *args;
   if (a.N <= 0 || a.groups <= 0) return 0;
   if (a.K <= 0 || (tm != GV_ROWS && tm != 8 && tm != 16 && tm != 64) || a.epi < 0 || a.epi > 5) return ODI_ERR_ARGUMENT;
-  if (dtype == 1 && vector_loads(a)) return launch_mma(a, max_tiles, tm, stream);
+  const bool vec = vector_loads(a);
+  if (dtype == 1 && vec && tm != 64) return launch_mma(a, max_tiles, tm, stream);
   if (tm == 8 && a.tile_group == nullptr) return ODI_ERR_UNSUPPORTED;      // a table's tiles of 8 rows fit the form for 16
   if (tm == GV_ROWS) {
     if (dtype != 0 || !odi_grouped_gemm_takes_few_rows(args)) return ODI_ERR_UNSUPPORTED;      // bf16 operands that allow it have left above
@@ -516,8 +518,9 @@ extern "C" int odi_grouped_gemm(const GroupedArgs* args, int max_tiles, int tm, 
   do { if (tm == 64) { if (gated) ODI_GG(T, 64, true, VEC); else ODI_GG(T, 64, false, VEC); } \
        else { if (gated) ODI_GG(T, 16, true, VEC); else ODI_GG(T, 16, false, VEC); } } while (0)
   const bool gated = a.epi == 2;
-  if (dtype == 1) ODI_GG_FORMS(bf16, false);      // with aligned operands on the tensor cores, above
-  else if (vector_loads(a)) ODI_GG_FORMS(float, true);
+  if (dtype == 1 && vec) { if (gated) ODI_GG(bf16, 64, true, true); else ODI_GG(bf16, 64, false, true); }      // tiles of fewer rows: above
+  else if (dtype == 1) ODI_GG_FORMS(bf16, false);
+  else if (vec) ODI_GG_FORMS(float, true);
   else ODI_GG_FORMS(float, false);
 #undef ODI_GG_FORMS
 #undef ODI_GG

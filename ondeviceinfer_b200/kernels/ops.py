@@ -1188,10 +1188,24 @@ def grouped_tensor_ok(K_values: Sequence[int], dtype: torch.dtype) -> bool:
     return dtype == torch.bfloat16 and all(K % 8 == 0 for K in K_values)
 
 
+def grouped_heads_tile(heads: int, M: int, N: int, K: int) -> int:
+    """Row tile of a bf16 product per head with aligned operands: 8 or 16 on the tensor cores, or 64 on the CUDA cores where
+    few k leave a tensor-core block of 16 x 16 outputs little but its start and end, and the rows fill the chip."""
+    # The times of both by what 1,078 shapes of 2 to 64 heads measured (us; a block of 16 x 16 outputs, a tile of 64 x 64, by the k).  16
+    # heads, tensor cores and tiles, M x N x K: 500 x 256 x 64 24 and 13, 2,048 x 512 x 64 172 and 75, 500 x 512 x 128 51 and 36, 2,048 x 512 x
+    # 128 197 and 133; but 200 x 512 x 128 22 and 25, 100 x 256 x 64 6.8 and 8.1, 2,048 x 64 x 256 32 and 41.
+    k = -(-K // 32) * 32
+    tensor = 1.4 + heads * -(-M // 16) * -(-N // 16) * max(0.00255, 0.0021 + 0.000007 * k)
+    if 1.0 + 0.047 * k + heads * -(-M // 64) * -(-N // 64) * (0.0025 + 0.000218 * k) < tensor:
+        return 64
+    return grouped_rows_tile(M, tensor=True)
+
+
 def grouped_gemm_heads(a: torch.Tensor, w: torch.Tensor, c: torch.Tensor, *, a_col: int, a_stride: int, c_col: int,
                        c_stride: int, K: int, out_f32: bool = False) -> None:
     """One product per head in one launch: for head g, ``c[:, c_col + g c_stride : +N] = a[:, a_col + g a_stride :
-    +K] w[g]^T`` with ``w`` [heads, N, K]; ``a`` and ``c`` are 2-D and contiguous, fp32 accumulation in k order."""
+    +K] w[g]^T`` with ``w`` [heads, N, K]; ``a`` and ``c`` are 2-D and contiguous, fp32 accumulation (``csrc/grouped_gemm.cu``
+    gives its order, the same for a row whatever rows are beside it in a form)."""
     _require(a, "a", w.dtype, 2)
     _require(w, "w", ndim=3)
     _require(c, "c", torch.float32 if out_f32 else w.dtype, 2)
@@ -1204,11 +1218,11 @@ def grouped_gemm_heads(a: torch.Tensor, w: torch.Tensor, c: torch.Tensor, *, a_c
                         None, None, None, None, None, a_stride, N * K, c_stride, a.shape[1], K, c.shape[1], M, N, K,
                         groups, 1, GROUPED_STORE_F32 if out_f32 else GROUPED_STORE, 0.0, 0.0, 0.0)
     lib = load_library("grouped_gemm")
-    # up to four rows: the form that streams the weights; five to eight rows too when the inner size is long (the
+    # float32, up to four rows: the form that streams the weights; five to eight rows too when the inner size is long (the
     # tile form would walk it in a few blocks per head), in two row tiles; else tiles of 16 or 64 rows
     few = M <= 2 * FEW_ROWS and (M <= FEW_ROWS or K >= 256) and bool(lib.odi_grouped_gemm_takes_few_rows(byref(args)))
     tensor = w.dtype == torch.bfloat16 and bool(lib.odi_grouped_gemm_takes_tensor(byref(args)))
-    tm = FEW_ROWS if few and not tensor else grouped_rows_tile(M, tensor=tensor)
+    tm = grouped_heads_tile(groups, M, N, K) if tensor else FEW_ROWS if few else grouped_rows_tile(M)
     _check(lib.odi_grouped_gemm(byref(args), c_int(0), c_int(tm), c_int(dtype_code(w.dtype)), _stream()), "grouped_gemm")
 
 

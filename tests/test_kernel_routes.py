@@ -1,0 +1,13 @@
+"""Which form of a kernel a call takes: the rules of the launchers, without a GPU."""
+
+import pytest
+
+from ondeviceinfer_b200.kernels import ops
+
+
+@pytest.mark.parametrize("heads,M,N,K,tile", [
+    (16, 1, 512, 64, 8), (16, 8, 256, 96, 8), (16, 9, 512, 64, 16), (16, 100, 256, 64, 16), (16, 100, 512, 128, 16),
+    (16, 500, 256, 64, 64), (16, 2048, 512, 64, 64), (16, 500, 512, 128, 64), (16, 500, 256, 96, 64),      # blocks of 16 x 16 outputs do too little
+    (16, 2048, 64, 256, 16), (16, 2048, 128, 512, 16), (4, 2048, 72, 40, 16)])
+def test_products_per_head_of_many_rows_and_few_k_go_in_tiles_of_64(heads, M, N, K, tile):
+    assert ops.grouped_heads_tile(heads, M, N, K) == tile

@@ -9,6 +9,7 @@ models without (``close``)."""
 
 import copy
 import json
+import math
 import subprocess
 import sys
 from pathlib import Path
@@ -238,6 +239,20 @@ def test_products_per_head(dtype, heads, K, N, M, a_gap, c_gap):
         bound = 1e-4 if dtype == torch.float32 else 2e-2 + 1e-2 * want.abs()      # one rounding of the result
         assert ((got - want).abs() <= bound).all()
         assert float(c[:, h * (N + c_gap) + N:(h + 1) * (N + c_gap)].abs().max()) == 0.0       # lanes between heads untouched
+
+
+@pytest.mark.parametrize("heads,M,N,K", [(4, 700, 300, 64), (6, 1031, 515, 128), (5, 1100, 391, 96), (40, 129, 321, 8)])
+def test_bf16_products_per_head_of_many_rows(heads, M, N, K):
+    """Few k and many rows: tiles of 64 rows, whole and with rows, features and k left over."""
+    assert ops.grouped_heads_tile(heads, M, N, K) == 64
+    g = torch.Generator().manual_seed(M)
+    a, w = torch.randn(M, heads * K, generator=g).bfloat16().cuda(), torch.randn(heads, N, K, generator=g).bfloat16().cuda()
+    c = torch.full((M, heads * N), math.nan, device="cuda")
+    ops.grouped_gemm_heads(a, w, c, a_col=0, a_stride=K, c_col=0, c_stride=N, K=K, out_f32=True)
+    x, f = a.view(M, heads, K).double(), w.double()
+    want = torch.einsum("mhk,hnk->mhn", x, f).reshape(M, -1)
+    bound = (K + 1) * 2.0 ** -24 * torch.einsum("mhk,hnk->mhn", x.abs(), f.abs()).reshape(M, -1)      # a rounding a product
+    assert bool(((c.double() - want).abs() <= bound).all())
 
 
 # ----------------------------------------------------------------------------- each mixer alone, whole models
