@@ -1616,6 +1616,16 @@ class _DeltaArgs(Structure):
 DELTA_CHUNK, DELTA_CHUNK_MIN_RUN, DELTA_CHUNK_MAX_SCRATCH = 16, 40, 1 << 30
 
 
+def chunk_floats(in_chunks: Optional[bool], dtype: torch.dtype, floats) -> int:
+    """Floats of scratch for a state mixer that takes runs in chunks, 0 token by token; ``floats(least)``: for runs of at least
+    so many tokens (None: what the mixer's rule says).  float32 goes token by token: its results for a sequence depend
+    neither on what else is in the batch nor on how its prompt is cut into passes, and chunks would make them do so (a
+    sum over a chunk is grouped by where the chunk begins).  In bfloat16 the products around the mixer do as well."""
+    if in_chunks is None:
+        return floats(None) if dtype == torch.bfloat16 else 0
+    return floats(1) if in_chunks else 0
+
+
 def delta_chunk_floats(n_tokens: int, n_seqs: int, heads: int, d: int, dv: int, least: Optional[int] = None) -> int:
     """Floats of scratch for a delta rule's run in chunks; 0 where it goes token by token: short runs, sizes that the
     chunk kernels do not take, more scratch than DELTA_CHUNK_MAX_SCRATCH bytes."""
@@ -1631,8 +1641,10 @@ DELTA_MAX_DIM = 480     # the recurrence stages 8 tokens of q, k and decay in 48
 def delta_rule(proj: torch.Tensor, decay_in: torch.Tensor, taps: torch.Tensor, a_log: torch.Tensor,
                dt_bias: torch.Tensor, norm_w: torch.Tensor, conv_state: Optional[torch.Tensor], state: torch.Tensor,
                out: torch.Tensor, cu_q, tok_seq, slots, *, n_seqs: int, heads: int, kv_heads: int, d: int, dv: int,
-               eps: float, unit_eps: float) -> None:
+               eps: float, unit_eps: float, in_chunks: Optional[bool] = None) -> None:
     """The channel-wise gated delta rule between its input products and its output product (``csrc/delta.cu``).
+    ``in_chunks`` chooses between runs in chunks, where their kernels take the sizes, and token by token (sweeps and tests);
+    None: by the rule (:func:`chunk_floats`).
 
     ``proj`` [tokens, C + heads]: q, k and v channels before their convolutions (C = 2 kv_heads d + heads dv), then
     one beta logit per head.  ``decay_in`` fp32 [tokens, heads d + heads dv]: the decay's inner term per head and
@@ -1658,7 +1670,7 @@ def delta_rule(proj: torch.Tensor, decay_in: torch.Tensor, taps: torch.Tensor, a
             raise KernelError("the convolution state does not fit the taps")
     dev = proj.device
     conv_out = qkg = beta = chunks = None
-    scratch = delta_chunk_floats(n, n_seqs, heads, d, dv)
+    scratch = chunk_floats(in_chunks, proj.dtype, lambda least: delta_chunk_floats(n, n_seqs, heads, d, dv, least))
     if scratch:
         chunks = torch.empty(scratch, dtype=torch.float32, device=dev)
     else:
@@ -1690,16 +1702,25 @@ HEAD_DELTA_MAX_DIM, HEAD_DELTA_MAX_TAPS = 512, 16
 HEAD_DELTA_CHUNK_MAX_HEADS, HEAD_DELTA_CHUNK_MIN_RUN = 64, 192
 
 
+def head_delta_chunk_floats(n_tokens: int, n_seqs: int, heads: int, d: int, dv: int, least: Optional[int] = None) -> int:
+    """As :func:`delta_chunk_floats`, for the rule with one decay per head."""
+    if least is None:
+        if heads * n_seqs > HEAD_DELTA_CHUNK_MAX_HEADS:
+            return 0
+        least = HEAD_DELTA_CHUNK_MIN_RUN
+    return delta_chunk_floats(n_tokens, n_seqs, heads, d, dv, least)
+
+
 def head_delta(proj: torch.Tensor, ab: torch.Tensor, taps: torch.Tensor, a_log: torch.Tensor, dt_bias: torch.Tensor,
                norm_w: torch.Tensor, conv_state: Optional[torch.Tensor], state: torch.Tensor, out: torch.Tensor, cu_q, tok_seq,
                slots, *, n_seqs: int, max_q_len: int, heads: int, kv_heads: int, d: int, dv: int, eps: float,
-               unit_eps: float) -> None:
+               unit_eps: float, in_chunks: Optional[bool] = None) -> None:
     """The gated delta rule with one decay per head between its products (``csrc/delta_head.cu``): ``proj`` [tokens,
     2 kv_heads d + 2 heads dv] = q, k and v channels before their convolutions, then the output gate's logits; ``ab``
     fp32 [tokens, 2 heads] = the decay's inner term, then the step size's logit; ``taps`` fp32 [K, C], C = 2 kv_heads d +
     heads dv (a row per tap, the last one the current token's); ``conv_state`` [slots, K - 1, C] and ``state`` [slots, heads, d, dv] are fp32 rows of the cache, advanced in
     place over all tokens that each sequence brings (``max_q_len``: the most that one brings); ``out`` [tokens, heads dv]
-    receives the normed, gated read-outs in the dtype of ``proj``."""
+    receives the normed, gated read-outs in the dtype of ``proj``.  ``in_chunks`` as in :func:`delta_rule`."""
     _require(proj, "proj", ndim=2)
     _require(ab, "ab", torch.float32, 2)
     _require(out, "out", proj.dtype, 2)
@@ -1721,9 +1742,7 @@ def head_delta(proj: torch.Tensor, ab: torch.Tensor, taps: torch.Tensor, a_log: 
     dev = proj.device
     qk = torch.empty((n, kv_heads, 2, d), dtype=torch.float32, device=dev)
     gb = torch.empty((n, heads, 2), dtype=torch.float32, device=dev)
-    scratch = 0
-    if heads * n_seqs <= HEAD_DELTA_CHUNK_MAX_HEADS:
-        scratch = delta_chunk_floats(n, n_seqs, heads, d, dv, HEAD_DELTA_CHUNK_MIN_RUN)
+    scratch = chunk_floats(in_chunks, proj.dtype, lambda least: head_delta_chunk_floats(n, n_seqs, heads, d, dv, least))
     chunks = torch.empty(scratch, dtype=torch.float32, device=dev) if scratch else None
     coefs = torch.empty(((n + 3) // 4 if max_q_len >= 4 and not scratch else 0, heads, 32), dtype=torch.float32, device=dev)
     o = torch.empty((n, heads * dv), dtype=torch.float32, device=dev)
@@ -2079,10 +2098,12 @@ SSD_MAX_STATE, SSD_MAX_TAPS = 256, 16
 SSD_CHUNK, SSD_CHUNK_MIN_RUN, SSD_CHUNK_MIN_TOKENS, SSD_CHUNK_MAX_SCRATCH = 64, 128, 1024, 1 << 30
 
 
-def ssd_chunk_floats(n_tokens: int, n_seqs: int, heads: int, head_dim: int, state_dim: int, groups: int) -> int:
+def ssd_chunk_floats(n_tokens: int, n_seqs: int, heads: int, head_dim: int, state_dim: int, groups: int,
+                     least: Optional[int] = None) -> int:
     """Floats of scratch for a state-space scan in chunks (the chunks' states, products of B and C, decays); 0 where it goes
     token by token: short runs, sizes that the chunk kernels do not take, more scratch than SSD_CHUNK_MAX_SCRATCH bytes."""
-    if (n_tokens < max(SSD_CHUNK_MIN_RUN * n_seqs, SSD_CHUNK_MIN_TOKENS) or state_dim % SSD_CHUNK != 0 or head_dim % 4 != 0
+    fewest = max(SSD_CHUNK_MIN_RUN * n_seqs, SSD_CHUNK_MIN_TOKENS) if least is None else least * n_seqs
+    if (n_tokens < fewest or state_dim % SSD_CHUNK != 0 or head_dim % 4 != 0
             or heads * -(-head_dim // SSD_CHUNK) * (state_dim // SSD_CHUNK) + groups > 65535):
         return 0
     floats = (n_tokens // SSD_CHUNK + n_seqs) * (heads * state_dim * head_dim + groups * SSD_CHUNK * SSD_CHUNK + heads)
@@ -2092,11 +2113,11 @@ def ssd_chunk_floats(n_tokens: int, n_seqs: int, heads: int, head_dim: int, stat
 def ssd_mix(proj: torch.Tensor, conv_w: torch.Tensor, conv_b: torch.Tensor, dt_bias: torch.Tensor, a_log: torch.Tensor,
             d_skip: torch.Tensor, norm_w: torch.Tensor, conv_state: Optional[torch.Tensor], state: torch.Tensor,
             out: torch.Tensor, cu_q, tok_seq, slots, *, n_seqs: int, heads: int, head_dim: int, state_dim: int,
-            groups: int, norm_groups: int, eps: float) -> None:
+            groups: int, norm_groups: int, eps: float, in_chunks: Optional[bool] = None) -> None:
     """The state-space mixer between its projections (``csrc/ssd.cu``): ``proj`` [tokens, 2 inner + 2 G N + heads]
     = [z | x | B | C | dt] in the compute dtype, ``out`` [tokens, inner] in the same; ``conv_state``
     [slots, taps - 1, inner + 2 G N] and ``state`` [slots, heads, N, P] are fp32 rows of the cache, advanced in place
-    over all tokens that each sequence brings."""
+    over all tokens that each sequence brings.  ``in_chunks`` as in :func:`delta_rule`."""
     _require(proj, "proj", ndim=2)
     _require(out, "out", proj.dtype, 2)
     n = proj.shape[0]
@@ -2116,7 +2137,9 @@ def ssd_mix(proj: torch.Tensor, conv_w: torch.Tensor, conv_b: torch.Tensor, dt_b
             raise KernelError("ssd_mix: the convolution state is [slots, taps - 1, channels]")
     xbc = torch.empty((n, C), dtype=torch.float32, device=proj.device)
     y = torch.empty((n, inner), dtype=torch.float32, device=proj.device)
-    scratch = ssd_chunk_floats(n, n_seqs, heads, head_dim, state_dim, groups) if state.data_ptr() % 16 == 0 else 0
+    scratch = 0
+    if state.data_ptr() % 16 == 0:
+        scratch = chunk_floats(in_chunks, proj.dtype, lambda least: ssd_chunk_floats(n, n_seqs, heads, head_dim, state_dim, groups, least))
     chunks = torch.empty(scratch, dtype=torch.float32, device=proj.device) if scratch else None
     args = _SsdArgs(_ptr(proj), _ptr(conv_w), _ptr(conv_b), _ptr(dt_bias), _ptr(a_log), _ptr(d_skip), _ptr(norm_w),
                     _ptr(conv_state if taps > 1 else None), _ptr(state), _ptr(xbc), _ptr(y), _ptr(chunks), _ptr(out), _ptr(cu_q),

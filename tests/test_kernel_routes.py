@@ -1,6 +1,7 @@
 """Which form of a kernel a call takes: the rules of the launchers, without a GPU."""
 
 import pytest
+import torch
 
 from ondeviceinfer_b200.kernels import ops
 
@@ -11,3 +12,9 @@ from ondeviceinfer_b200.kernels import ops
     (16, 2048, 64, 256, 16), (16, 2048, 128, 512, 16), (4, 2048, 72, 40, 16)])
 def test_products_per_head_of_many_rows_and_few_k_go_in_tiles_of_64(heads, M, N, K, tile):
     assert ops.grouped_heads_tile(heads, M, N, K) == tile
+
+
+def test_only_bfloat16_takes_runs_in_chunks():
+    floats = lambda least: 7 if least is None else 100 + least
+    assert [ops.chunk_floats(None, dtype, floats) for dtype in (torch.bfloat16, torch.float32)] == [7, 0]
+    assert ops.chunk_floats(True, torch.float32, floats) == 101 and ops.chunk_floats(False, torch.bfloat16, floats) == 0

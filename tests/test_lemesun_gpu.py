@@ -121,7 +121,7 @@ def test_delta_rule_in_chunks_of_tokens(d, dv, heads, kv_heads, taps):
     dev = {n: t.cuda() for n, t in w.items()}
     ints = lambda *x: torch.tensor(x, dtype=torch.int32, device="cuda")
 
-    def run():
+    def run(in_chunks):
         state = torch.zeros(6, heads, d, dv, device="cuda")
         state[2] = 7.0                              # a slot of somebody else: must stay as it is
         conv_state = torch.zeros(6, taps - 1, C, device="cuda") if taps > 1 else None
@@ -134,7 +134,7 @@ def test_delta_rule_in_chunks_of_tokens(d, dv, heads, kv_heads, taps):
             out = torch.empty(cu[-1], heads * dv, device="cuda")
             ops.delta_rule(piece(projs), piece(inners), dev["taps"], dev["A_log"], dev["dt_bias"], dev["norm"], conv_state, state, out,
                            ints(*cu), ints(*[s for s, n in enumerate(lens) for _ in range(n)]), ints(*slots), n_seqs=len(lens),
-                           heads=heads, kv_heads=kv_heads, d=d, dv=dv, eps=eps, unit_eps=1e-6)
+                           heads=heads, kv_heads=kv_heads, d=d, dv=dv, eps=eps, unit_eps=1e-6, in_chunks=in_chunks)
             for s, n in enumerate(lens):
                 got[s].append(out[cu[s]:cu[s + 1]].cpu())
                 at[s] += n
@@ -142,15 +142,39 @@ def test_delta_rule_in_chunks_of_tokens(d, dv, heads, kv_heads, taps):
         pieces = [(torch.cat(g).double(), state[slot].cpu().double()) for g, slot in zip(got, slots)]
         return [float((a - b).norm() / b.norm()) for p, q in zip(pieces, want) for a, b in zip(p, q)]
 
-    assert ops.delta_chunk_floats(sum(cuts[0]), 4, heads, d, dv) > 0
-    chunked, least = run(), ops.DELTA_CHUNK_MIN_RUN
-    ops.DELTA_CHUNK_MIN_RUN = 1 << 30
-    try:
-        single = run()
-    finally:
-        ops.DELTA_CHUNK_MIN_RUN = least
+    assert ops.delta_chunk_floats(sum(cuts[0]), 4, heads, d, dv, 1) > 0
+    chunked, single = run(True), run(False)
     assert max(chunked) < 5e-6 and max(single) < 5e-6      # sums of a hundred products of 2^-24 each
     assert sum(chunked) <= 1.25 * sum(single)
+
+
+def test_float32_delta_rule_depends_on_neither_the_batch_nor_the_cut():
+    """A run of 300 tokens alone, beside others, and in passes: the same bits."""
+    heads, d, lens = 2, 64, [300, 1, 70, 1]
+    gen = torch.Generator().manual_seed(5)
+    C = 3 * heads * d
+    proj, inner = torch.randn(sum(lens), C + heads, generator=gen).cuda(), torch.randn(sum(lens), 2 * heads * d, generator=gen).cuda()
+    taps, norm = (torch.randn(C, 4, generator=gen) * 0.5).cuda(), torch.ones(d, device="cuda")
+    a_log, bias = torch.rand(heads, generator=gen).cuda(), (torch.randn(heads * d, generator=gen) - 3).cuda()
+    ints = lambda *x: torch.tensor(x, dtype=torch.int32, device="cuda")
+
+    def run(passes):      # each a list of (sequence, first token, tokens)
+        state, conv_state = torch.zeros(4, heads, d, d, device="cuda"), torch.zeros(4, 3, C, device="cuda")
+        got = []
+        for runs in passes:
+            rows = torch.cat([torch.arange(sum(lens[:s]) + first, sum(lens[:s]) + first + n) for s, first, n in runs]).cuda()
+            cu = [sum(n for _, _, n in runs[:i]) for i in range(len(runs) + 1)]
+            out = torch.empty(cu[-1], heads * d, device="cuda")
+            ops.delta_rule(proj[rows], inner[rows], taps, a_log, bias, norm, conv_state, state, out, ints(*cu),
+                           ints(*[i for i, r in enumerate(runs) for _ in range(r[2])]), ints(*[r[0] for r in runs]), n_seqs=len(runs),
+                           heads=heads, kv_heads=heads, d=d, dv=d, eps=1e-6, unit_eps=1e-6)
+            got += [out[cu[i]:cu[i + 1]] for i, r in enumerate(runs) if r[0] == 0]
+        return torch.cat(got), state[0]
+
+    alone, state = run([[(0, 0, 300)]])
+    for passes in ([[(0, 0, 300), (1, 0, 1), (2, 0, 70), (3, 0, 1)]], [[(0, 0, 170)], [(2, 0, 70), (0, 170, 129)], [(0, 299, 1)]]):
+        got, end = run(passes)
+        assert torch.equal(got, alone) and torch.equal(end, state)
 
 
 def test_offset_norm_scales_in_fp32():

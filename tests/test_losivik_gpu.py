@@ -11,7 +11,6 @@ largest row error is bounded only for models without them."""
 import copy
 import json
 import math
-import math
 import subprocess
 import sys
 from pathlib import Path
@@ -300,7 +299,7 @@ def test_state_space_scan_in_chunks_of_tokens(heads, P, N, G, taps, parts):
     want = [plain.state_space({k: v.double() for k, v in w.items()}, "", m, p.double(), 1e-5) for p in projs]
     dev = {k: v.float().cuda() for k, v in w.items()}
 
-    def run(projs):
+    def run(projs, in_chunks):
         state = torch.zeros(6, heads, N, P, device="cuda")
         conv_state = torch.zeros(6, taps - 1, C, device="cuda") if taps > 1 else None
         state[2].fill_(7.0)          # a slot of somebody else: must stay as it is
@@ -313,7 +312,7 @@ def test_state_space_scan_in_chunks_of_tokens(heads, P, N, G, taps, parts):
             ops.ssd_mix(torch.cat([x[o:o + n] for x, o, n in zip(projs, at, lens)]).cuda(), dev["conv"], dev["conv.b"], dev["dt_bias"],
                         dev["A_log"], dev["D"], dev["norm"], conv_state, state, out, ints(*cu),
                         ints(*[s for s, n in enumerate(lens) for _ in range(n)]), ints(*slots), n_seqs=len(lens), heads=heads, head_dim=P,
-                        state_dim=N, groups=G, norm_groups=parts, eps=1e-5)
+                        state_dim=N, groups=G, norm_groups=parts, eps=1e-5, in_chunks=in_chunks)
             for s, n in enumerate(lens):
                 got[s].append(out[cu[s]:cu[s + 1]].cpu().double())
                 at[s] += n
@@ -322,19 +321,43 @@ def test_state_space_scan_in_chunks_of_tokens(heads, P, N, G, taps, parts):
 
     off = lambda got: [float((a - b).norm() / b.norm()) for a, b in zip(got, want)]
     assert ops.ssd_chunk_floats(sum(cuts[0]), 4, heads, P, N, G) > 0
-    (chunked, state), least = run(projs), ops.SSD_CHUNK_MIN_RUN
-    ops.SSD_CHUNK_MIN_RUN = 1 << 30
-    try:
-        single, state_single = run(projs)
-    finally:
-        ops.SSD_CHUNK_MIN_RUN = least
+    (chunked, state), (single, state_single) = run(projs, True), run(projs, False)
     assert max(off(chunked)) < 5e-6 and max(off(single)) < 5e-6      # sums of a few hundred products of 2^-24 each
     assert sum(off(chunked)) <= 1.25 * sum(off(single))
     torch.testing.assert_close(state, state_single, atol=2e-5, rtol=2e-5)
     broken = [p.clone() for p in projs]
     broken[0][100, inner:] = math.nan      # in the middle of a chunk
-    got = run(broken)[0][0]
+    got = run(broken, True)[0][0]
     assert bool(torch.equal(got[:100], chunked[0][:100])) and not bool(torch.isfinite(got[100:]).any())
+
+
+def test_float32_state_space_mixer_depends_on_neither_the_batch_nor_the_cut():
+    """A run of 1,100 tokens alone, beside others, and in passes: the same bits."""
+    heads, P, N, lens = 2, 64, 64, [1100, 1, 70, 3]
+    gen = torch.Generator().manual_seed(6)
+    inner, C = heads * P, heads * P + 2 * N
+    proj = torch.randn(sum(lens), inner + C + heads, generator=gen).cuda()
+    conv, conv_b = (torch.randn(C, 4, generator=gen) * 0.5).cuda(), (torch.randn(C, generator=gen) * 0.1).cuda()
+    dt_bias, a_log, skip = (torch.randn(heads, generator=gen).cuda() for _ in range(3))
+    norm = torch.ones(inner, device="cuda")
+
+    def run(passes):      # each a list of (sequence, first token, tokens)
+        state, conv_state = torch.zeros(4, heads, N, P, device="cuda"), torch.zeros(4, 3, C, device="cuda")
+        got = []
+        for runs in passes:
+            rows = torch.cat([torch.arange(sum(lens[:s]) + first, sum(lens[:s]) + first + n) for s, first, n in runs]).cuda()
+            cu = [sum(n for _, _, n in runs[:i]) for i in range(len(runs) + 1)]
+            out = torch.empty(cu[-1], inner, device="cuda")
+            ops.ssd_mix(proj[rows], conv, conv_b, dt_bias, a_log, skip, norm, conv_state, state, out, ints(*cu),
+                        ints(*[i for i, r in enumerate(runs) for _ in range(r[2])]), ints(*[r[0] for r in runs]), n_seqs=len(runs),
+                        heads=heads, head_dim=P, state_dim=N, groups=1, norm_groups=1, eps=1e-5)
+            got += [out[cu[i]:cu[i + 1]] for i, r in enumerate(runs) if r[0] == 0]
+        return torch.cat(got), state[0]
+
+    alone, state = run([[(0, 0, 1100)]])
+    for passes in ([[(0, 0, 1100), (1, 0, 1), (2, 0, 70), (3, 0, 3)]], [[(0, 0, 555)], [(2, 0, 70), (0, 555, 544)], [(0, 1099, 1)]]):
+        got, end = run(passes)
+        assert torch.equal(got, alone) and torch.equal(end, state)
 
 
 # ----------------------------------------------------------------------------- attention with kept first positions

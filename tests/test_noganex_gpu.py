@@ -412,7 +412,7 @@ def test_delta_rule_in_chunks_of_tokens(heads, kv_heads, d, dv, taps):
     dev = {k: t.float().cuda() for k, t in w.items()}
     dev["taps"] = dev["taps"].t().contiguous()
 
-    def run():
+    def run(in_chunks):
         state = torch.zeros(6, heads, d, dv, device="cuda")
         state[2].fill_(7.0)                      # a slot of somebody else: must stay as it is
         conv_state = torch.zeros(6, taps - 1, C, device="cuda") if taps > 1 else None
@@ -425,20 +425,16 @@ def test_delta_rule_in_chunks_of_tokens(heads, kv_heads, d, dv, taps):
             out = torch.empty(cu[-1], v, device="cuda")
             ops.head_delta(piece(projs), piece(abs_), dev["taps"], dev["A_log"], dev["dt_bias"], dev["norm"], conv_state, state, out,
                            ints(*cu), ints(*[s for s, n in enumerate(lens) for _ in range(n)]), ints(*slots), n_seqs=len(lens),
-                           max_q_len=max(lens), heads=heads, kv_heads=kv_heads, d=d, dv=dv, eps=1e-5, unit_eps=1e-6)
+                           max_q_len=max(lens), heads=heads, kv_heads=kv_heads, d=d, dv=dv, eps=1e-5, unit_eps=1e-6,
+                           in_chunks=in_chunks)
             for s, n in enumerate(lens):
                 got[s].append(out[cu[s]:cu[s + 1]].cpu().double())
                 at[s] += n
         assert at == lengths and bool((state[2] == 7.0).all())
         return [float((torch.cat(g) - x).norm() / x.norm()) for g, x in zip(got, want)], state
 
-    assert ops.delta_chunk_floats(sum(cuts[0]), 4, heads, d, dv, ops.HEAD_DELTA_CHUNK_MIN_RUN) > 0
-    (chunked, state), least = run(), ops.HEAD_DELTA_CHUNK_MIN_RUN
-    ops.HEAD_DELTA_CHUNK_MIN_RUN = 1 << 30
-    try:
-        fours, state_fours = run()
-    finally:
-        ops.HEAD_DELTA_CHUNK_MIN_RUN = least
+    assert ops.head_delta_chunk_floats(sum(cuts[0]), 4, heads, d, dv, 1) > 0
+    (chunked, state), (fours, state_fours) = run(True), run(False)
     assert max(chunked) < 5e-6 and max(fours) < 5e-6      # sums of a hundred products of 2^-24 each
     assert sum(chunked) <= 1.25 * sum(fours)
     torch.testing.assert_close(state, state_fours, atol=2e-5, rtol=2e-5)
