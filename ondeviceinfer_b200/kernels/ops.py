@@ -1696,16 +1696,19 @@ class _HeadDeltaArgs(Structure):
 
 HEAD_DELTA_MAX_DIM, HEAD_DELTA_MAX_TAPS = 512, 16
 # In chunks (csrc/delta_chunk.cuh) where a few long sequences leave the chip to chains of their tokens: at most this many heads in
-# all, at least so many tokens a sequence.  Measured against four tokens at a time, the mixer, us: 16 heads of 128 x 128, one
+# all, at least so many tokens a sequence; with heads of 128, whose chunks cost more work than four tokens at a time do, also at
+# most so many heads' worth of the longest run: that run's chain must be what the step waits for (us, chunks and fours: 16 heads,
+# 2 x 1,000 tokens 305 and 324, 3 x 1,000 433 and 413, 4 x 200 129 and 116, 1,000 + 500 + 250 307 and 329; 32 heads, 2 x 256 172 and 156,
+# 1,000 + 500 518 and 495, 800 280 and 290).  Measured against four tokens at a time, the mixer, us: 16 heads of 128 x 128, one
 # sequence of 2,048 tokens 334 and 432, 256 57 and 67, 128 42 and 42; 333 + 769 + 1,777 tokens 546 and 600; 8 x 512 544 and 430; heads
 # of 64 x 64: 2,048 256 and 383, 333 + 769 + 1,777 295 and 514, 8 x 512 288 and 264.
-HEAD_DELTA_CHUNK_MAX_HEADS, HEAD_DELTA_CHUNK_MIN_RUN = 64, 192
+HEAD_DELTA_CHUNK_MAX_HEADS, HEAD_DELTA_CHUNK_MIN_RUN, HEAD_DELTA_CHUNK_MAX_LONGEST = 64, 192, 32
 
 
-def head_delta_chunk_floats(n_tokens: int, n_seqs: int, heads: int, d: int, dv: int, least: Optional[int] = None) -> int:
+def head_delta_chunk_floats(n_tokens: int, n_seqs: int, max_q_len: int, heads: int, d: int, dv: int, least: Optional[int] = None) -> int:
     """As :func:`delta_chunk_floats`, for the rule with one decay per head."""
     if least is None:
-        if heads * n_seqs > HEAD_DELTA_CHUNK_MAX_HEADS:
+        if heads * n_seqs > HEAD_DELTA_CHUNK_MAX_HEADS or (d > 64 and heads * n_tokens > HEAD_DELTA_CHUNK_MAX_LONGEST * max_q_len):
             return 0
         least = HEAD_DELTA_CHUNK_MIN_RUN
     return delta_chunk_floats(n_tokens, n_seqs, heads, d, dv, least)
@@ -1742,7 +1745,7 @@ def head_delta(proj: torch.Tensor, ab: torch.Tensor, taps: torch.Tensor, a_log: 
     dev = proj.device
     qk = torch.empty((n, kv_heads, 2, d), dtype=torch.float32, device=dev)
     gb = torch.empty((n, heads, 2), dtype=torch.float32, device=dev)
-    scratch = chunk_floats(in_chunks, proj.dtype, lambda least: head_delta_chunk_floats(n, n_seqs, heads, d, dv, least))
+    scratch = chunk_floats(in_chunks, proj.dtype, lambda least: head_delta_chunk_floats(n, n_seqs, max_q_len, heads, d, dv, least))
     chunks = torch.empty(scratch, dtype=torch.float32, device=dev) if scratch else None
     coefs = torch.empty(((n + 3) // 4 if max_q_len >= 4 and not scratch else 0, heads, 32), dtype=torch.float32, device=dev)
     o = torch.empty((n, heads * dv), dtype=torch.float32, device=dev)

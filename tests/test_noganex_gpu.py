@@ -433,7 +433,7 @@ def test_delta_rule_in_chunks_of_tokens(heads, kv_heads, d, dv, taps):
         assert at == lengths and bool((state[2] == 7.0).all())
         return [float((torch.cat(g) - x).norm() / x.norm()) for g, x in zip(got, want)], state
 
-    assert ops.head_delta_chunk_floats(sum(cuts[0]), 4, heads, d, dv, 1) > 0
+    assert ops.head_delta_chunk_floats(sum(cuts[0]), 4, max(cuts[0]), heads, d, dv, 1) > 0
     (chunked, state), (fours, state_fours) = run(True), run(False)
     assert max(chunked) < 5e-6 and max(fours) < 5e-6      # sums of a hundred products of 2^-24 each
     assert sum(chunked) <= 1.25 * sum(fours)
