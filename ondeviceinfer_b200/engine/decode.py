@@ -141,6 +141,16 @@ class _DecodeContext(StepDescription):
         return self._planned_bounds
 
 
+def write_tokens(pinned: torch.Tensor, view: np.ndarray, n: int, tokens) -> None:
+    """The ``n`` tokens of a step into pinned memory (``view``: the same as a numpy array).  Plain numbers go there without a
+    tensor on the way, since the GPU waits for this; whatever else ``torch.as_tensor`` takes goes by it, and what it refuses it
+    refuses."""
+    if isinstance(tokens, (list, tuple)) and len(tokens) == n and all(type(t) is int and 0 <= t <= 0x7fffffff for t in tokens):
+        view[:n] = tokens
+    else:
+        pinned[:n] = torch.as_tensor(tokens, dtype=torch.int32)
+
+
 class DecodeRunner:
     def __init__(self, model, cache, *, temperature: float = 0.0, seed: int = 0) -> None:
         # The cache keeps its runners (ondeviceinfer_b200.api.decode_runner); the runner must not keep the cache
@@ -354,10 +364,7 @@ class DecodeRunner:
             if self._pinned_tokens is None or self._pinned_tokens.numel() < n:
                 self._pinned_tokens = torch.empty(max(n, 64), dtype=torch.int32).pin_memory()
                 self._tokens_view = self._pinned_tokens.numpy()
-            if isinstance(host_tokens, (list, tuple)):      # without a tensor on the way: the GPU waits for this
-                self._tokens_view[:n] = host_tokens
-            else:
-                self._pinned_tokens[:n] = torch.as_tensor(host_tokens, dtype=torch.int32)
+            write_tokens(self._pinned_tokens, self._tokens_view, n, host_tokens)
             self.ctx.token_ids[:n].copy_(self._pinned_tokens[:n], non_blocking=True)
         self.step_device(1)
         # the sampled tokens back through pinned memory, and with them the kernels' error word: two asynchronous

@@ -198,3 +198,22 @@ def test_runner_follows_the_sequences_through_graphs_captures_and_dropped_rows(c
     assert len(runner._graphs) == graphs_before
     runner.step_device(1)
     assert runner.ctx.token_ids[:2].tolist() == [(1 + 300) % VOCAB, (2 + 280) % VOCAB]
+
+
+@pytest.mark.parametrize("tokens", [
+    [1, 2, 3], (4, 5, 6), [True, False, True], [1.7, 2.0, 3.0], [[1, 2, 3]], [-1, 0, 1], [7], torch.tensor([1, 2, 3]),
+    [torch.tensor(3), torch.tensor(4), torch.tensor(5)],                                       # scalars, on a GPU as well
+    ["5", "6", "7"], [2 ** 31, 0, 0], [1, 2], [], [None, 1, 2], [math.nan, 1, 2]])            # refused
+def test_the_tokens_of_a_step_are_those_that_a_tensor_takes(tokens):
+    def attempt(write):
+        pinned = torch.full((4,), -9, dtype=torch.int32)
+        try:
+            write(pinned)
+        except Exception as error:
+            return type(error)
+        return pinned.tolist()
+
+    def by_tensor(pinned):
+        pinned[:3] = torch.as_tensor(tokens, dtype=torch.int32)
+
+    assert attempt(lambda pinned: decode_module.write_tokens(pinned, pinned.numpy(), 3, tokens)) == attempt(by_tensor)
