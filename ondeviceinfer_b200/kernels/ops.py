@@ -1183,9 +1183,10 @@ def grouped_few_rows_ok(K_values: Sequence[int], dtype: torch.dtype) -> bool:
     return all(K % 8 == 0 and 4 * FEW_ROWS * K <= 200 * 1024 for K in K_values)
 
 
-def grouped_tensor_ok(K_values: Sequence[int], dtype: torch.dtype) -> bool:
-    """Whether products over these inner sizes run on the tensor cores (bf16, rows in pieces of 16 bytes)."""
-    return dtype == torch.bfloat16 and all(K % 8 == 0 for K in K_values)
+def grouped_tensor_ok(K_values: Sequence[int], dtype: torch.dtype, *operands: torch.Tensor) -> bool:
+    """Whether products over these inner sizes, of these operands, run on the tensor cores (bf16, rows in pieces of 16 bytes
+    from 16-byte borders on).  A table of row tiles is made for one or the other form."""
+    return dtype == torch.bfloat16 and all(K % 8 == 0 for K in K_values) and all(t.data_ptr() % 16 == 0 for t in operands)
 
 
 def grouped_heads_tile(heads: int, M: int, N: int, K: int) -> int:

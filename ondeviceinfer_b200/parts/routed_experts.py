@@ -108,9 +108,10 @@ class RoutedExperts(Part):
         ops.moe_route(logits, self.correction, ids, weights, n_groups=s.num_groups, keep=s.keep_groups,
                       sigmoid=s.scoring == "sigmoid", renormalise=s.renormalise, scale=s.weight_scale)
         # single-token steps, a few rows per expert: the grouped product that streams weights through registers
+        experts = (self.w_gate_up, self.w_down) if s.num_experts > 0 else ()
         few_ok = ops.grouped_few_rows_ok((s.hidden_size, s.expert_size), x.dtype)
         table = ops.RoutingTable(n, s.top_k, max(s.num_experts, 1), dev, few_rows_ok=few_ok,
-                                 tensor=ops.grouped_tensor_ok((s.hidden_size, s.expert_size), x.dtype))
+                                 tensor=ops.grouped_tensor_ok((s.hidden_size, s.expert_size), x.dtype, x, *experts))
         expert_out = torch.empty((table.n_pairs, s.hidden_size), dtype=torch.float32, device=dev)
         if s.num_experts > 0:
             ops.moe_group(ids, self.counts, table)

@@ -72,7 +72,7 @@ class TableExperts(Part):
         ops.moe_table_route(self.table, ctx.token_ids, ids, weights, n_experts=s.num_experts, weight=1.0 / s.top_k)
         few_ok = ops.grouped_few_rows_ok((s.hidden_size, s.expert_size), x.dtype)
         table = ops.RoutingTable(n, s.top_k, s.num_experts, dev, few_rows_ok=few_ok,
-                                 tensor=ops.grouped_tensor_ok((s.hidden_size, s.expert_size), x.dtype))
+                                 tensor=ops.grouped_tensor_ok((s.hidden_size, s.expert_size), x.dtype, x, self.w_up, self.w_down))
         ops.moe_group(ids, self.counts, table)
         act = torch.empty((table.n_pairs, s.expert_size), dtype=x.dtype, device=dev)
         expert_out = None

@@ -27,3 +27,14 @@ def test_only_bfloat16_takes_runs_in_chunks():
     (16, 64, [512] * 4, True), (32, 64, [256, 256], True), (16, 64, [512] * 5, False), (16, 64, [128], False), (16, 96, [2048], False)])
 def test_head_delta_goes_in_chunks_where_a_run_is_what_the_step_waits_for(heads, d, lens, chunks):
     assert (ops.head_delta_chunk_floats(sum(lens), len(lens), max(lens), heads, d, d) > 0) == chunks
+
+
+def test_operands_off_the_16_byte_borders_keep_the_tiles_of_the_cuda_cores():
+    whole = torch.zeros(65, dtype=torch.bfloat16)
+    aligned, off = whole[:64], whole[1:]
+    assert aligned.data_ptr() % 16 == 0
+    ok = lambda *operands: ops.grouped_tensor_ok((64, 8), torch.bfloat16, *operands)
+    assert ok() and ok(aligned, aligned) and not ok(aligned, off)
+    assert not ops.grouped_tensor_ok((64, 12), torch.bfloat16, aligned) and not ops.grouped_tensor_ok((64, 8), torch.float32)
+    tiles = lambda pairs, *operands: ops.RoutingTable(pairs, 1, 2, "cpu", tensor=ok(*operands)).tm
+    assert [tiles(n, aligned) for n in (16, 17, 100)] == [8, 16, 16] and [tiles(n, off) for n in (16, 64, 65, 100)] == [16, 16, 64, 64]
