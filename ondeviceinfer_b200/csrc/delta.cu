@@ -245,25 +245,34 @@ __global__ void delta_values_kernel(DeltaArgs a) {
   for (int i = threadIdx.x; i < n; i += blockDim.x) a.o[(size_t)t * n + i] = to_f<T>(v[i]);
 }
 
-// One warp per (token, head).
+// One warp per (token, head); blocks of four heads of a token (no 64-bit division in a step of single tokens).
 template <typename T>
 __global__ void __launch_bounds__(128)
 delta_out_norm_kernel(DeltaArgs a) {
   pdl_launch_dependents();
   pdl_wait();
-  const int lane = threadIdx.x & 31;
-  const long item = (long)blockIdx.x * 4 + (threadIdx.x >> 5);
-  if (item >= (long)a.n_tokens * a.heads) return;
-  const size_t t = item / a.heads;
-  const int h = (int)(item % a.heads);
+  const int lane = threadIdx.x & 31, h = blockIdx.y * 4 + (threadIdx.x >> 5);
+  if (h >= a.heads) return;
+  const size_t t = blockIdx.x, item = t * a.heads + h;
   const float* o = a.o + item * a.dv;
   const float* gate = a.decay_in + t * a.ld_decay + a.heads * D + (size_t)h * a.dv;
-  float ss = 0.f;
-  for (int i = lane; i < a.dv; i += 32) ss = fmaf(o[i], o[i], ss);
+  T* out = (T*)a.out + item * a.dv;
+  float v[4], z[4], w[4], ss = 0.f;      // the first 128 columns: everything requested before anything waits
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const int i = lane + 32 * k;
+    const bool in = i < a.dv;
+    v[k] = in ? o[i] : 0.f; z[k] = in ? gate[i] : 0.f; w[k] = in ? a.norm_w[i] : 0.f;
+  }
+#pragma unroll
+  for (int k = 0; k < 4; ++k) ss = fmaf(v[k], v[k], ss);
+  for (int i = lane + 128; i < a.dv; i += 32) ss = fmaf(o[i], o[i], ss);
   ss = warp_sum(ss);
   const float inv = 1.0f / sqrtf(ss / (float)a.dv + a.eps);
-  T* out = (T*)a.out + item * a.dv;
-  for (int i = lane; i < a.dv; i += 32) out[i] = from_f<T>(o[i] * inv * a.norm_w[i] / (1.f + expf(-gate[i])));
+#pragma unroll
+  for (int k = 0; k < 4; ++k)
+    if (lane + 32 * k < a.dv) out[lane + 32 * k] = from_f<T>(v[k] * inv * w[k] / (1.f + expf(-z[k])));
+  for (int i = lane + 128; i < a.dv; i += 32) out[i] = from_f<T>(o[i] * inv * a.norm_w[i] / (1.f + expf(-gate[i])));
 }
 
 #if D % 64 == 0 && D <= 128
@@ -354,7 +363,7 @@ static int launch_chunks(const DeltaArgs& a, const DeltaChunkArgs& c, cudaStream
     odi_rc = launch_pdl((delta_conv_state_kernel<T>), dim3(a.n_seqs, (a.C + 255) / 256), dim3(256), 0, stream, a);
   if (odi_rc == 0) odi_rc = dc_launch<D>(c, stream);
   if (odi_rc == 0)
-    odi_rc = launch_pdl((delta_out_norm_kernel<T>), dim3((unsigned)(((long)a.n_tokens * a.heads + 3) / 4)), dim3(128), 0, stream, a);
+    odi_rc = launch_pdl((delta_out_norm_kernel<T>), dim3(a.n_tokens, (a.heads + 3) / 4), dim3(128), 0, stream, a);
   return launch_status();
 }
 #endif
@@ -394,7 +403,7 @@ extern "C" int odi_delta_rule(const DeltaArgs* args, int dtype, cudaStream_t str
     odi_rc = launch_pdl((delta_values_kernel<bf16>), dim3(a.n_tokens), dim3(128), 0, stream, a);
   }
   odi_rc = launch_pdl(delta_rule_kernel, rgrid, dim3(CB * RS), 0, stream, a);
-  const dim3 ngrid((unsigned)(((long)a.n_tokens * a.heads + 3) / 4));
+  const dim3 ngrid(a.n_tokens, (a.heads + 3) / 4);
   if (dtype == 0) odi_rc = launch_pdl((delta_out_norm_kernel<float>), ngrid, dim3(128), 0, stream, a);
   else odi_rc = launch_pdl((delta_out_norm_kernel<bf16>), ngrid, dim3(128), 0, stream, a);
   return launch_status();
