@@ -87,6 +87,7 @@ template <> __device__ __forceinline__ float4 ssd_load4<bf16>(const bf16* p) {
 // of 2,304 channels: 13 us against 45; the bytes take 4).  Tokens that reach back before their run's start, or lie on both sides of a
 // border between runs, go one by one.
 #define SSD_CT 8
+#define SSD_CONV4_LEAST (1L << 19)      // inputs in all from which that pays
 template <typename T>
 __global__ void __launch_bounds__(128)
 ssd_conv4_kernel(SsdArgs a) {
@@ -686,7 +687,9 @@ static int ssd_launch(const SsdArgs& a, cudaStream_t stream) {
   // rows and parts of rows in pieces of four elements
   const bool vec4 = inner % 4 == 0 && a.ld % 4 == 0 && (uintptr_t)a.proj % (4 * sizeof(T)) == 0 && (uintptr_t)a.out % (4 * sizeof(T)) == 0 &&
                     (((uintptr_t)a.y | (uintptr_t)a.norm_w | (uintptr_t)a.xbc | (uintptr_t)a.conv_w | (uintptr_t)a.conv_b | (uintptr_t)a.conv_state) & 15) == 0;
-  if (vec4 && C % 4 == 0 && a.taps == 4 && a.n_tokens >= 2 * SSD_CT * a.n_seqs)
+  // the pieces of eight tokens where there are enough of them: below, their longer way through a block is not made up for (one run of 16
+  // tokens of 640 channels 14.8 us the mixer against 10.9, of 40 19.9 against 16.6; 100 tokens of 2,304 50 and 50)
+  if (vec4 && C % 4 == 0 && a.taps == 4 && a.n_tokens >= 2 * SSD_CT * a.n_seqs && (long)a.n_tokens * C >= SSD_CONV4_LEAST)
     odi_rc = launch_pdl((ssd_conv4_kernel<T>), dim3((a.n_tokens + SSD_CT - 1) / SSD_CT, (C / 4 + 127) / 128), dim3(128), 0, stream, a);
   else
     odi_rc = launch_pdl((ssd_conv_kernel<T>), dim3(a.n_tokens, (C + 255) / 256), dim3(256), 0, stream, a);
@@ -706,6 +709,9 @@ static int ssd_launch(const SsdArgs& a, cudaStream_t stream) {
   // sequence has nothing else to run beside it.  (Measured at 32 heads of 64 columns, 128 rows, 2,048 tokens: 32
   // columns 1,080 us, 8 columns 545 us, 8 columns over 16 lanes each 640 us.)
   const bool narrow = (long)((a.P + 31) / 32) * a.heads * a.n_seqs < 2 * 148;
+  // Few blocks that live long start only when the kernel before has left: started early they are packed several to a
+  // multiprocessor beside it and stay there (8 heads of 64 x 64, one run of 600 tokens: 129 to 271 us by what ran before).
+  const bool spread = narrow && a.n_tokens >= 32 * (long)a.n_seqs;
   const int cols = narrow ? 8 : SSD_COLS;
   const dim3 grid((a.P + cols - 1) / cols, a.heads, a.n_seqs);
   const size_t smem = 2 * sizeof(float) * (SSD_TCH * (2 * (size_t)a.N + cols) + 2 * SSD_TCH);
@@ -716,7 +722,10 @@ static int ssd_launch(const SsdArgs& a, cudaStream_t stream) {
     do { if (smem > 48 * 1024) { \
            const cudaError_t e = cudaFuncSetAttribute(ssd_scan_kernel<T, NPT, VEC, COLS, LANES>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
            if (e != cudaSuccess) return (int)e; } \
-         odi_rc = launch_pdl((ssd_scan_kernel<T, NPT, VEC, COLS, LANES>), grid, dim3(COLS * LANES), smem, stream, a); } while (0)
+         if (spread) { \
+           ssd_scan_kernel<T, NPT, VEC, COLS, LANES><<<grid, dim3(COLS * LANES), smem, stream>>>(a); \
+           odi_rc = (int)cudaPeekAtLastError(); \
+         } else odi_rc = launch_pdl((ssd_scan_kernel<T, NPT, VEC, COLS, LANES>), grid, dim3(COLS * LANES), smem, stream, a); } while (0)
 #define ODI_SCAN(NPT_WIDE, NPT_NARROW) \
     do { if (vec) { if (narrow) ODI_SCAN_FORM(NPT_NARROW, true, 8, 8); else ODI_SCAN_FORM(NPT_WIDE, true, 32, 8); } \
          else { if (narrow) ODI_SCAN_FORM(NPT_NARROW, false, 8, 8); else ODI_SCAN_FORM(NPT_WIDE, false, 32, 8); } } while (0)

@@ -360,6 +360,37 @@ def test_float32_state_space_mixer_depends_on_neither_the_batch_nor_the_cut():
         assert torch.equal(got, alone) and torch.equal(end, state)
 
 
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("heads,P,N,lens", [(4, 20, 32, [16]), (16, 64, 64, [460]), (16, 64, 64, [17, 203, 40, 1, 99, 120]), (32, 64, 128, [8, 226])])
+def test_convolution_in_pieces_of_eight_tokens(dtype, heads, P, N, lens):
+    """Steps below and above the number of inputs from which the convolution takes eight tokens at a time: runs that begin, end and
+    meet anywhere in a piece, behind three earlier tokens of theirs; the same bits as token by token."""
+    gen = torch.Generator().manual_seed(sum(lens))
+    inner, C, n = heads * P, heads * P + 2 * N, sum(lens)
+    proj = torch.randn(n, inner + C + heads, generator=gen).to(dtype).cuda()
+    conv, conv_b = (torch.randn(C, 4, generator=gen) * 0.5).cuda(), (torch.randn(C, generator=gen) * 0.1).cuda()
+    dt_bias, a_log, skip = (torch.randn(heads, generator=gen).cuda() for _ in range(3))
+    norm, before = torch.ones(inner, device="cuda"), torch.randn(len(lens), 3, C, generator=gen).cuda()
+    starts = [sum(lens[:s]) for s in range(len(lens))]
+
+    def run(steps):      # each a list of (sequence, first token, tokens)
+        state, conv_state = torch.zeros(len(lens), heads, N, P, device="cuda"), before.clone()
+        got = torch.empty(n, inner, dtype=dtype, device="cuda")
+        for runs in steps:
+            rows = torch.cat([torch.arange(starts[s] + first, starts[s] + first + m) for s, first, m in runs]).cuda()
+            cu = [sum(m for _, _, m in runs[:i]) for i in range(len(runs) + 1)]
+            out = torch.empty(cu[-1], inner, dtype=dtype, device="cuda")
+            ops.ssd_mix(proj[rows], conv, conv_b, dt_bias, a_log, skip, norm, conv_state, state, out, ints(*cu),
+                        ints(*[i for i, r in enumerate(runs) for _ in range(r[2])]), ints(*[r[0] for r in runs]), n_seqs=len(runs),
+                        heads=heads, head_dim=P, state_dim=N, groups=1, norm_groups=1, eps=1e-5, in_chunks=False)
+            got[rows] = out
+        return got, conv_state
+
+    whole, end = run([[(s, 0, m) for s, m in enumerate(lens)]])
+    single, end_single = run([[(s, t, 1) for s, m in enumerate(lens) if t < m] for t in range(max(lens))])
+    assert torch.equal(whole, single) and torch.equal(end, end_single)
+
+
 # ----------------------------------------------------------------------------- attention with kept first positions
 
 
