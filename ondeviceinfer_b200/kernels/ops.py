@@ -2098,16 +2098,22 @@ class _SsdArgs(Structure):
 SSD_MAX_STATE, SSD_MAX_TAPS = 256, 16
 # The scan of runs of tokens goes 64 tokens at a time when a sequence brings this many on average (the mixer of 32 heads of 128 x
 # 64, us in chunks and token by token: 64 tokens 57, 38; 128 63, 60; 8 x 100 99, 107; 512 79, 152), and a step so many in all: with fewer
-# the host's launches are the bound of the models that have it, and the chunks are two launches more.
-SSD_CHUNK, SSD_CHUNK_MIN_RUN, SSD_CHUNK_MIN_TOKENS, SSD_CHUNK_MAX_SCRATCH = 64, 128, 1024, 1 << 30
+# the host's launches are the bound of the models that have it, and the chunks are two launches more.  Longer runs for heads whose
+# columns are no multiple of 64, which the chunks pad to it (16 heads of 256 x 32: 8 x 130 tokens 115 and 88, 64 x 128 473 and 400, 8 x 256
+# 133 and 157; 4 of 64 x 20: 8 x 130 44 and 35, 8 x 256 48 and 63).
+SSD_CHUNK, SSD_CHUNK_MIN_RUN, SSD_CHUNK_MIN_RUN_PADDED, SSD_CHUNK_MIN_TOKENS, SSD_CHUNK_MAX_SCRATCH = 64, 128, 256, 1024, 1 << 30
 
 
 def ssd_chunk_floats(n_tokens: int, n_seqs: int, heads: int, head_dim: int, state_dim: int, groups: int,
                      least: Optional[int] = None) -> int:
     """Floats of scratch for a state-space scan in chunks (the chunks' states, products of B and C, decays); 0 where it goes
     token by token: short runs, sizes that the chunk kernels do not take, more scratch than SSD_CHUNK_MAX_SCRATCH bytes."""
-    fewest = max(SSD_CHUNK_MIN_RUN * n_seqs, SSD_CHUNK_MIN_TOKENS) if least is None else least * n_seqs
-    if (n_tokens < fewest or state_dim % SSD_CHUNK != 0 or head_dim % 4 != 0
+    if least is None:
+        least = SSD_CHUNK_MIN_RUN if head_dim % SSD_CHUNK == 0 else SSD_CHUNK_MIN_RUN_PADDED
+        too_few = n_tokens < max(least * n_seqs, SSD_CHUNK_MIN_TOKENS)
+    else:
+        too_few = n_tokens < least * n_seqs
+    if (too_few or state_dim % SSD_CHUNK != 0 or head_dim % 4 != 0
             or heads * -(-head_dim // SSD_CHUNK) * (state_dim // SSD_CHUNK) + groups > 65535):
         return 0
     floats = (n_tokens // SSD_CHUNK + n_seqs) * (heads * state_dim * head_dim + groups * SSD_CHUNK * SSD_CHUNK + heads)

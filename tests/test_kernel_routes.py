@@ -38,3 +38,11 @@ def test_operands_off_the_16_byte_borders_keep_the_tiles_of_the_cuda_cores():
     assert not ops.grouped_tensor_ok((64, 12), torch.bfloat16, aligned) and not ops.grouped_tensor_ok((64, 8), torch.float32)
     tiles = lambda pairs, *operands: ops.RoutingTable(pairs, 1, 2, "cpu", tensor=ok(*operands)).tm
     assert [tiles(n, aligned) for n in (16, 17, 100)] == [8, 16, 16] and [tiles(n, off) for n in (16, 64, 65, 100)] == [16, 16, 64, 64]
+
+
+@pytest.mark.parametrize("P,N,lens,chunks", [
+    (64, 128, [2048], True), (64, 128, [1023], False), (64, 128, [128] * 8, True), (64, 128, [127] * 9, False),
+    (32, 256, [130] * 8, False), (20, 64, [130] * 8, False), (32, 256, [256] * 8, True), (32, 256, [1100], True),      # padded to 64 columns
+    (64, 48, [2048], False), (6, 64, [2048], False)])
+def test_state_space_scan_goes_in_chunks_from_the_runs_that_win_by_it(P, N, lens, chunks):
+    assert (ops.ssd_chunk_floats(sum(lens), len(lens), 16, P, N, 1) > 0) == chunks
