@@ -1178,9 +1178,9 @@ def grouped_rows_tile(rows_per_group: float, few_rows_ok: bool = False, tensor: 
 
 
 def grouped_few_rows_ok(K_values: Sequence[int], dtype: torch.dtype) -> bool:
-    """Whether products over these inner sizes can take the form for few rows (multiples of 8, and four rows of
-    floats within the shared memory of a block)."""
-    return all(K % 8 == 0 and 4 * FEW_ROWS * K <= 200 * 1024 for K in K_values)
+    """Whether products over these inner sizes can take the form for few rows (float32, multiples of 8, and four rows
+    within the shared memory of a block; bf16 goes on the tensor cores or in tiles)."""
+    return dtype == torch.float32 and all(K % 8 == 0 and 4 * FEW_ROWS * K <= 200 * 1024 for K in K_values)
 
 
 def grouped_tensor_ok(K_values: Sequence[int], dtype: torch.dtype, *operands: torch.Tensor) -> bool:

@@ -107,7 +107,7 @@ class RoutedExperts(Part):
         weights = torch.empty((n, s.top_k), dtype=torch.float32, device=dev)
         ops.moe_route(logits, self.correction, ids, weights, n_groups=s.num_groups, keep=s.keep_groups,
                       sigmoid=s.scoring == "sigmoid", renormalise=s.renormalise, scale=s.weight_scale)
-        # single-token steps, a few rows per expert: the grouped product that streams weights through registers
+        # float32 steps of a few rows per expert: the grouped product that streams weights through registers
         experts = (self.w_gate_up, self.w_down) if s.num_experts > 0 else ()
         few_ok = ops.grouped_few_rows_ok((s.hidden_size, s.expert_size), x.dtype)
         table = ops.RoutingTable(n, s.top_k, max(s.num_experts, 1), dev, few_rows_ok=few_ok,

@@ -36,8 +36,10 @@ def test_operands_off_the_16_byte_borders_keep_the_tiles_of_the_cuda_cores():
     ok = lambda *operands: ops.grouped_tensor_ok((64, 8), torch.bfloat16, *operands)
     assert ok() and ok(aligned, aligned) and not ok(aligned, off)
     assert not ops.grouped_tensor_ok((64, 12), torch.bfloat16, aligned) and not ops.grouped_tensor_ok((64, 8), torch.float32)
-    tiles = lambda pairs, *operands: ops.RoutingTable(pairs, 1, 2, "cpu", tensor=ok(*operands)).tm
-    assert [tiles(n, aligned) for n in (16, 17, 100)] == [8, 16, 16] and [tiles(n, off) for n in (16, 64, 65, 100)] == [16, 16, 64, 64]
+    few = ops.grouped_few_rows_ok((64, 8), torch.bfloat16)      # the form for few rows is float32's
+    tiles = lambda pairs, *operands: ops.RoutingTable(pairs, 1, 2, "cpu", few_rows_ok=few, tensor=ok(*operands)).tm
+    assert [tiles(n, aligned) for n in (2, 16, 17, 100)] == [8, 8, 16, 16] and [tiles(n, off) for n in (2, 16, 64, 65, 100)] == [16, 16, 16, 64, 64]
+    assert ops.RoutingTable(2, 1, 2, "cpu", few_rows_ok=ops.grouped_few_rows_ok((64, 8), torch.float32)).tm == 4
 
 
 @pytest.mark.parametrize("P,N,lens,chunks", [

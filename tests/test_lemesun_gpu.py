@@ -223,9 +223,13 @@ def test_routed_products_against_a_loop_over_pairs(dtype, tokens, K, F):
     w_d = (torch.randn(E, K, F, generator=g) / F ** 0.5).to(dtype)
     ids = torch.stack([torch.randperm(E + ident, generator=g)[:top] for _ in range(tokens)]).int()
     weights = torch.rand(tokens, top, generator=g)
-    # aligned sizes and few rows per expert: the form that streams the weights through registers
-    table = ops.RoutingTable(tokens, top, E, "cuda", few_rows_ok=ops.grouped_few_rows_ok((K, F), dtype))
-    assert table.tm == (4 if K % 8 == 0 and tokens <= 5 else 16 if tokens <= 5 else 64)
+    # aligned sizes: bf16 on the tensor cores; float32 with few rows per expert in the form that streams the weights through registers
+    table = ops.RoutingTable(tokens, top, E, "cuda", few_rows_ok=ops.grouped_few_rows_ok((K, F), dtype),
+                             tensor=ops.grouped_tensor_ok((K, F), dtype))
+    if dtype == torch.bfloat16 and K % 8 == 0:
+        assert table.tm == (8 if tokens <= 5 else 16)
+    else:
+        assert table.tm == (4 if K % 8 == 0 and tokens <= 5 else 16 if tokens <= 5 else 64)
     counts = torch.zeros(E, dtype=torch.int32, device="cuda")
     ops.moe_group(ids.cuda(), counts, table)
     assert int(counts.abs().sum()) == 0                    # left clean for the next step
@@ -249,8 +253,8 @@ def test_routed_products_against_a_loop_over_pairs(dtype, tokens, K, F):
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("heads,K,N,M,a_gap,c_gap", [(3, 10, 7, 37, 2, 4), (4, 16, 12, 3, 8, 4), (4, 16, 12, 7, 8, 4),
                                                      (2, 24, 70, 130, 8, 2),
-                                                     (3, 264, 20, 7, 8, 4), (4, 512, 40, 8, 0, 8), (2, 256, 9, 5, 8, 3),   # five to eight rows, long inner size: two row tiles of the form for few rows
-                                                     (2400, 16, 320, 3, 8, 4)])     # bf16: more than 32 items a warp
+                                                     (3, 264, 20, 7, 8, 4), (4, 512, 40, 8, 0, 8), (2, 256, 9, 5, 8, 3),   # five to eight rows, long inner size: float32 in two row tiles of the form for few rows
+                                                     (2400, 16, 320, 3, 8, 4)])     # many heads
 def test_products_per_head(dtype, heads, K, N, M, a_gap, c_gap):
     g = torch.Generator().manual_seed(3)
     a = torch.randn(M, heads * (K + a_gap) + 8, generator=g).to(dtype)     # a head's K lanes lie K + a_gap apart

@@ -210,7 +210,7 @@ def test_ungated_experts_with_weights_on_their_inputs(dtype, n, H, F, n_experts,
     ids = torch.empty(n, top, dtype=torch.int32, device="cuda")
     weights = torch.empty(n, top, dtype=torch.float32, device="cuda")
     ops.moe_route(logits.cuda(), None, ids, weights, n_groups=1, keep=1, sigmoid=True)
-    table = ops.RoutingTable(n, top, n_experts, "cuda")
+    table = ops.RoutingTable(n, top, n_experts, "cuda", tensor=ops.grouped_tensor_ok((H, F), dtype))
     counts = torch.zeros(n_experts, dtype=torch.int32, device="cuda")
     ops.moe_group(ids, counts, table)
     rows = torch.empty(n * top, H, dtype=dtype, device="cuda")

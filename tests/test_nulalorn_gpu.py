@@ -291,7 +291,8 @@ def test_table_routed_experts_against_a_loop_over_tokens(dtype, tokens, experts,
     weights = torch.empty((tokens, top), dtype=torch.float32, device="cuda")
     ops.moe_table_route(table.cuda(), ids_in.cuda(), ids, weights, n_experts=experts, weight=1.0 / top)
     assert torch.equal(ids.cpu(), table[ids_in.long()]) and float((weights - 1.0 / top).abs().max()) == 0
-    routing = ops.RoutingTable(tokens, top, experts, "cuda", few_rows_ok=ops.grouped_few_rows_ok((K, F), dtype))
+    routing = ops.RoutingTable(tokens, top, experts, "cuda", few_rows_ok=ops.grouped_few_rows_ok((K, F), dtype),
+                               tensor=ops.grouped_tensor_ok((K, F), dtype))
     counts = torch.zeros(experts, dtype=torch.int32, device="cuda")
     ops.moe_group(ids, counts, routing)
     act = torch.empty((tokens * top, F), dtype=dtype, device="cuda")
@@ -307,19 +308,19 @@ def test_table_routed_experts_against_a_loop_over_tokens(dtype, tokens, experts,
     assert (acc.cpu().double() - want).abs().max() < (2e-5 if dtype == torch.float32 else 3e-2)
 
 
-@pytest.mark.parametrize("tokens,experts,top,K,F", [(7, 5, 3, 616, 1016),       # three chunks of k, the last one partial
-                                                    (6, 12, 2, 264, 4096),       # a list long enough for items of 8 weight rows
-                                                    (3, 4, 4, 136, 12800),       # the widest rows the form takes
+@pytest.mark.parametrize("tokens,experts,top,K,F", [(7, 5, 3, 616, 1016),       # two pieces of k a warp, the last of them partial
+                                                    (6, 12, 2, 264, 4096),       # many blocks of features
+                                                    (3, 4, 4, 136, 12800),       # long inner sizes: 25 pieces of k a warp
                                                     (1, 2, 1, 8, 8)])
-def test_single_token_expert_products_that_walk_item_lists(tokens, experts, top, K, F):
-    """bf16 products of a few rows per expert: every warp walks its own list of (tile, weight rows) items."""
+def test_single_token_expert_products(tokens, experts, top, K, F):
+    """bf16 products of a few rows per expert: tiles of eight rows, most of them empty."""
     g = torch.Generator().manual_seed(K)
     ids = torch.stack([torch.randperm(experts, generator=g)[:top] for _ in range(tokens)]).int().cuda()
     x = torch.randn(tokens, K, generator=g).bfloat16().cuda()
     w_up = (torch.randn(experts, F, K, generator=g) / K ** 0.5).bfloat16().cuda()
     w_down = (torch.randn(experts, K, F, generator=g) / F ** 0.5).bfloat16().cuda()
-    assert ops.grouped_few_rows_ok((K, F), torch.bfloat16)
-    routing = ops.RoutingTable(tokens, top, experts, "cuda", few_rows_ok=True)
+    routing = ops.RoutingTable(tokens, top, experts, "cuda", tensor=ops.grouped_tensor_ok((K, F), torch.bfloat16))
+    assert routing.tm == 8
     counts = torch.zeros(experts, dtype=torch.int32, device="cuda")
     ops.moe_group(ids, counts, routing)
     act = torch.empty((tokens * top, F), dtype=torch.bfloat16, device="cuda")
