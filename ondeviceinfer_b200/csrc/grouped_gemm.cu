@@ -1,6 +1,8 @@
-// Grouped matrix product on the CUDA cores: many small products C_g = A_g W_g^T in one launch, each group with
-// a weight matrix of its own.  fp32 accumulation over k = 0..K-1 in that order for every output element,
-// whatever else is in the launch, for both element types (T = float: the true 32-bit path; T = bf16).
+// Grouped matrix product: many small products C_g = A_g W_g^T in one launch, each group with a weight matrix of its own, fp32
+// accumulation in an order that no other row of the launch changes.  T = float (the true 32-bit path): on the CUDA cores, over
+// k = 0..K-1 in that order, or for groups of a few rows a lane's k and then the lanes by a tree.  T = bf16 with aligned operands: on
+// the tensor cores (grouped_mma_kernel says how its sums are grouped); else, and for products per head of many rows and few
+// k, as float in tiles.
 //
 // Two ways to say which rows belong to which group:
 //  * dense (tile table null): every group has the same M rows; group g reads columns [g * a_group_off, +K) of
@@ -13,8 +15,8 @@
 // g = min(gate, limit), u = clamp(up, -limit, limit), C = g * sigmoid(alpha * g) * (u + up_shift) as T), 3 the exact
 // (erf) GELU of the sum as T, 4 its tanh form, 5 the square of max(sum, 0) as T.
 //
-// Tile: TM rows x 64 features per block of 256 threads, K in slices of 16 or 32 through shared memory (fp32).
-// TM = 64 (4 x 4 outputs a thread) or 16 (1 x 4), chosen by the caller from the rows a group has; for groups
+// Tile on the CUDA cores: TM rows x 64 features per block of 256 threads, K in slices of 16 or 32 through shared memory (fp32).
+// TM = 64 (4 x 4 outputs a thread) or 16 (1 x 4), chosen by the caller from the rows a group has; for float groups
 // of a few rows there is a form that streams the weights through registers only (grouped_gemv_kernel).
 #include "common.cuh"
 

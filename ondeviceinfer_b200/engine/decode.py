@@ -236,7 +236,7 @@ class DecodeRunner:
         cache, slots = self.cache, self.live_slots
         before = [[len(group.slot_pages[s]) for s in slots] for group in cache.kv_groups]
         if not cache.reserve(slots, [ahead] * len(slots)):
-            return                             # 63 steps of 64
+            return                             # a sequence takes a page every 64 steps
         for g, group in enumerate(cache.kv_groups):
             for i, slot in enumerate(slots):
                 pages = group.slot_pages[slot]
