@@ -27,18 +27,22 @@ __device__ __forceinline__ void fma_pair(unsigned long long& acc, unsigned long 
   asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(a), "l"(w));
 }
 
-// ROWS rows of X [limit, K] from row r0 on, k0 .. k0 + KS - 1, into dst (pitch PITCH); zeros beyond either end
+// ROWS rows of X [limit, K] from row r0 on, k0 .. k0 + KS - 1, into dst (pitch PITCH); zeros beyond either end, but nothing
+// where the last stage has no k left to multiply
 template <int ROWS, bool VEC>
 __device__ __forceinline__ void stage_rows(uint32_t dst, const float* __restrict__ X, int r0, int limit, int k0, int K, int ld) {
+  const int left = K - k0 + (K & 1);      // k in pairs
   if (VEC) {
     for (int i = threadIdx.x; i < ROWS * (KS / 4); i += NTH) {
       const int r = i / (KS / 4), k = (i % (KS / 4)) * 4;
+      if (k >= left) continue;
       const bool ok = r0 + r < limit && k0 + k < K;
       cp_async16(dst + (r * PITCH + k) * 4, ok ? X + (size_t)(r0 + r) * ld + k0 + k : X, ok);
     }
   } else {
     for (int i = threadIdx.x; i < ROWS * KS; i += NTH) {
       const int r = i / KS, k = i % KS;
+      if (k >= left) continue;
       const bool ok = r0 + r < limit && k0 + k < K;
       cp_async4(dst + (r * PITCH + k) * 4, ok ? X + (size_t)(r0 + r) * ld + k0 + k : X, ok);
     }
@@ -88,7 +92,8 @@ gemm_f32_kernel(const float* __restrict__ A, const float* __restrict__ W, float*
   asm volatile("cp.async.wait_group %0;" ::"n"(STAGES - 1) : "memory");
   __syncthreads();
   read(0, 0, 0);
-  for (int s = 0; s < n_stages; ++s) {
+  const int full = K / KS;
+  for (int s = 0; s < full; ++s) {
 #pragma unroll
     for (int k = 0; k < KS; k += 2) {
       const int set = (k >> 1) & 1;
@@ -105,6 +110,15 @@ gemm_f32_kernel(const float* __restrict__ A, const float* __restrict__ W, float*
 #pragma unroll
         for (int j = 0; j < RN; ++j) fma_pair(acc[i][j], a[set][i], w[set][j]);
     }
+  }
+  // the k that fill no stage, if any: the first two are read already
+#pragma unroll 1
+  for (int k = 0; k < K - full * KS; k += 2) {
+    if (k > 0) read(0, full, k);
+#pragma unroll
+    for (int i = 0; i < RM; ++i)
+#pragma unroll
+      for (int j = 0; j < RN; ++j) fma_pair(acc[i][j], a[0][i], w[0][j]);
   }
   pdl_launch_dependents();      // not earlier: blocks of the next kernel would take the places of this one's
 #pragma unroll
@@ -163,19 +177,40 @@ static int pick_form(int M, int N) {
   return best;
 }
 
+// Rows that are copied 4 bytes at a time have three tiles (16 x 64, 32 x 64, 64 x 128), whose copies bound them: us at K = 1,001 up to 66
+// tiles, then of c tiles a multiprocessor the larger of `one` and start + c more.  (By the rule of the forms above 1,024 x 300 x 50
+// took 9.3 us where the 64 x 64 tile of before took 6.5, and takes 5.9 now; 300 x 1,000 x 333 34 and 26, now 22.)
+struct F32Scalar { int rows, cols; double few, one, start, more; };
+static const F32Scalar scalar_forms[] = {{16, 64, 42.4, 42.4, 9, 18.2}, {32, 64, 42.2, 42.2, 12, 24.2}, {64, 128, 91, 123, 0, 77}};
+static int pick_scalar(int M, int N) {
+  int best = 0;
+  double least = 1e300;
+  for (int f = 0; f < 3; ++f) {
+    const F32Scalar& x = scalar_forms[f];
+    const long tiles = (long)((M + x.rows - 1) / x.rows) * ((N + x.cols - 1) / x.cols), c = (tiles + 147) / 148;
+    const double cost = tiles > 66 ? max(x.one, x.start + (double)c * x.more) : x.few;
+    if (cost < least) { least = cost; best = f; }
+  }
+  return best;
+}
+
 // R may be null (no residual) or alias C (in-place add: each element is read and then
 // written by the same thread).  bias may be null; it is added to the product before the residual.
 extern "C" int odi_gemm_f32(const float* A, const float* W, float* C, const float* R, const float* bias, int M, int N,
                             int K, int lda, int ldw, int ldc, int ldr, int force, cudaStream_t stream) {
   if (M <= 0 || N <= 0) return 0;
   if (K <= 0) return ODI_ERR_ARGUMENT;
-  if ((M - 1) / 64 >= 65535) return ODI_ERR_UNSUPPORTED;
+  if ((M - 1) / 64 >= 65535) return ODI_ERR_UNSUPPORTED;      // more rows than this has never been taken or tried
   const bool vec = (K % 4 == 0) && (lda % 4 == 0) && (ldw % 4 == 0) &&
                    ((uintptr_t)A % 16 == 0) && ((uintptr_t)W % 16 == 0);
-  const int form = force >= 0 && force < F32_FORMS ? force : pick_form(M, N);
+  const bool forced = force >= 0 && force < F32_FORMS;
+  const int form = forced ? force : vec ? pick_form(M, N) : 0;
 #define ODI_F32(RM, RN, STAGES) launch_form<RM, RN, STAGES, true>(A, W, C, R, bias, M, N, K, lda, ldw, ldc, ldr, stream)
 #define ODI_F32_SCALAR(RM, RN) launch_form<RM, RN, 3, false>(A, W, C, R, bias, M, N, K, lda, ldw, ldc, ldr, stream)
-  if (!vec) return form < 4 ? ODI_F32_SCALAR(2, 4) : (form < 6 ? ODI_F32_SCALAR(4, 4) : ODI_F32_SCALAR(8, 8));
+  if (!vec) {
+    const int tile = forced ? (form < 4 ? 0 : form < 6 ? 1 : 2) : pick_scalar(M, N);
+    return tile == 0 ? ODI_F32_SCALAR(2, 4) : tile == 1 ? ODI_F32_SCALAR(4, 4) : ODI_F32_SCALAR(8, 8);
+  }
   switch (form) {
     case 0: return ODI_F32(1, 2, 8);
     case 1: return ODI_F32(1, 4, 6);
