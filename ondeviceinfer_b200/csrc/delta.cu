@@ -284,7 +284,7 @@ __global__ void __launch_bounds__(2 * D)
 delta_parts_kernel(DeltaArgs a, DeltaChunkArgs c) {
   pdl_launch_dependents();
   pdl_wait();
-  __shared__ DeltaChunkShared<D> sh;
+  __shared__ DeltaChunkShared<D, false> sh;
   const int h = blockIdx.y, src = h / (a.heads / a.kv_heads);
   int seq, first, nt;
   if (!run_chunk<DC>(a.cu_q, a.n_seqs, blockIdx.x, sh.found, seq, first, nt)) return;
@@ -350,7 +350,7 @@ delta_parts_kernel(DeltaArgs a, DeltaChunkArgs c) {
   __syncthreads();
   // the values of this thread's columns: all its tokens at once when it comes to a new column
   float v[DC];
-  dc_parts<D>(sh, c, blockIdx.x, h, [&](int t, int col) {
+  dc_parts<D, false>(sh, c, blockIdx.x, h, [&](int t, int col) {
     if (t == 0) convolved(2 * a.kv_heads * D + h * a.dv + col, v);
     return v[t];
   });

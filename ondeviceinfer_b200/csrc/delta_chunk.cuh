@@ -2,7 +2,8 @@
 // per head, which is then every channel's).
 //
 // Per sequence and head, with S [D, dv] the state before the chunk, g_t [D] the decays of token t, G_t = g_0 .. g_t and
-// D_ts = g_(s+1) .. g_t (products lane by lane; nothing is divided, so no decay is too small), the recurrence
+// D_ts = g_(s+1) .. g_t (products lane by lane, with one decay a head once for all and rounded once; nothing is divided, so no decay
+// is too small), the recurrence
 //     S <- diag(g) S;   u = beta (v - S^T k);   S <- S + k u^T;   o = S^T q
 // unrolls over the chunk to
 //     u_t = beta_t (v_t - (G_t k_t)^T S - sum_(s<t) A_ts u_s),      A_ts = k_t . (D_ts k_s)
@@ -35,19 +36,34 @@ struct DeltaChunkArgs {
   int n_seqs, heads, dv;
 };
 
-template <int D>
+template <int D, bool HEAD>
 struct DeltaChunkShared {
-  float q[DC][D], k[DC][D], g[DC][D];
+  float q[DC][D], k[DC][D];
+  float g[HEAD ? DC + 1 : DC][HEAD ? DC : D];      // decays per token and channel; HEAD: dc_head_decays
   __align__(16) float A[DC][DC];
   __align__(16) float B[DC][DC];
   float beta[DC];
   int found[3];
 };
 
+// One decay a head: row s the products D_ts of the tokens behind s (1 at s, 0 before), the last row G_t.  By the block's first warp,
+// whose lanes hold a token's decay each (1 from lane DC on).
+template <typename Shared>
+__device__ __forceinline__ void dc_head_decays(Shared& sh, float own) {
+  const int s = threadIdx.x;
+  DecayProduct run;
+#pragma unroll
+  for (int t = 0; t < DC; ++t) {
+    const float g = __shfl_sync(0xffffffffu, own, t);
+    if (t > s || s == DC) run.times(g);
+    if (s <= DC) sh.g[s][t] = t < s && s < DC ? 0.f : run.value();
+  }
+}
+
 // The parts of a chunk from its unit vectors, decays and step sizes in shared memory (written before a barrier) and
 // its values; by all threads of a block of whole warps, D + dv columns in turn.
-template <int D, typename Value>
-__device__ __forceinline__ void dc_parts(DeltaChunkShared<D>& sh, const DeltaChunkArgs& a, int b, int h, Value value) {
+template <int D, bool HEAD, typename Value>
+__device__ __forceinline__ void dc_parts(DeltaChunkShared<D, HEAD>& sh, const DeltaChunkArgs& a, int b, int h, Value value) {
   static_assert(D % 32 == 0, "lanes own whole channels");
   constexpr int NI = D / 32;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, n_warps = blockDim.x >> 5;
@@ -63,7 +79,7 @@ __device__ __forceinline__ void dc_parts(DeltaChunkShared<D>& sh, const DeltaChu
       if (t >= s) {
 #pragma unroll
         for (int e = 0; e < NI; ++e) {
-          if (t > s) w[e] *= sh.g[t][lane + 32 * e];
+          if (!HEAD && t > s) w[e] *= sh.g[t][lane + 32 * e];
           r[t] = fmaf(w[e], sh.k[t][lane + 32 * e], r[t]);
           r[DC + t] = fmaf(w[e], sh.q[t][lane + 32 * e], r[DC + t]);
         }
@@ -78,7 +94,8 @@ __device__ __forceinline__ void dc_parts(DeltaChunkShared<D>& sh, const DeltaChu
         r[i] = keep + __shfl_xor_sync(0xffffffffu, give, m);
       }
     }
-    (lane < DC ? sh.A : sh.B)[lane & (DC - 1)][s] = r[0];      // column s; A's diagonal and what lies above are not read
+    const float decayed = HEAD ? r[0] * sh.g[s][lane & (DC - 1)] : r[0];
+    (lane < DC ? sh.A : sh.B)[lane & (DC - 1)][s] = decayed;      // column s; A's diagonal and what lies above are not read
   }
   __syncthreads();
   const size_t item = (size_t)b * a.heads + h;
@@ -89,11 +106,11 @@ __device__ __forceinline__ void dc_parts(DeltaChunkShared<D>& sh, const DeltaChu
     float w[DC], decay = 1.f;
 #pragma unroll
     for (int t = 0; t < DC; ++t) {
-      if (is_k) decay *= sh.g[t][c];
-      float x = is_k ? sh.k[t][c] * decay : value(t, c - D);
+      if (is_k) decay = HEAD ? sh.g[HEAD ? DC : 0][t] : decay * sh.g[t][c];
+      float x = 0.f;      // summed before it is taken off: one rounding of the larger number
 #pragma unroll
-      for (int s = 0; s < t; ++s) x = fmaf(-sh.A[t][s], w[s], x);
-      w[t] = sh.beta[t] * x;
+      for (int s = 0; s < t; ++s) x = fmaf(sh.A[t][s], w[s], x);
+      w[t] = sh.beta[t] * (is_k ? fmaf(sh.k[t][c], decay, -x) : value(t, c - D) - x);
     }
     float run = 1.f, tail = 1.f;
 #pragma unroll
@@ -102,7 +119,7 @@ __device__ __forceinline__ void dc_parts(DeltaChunkShared<D>& sh, const DeltaChu
 #pragma unroll
       for (int s = 0; s <= t; ++s) x = fmaf(sh.B[t][s], w[s], x);
       if (is_k) {
-        run *= sh.g[t][c];
+        run = HEAD ? sh.g[HEAD ? DC : 0][t] : run * sh.g[t][c];
         wk[t * D + c] = w[t];
         wk[(DC + t) * D + c] = fmaf(sh.q[t][c], run, -x);
       } else {
@@ -113,8 +130,8 @@ __device__ __forceinline__ void dc_parts(DeltaChunkShared<D>& sh, const DeltaChu
     if (is_k) {
 #pragma unroll
       for (int t = DC - 1; t >= 0; --t) {
-        wk[(2 * DC + t) * D + c] = sh.k[t][c] * tail;
-        tail *= sh.g[t][c];
+        wk[(2 * DC + t) * D + c] = sh.k[t][c] * (HEAD ? sh.g[t][DC - 1] : tail);
+        if (!HEAD) tail *= sh.g[t][c];
       }
       wk[3 * DC * D + c] = decay;
     }

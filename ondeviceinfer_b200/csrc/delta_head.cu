@@ -649,25 +649,26 @@ __global__ void __launch_bounds__(2 * D, D == 64 ? 6 : 3)      // three resp. si
 hd_parts_kernel(HeadDeltaArgs a, DeltaChunkArgs c) {
   pdl_launch_dependents();
   pdl_wait();
-  __shared__ DeltaChunkShared<D> sh;
+  __shared__ DeltaChunkShared<D, true> sh;
   const int h = blockIdx.y, kvh = h / (a.heads / a.kv_heads);
   int seq, first, nt;
   if (!run_chunk<DC>(a.cu_q, a.n_seqs, blockIdx.x, sh.found, seq, first, nt)) return;
   const size_t tok = (size_t)a.cu_q[seq] + first;
   const float* qk = a.qk + (tok * a.kv_heads + kvh) * 2 * D;
+  const float decay = (int)threadIdx.x < nt ? a.gb[((tok + threadIdx.x) * a.heads + h) * 2] : 1.f;      // nt <= DC
   for (int x = threadIdx.x; x < DC * D; x += blockDim.x) {
     const int t = x / D, i = x % D;
     const bool in = t < nt;
     const float* row = qk + (size_t)t * a.kv_heads * 2 * D;
     sh.q[t][i] = in ? row[i] : 0.f;
     sh.k[t][i] = in ? row[D + i] : 0.f;
-    sh.g[t][i] = in ? a.gb[((tok + t) * a.heads + h) * 2] : 1.f;
   }
+  if (threadIdx.x < 32) dc_head_decays(sh, decay);
   if (threadIdx.x < DC) sh.beta[threadIdx.x] = (int)threadIdx.x < nt ? a.gb[((tok + threadIdx.x) * a.heads + h) * 2 + 1] : 0.f;
   __syncthreads();
   const float* v = a.o + (tok * a.heads + h) * a.dv;
   const size_t step = (size_t)a.heads * a.dv;
-  dc_parts<D>(sh, c, blockIdx.x, h, [&](int t, int col) { return t < nt ? v[t * step + col] : 0.f; });
+  dc_parts<D, true>(sh, c, blockIdx.x, h, [&](int t, int col) { return t < nt ? v[t * step + col] : 0.f; });
 }
 
 template <int D>

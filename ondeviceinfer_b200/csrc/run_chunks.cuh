@@ -19,3 +19,20 @@ __device__ __forceinline__ bool run_chunk(const int* cu_q, int n_seqs, int b, in
   seq = found[0]; first = found[1]; nt = found[2];
   return seq >= 0;
 }
+
+// A product of decays carried as two floats and rounded once at the end: in the sums over a state's rows the errors of a chunk's
+// decays, which all rows share, do not even out as those of rows that round by themselves do.
+struct DecayProduct {
+  float hi = 1.f, lo = 0.f;
+  __device__ __forceinline__ void times(float a) {
+    const float p = __fmul_rn(hi, a);
+    lo = fmaf(lo, a, fmaf(hi, a, -p));
+    hi = p;
+  }
+  __device__ __forceinline__ void times(const DecayProduct& o) {
+    const float p = __fmul_rn(hi, o.hi);
+    lo = fmaf(hi, o.lo, fmaf(lo, o.hi, fmaf(hi, o.hi, -p)));
+    hi = p;
+  }
+  __device__ __forceinline__ float value() const { return hi + lo; }
+};

@@ -349,8 +349,8 @@ ssd_scan_kernel(SsdArgs a) {
 //           group: the products C_t . B_s, which the heads of a group share;
 //  pass     per element of S: E of every chunk gives way to the state before it;
 //  outputs  every chunk and head at once: y.
-// All of it plain fp32 multiply-adds, as token by token, where a sequence's tokens were one chain of them.  The mixer between its
-// products, 32 heads of 128 x 64, us (in chunks, token by token): 2,048 tokens 187, 564; 2 x 1,024 183, 350; 8 x 1,000 715, 961;
+// The products of decays are rounded once (DecayProduct); all else is plain fp32 multiply-adds, as token by token, where a
+// sequence's tokens were one chain of them.  The mixer between its products, 32 heads of 128 x 64, us (in chunks, token by token): 2,048 tokens 187, 564; 2 x 1,024 183, 350; 8 x 1,000 715, 961;
 // 512 79, 152; 128 63, 60.  What bounds outputs (66 us of those 187) and states (54) is shared memory: three 16-byte reads per 32
 // multiply-adds of a thread.
 #define SSD_L 64
@@ -461,11 +461,27 @@ ssd_states_kernel(SsdArgs a) {
   const int h = blockIdx.y / (p_tiles * n_tiles), p0 = blockIdx.y / n_tiles % p_tiles * SSD_L, n0 = blockIdx.y % n_tiles * SSD_L;
   ssd_chunk_steps<T>(a, h, tok, nt, dt_s, a_s);
   __syncthreads();
-  if (tid == 0) {                                 // D_last,s dt_s, from the last token on
-    float tail = 1.f;
-#pragma unroll 16
-    for (int s = SSD_L - 1; s >= 0; --s) { w_s[s] = tail * dt_s[s]; tail *= a_s[s]; }
-    if (p0 == 0 && n0 == 0) out.gamma[(size_t)blockIdx.x * a.heads + h] = tail;
+  if (tid < 32) {                                 // D_last,s dt_s: a lane two tokens, the products of all behind them by shuffles
+    const float a0 = a_s[2 * tid], a1 = a_s[2 * tid + 1];
+    DecayProduct run, other;                      // of this lane's tokens and those behind them
+    run.times(a0);
+    run.times(a1);
+#pragma unroll
+    for (int m = 1; m < 32; m <<= 1) {
+      other.hi = __shfl_down_sync(0xffffffffu, run.hi, m);
+      other.lo = __shfl_down_sync(0xffffffffu, run.lo, m);
+      if (tid + m < 32) run.times(other);
+    }
+    if (tid == 0 && p0 == 0 && n0 == 0) out.gamma[(size_t)blockIdx.x * a.heads + h] = run.value();
+    other.hi = __shfl_down_sync(0xffffffffu, run.hi, 1);
+    other.lo = __shfl_down_sync(0xffffffffu, run.lo, 1);
+    if (tid == 31) other = DecayProduct();
+    DecayProduct last = other;
+    last.times(dt_s[2 * tid + 1]);
+    other.times(a1);
+    other.times(dt_s[2 * tid]);
+    w_s[2 * tid + 1] = last.value();
+    w_s[2 * tid] = other.value();
   }
   const float* Bg = rows + inner + (size_t)(h / (a.heads / a.G)) * a.N + n0;
   const float* X = rows + (size_t)h * a.P + p0;
@@ -545,16 +561,17 @@ ssd_outputs_kernel(SsdArgs a) {
   ssd_chunk_steps<T>(a, h, tok, nt, dt_s, a_s);
   __syncthreads();
   if (tid < SSD_L) {                              // a thread a token s: its decays on the way to every later token
-    float d = dt_s[tid];
+    DecayProduct d;
+    d.hi = dt_s[tid];
 #pragma unroll 16
     for (int t = 0; t < SSD_L; ++t) {
-      if (t > tid) d *= a_s[t];
-      Ds[tid * SSD_PAD + t] = t < tid ? 0.f : d;
+      if (t > tid) d.times(a_s[t]);
+      Ds[tid * SSD_PAD + t] = t < tid ? 0.f : d.value();
     }
   } else if (tid == SSD_L) {
-    float run = 1.f;
+    DecayProduct run;
 #pragma unroll 16
-    for (int t = 0; t < SSD_L; ++t) { run *= a_s[t]; g_s[t] = run; }
+    for (int t = 0; t < SSD_L; ++t) { run.times(a_s[t]); g_s[t] = run.value(); }
   }
   const int mt = tid >> 4, nn = tid & 15;
   float acc[8][4] = {};
