@@ -1699,11 +1699,11 @@ HEAD_DELTA_MAX_DIM, HEAD_DELTA_MAX_TAPS = 512, 16
 # In chunks (csrc/delta_chunk.cuh) where a few long sequences leave the chip to chains of their tokens: at most this many heads in
 # all, at least so many tokens a sequence; with heads of 128, whose chunks cost more work than four tokens at a time do, also at
 # most so many heads' worth of the longest run: that run's chain must be what the step waits for (us, chunks and fours: 16 heads,
-# 2 x 1,000 tokens 305 and 324, 3 x 1,000 433 and 413, 4 x 200 129 and 116, 1,000 + 500 + 250 307 and 329; 32 heads, 2 x 256 172 and 156,
-# 1,000 + 500 518 and 495, 800 280 and 290).  Measured against four tokens at a time, the mixer, us: 16 heads of 128 x 128, one
-# sequence of 2,048 tokens 334 and 432, 256 57 and 67, 128 42 and 42; 333 + 769 + 1,777 tokens 546 and 600; 8 x 512 544 and 430; heads
-# of 64 x 64: 2,048 256 and 383, 333 + 769 + 1,777 295 and 514, 8 x 512 288 and 264.
-HEAD_DELTA_CHUNK_MAX_HEADS, HEAD_DELTA_CHUNK_MIN_RUN, HEAD_DELTA_CHUNK_MAX_LONGEST = 64, 192, 32
+# 2 x 1,000 tokens 309 and 322, 3 x 1,000 440 and 412, 4 x 200 130 and 115, 1,000 + 500 + 250 310 and 328; 32 heads, 2 x 256 177 and 151,
+# 1,000 + 500 529 and 493, 800 285 and 285).  Measured against four tokens at a time, the mixer, us: 16 heads of 128 x 128, one
+# sequence of 2,048 tokens 338 and 431, 800 140 and 178, 192 49 and 53 (4 heads 46 and 45); 333 + 769 + 1,777 tokens 553 and 598; 8 x
+# 512 543 and 428; heads of 64 x 64: 2,048 247 and 368, 333 + 769 + 1,777 283 and 492, 8 x 512 261 and 229.
+HEAD_DELTA_CHUNK_MAX_HEADS, HEAD_DELTA_CHUNK_MIN_RUN, HEAD_DELTA_CHUNK_MAX_LONGEST = 64, 224, 32
 
 
 def head_delta_chunk_floats(n_tokens: int, n_seqs: int, max_q_len: int, heads: int, d: int, dv: int, least: Optional[int] = None) -> int:

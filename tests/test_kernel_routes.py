@@ -24,7 +24,7 @@ def test_only_bfloat16_takes_runs_in_chunks():
     (16, 128, [2048], True), (16, 128, [333, 769, 1777], True), (16, 128, [1000, 1000], True), (16, 128, [1000, 500, 250], True),
     (16, 128, [1000] * 3, False), (16, 128, [512] * 4, False), (16, 128, [200] * 4, False), (32, 128, [256, 256], False),
     (32, 128, [1000, 500], False), (32, 128, [800], True), (8, 128, [512] * 4, True),      # heads of 128: the longest run's chain
-    (16, 64, [512] * 4, True), (32, 64, [256, 256], True), (16, 64, [512] * 5, False), (16, 64, [128], False), (16, 96, [2048], False)])
+    (16, 64, [512] * 4, True), (32, 64, [256, 256], True), (16, 64, [512] * 5, False), (16, 64, [223], False), (4, 128, [224], True), (16, 96, [2048], False)])
 def test_head_delta_goes_in_chunks_where_a_run_is_what_the_step_waits_for(heads, d, lens, chunks):
     assert (ops.head_delta_chunk_floats(sum(lens), len(lens), max(lens), heads, d, d) > 0) == chunks
 
