@@ -80,11 +80,13 @@ def routed(case):
 # ----------------------------------------------------------------------------- kernels against plain functions
 
 
-def delta_by_token(proj, inner, w, m, eps):
-    """The mixer between its products, token by token in 64 bits: (out [T, heads dv], final state [heads, d, dv])."""
+def delta_by_token(proj, inner, w, m, eps, dtype):
+    """The mixer between its products, token by token in 64 bits, what leaves the convolutions rounded to ``dtype``:
+    (out [T, heads dv], final state [heads, d, dv])."""
     H, G, d, dv = m["heads"], m["kv_heads"], m["dim"], m["vdim"]
     T, C = proj.shape[0], 2 * G * d + H * dv
     y = plain.causal_conv_silu(proj[:, :C], w["taps"])
+    y = y if dtype == torch.float32 else y.to(dtype).double()
     unit = lambda x: x / torch.sqrt((x * x).sum(-1, keepdim=True) + 1e-6)
     q = (unit(y[:, :G * d].view(T, G, d)) * d ** -0.5).repeat_interleave(H // G, 1)
     k = unit(y[:, G * d:2 * G * d].view(T, G, d)).repeat_interleave(H // G, 1)
@@ -101,27 +103,28 @@ def delta_by_token(proj, inner, w, m, eps):
     return out.reshape(T, H * dv), S
 
 
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("d,dv,heads,kv_heads,taps", [(64, 64, 3, 3, 4), (64, 20, 4, 2, 1), (128, 100, 2, 1, 3), (128, 128, 2, 2, 4)])
-def test_delta_rule_in_chunks_of_tokens(d, dv, heads, kv_heads, taps):
+def test_delta_rule_in_chunks_of_tokens(dtype, d, dv, heads, kv_heads, taps):
     """Runs around the chunks' edges, one of a single token among them, continued by a second step, with decays from one
     to those that wipe the state; against the recurrence token by token in 64 bits, and no further off than the token by
-    token kernel."""
+    token kernel.  A token that is not a number reaches no token before it."""
     gen = torch.Generator().manual_seed(d + dv + heads)
     C, cuts, slots, eps = 2 * kv_heads * d + heads * dv, [[97, 16, 1, 60], [48, 33, 31, 80]], [3, 0, 4, 1], 1e-5
     m = {"heads": heads, "kv_heads": kv_heads, "dim": d, "vdim": dv}
     w = {"taps": torch.randn(C, taps, generator=gen) * 0.5, "A_log": torch.log(0.02 + 8 * torch.rand(heads, generator=gen)),
          "dt_bias": torch.randn(heads * d, generator=gen) - 3, "norm": 1 + 0.1 * torch.randn(dv, generator=gen)}
     lengths = [a + b for a, b in zip(*cuts)]
-    projs = [torch.randn(L, C + heads, generator=gen) for L in lengths]
+    projs = [torch.randn(L, C + heads, generator=gen).to(dtype) for L in lengths]
     inners = [torch.randn(L, heads * (d + dv), generator=gen) for L in lengths]
     inners[0][20:22, :heads * d] = 400.0            # decays of zero inside a chunk
     inners[1][:, :d // 2] = -60.0                   # half of a head's channels keep everything
     wide = {n: t.double() for n, t in w.items()}
-    want = [delta_by_token(p.double(), i.double(), wide, m, eps) for p, i in zip(projs, inners)]
+    want = [delta_by_token(p.double(), i.double(), wide, m, eps, dtype) for p, i in zip(projs, inners)]
     dev = {n: t.cuda() for n, t in w.items()}
     ints = lambda *x: torch.tensor(x, dtype=torch.int32, device="cuda")
 
-    def run(in_chunks):
+    def run(in_chunks, projs=projs):
         state = torch.zeros(6, heads, d, dv, device="cuda")
         state[2] = 7.0                              # a slot of somebody else: must stay as it is
         conv_state = torch.zeros(6, taps - 1, C, device="cuda") if taps > 1 else None
@@ -131,7 +134,7 @@ def test_delta_rule_in_chunks_of_tokens(d, dv, heads, kv_heads, taps):
             for n in lens:
                 cu.append(cu[-1] + n)
             piece = lambda all_: torch.cat([x[o:o + n] for x, o, n in zip(all_, at, lens)]).cuda()
-            out = torch.empty(cu[-1], heads * dv, device="cuda")
+            out = torch.empty(cu[-1], heads * dv, dtype=dtype, device="cuda")
             ops.delta_rule(piece(projs), piece(inners), dev["taps"], dev["A_log"], dev["dt_bias"], dev["norm"], conv_state, state, out,
                            ints(*cu), ints(*[s for s, n in enumerate(lens) for _ in range(n)]), ints(*slots), n_seqs=len(lens),
                            heads=heads, kv_heads=kv_heads, d=d, dv=dv, eps=eps, unit_eps=1e-6, in_chunks=in_chunks)
@@ -139,13 +142,25 @@ def test_delta_rule_in_chunks_of_tokens(d, dv, heads, kv_heads, taps):
                 got[s].append(out[cu[s]:cu[s + 1]].cpu())
                 at[s] += n
         assert at == lengths and bool((state[2] == 7.0).all())
-        pieces = [(torch.cat(g).double(), state[slot].cpu().double()) for g, slot in zip(got, slots)]
-        return [float((a - b).norm() / b.norm()) for p, q in zip(pieces, want) for a, b in zip(p, q)]
+        return [torch.cat(g).double() for g in got], [state[slot].cpu().double() for slot in slots]
+
+    def off(got, of):
+        return [float((a - b).norm() / b.norm()) for p, q in zip(got, of) for a, b in zip(p, q)]
 
     assert ops.delta_chunk_floats(sum(cuts[0]), 4, heads, d, dv, 1) > 0
-    chunked, single = run(True), run(False)
-    assert max(chunked) < 5e-6 and max(single) < 5e-6      # sums of a hundred products of 2^-24 each
-    assert sum(chunked) <= 1.25 * sum(single)
+    chunked, single, exact = run(True), run(False), tuple(zip(*want))
+    if dtype == torch.float32:
+        assert max(off(chunked, exact)) < 5e-6 and max(off(single, exact)) < 5e-6      # sums of a hundred products of 2^-24 each
+        assert sum(off(chunked, exact)) <= 1.25 * sum(off(single, exact))
+    else:
+        # a rounding of the output (2^-9); before it the two forms work on the same rounded inputs in fp32, which differ from the
+        # 64-bit ones where a convolution lies at the middle of two bf16 numbers: about one in 10,000, by 2^-8
+        assert max(off(chunked, exact)) < 2.0 ** -9 + 3e-4
+        assert max(off(chunked[1:], single[1:])) < 1e-5 and max(off(chunked[:1], single[:1])) < 3e-4
+    broken = [p.clone() for p in projs]
+    broken[0][40, :C] = math.nan                    # in the middle of a chunk
+    got = run(True, broken)[0][0]
+    assert bool(torch.equal(got[:40], chunked[0][0][:40])) and not bool(torch.isfinite(got[40:]).any())
 
 
 def test_float32_delta_rule_depends_on_neither_the_batch_nor_the_cut():
@@ -318,6 +333,22 @@ def test_prefill_then_long_decoding_over_page_borders(case, dtype, tmp_path_fact
     slot = cache.alloc()
     rows = [model.step(cache, [slot], [[t]], "last") for t in tokens[:12]]
     close(torch.cat(rows), expected(case, tokens)[:12], dtype, f"{case} from the first token", routed(case))
+
+
+def test_bf16_model_whose_prompts_go_in_chunks(tmp_path):
+    """Heads of 64 and of 128: a prompt and a portion long enough for chunks of 16 tokens, single tokens between them."""
+    cfg = plain.model_config(53, 32, 1e-6, [plain.delta_layer(2, 1, 64, 36, 4, None), plain.delta_layer(1, 1, 128, 20, 3, None)])
+    weights = plain.random_weights(cfg, 27)
+    assert all(ops.delta_chunk_floats(n, 1, h, d, v) > 0 for n in (150, 95) for h, d, v in ((2, 64, 36), (1, 128, 20)))
+    model = odi.load_resident_model(write_model_folder(tmp_path / "model", cfg, weights), dtype="bfloat16")
+    tokens = plain.random_prompts(cfg, [275], 12)[0]
+    want = plain.forward(cfg, plain.widened(weights), tokens).float()
+    cache = model.make_cache(max_tokens=320, max_seqs=1)
+    slot = cache.alloc()
+    rows = [model.step(cache, [slot], [tokens[:150]], "all")]
+    rows += [model.step(cache, [slot], [[t]], "last") for t in tokens[150:180]]
+    rows.append(model.step(cache, [slot], [tokens[180:]], "all"))
+    close(torch.cat(rows), want, "bfloat16", "a prompt in chunks, single tokens, a portion", False)
 
 
 @pytest.mark.parametrize("dtype", DTYPES)

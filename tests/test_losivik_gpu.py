@@ -280,8 +280,9 @@ def test_state_space_mixer_over_cut_sequences(dtype, heads, P, N, G, taps, parts
                                                                            else dict(atol=3e-2, rtol=3e-2)))
 
 
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("heads,P,N,G,taps,parts", [(4, 64, 128, 2, 4, 1), (3, 20, 64, 1, 1, 3), (2, 100, 192, 2, 2, 1)])
-def test_state_space_scan_in_chunks_of_tokens(heads, P, N, G, taps, parts):
+def test_state_space_scan_in_chunks_of_tokens(dtype, heads, P, N, G, taps, parts):
     """Runs around the chunks' edges, one of a single token among them, continued by a second step, with decays down to
     those that wipe the state; against the recurrence over each whole sequence, and no further off than the token by token
     kernel.  A token that is not a number reaches no token before it."""
@@ -289,7 +290,7 @@ def test_state_space_scan_in_chunks_of_tokens(heads, P, N, G, taps, parts):
     inner, C = heads * P, heads * P + 2 * G * N
     M, slots, cuts = inner + C + heads, [3, 0, 4, 1], [[890, 64, 1, 70], [63, 129, 800, 75]]
     lengths = [a + b for a, b in zip(*cuts)]
-    projs = [torch.randn(L, M, generator=gen) for L in lengths]
+    projs = [torch.randn(L, M, generator=gen).to(dtype) for L in lengths]
     projs[0][40:42, -heads:] = 300.0             # the state is wiped inside a chunk
     w = {"in": torch.eye(M, dtype=torch.float64), "o": torch.eye(inner, dtype=torch.float64),
          "conv": torch.randn(C, taps, generator=gen) * 0.5, "conv.b": torch.randn(C, generator=gen) * 0.1,
@@ -308,7 +309,7 @@ def test_state_space_scan_in_chunks_of_tokens(heads, P, N, G, taps, parts):
             cu = [0]
             for n in lens:
                 cu.append(cu[-1] + n)
-            out = torch.empty(cu[-1], inner, device="cuda")
+            out = torch.empty(cu[-1], inner, dtype=dtype, device="cuda")
             ops.ssd_mix(torch.cat([x[o:o + n] for x, o, n in zip(projs, at, lens)]).cuda(), dev["conv"], dev["conv.b"], dev["dt_bias"],
                         dev["A_log"], dev["D"], dev["norm"], conv_state, state, out, ints(*cu),
                         ints(*[s for s, n in enumerate(lens) for _ in range(n)]), ints(*slots), n_seqs=len(lens), heads=heads, head_dim=P,
@@ -322,8 +323,9 @@ def test_state_space_scan_in_chunks_of_tokens(heads, P, N, G, taps, parts):
     off = lambda got: [float((a - b).norm() / b.norm()) for a, b in zip(got, want)]
     assert ops.ssd_chunk_floats(sum(cuts[0]), 4, heads, P, N, G) > 0
     (chunked, state), (single, state_single) = run(projs, True), run(projs, False)
-    assert max(off(chunked)) < 5e-6 and max(off(single)) < 5e-6      # sums of a few hundred products of 2^-24 each
-    assert sum(off(chunked)) <= 1.25 * sum(off(single))
+    rounding = 0.0 if dtype == torch.float32 else 2.0 ** -9      # of the output; all before it is fp32 in both
+    assert max(off(chunked)) < rounding + 5e-6 and max(off(single)) < rounding + 5e-6      # sums of a few hundred products of 2^-24 each
+    assert sum(off(chunked)) <= (1.25 if dtype == torch.float32 else 1.01) * sum(off(single))
     torch.testing.assert_close(state, state_single, atol=2e-5, rtol=2e-5)
     broken = [p.clone() for p in projs]
     broken[0][100, inner:] = math.nan      # in the middle of a chunk
@@ -760,6 +762,24 @@ def test_command_line_writes_a_random_model_and_generates_from_it(tmp_path):
         assert float(logits.max() - logits[token]) < 1e-4
         ids.append(token)
     assert len(ids) == 9
+
+
+def test_bf16_model_whose_prompts_go_in_chunks(tmp_path):
+    """States of 64 rows: a prompt long enough for the scan in chunks of 64 tokens, then single tokens and a portion."""
+    cfg = plain._config(120, 64, [
+        {"type": "parallel", "mixer": plain._pair(4, 2, 16, 32, 0.25, 30, 70, 4, 20, 64, 2, 4, 1), "mlp": plain._dense(48, 1.2)},
+        {"type": "parallel", "mixer": plain._pair(2, 1, 32, 16, 0.18, 129, 1, 2, 64, 128, 1, 2, 1), "mlp": None}])
+    weights = plain.random_weights(cfg, 312)
+    assert ops.ssd_chunk_floats(1100, 1, 4, 20, 64, 2) > 0 and ops.ssd_chunk_floats(1100, 1, 2, 64, 128, 1) > 0
+    model = odi.load_resident_model(write_model_folder(tmp_path / "model", cfg, weights), dtype="bfloat16")
+    tokens = plain.random_prompts(cfg, [1150], 12)[0]
+    want = plain.forward(cfg, weights, tokens).float()
+    cache = model.make_cache(max_tokens=1216, max_seqs=1)
+    slot = cache.alloc()
+    rows = [model.step(cache, [slot], [tokens[:1100]], "all")]
+    rows += [model.step(cache, [slot], [[t]], "last") for t in tokens[1100:1130]]
+    rows.append(model.step(cache, [slot], [tokens[1130:]], "all"))
+    close(torch.cat(rows), want, "bfloat16", "a prompt in chunks, single tokens, a portion", flips=False)
 
 
 @pytest.mark.parametrize("dtype", DTYPES)

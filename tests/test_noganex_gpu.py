@@ -391,15 +391,17 @@ def test_delta_rule_over_cut_sequences(dtype, heads, kv_heads, d, dv, taps):
                                                                            else dict(atol=4e-2, rtol=2e-2)))
 
 
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("heads,kv_heads,d,dv,taps", [(4, 2, 64, 64, 4), (3, 3, 64, 20, 1), (2, 1, 128, 100, 3), (2, 2, 128, 128, 4)])
-def test_delta_rule_in_chunks_of_tokens(heads, kv_heads, d, dv, taps):
+def test_delta_rule_in_chunks_of_tokens(dtype, heads, kv_heads, d, dv, taps):
     """Runs around the chunks' edges, one of a single token among them, continued by a second step, with decays from one to
-    those that wipe the state; against the recurrence in 64 bits, and no further off than four tokens at a time."""
+    those that wipe the state; against the recurrence in 64 bits, and no further off than four tokens at a time.  A token that is
+    not a number reaches no token before it."""
     gen = torch.Generator().manual_seed(heads * d + dv)
     v = heads * dv
     C, cuts, slots = 2 * kv_heads * d + v, [[691, 16, 1, 80], [64, 97, 63, 545]], [3, 0, 4, 1]
     lengths = [a + b for a, b in zip(*cuts)]
-    projs = [torch.randn(L, C + v, generator=gen) for L in lengths]
+    projs = [torch.randn(L, C + v, generator=gen).to(dtype) for L in lengths]
     abs_ = [torch.randn(L, 2 * heads, generator=gen) for L in lengths]
     abs_[0][20:22, 0] = 500.0                    # wiped inside a chunk
     abs_[1][:, 0] = -80.0                        # no decay at all
@@ -412,7 +414,7 @@ def test_delta_rule_in_chunks_of_tokens(heads, kv_heads, d, dv, taps):
     dev = {k: t.float().cuda() for k, t in w.items()}
     dev["taps"] = dev["taps"].t().contiguous()
 
-    def run(in_chunks):
+    def run(in_chunks, projs=projs):
         state = torch.zeros(6, heads, d, dv, device="cuda")
         state[2].fill_(7.0)                      # a slot of somebody else: must stay as it is
         conv_state = torch.zeros(6, taps - 1, C, device="cuda") if taps > 1 else None
@@ -422,7 +424,7 @@ def test_delta_rule_in_chunks_of_tokens(heads, kv_heads, d, dv, taps):
             for n in lens:
                 cu.append(cu[-1] + n)
             piece = lambda all_: torch.cat([x[o:o + n] for x, o, n in zip(all_, at, lens)]).cuda()
-            out = torch.empty(cu[-1], v, device="cuda")
+            out = torch.empty(cu[-1], v, dtype=dtype, device="cuda")
             ops.head_delta(piece(projs), piece(abs_), dev["taps"], dev["A_log"], dev["dt_bias"], dev["norm"], conv_state, state, out,
                            ints(*cu), ints(*[s for s, n in enumerate(lens) for _ in range(n)]), ints(*slots), n_seqs=len(lens),
                            max_q_len=max(lens), heads=heads, kv_heads=kv_heads, d=d, dv=dv, eps=1e-5, unit_eps=1e-6,
@@ -431,13 +433,20 @@ def test_delta_rule_in_chunks_of_tokens(heads, kv_heads, d, dv, taps):
                 got[s].append(out[cu[s]:cu[s + 1]].cpu().double())
                 at[s] += n
         assert at == lengths and bool((state[2] == 7.0).all())
-        return [float((torch.cat(g) - x).norm() / x.norm()) for g, x in zip(got, want)], state
+        return [torch.cat(g) for g in got], state
+
+    off = lambda got: [float((a - b).norm() / b.norm()) for a, b in zip(got, want)]
 
     assert ops.head_delta_chunk_floats(sum(cuts[0]), 4, max(cuts[0]), heads, d, dv, 1) > 0
     (chunked, state), (fours, state_fours) = run(True), run(False)
-    assert max(chunked) < 5e-6 and max(fours) < 5e-6      # sums of a hundred products of 2^-24 each
-    assert sum(chunked) <= 1.25 * sum(fours)
+    rounding = 0.0 if dtype == torch.float32 else 2.0 ** -9      # of the output; all before it is fp32 in both
+    assert max(off(chunked)) < rounding + 5e-6 and max(off(fours)) < rounding + 5e-6      # sums of a hundred products of 2^-24 each
+    assert sum(off(chunked)) <= (1.25 if dtype == torch.float32 else 1.01) * sum(off(fours))
     torch.testing.assert_close(state, state_fours, atol=2e-5, rtol=2e-5)
+    broken = [p.clone() for p in projs]
+    broken[0][100, :C] = math.nan                # in the middle of a chunk
+    got = run(True, broken)[0][0]
+    assert bool(torch.equal(got[:100], chunked[0][:100])) and not bool(torch.isfinite(got[100:]).any())
 
 
 @pytest.mark.parametrize("d", [64, 128])
@@ -734,6 +743,22 @@ def test_command_line_writes_a_random_model_and_generates_from_it(tmp_path):
         assert float(logits.max() - logits[token]) < 1e-4
         ids.append(token)
     assert len(ids) == 9
+
+
+def test_bf16_model_whose_prompts_go_in_chunks(tmp_path):
+    """Heads of 64 and of 128: a prompt and a portion long enough for chunks of 16 tokens, single tokens between them."""
+    cfg = plain._config(97, 64, [(plain._delta(2, 1, 64, 36, 4), plain._dense(48), None), (plain._delta(1, 1, 128, 20, 3), None, None)])
+    weights = plain.random_weights(cfg, 313)
+    assert all(ops.head_delta_chunk_floats(n, 1, n, h, d, v) > 0 for n in (240, 235) for h, d, v in ((2, 64, 36), (1, 128, 20)))
+    model = odi.load_resident_model(write_model_folder(tmp_path / "model", cfg, weights), dtype="bfloat16")
+    tokens = plain.random_prompts(cfg, [505], 12)[0]
+    want = plain.forward(cfg, weights, tokens).float()
+    cache = model.make_cache(max_tokens=512, max_seqs=1)
+    slot = cache.alloc()
+    rows = [model.step(cache, [slot], [tokens[:240]], "all")]
+    rows += [model.step(cache, [slot], [[t]], "last") for t in tokens[240:270]]
+    rows.append(model.step(cache, [slot], [tokens[270:]], "all"))
+    close(torch.cat(rows), want, "bfloat16", "a prompt in chunks, single tokens, a portion", flips=False)
 
 
 @pytest.mark.parametrize("dtype", DTYPES)
