@@ -18,8 +18,8 @@
 // Everything is fp32, as token by token.  A last chunk of fewer tokens is filled with tokens that do nothing (k, q, v
 // and beta 0, g 1).
 //
-// What bounds it: the scan's chain of latencies (1.25 us a chunk of one sequence, a quarter of which is instruction issue);
-// with many sequences its reads of shared memory.  The scratch has a slot per chunk (run_chunks.cuh).
+// What bounds it: the scan's chain of latencies (1.5 us a chunk of one sequence with heads of 64, 1.9 with heads of 128, a third or
+// more of it instruction issue); with many sequences its reads of shared memory.  The scratch has a slot per chunk (run_chunks.cuh).
 #pragma once
 #include "run_chunks.cuh"
 

@@ -350,9 +350,9 @@ ssd_scan_kernel(SsdArgs a) {
 //  pass     per element of S: E of every chunk gives way to the state before it;
 //  outputs  every chunk and head at once: y.
 // The products of decays are rounded once (DecayProduct); all else is plain fp32 multiply-adds, as token by token, where a
-// sequence's tokens were one chain of them.  The mixer between its products, 32 heads of 128 x 64, us (in chunks, token by token): 2,048 tokens 187, 564; 2 x 1,024 183, 350; 8 x 1,000 715, 961;
-// 512 79, 152; 128 63, 60.  What bounds outputs (66 us of those 187) and states (54) is shared memory: three 16-byte reads per 32
-// multiply-adds of a thread.
+// sequence's tokens were one chain of them.  The mixer between its products, 32 heads of 128 x 64, us (in chunks, token by token):
+// 2,048 tokens 187, 564; 2 x 1,024 183, 350; 8 x 1,000 715, 961; 512 79, 152; 128 63, 60.  What bounds outputs (66 us of those 187)
+// and states (54) is shared memory: three 16-byte reads per 32 multiply-adds of a thread.
 #define SSD_L 64
 
 // dt_t and a_t of the chunk's tokens into shared memory; tokens behind the run's end have dt 0, a 1
