@@ -145,10 +145,13 @@ def write_tokens(pinned: torch.Tensor, view: np.ndarray, n: int, tokens) -> None
     """The ``n`` tokens of a step into pinned memory (``view``: the same as a numpy array).  Plain numbers go there without a
     tensor on the way, since the GPU waits for this; whatever else ``torch.as_tensor`` takes goes by it, and what it refuses it
     refuses."""
-    if isinstance(tokens, (list, tuple)) and len(tokens) == n and all(type(t) is int and 0 <= t <= 0x7fffffff for t in tokens):
-        view[:n] = tokens
-    else:
-        pinned[:n] = torch.as_tensor(tokens, dtype=torch.int32)
+    if isinstance(tokens, (list, tuple)) and len(tokens) == n and set(map(type, tokens)) == {int}:
+        try:
+            view[:n] = tokens
+            return
+        except OverflowError:      # refused below
+            pass
+    pinned[:n] = torch.as_tensor(tokens, dtype=torch.int32)
 
 
 class DecodeRunner:
