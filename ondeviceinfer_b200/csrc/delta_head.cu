@@ -655,14 +655,21 @@ hd_parts_kernel(HeadDeltaArgs a, DeltaChunkArgs c) {
   const size_t tok = (size_t)a.cu_q[seq] + first;
   const float* qk = a.qk + (tok * a.kv_heads + kvh) * 2 * D;
   const float decay = (int)threadIdx.x < nt ? a.gb[((tok + threadIdx.x) * a.heads + h) * 2] : 1.f;      // nt <= DC
-  for (int x = threadIdx.x; x < DC * D; x += blockDim.x) {
-    const int t = x / D, i = x % D;
-    const bool in = t < nt;
+  float qv[DC / 2], kv[DC / 2];
+#pragma unroll
+  for (int j = 0; j < DC / 2; ++j) {
+    const int t = 2 * j + (int)threadIdx.x / D, i = threadIdx.x % D;
     const float* row = qk + (size_t)t * a.kv_heads * 2 * D;
-    sh.q[t][i] = in ? row[i] : 0.f;
-    sh.k[t][i] = in ? row[D + i] : 0.f;
+    qv[j] = t < nt ? row[i] : 0.f;
+    kv[j] = t < nt ? row[D + i] : 0.f;
   }
-  if (threadIdx.x < 32) dc_head_decays(sh, decay);
+  if (threadIdx.x < 32) dc_head_decays(sh, decay);      // while those are on their way
+#pragma unroll
+  for (int j = 0; j < DC / 2; ++j) {
+    const int t = 2 * j + (int)threadIdx.x / D, i = threadIdx.x % D;
+    sh.q[t][i] = qv[j];
+    sh.k[t][i] = kv[j];
+  }
   if (threadIdx.x < DC) sh.beta[threadIdx.x] = (int)threadIdx.x < nt ? a.gb[((tok + threadIdx.x) * a.heads + h) * 2 + 1] : 0.f;
   __syncthreads();
   const float* v = a.o + (tok * a.heads + h) * a.dv;
