@@ -27,29 +27,30 @@ __device__ __forceinline__ void fma_pair(unsigned long long& acc, unsigned long 
   asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(a), "l"(w));
 }
 
-// ROWS rows of X [limit, K] from row r0 on, k0 .. k0 + KS - 1, into dst (pitch PITCH); zeros beyond either end, but nothing
+// ROWS rows of X [limit, K] from row r0 on, k0 .. k0 + KS - 1, into dst (pitch PITCH); zeros beyond either end, TAIL: but nothing
 // where the last stage has no k left to multiply
-template <int ROWS, bool VEC>
+template <int ROWS, bool VEC, bool TAIL>
 __device__ __forceinline__ void stage_rows(uint32_t dst, const float* __restrict__ X, int r0, int limit, int k0, int K, int ld) {
   const int left = K - k0 + (K & 1);      // k in pairs
   if (VEC) {
     for (int i = threadIdx.x; i < ROWS * (KS / 4); i += NTH) {
       const int r = i / (KS / 4), k = (i % (KS / 4)) * 4;
-      if (k >= left) continue;
+      if (TAIL && k >= left) continue;
       const bool ok = r0 + r < limit && k0 + k < K;
       cp_async16(dst + (r * PITCH + k) * 4, ok ? X + (size_t)(r0 + r) * ld + k0 + k : X, ok);
     }
   } else {
     for (int i = threadIdx.x; i < ROWS * KS; i += NTH) {
       const int r = i / KS, k = i % KS;
-      if (k >= left) continue;
+      if (TAIL && k >= left) continue;
       const bool ok = r0 + r < limit && k0 + k < K;
       cp_async4(dst + (r * PITCH + k) * 4, ok ? X + (size_t)(r0 + r) * ld + k0 + k : X, ok);
     }
   }
 }
 
-template <int RM, int RN, int STAGES, bool VEC>
+// TAIL: K may be no multiple of KS
+template <int RM, int RN, int STAGES, bool VEC, bool TAIL>
 __global__ void __launch_bounds__(NTH)
 gemm_f32_kernel(const float* __restrict__ A, const float* __restrict__ W, float* C,
                 const float* R, const float* __restrict__ bias, int M, int N, int K, int lda, int ldw, int ldc, int ldr) {
@@ -65,8 +66,8 @@ gemm_f32_kernel(const float* __restrict__ A, const float* __restrict__ W, float*
   auto issue = [&](int s) {
     if (s < n_stages) {
       const uint32_t dst = base + (s % STAGES) * STAGE * 4;
-      stage_rows<BM, VEC>(dst, A, m0, M, s * KS, K, lda);
-      stage_rows<BN, VEC>(dst + BM * PITCH * 4, W, n0, N, s * KS, K, ldw);
+      stage_rows<BM, VEC, TAIL>(dst, A, m0, M, s * KS, K, lda);
+      stage_rows<BN, VEC, TAIL>(dst + BM * PITCH * 4, W, n0, N, s * KS, K, ldw);
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
   };
@@ -92,7 +93,7 @@ gemm_f32_kernel(const float* __restrict__ A, const float* __restrict__ W, float*
   asm volatile("cp.async.wait_group %0;" ::"n"(STAGES - 1) : "memory");
   __syncthreads();
   read(0, 0, 0);
-  const int full = K / KS;
+  const int full = TAIL ? K / KS : n_stages;
   for (int s = 0; s < full; ++s) {
 #pragma unroll
     for (int k = 0; k < KS; k += 2) {
@@ -111,14 +112,15 @@ gemm_f32_kernel(const float* __restrict__ A, const float* __restrict__ W, float*
         for (int j = 0; j < RN; ++j) fma_pair(acc[i][j], a[set][i], w[set][j]);
     }
   }
-  // the k that fill no stage, if any: the first two are read already
+  if (TAIL) {      // the k that fill no stage, if any: the first two are read already
 #pragma unroll 1
-  for (int k = 0; k < K - full * KS; k += 2) {
-    if (k > 0) read(0, full, k);
+    for (int k = 0; k < K - full * KS; k += 2) {
+      if (k > 0) read(0, full, k);
 #pragma unroll
-    for (int i = 0; i < RM; ++i)
+      for (int i = 0; i < RM; ++i)
 #pragma unroll
-      for (int j = 0; j < RN; ++j) fma_pair(acc[i][j], a[0][i], w[0][j]);
+        for (int j = 0; j < RN; ++j) fma_pair(acc[i][j], a[0][i], w[0][j]);
+    }
   }
   pdl_launch_dependents();      // not earlier: blocks of the next kernel would take the places of this one's
 #pragma unroll
@@ -137,7 +139,7 @@ gemm_f32_kernel(const float* __restrict__ A, const float* __restrict__ W, float*
   }
 }
 
-template <int RM, int RN, int STAGES, bool VEC>
+template <int RM, int RN, int STAGES, bool VEC, bool TAIL>
 static int launch_form(const float* A, const float* W, float* C, const float* R, const float* bias, int M, int N, int K,
                        int lda, int ldw, int ldc, int ldr, cudaStream_t stream) {
   constexpr size_t smem = sizeof(float) * STAGES * (8 * RM + 16 * RN) * PITCH;
@@ -145,10 +147,10 @@ static int launch_form(const float* A, const float* W, float* C, const float* R,
   if (tiles > 0x7fffffffL) return ODI_ERR_UNSUPPORTED;
   const dim3 grid((unsigned)tiles);
   if (smem > 48 * 1024) {
-    const cudaError_t e = cudaFuncSetAttribute(gemm_f32_kernel<RM, RN, STAGES, VEC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    const cudaError_t e = cudaFuncSetAttribute(gemm_f32_kernel<RM, RN, STAGES, VEC, TAIL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return (int)e;
   }
-  odi_rc = launch_pdl((gemm_f32_kernel<RM, RN, STAGES, VEC>), grid, dim3(NTH), smem, stream, A, W, C, R, bias, M, N, K, lda, ldw, ldc, ldr);
+  odi_rc = launch_pdl((gemm_f32_kernel<RM, RN, STAGES, VEC, TAIL>), grid, dim3(NTH), smem, stream, A, W, C, R, bias, M, N, K, lda, ldw, ldc, ldr);
   return launch_status();
 }
 
@@ -205,8 +207,11 @@ extern "C" int odi_gemm_f32(const float* A, const float* W, float* C, const floa
                    ((uintptr_t)A % 16 == 0) && ((uintptr_t)W % 16 == 0);
   const bool forced = force >= 0 && force < F32_FORMS;
   const int form = forced ? force : vec ? pick_form(M, N) : 0;
-#define ODI_F32(RM, RN, STAGES) launch_form<RM, RN, STAGES, true>(A, W, C, R, bias, M, N, K, lda, ldw, ldc, ldr, stream)
-#define ODI_F32_SCALAR(RM, RN) launch_form<RM, RN, 3, false>(A, W, C, R, bias, M, N, K, lda, ldw, ldc, ldr, stream)
+  // a loop of its own for whole stages: with the tail behind it the same one took 2.4 % longer (185 x 24,576 x 4,096)
+#define ODI_F32(RM, RN, STAGES) \
+  (K % KS == 0 ? launch_form<RM, RN, STAGES, true, false>(A, W, C, R, bias, M, N, K, lda, ldw, ldc, ldr, stream) \
+               : launch_form<RM, RN, STAGES, true, true>(A, W, C, R, bias, M, N, K, lda, ldw, ldc, ldr, stream))
+#define ODI_F32_SCALAR(RM, RN) launch_form<RM, RN, 3, false, true>(A, W, C, R, bias, M, N, K, lda, ldw, ldc, ldr, stream)
   if (!vec) {
     const int tile = forced ? (form < 4 ? 0 : form < 6 ? 1 : 2) : pick_scalar(M, N);
     return tile == 0 ? ODI_F32_SCALAR(2, 4) : tile == 1 ? ODI_F32_SCALAR(4, 4) : ODI_F32_SCALAR(8, 8);
