@@ -49,7 +49,7 @@ __device__ __forceinline__ void stage_rows(uint32_t dst, const float* __restrict
   }
 }
 
-// TAIL: K may be no multiple of KS
+// TAIL: the k that fill no stage go behind the loop, else they are one more stage, filled with zeros
 template <int RM, int RN, int STAGES, bool VEC, bool TAIL>
 __global__ void __launch_bounds__(NTH)
 gemm_f32_kernel(const float* __restrict__ A, const float* __restrict__ W, float* C,
@@ -183,7 +183,7 @@ static int pick_form(int M, int N) {
 // tiles, then of c tiles a multiprocessor the larger of `one` and start + c more.  (By the rule of the forms above 1,024 x 300 x 50
 // took 9.3 us where the 64 x 64 tile of before took 6.5, and takes 5.9 now; 300 x 1,000 x 333 34 and 26, now 22.)
 struct F32Scalar { int rows, cols; double few, one, start, more; };
-static const F32Scalar scalar_forms[] = {{16, 64, 42.4, 42.4, 9, 18.2}, {32, 64, 42.2, 42.2, 12, 24.2}, {64, 128, 91, 123, 0, 77}};
+static const F32Scalar scalar_forms[] = {{16, 64, 42.4, 42.4, 9, 18.2}, {32, 64, 42.5, 42.5, 12, 24.2}, {64, 128, 91, 123, 0, 77}};
 static int pick_scalar(int M, int N) {
   int best = 0;
   double least = 1e300;
@@ -207,11 +207,15 @@ extern "C" int odi_gemm_f32(const float* A, const float* W, float* C, const floa
                    ((uintptr_t)A % 16 == 0) && ((uintptr_t)W % 16 == 0);
   const bool forced = force >= 0 && force < F32_FORMS;
   const int form = forced ? force : vec ? pick_form(M, N) : 0;
-  // a loop of its own for whole stages: with the tail behind it the same one took 2.4 % longer (185 x 24,576 x 4,096)
+  // the tail only for a few k: elsewhere the loop with it takes longer than the zeros of the last stage that it saves (185 x 24,576 x 4,096
+  // 2.4 %, 1,024 x 64 x 1,001 50 us against 42; but 4,096 x 2,048 x 10 19 against 31)
+  const bool tail = K <= 40 && K % KS != 0;
 #define ODI_F32(RM, RN, STAGES) \
-  (K % KS == 0 ? launch_form<RM, RN, STAGES, true, false>(A, W, C, R, bias, M, N, K, lda, ldw, ldc, ldr, stream) \
-               : launch_form<RM, RN, STAGES, true, true>(A, W, C, R, bias, M, N, K, lda, ldw, ldc, ldr, stream))
-#define ODI_F32_SCALAR(RM, RN) launch_form<RM, RN, 3, false, true>(A, W, C, R, bias, M, N, K, lda, ldw, ldc, ldr, stream)
+  (tail ? launch_form<RM, RN, STAGES, true, true>(A, W, C, R, bias, M, N, K, lda, ldw, ldc, ldr, stream) \
+        : launch_form<RM, RN, STAGES, true, false>(A, W, C, R, bias, M, N, K, lda, ldw, ldc, ldr, stream))
+#define ODI_F32_SCALAR(RM, RN) \
+  (tail ? launch_form<RM, RN, 3, false, true>(A, W, C, R, bias, M, N, K, lda, ldw, ldc, ldr, stream) \
+        : launch_form<RM, RN, 3, false, false>(A, W, C, R, bias, M, N, K, lda, ldw, ldc, ldr, stream))
   if (!vec) {
     const int tile = forced ? (form < 4 ? 0 : form < 6 ? 1 : 2) : pick_scalar(M, N);
     return tile == 0 ? ODI_F32_SCALAR(2, 4) : tile == 1 ? ODI_F32_SCALAR(4, 4) : ODI_F32_SCALAR(8, 8);
