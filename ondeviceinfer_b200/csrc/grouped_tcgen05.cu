@@ -28,6 +28,7 @@
 #define EPI_RELU2 3
 #define EPI_STORE_F32 5
 #define EPI_GATED_CLAMP 4  // g sigmoid(alpha g) (u + shift) of g <= limit, |u| <= limit
+#define EPI_RELU2_ROUNDED 6      // max(z, 0)^2 of the sum as bf16 holds it: what a product that stores bf16 and an activation behind it give
 
 #define BF 128             // weight rows per CTA
 #define BK 64              // k per stage
@@ -173,6 +174,7 @@ __device__ __forceinline__ float plain(float v) {
   if (EPI == EPI_GELU) return gelu_erf_f(v);
   if (EPI == EPI_GELU_TANH) return gelu_tanh_f(v);
   if (EPI == EPI_RELU2) { const float r = fmaxf(v, 0.f); return r * r; }
+  if (EPI == EPI_RELU2_ROUNDED) { const float r = fmaxf(__bfloat162float(__float2bfloat16_rn(v)), 0.f); return r * r; }
   return v;
 }
 
@@ -472,6 +474,7 @@ extern "C" int odi_grouped_tcgen05(const void* x, const void* w, void* out, cons
     case EPI_GELU: return launch<EPI_GELU>(mx, mw, a, pairs, stream);
     case EPI_GELU_TANH: return launch<EPI_GELU_TANH>(mx, mw, a, pairs, stream);
     case EPI_RELU2: return launch<EPI_RELU2>(mx, mw, a, pairs, stream);
+    case EPI_RELU2_ROUNDED: return launch<EPI_RELU2_ROUNDED>(mx, mw, a, pairs, stream);
     case EPI_STORE_F32: return launch<EPI_STORE_F32>(mx, mw, a, pairs, stream);
     case EPI_GATED_CLAMP: return launch<EPI_GATED_CLAMP>(mx, mw, a, pairs, stream);
   }

@@ -1318,11 +1318,11 @@ def grouped_tcgen05_ok(dtype: torch.dtype, *weights: torch.Tensor) -> bool:
 
 
 def grouped_gemm_sorted(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, offsets: torch.Tensor, *, epi: int, limit: float = 0.0,
-                        alpha: float = 1.0, up_shift: float = 1.0) -> None:
+                        alpha: float = 1.0, up_shift: float = 1.0, round_sums: bool = False) -> None:
     """Rows offsets[e] .. offsets[e + 1] - 1 of ``x`` (bf16, sorted by expert) through ``w[e]`` on the tcgen05 tensor cores, for steps
     whose experts get some dozens of rows and more (:func:`grouped_tcgen05_ok`); out [rows, features] bf16 (fp32 for ``GROUPED_STORE_F32``),
     epilogues of :func:`grouped_gemm_routed`.  ``offsets``: int32 [experts + 1] on the device; rows of ``out`` beyond the last are
-    left as they are."""
+    left as they are.  ``round_sums`` (``GROUPED_RELU2``): the activation of the sums as bfloat16 holds them."""
     _require(x, "x", torch.bfloat16, 2)
     _require(w, "w", torch.bfloat16, 3)
     _require(out, "out", torch.float32 if epi == GROUPED_STORE_F32 else torch.bfloat16, 2)
@@ -1330,14 +1330,14 @@ def grouped_gemm_sorted(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, off
     groups, w_rows, K = w.shape
     n_out = w_rows // 2 if epi == GROUPED_GATED_CLAMP else w_rows
     if (epi not in _GROUPED_TCGEN05_EPILOGUES or x.shape[1] != K or out.shape != (x.shape[0], n_out) or offsets.numel() != groups + 1
-            or (epi == GROUPED_GATED_CLAMP and w_rows % 2)):
+            or (epi == GROUPED_GATED_CLAMP and w_rows % 2) or (round_sums and epi != GROUPED_RELU2)):
         raise KernelError(f"grouped product: epilogue {epi}, x {tuple(x.shape)}, w {tuple(w.shape)}, out {tuple(out.shape)}, "
                           f"{offsets.numel()} offsets do not fit")
     _, _, status = _gemm_buffers(w.device, 0)
     lib = load_library("grouped_tcgen05")
     _check(lib.odi_grouped_tcgen05(_ptr(x), _ptr(w), _ptr(out), _ptr(offsets), c_int(x.shape[0]), c_int(groups), c_int(n_out), c_int(K),
-                                   c_int(w_rows), c_int(_GROUPED_TCGEN05_EPILOGUES[epi]), c_float(limit), c_float(alpha), c_float(up_shift),
-                                   _ptr(status), _stream()), "grouped_tcgen05")
+                                   c_int(w_rows), c_int(6 if round_sums else _GROUPED_TCGEN05_EPILOGUES[epi]), c_float(limit), c_float(alpha),
+                                   c_float(up_shift), _ptr(status), _stream()), "grouped_tcgen05")
 
 
 def moe_route(logits: torch.Tensor, correction: Optional[torch.Tensor], ids: torch.Tensor, weights: torch.Tensor, *,

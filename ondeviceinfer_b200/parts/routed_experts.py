@@ -16,7 +16,7 @@ Steps of ``forward`` (no step waits for the host):
 
 Options of the spec: experts (and the shared one) that are SiLU gates without limits, the same kernels with other
 constants; weights divided by their sum and multiplied by a constant (in the routing kernel); sigmoid scores instead of the softmax (a flag of the routing kernel); ungated experts with the
-squared ReLU (one up matrix per expert, the activation in the grouped product's epilogue); weights that multiply the experts' inputs (the rows are gathered in the
+squared ReLU (one up matrix per expert, the activation in the grouped product's epilogue, of many rows on the sums as bfloat16 holds them); weights that multiply the experts' inputs (the rows are gathered in the
 sorted order and multiplied by their pair's weight in fp32 on the way, ``ops.moe_gather``; the combine then adds
 the chosen rows unweighted).
 """
@@ -31,12 +31,15 @@ from ..config.specs import RoutedExpertsSpec
 from ..kernels import ops
 from ..weights.tensors import TensorDecl
 from .base import Part, register_part
-from .linear import activated_linear, clamped_gated_linear, gated_linear, linear
+from .linear import clamped_gated_linear, gated_linear, linear
 
 
 # From this many rows per expert on (on average) the experts of a bfloat16 step go to tcgen05 over gathered rows.  Measured, gather and both
 # products against the form that gathers in its loads (mma.sync), us, 30 experts of 2,048 and 1,024: 4 rows 77 / 71, 8 77 / 79, 16 78 / 121,
 # 32 80 / 187; 128 experts of 1,024 and 512: 4 77 / 77, 8 78 / 96, 15 79 / 142.
+# Ungated experts go there only with ROWS_PER_EXPERT_ROUNDED rows, and their sums, like the shared expert's, are rounded before the squared
+# ReLU (max(z, 0)^2 of a bfloat16 product, as an activation behind it gives): their layers weigh the experts' inputs by a router's
+# scores, and rounded once, after the activation, they moved the logits by 0.027 of their norm where two scores nearly tied.
 ROWS_PER_EXPERT_FOR_TCGEN05 = 8
 # From this many on the experts' outputs are rounded to the compute dtype (half the bytes of many rows), and experts that tcgen05 refuses run
 # one by one through linear().
@@ -122,13 +125,13 @@ class RoutedExperts(Part):
             ops.moe_group(ids, self.counts, table)
             act = torch.empty((table.n_pairs, s.expert_size), dtype=x.dtype, device=dev)
             first_epi = ops.GROUPED_GATED_CLAMP if self.gated else ops.GROUPED_RELU2
-            tcgen05 = x.dtype == torch.bfloat16 and ops.grouped_tcgen05_ok(x.dtype, self.w_gate_up, self.w_down)
             many = x.dtype == torch.bfloat16 and table.n_pairs >= ROWS_PER_EXPERT_ROUNDED * s.num_experts
-            if tcgen05 and table.n_pairs >= ROWS_PER_EXPERT_FOR_TCGEN05 * s.num_experts:
+            tcgen05 = table.n_pairs >= ROWS_PER_EXPERT_FOR_TCGEN05 * s.num_experts if self.gated else many and not torch.cuda.is_current_stream_capturing()
+            if tcgen05 and ops.grouped_tcgen05_ok(x.dtype, self.w_gate_up, self.w_down):
                 rows = torch.empty((table.n_pairs, s.hidden_size), dtype=x.dtype, device=dev)
                 ops.moe_gather(x, table, rows, weights if s.weight_on_input else None)
                 ops.grouped_gemm_sorted(rows, self.w_gate_up, act, table.offsets, epi=first_epi, limit=self.limit, alpha=self.gate_alpha,
-                                        up_shift=self.up_shift)
+                                        up_shift=self.up_shift, round_sums=not self.gated)
                 # the gathered rows were read by the first product: of many rows the outputs, of the same size, take their place
                 expert_out = rows if many else wide_out()
                 ops.grouped_gemm_sorted(act, self.w_down, expert_out, table.offsets, epi=ops.GROUPED_STORE if many else ops.GROUPED_STORE_F32)
@@ -161,7 +164,9 @@ class RoutedExperts(Part):
     def _activated(self, x, weight, limit):
         if self.gated:
             return clamped_gated_linear(x, weight, limit, self.gate_alpha, self.up_shift)
-        return activated_linear(x, weight, "relu2")
+        out = linear(x, weight)
+        ops.activation(out, out, "relu2")
+        return out
 
     def _experts_one_by_one(self, x, table, act, expert_out, weights) -> None:
         """The experts' outputs in the sorted order of pairs, into ``expert_out``."""

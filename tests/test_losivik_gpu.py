@@ -199,6 +199,54 @@ def test_router_with_sigmoid_scores_against_the_plain_choice():
         torch.testing.assert_close(weights.cpu().double(), scores, atol=1e-6, rtol=1e-6)
 
 
+# whole tiles of rows (each expert gets every token), fewer rows than tcgen05 takes, more tokens than a fused epilogue takes
+@pytest.mark.parametrize("n", [8, 64, 1024])
+def test_activations_are_of_the_products_as_bfloat16_holds_them(n):
+    """Ungated experts of many rows, their shared expert and the clamped gated feed-forward: the activation of the rounded product, bit for
+    bit; with few rows an expert the sums of the grouped product that gathers in its loads, as they are."""
+    from ondeviceinfer_b200.config.specs import ClampedGatedMLPSpec, RoutedExpertsSpec
+    from ondeviceinfer_b200.parts import Runtime, build_part
+    from ondeviceinfer_b200.parts.linear import linear
+    gen = torch.Generator().manual_seed(n)
+    H, F, E = 128, 64, 2
+    matrix = lambda *shape: (torch.randn(*shape, generator=gen) / math.sqrt(shape[-1])).bfloat16().cuda()
+    x = torch.randn(n, H, generator=gen).bfloat16().cuda()
+    runtime = Runtime(dtype=torch.bfloat16, device=torch.device("cuda"))
+    mlp = build_part(ClampedGatedMLPSpec(hidden_size=H, intermediate_size=F, prefix="", limit=1.5, alpha=1.2,
+                                         names=(("gate", "gate"), ("up", "up"), ("down", "down"))))
+    experts = build_part(RoutedExpertsSpec(hidden_size=H, expert_size=F, num_experts=E, num_identity=0, top_k=E, num_groups=1, keep_groups=1,
+                                           limit=0.0, prefix="", has_correction=False, shared_size=F, scoring="sigmoid", expert_form="relu2",
+                                           weight_on_input=True))
+    for part in (mlp, experts):
+        w = {d.name: matrix(*d.shape) for d in part.tensor_decls()}
+        part.load(type("Fetch", (), {"matrix": staticmethod(w.__getitem__), "vector": staticmethod(w.__getitem__)}), runtime)
+    act = torch.empty(n, F, dtype=torch.bfloat16, device="cuda")
+    ops.gated_clamp(linear(x, mlp.w_gate_up), act, 1.5, 1.2)
+    assert torch.equal(mlp.forward(x, None, None), linear(act, mlp.w_down, out_dtype=torch.float32))
+
+    ids, weights = torch.empty(n, E, dtype=torch.int32, device="cuda"), torch.empty(n, E, device="cuda")
+    ops.moe_route(linear(x, experts.w_router, out_dtype=torch.float32), None, ids, weights, n_groups=1, keep=1, sigmoid=True)
+    table = ops.RoutingTable(n, E, E, "cuda", tensor=ops.grouped_tensor_ok((H, F), torch.bfloat16, x, experts.w_gate_up, experts.w_down))
+    ops.moe_group(ids, experts.counts, table)
+    rows, act = (torch.empty(n * E, width, dtype=torch.bfloat16, device="cuda") for width in (H, F))
+    ops.moe_gather(x, table, rows, weights)
+    if n >= 32:
+        ops.grouped_gemm_sorted(rows, experts.w_gate_up, act, table.offsets, epi=ops.GROUPED_STORE)
+        ops.activation(act, act, "relu2")
+        out = torch.empty(n * E, H, dtype=torch.bfloat16, device="cuda")
+        ops.grouped_gemm_sorted(act, experts.w_down, out, table.offsets, epi=ops.GROUPED_STORE)
+    else:
+        ops.grouped_gemm_routed(rows, experts.w_gate_up, act, table, gather=False, epi=ops.GROUPED_RELU2)
+        out = torch.empty(n * E, H, device="cuda")
+        ops.grouped_gemm_routed(act, experts.w_down, out, table, gather=False, epi=ops.GROUPED_STORE_F32)
+    want = torch.empty(n, H, device="cuda")
+    ops.moe_combine(want, out, x, ids, None, table, assign=True)
+    shared = linear(x, experts.w_shared_gate_up)
+    ops.activation(shared, shared, "relu2")
+    linear(shared, experts.w_shared_down, residual=want)
+    assert torch.equal(experts.forward(x, None, None), want)
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("n,H,F,n_experts,top", [(1, 16, 8, 3, 2), (9, 40, 24, 5, 3), (300, 64, 32, 4, 1)])
 def test_ungated_experts_with_weights_on_their_inputs(dtype, n, H, F, n_experts, top):
