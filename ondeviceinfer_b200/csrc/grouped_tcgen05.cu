@@ -312,16 +312,17 @@ grouped_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_c
       if (ok && !warp_wait(acc_full + 8 * buf, (uint32_t)(local >> 1) & 1u, abort_ptr)) ok = false;
       tc_fence_after();
       const uint32_t src = tmem + ((uint32_t)(lane_group * 32) << 16) + buf * MAX_BN + c0;
+      // columns that hold rows: no more are loaded than are waited for, so that no load lands in registers that have another use by then
+      const int mine_cols = min(half, t.cols - c0);      // the same for the warps that exchange
       uint32_t next[16];                       // the next 16 columns: on their way while these are worked on
-      tmem_ld16(src, next);
-      for (int c = 0; c < half; c += 16) {
-        const int left = t.cols - c0 - c;      // rows of these 16
-        if (left <= 0) break;                  // the same for the warps that exchange
+      if (mine_cols > 0) tmem_ld16(src, next);
+      for (int c = 0; c < mine_cols; c += 16) {
+        const int left = mine_cols - c;        // rows of these 16 (and more)
         float v[16];
         tmem_wait16(next);
 #pragma unroll
         for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(next[i]);
-        if (c + 16 < half) tmem_ld16(src + c + 16, next);
+        if (c + 16 < mine_cols) tmem_ld16(src + c + 16, next);
         if (EPI == EPI_STORE_F32) {
           float* to = (float*)a.out + (size_t)(t.t0 + c0 + c) * a.N + n;
 #pragma unroll
@@ -375,7 +376,6 @@ grouped_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_c
           to += 2 * (size_t)a.N;
         }
       }
-      asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive_cluster(leader_empty + 8 * buf);

@@ -1,0 +1,23 @@
+"""What the tcgen05 kernels' sources have to keep and no run can show for certain (no GPU)."""
+
+import re
+from pathlib import Path
+
+import ondeviceinfer_b200
+
+CSRC = Path(ondeviceinfer_b200.__file__).parent / "csrc"
+
+
+def _code(name):
+    return re.sub(r"//[^\n]*", "", (CSRC / name).read_text())
+
+
+def test_no_load_from_tensor_memory_is_left_on_its_way():
+    """tcgen05.ld writes its registers when it likes until the wait that names them.  The grouped product's epilogue asks for 16 columns ahead:
+    it may ask for no more of them than its loop goes through and waits for, and the loop may not be left in between."""
+    text = _code("grouped_tcgen05.cu")
+    loop = re.search(r"for \(int c = 0; c < (\w+); c \+= 16\) \{(.*?)tc_fence_before\(\)", text, re.S)
+    bound, body = loop.group(1), loop.group(2)
+    loads = re.findall(r"^(.*)tmem_ld16\(src", text, re.M)
+    assert [load.strip() for load in loads] == [f"if ({bound} > 0)", f"if (c + 16 < {bound})"]
+    assert "break" not in body and body.index("tmem_wait16(next)") < body.index("tmem_ld16(")
