@@ -144,6 +144,11 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
   *abort_flag = 1;
   return false;
 }
+// The same by a whole warp, with one answer for all of its lanes, which it also rejoins: a lane that fell behind by a lap of a ring would
+// wait for a phase that has come and gone.
+__device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
+  return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag));
+}
 __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, int x, int y, uint32_t bar) {
   asm volatile(
       "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
@@ -519,12 +524,12 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
       const bool issues = elect_one();
       constexpr uint32_t idesc_s = idesc_bf16(BM, BNK, false);
       constexpr uint32_t idesc_o = idesc_bf16(BM, D, true);
-      bool ok = mbar_wait(q_full, 0, abort_ptr);
+      bool ok = warp_wait(q_full, 0, abort_ptr);
       auto issue_s = [&](int j) -> bool {
         const int b = j & 1;
         for (int g = 0; g < KH; ++g) {
           const int n = j * KH + g, s = n % KRING;
-          if (!mbar_wait(k_full + 8 * s, (uint32_t)(n / KRING) & 1u, abort_ptr)) return false;
+          if (!warp_wait(k_full + 8 * s, (uint32_t)(n / KRING) & 1u, abort_ptr)) return false;
           tc_fence_after();
           const uint32_t k_addr = smem_u32(k_smem + (size_t)s * KV_BYTES);
           if (!issues) continue;
@@ -550,11 +555,11 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
         if (j + 1 < n_tiles) ok = issue_s(j + 1);      // the next page's scores run under this page's softmax
         if (!ok) break;
         const int s = j % RING, b = j & 1;
-        if (!mbar_wait(v_full + 8 * s, (uint32_t)(j / RING) & 1u, abort_ptr)) { ok = false; break; }
+        if (!warp_wait(v_full + 8 * s, (uint32_t)(j / RING) & 1u, abort_ptr)) { ok = false; break; }
         const uint64_t dv = desc_mn_major(smem_u32(v_smem + (size_t)s * KV_BYTES));
 #pragma unroll
         for (int t = 0; t < TILES; ++t) {
-          if (!mbar_wait(p_full + 16 * t + 8 * b, (uint32_t)(j >> 1) & 1u, abort_ptr)) { ok = false; break; }
+          if (!warp_wait(p_full + 16 * t + 8 * b, (uint32_t)(j >> 1) & 1u, abort_ptr)) { ok = false; break; }
           tc_fence_after();
           if (!issues) continue;
 #pragma unroll

@@ -108,6 +108,11 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
   *abort_flag = 1;
   return false;
 }
+// The same by a whole warp, with one answer for all of its lanes, which it also rejoins: a lane that fell behind by a lap of a ring would
+// wait for a phase that has come and gone.
+__device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
+  return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag));
+}
 // A staged tile (128 rows of 128 bytes, 128-byte swizzle) to global memory: plain store, or fp32 add.
 __device__ __forceinline__ void tma_store_2d(const CUtensorMap* map, uint32_t src, int x, int y) {
   asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%2, %3}], [%1];"
@@ -401,11 +406,11 @@ gemm_prefill_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
       Segment sg;
       for (; ok && segment_of(a, pair, n_pairs, total_tiles, total_kb, local, sg); ++local) {
         const int buf = local & 1;
-        if (local >= 2 && !mbar_wait(acc_empty0 + 8 * buf, (((uint32_t)(local >> 1) & 1u) ^ 1u), abort_ptr)) { ok = false; break; }
+        if (local >= 2 && !warp_wait(acc_empty0 + 8 * buf, (((uint32_t)(local >> 1) & 1u) ^ 1u), abort_ptr)) { ok = false; break; }
         tc_fence_after();
         for (int kb = sg.kb0; kb < sg.kb1; ++kb, ++it) {
           const int s = it % STAGES;
-          if (!mbar_wait(full0 + 8 * s, (uint32_t)(it / STAGES) & 1u, abort_ptr)) { ok = false; break; }
+          if (!warp_wait(full0 + 8 * s, (uint32_t)(it / STAGES) & 1u, abort_ptr)) { ok = false; break; }
           tc_fence_after();
           const uint32_t sa = smem_u32(smem + (size_t)s * STAGE_BYTES);
           const uint64_t da = smem_desc_k_sw128(sa), db = smem_desc_k_sw128(sa + A_BYTES);

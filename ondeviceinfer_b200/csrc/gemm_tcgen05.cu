@@ -131,6 +131,11 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
   *abort_flag = 1;
   return false;
 }
+// The same by a whole warp, with one answer for all of its lanes, which it also rejoins: a lane that fell behind by a lap of a ring would
+// wait for a phase that has come and gone.
+__device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag, int* status, int code) {
+  return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag, status, code));
+}
 __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, int x, int y, uint32_t bar) {
   asm volatile(
       "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
@@ -388,12 +393,12 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
       const bool issues = elect_one();
       constexpr uint32_t idesc = instr_desc_bf16(BM, BN);
       // MERGE: every token tile of this CTA is ready at once (the first `ready` barrier)
-      bool ok = !MERGE || mbar_wait(ready0, 0, abort_ptr, a.status, GEMM_ERR_TIMEOUT_MMA);
+      bool ok = !MERGE || warp_wait(ready0, 0, abort_ptr, a.status, GEMM_ERR_TIMEOUT_MMA);
       for (int i = 0; i < kb_count && ok; ++i) {
         const int s = i % STAGES;
         const uint32_t phase = (uint32_t)(i / STAGES) & 1u;
-        if (!mbar_wait(full0 + 8 * s, phase, abort_ptr, a.status, GEMM_ERR_TIMEOUT_MMA) ||
-            (NORM && !mbar_wait(ready0 + 8 * s, phase, abort_ptr, a.status, GEMM_ERR_TIMEOUT_MMA))) {
+        if (!warp_wait(full0 + 8 * s, phase, abort_ptr, a.status, GEMM_ERR_TIMEOUT_MMA) ||
+            (NORM && !warp_wait(ready0 + 8 * s, phase, abort_ptr, a.status, GEMM_ERR_TIMEOUT_MMA))) {
           ok = false; break;
         }
         tc_fence_after();

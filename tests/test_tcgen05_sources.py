@@ -3,6 +3,8 @@
 import re
 from pathlib import Path
 
+import pytest
+
 import ondeviceinfer_b200
 
 CSRC = Path(ondeviceinfer_b200.__file__).parent / "csrc"
@@ -21,3 +23,20 @@ def test_no_load_from_tensor_memory_is_left_on_its_way():
     loads = re.findall(r"^(.*)tmem_ld16\(src", text, re.M)
     assert [load.strip() for load in loads] == [f"if ({bound} > 0)", f"if (c + 16 < {bound})"]
     assert "break" not in body and body.index("tmem_wait16(next)") < body.index("tmem_ld16(")
+
+
+ISSUING = [p.name for p in sorted(CSRC.glob("*.cu")) if "elect_one()" in _code(p.name)]
+
+
+@pytest.mark.parametrize("name", ISSUING)
+def test_a_warp_that_issues_waits_as_one(name):
+    """The warps that issue MMAs go through their loops whole, and the lane that issues waits for nobody: every wait there has to rejoin the
+    warp (``warp_wait``), or a lane a lap of the ring behind waits for a phase that is over and, two seconds later, ends the block."""
+    text = _code(name)
+    at = text.index("elect_one()")
+    branch = text[at:text.index("} else ", text.index("umma_commit", at))]
+    assert "warp_wait(" in branch and "mbar_wait(" not in branch
+
+
+def test_the_kernels_that_issue_are_all_here():
+    assert ISSUING == ["attention_tcgen05.cu", "gemm_f32_split.cu", "gemm_prefill_tcgen05.cu", "gemm_tcgen05.cu", "grouped_tcgen05.cu"]
