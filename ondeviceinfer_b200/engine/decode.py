@@ -66,6 +66,7 @@ class _DecodeContext(StepDescription):
     (``REPLAY_ONLY``)."""
 
     REPLAY_ONLY = ("width", "max_pages", "streams", "steps", "active", "plan_key_splits")
+    captured = True
 
     def __init__(self, cache, width: int, max_pages: int, device, longest: int) -> None:
         super().__init__()

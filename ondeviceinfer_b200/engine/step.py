@@ -49,6 +49,7 @@ class StepDescription:
     ``page_table(g)``         ``(page_start [n_seqs + 1], page_ids)`` of key/value group g;
     ``key_splits(rows)``      how a split-key decode kernel may cut the sequences' keys;
     ``memo(key, make)``       a value shared by all layers of the step (rotary tables and the like);
+    ``captured``              whether the step is one of a graph: the run before the capture has to launch what the capture will;
     ``residual_sumsq``        the note a residual product leaves for the norm that follows it;
     ``stream_copy``           ``(stream, rows)``: the stream's rows in the compute dtype, left by the block that wrote them
                               (None: nobody left any);
@@ -65,7 +66,8 @@ class StepDescription:
     INTERFACE = ("token_ids", "tok_seq", "tok_pos", "cu_q", "past", "slots", "want_rows",
                  "n_seqs", "n_tokens", "n_want", "q_lens", "past_lens", "kv_lens", "max_q_len", "max_kv_len",
                  "slot_list", "residual_sumsq", "pending_residual_add", "defers_residual_add", "stream_copy",
-                 "page_table", "key_splits", "memo")
+                 "page_table", "key_splits", "memo", "captured")
+    captured = False
 
     def __init__(self) -> None:
         self._memo: Dict[object, object] = {}

@@ -42,8 +42,14 @@ from .linear import clamped_gated_linear, gated_linear, linear
 # scores, and rounded once, after the activation, they moved the logits by 0.027 of their norm where two scores nearly tied.
 ROWS_PER_EXPERT_FOR_TCGEN05 = 8
 # From this many on the experts' outputs are rounded to the compute dtype (half the bytes of many rows), and experts that tcgen05 refuses run
-# one by one through linear().
+# one by one through linear(), which waits for the host: neither in a step of a graph, whose outputs stay fp32 at any number of rows.
 ROWS_PER_EXPERT_ROUNDED = 32
+
+
+def rounds_outputs(dtype: torch.dtype, table: "ops.RoutingTable", ctx) -> bool:
+    """Whether the experts' outputs of a step are rounded to the compute dtype before they are combined."""
+    return (dtype == torch.bfloat16 and table.n_pairs >= ROWS_PER_EXPERT_ROUNDED * table.n_experts
+            and not getattr(ctx, "captured", False) and not torch.cuda.is_current_stream_capturing())
 
 
 class RoutedExperts(Part):
@@ -125,8 +131,8 @@ class RoutedExperts(Part):
             ops.moe_group(ids, self.counts, table)
             act = torch.empty((table.n_pairs, s.expert_size), dtype=x.dtype, device=dev)
             first_epi = ops.GROUPED_GATED_CLAMP if self.gated else ops.GROUPED_RELU2
-            many = x.dtype == torch.bfloat16 and table.n_pairs >= ROWS_PER_EXPERT_ROUNDED * s.num_experts
-            tcgen05 = table.n_pairs >= ROWS_PER_EXPERT_FOR_TCGEN05 * s.num_experts if self.gated else many and not torch.cuda.is_current_stream_capturing()
+            many = rounds_outputs(x.dtype, table, ctx)
+            tcgen05 = table.n_pairs >= ROWS_PER_EXPERT_FOR_TCGEN05 * s.num_experts if self.gated else many
             if tcgen05 and ops.grouped_tcgen05_ok(x.dtype, self.w_gate_up, self.w_down):
                 rows = torch.empty((table.n_pairs, s.hidden_size), dtype=x.dtype, device=dev)
                 ops.moe_gather(x, table, rows, weights if s.weight_on_input else None)
@@ -135,7 +141,7 @@ class RoutedExperts(Part):
                 # the gathered rows were read by the first product: of many rows the outputs, of the same size, take their place
                 expert_out = rows if many else wide_out()
                 ops.grouped_gemm_sorted(act, self.w_down, expert_out, table.offsets, epi=ops.GROUPED_STORE if many else ops.GROUPED_STORE_F32)
-            elif many and not torch.cuda.is_current_stream_capturing():
+            elif many:
                 expert_out = wide_out()
                 self._experts_one_by_one(x, table, act, expert_out, weights)
             elif s.weight_on_input:

@@ -22,7 +22,7 @@ from ..kernels import ops
 from ..weights.tensors import TensorDecl
 from .base import Part, register_part
 from .linear import activated_linear, linear
-from .routed_experts import ROWS_PER_EXPERT_FOR_TCGEN05, ROWS_PER_EXPERT_ROUNDED
+from .routed_experts import ROWS_PER_EXPERT_FOR_TCGEN05, rounds_outputs
 
 GROUPED_EPILOGUE = {"gelu_erf": ops.GROUPED_GELU_ERF, "gelu_tanh": ops.GROUPED_GELU_TANH}
 
@@ -85,7 +85,7 @@ class TableExperts(Part):
             rows = torch.empty((table.n_pairs, s.hidden_size), dtype=x.dtype, device=dev)
             ops.moe_gather(x, table, rows)
             ops.grouped_gemm_sorted(rows, self.w_up, act, table.offsets, epi=GROUPED_EPILOGUE[s.activation])
-            many = table.n_pairs >= ROWS_PER_EXPERT_ROUNDED * s.num_experts
+            many = rounds_outputs(x.dtype, table, ctx)
             # the gathered rows were read by the first product: of many rows the outputs, of the same size, take their place
             expert_out = rows if many else torch.empty((table.n_pairs, s.hidden_size), dtype=torch.float32, device=dev)
             ops.grouped_gemm_sorted(act, self.w_down, expert_out, table.offsets, epi=ops.GROUPED_STORE if many else ops.GROUPED_STORE_F32)

@@ -436,6 +436,52 @@ def test_grouped_products_of_sorted_rows(rows, N, K):
     assert ops.gemm_status() == 0
 
 
+@pytest.mark.parametrize("form", ["gated_clamp", "relu2", "table"])
+def test_experts_of_a_captured_step_keep_their_outputs_in_32_bits(form):
+    """64 rows an expert, from where on the outputs of a step that is launched kernel by kernel are rounded to bf16: in a graph, and in the run
+    before its capture, their weighted sum is that of fp32 rows."""
+    from ondeviceinfer_b200.config.specs import RoutedExpertsSpec, TableExpertsSpec
+    from ondeviceinfer_b200.engine.step import StepDescription
+    from ondeviceinfer_b200.parts import Runtime, build_part
+    gen = torch.Generator().manual_seed(5)
+    n, H, F, E = 64, 128, 64, 2
+    matrix = lambda *shape: (torch.randn(*shape, generator=gen) / math.sqrt(shape[-1])).bfloat16().to(DEV)
+    x = torch.randn(n, H, generator=gen).bfloat16().to(DEV)
+    if form == "table":
+        part = build_part(TableExpertsSpec(hidden_size=H, expert_size=F, num_experts=E, top_k=E, vocab_size=3, prefix=""))
+    else:
+        part = build_part(RoutedExpertsSpec(hidden_size=H, expert_size=F, num_experts=E, num_identity=0, top_k=E, num_groups=1, keep_groups=1,
+                                            limit=1.5, prefix="", has_correction=False, expert_form=form))
+    w = {d.name: torch.tensor([[0, 1]] * 3, dtype=torch.int32, device=DEV) if "distinct" in d.init else matrix(*d.shape)
+         for d in part.tensor_decls()}
+    part.load(type("Fetch", (), {name: staticmethod(w.__getitem__) for name in ("matrix", "vector", "integer")}),
+              Runtime(dtype=torch.bfloat16, device=torch.device(DEV)))
+
+    def step(captured):
+        ctx = StepDescription()
+        ctx.captured, ctx.token_ids = captured, torch.zeros(n, dtype=torch.int32, device=DEV)
+        return ctx
+
+    seen, real = [], ops.moe_combine
+    def combine(residual, expert_out, *args, **kw):
+        seen.append(expert_out.dtype)
+        return real(residual, expert_out, *args, **kw)
+    ops.moe_combine = combine
+    try:
+        eager = part.forward(x, step(False), None)
+        before = part.forward(x, step(True), None)
+        torch.cuda.synchronize()
+        graph, ctx = torch.cuda.CUDAGraph(), step(True)
+        with torch.cuda.graph(graph):
+            replayed = part.forward(x, ctx, None)
+    finally:
+        ops.moe_combine = real
+    graph.replay()
+    torch.cuda.synchronize()
+    assert seen == [torch.bfloat16, torch.float32, torch.float32] and torch.equal(replayed, before)
+    assert not torch.equal(eager, before) and torch.allclose(eager, before, atol=0.05, rtol=0.02)
+
+
 @pytest.mark.parametrize("tokens,I,K,biased", [(1, 8, 64, False), (257, 136, 72, True), (700, 256, 520, False)])
 def test_gemm_prefill_clamps_and_gates_in_its_epilogue(tokens, I, K, biased):
     torch.manual_seed(tokens + I)
