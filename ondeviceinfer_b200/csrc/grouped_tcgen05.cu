@@ -167,7 +167,10 @@ __device__ __forceinline__ float gelu_erf_f(float z) { return 0.5f * z * (1.0f +
 __device__ __forceinline__ float gated(const ExpertsArgs& a, float g, float u) {
   g = fminf(g, a.limit);
   u = fminf(fmaxf(u, -a.limit), a.limit);
-  return __fdividef(g, 1.f + __expf(-a.alpha * g)) * (u + a.shift);
+  const float d = 1.f + __expf(-a.alpha * g);
+  float r;
+  asm("rcp.approx.f32 %0, %1;" : "=f"(r) : "f"(d));
+  return (d > 8.5070592e37f ? g * r : __fdividef(g, d)) * (u + a.shift);      // __fdividef gives 0 for d beyond 2^126
 }
 template <int EPI>
 __device__ __forceinline__ float plain(float v) {

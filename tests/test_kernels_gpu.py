@@ -436,6 +436,31 @@ def test_grouped_products_of_sorted_rows(rows, N, K):
     assert ops.gemm_status() == 0
 
 
+@pytest.mark.parametrize("kind", ["silu", "gelu_tanh", "clamp", "experts"])
+def test_gates_over_the_whole_range_of_their_quotient(kind):
+    """Gates down to -88.5, where 1 + exp(-g) is beyond 2^126, times up values that lift the result to ordinary numbers; an infinite gate."""
+    g = torch.cat([torch.linspace(-88.5, 88.5, 3000), torch.tensor([math.inf])]).bfloat16().to(DEV)
+    if kind == "gelu_tanh":
+        g = g / 16      # -5.5: beyond, the cubic leaves nothing
+    up = 2.0 ** 100 if kind != "gelu_tanh" else 2.0 ** 20
+    x, w = torch.zeros(g.numel(), 64, dtype=torch.bfloat16, device=DEV), torch.zeros(2 * 128, 64, dtype=torch.bfloat16, device=DEV)
+    x[:, 0], x[:, 1], w[:128, 0], w[128:, 1] = g, up, 1.0, 1.0
+    x[-1, 1] = 1.0      # and w's zeros times infinity:
+    x[-1, 0] = 3.0e38 if kind != "gelu_tanh" else 8.0
+    out = torch.empty(g.numel(), 128, dtype=torch.bfloat16, device=DEV)
+    if kind == "experts":
+        ops.grouped_gemm_sorted(x, w[None], out, torch.tensor([0, g.numel()], dtype=torch.int32, device=DEV), epi=ops.GROUPED_GATED_CLAMP,
+                                limit=math.inf, alpha=1.0, up_shift=0.0)
+    else:
+        epi = {"silu": ops.EPI_SWIGLU, "gelu_tanh": ops.EPI_GEGLU, "clamp": ops.EPI_GATED_CLAMP}[kind]
+        ops.gemm_prefill_bf16(x, w, out, epi, limit=math.inf, alpha=1.0, up_shift=0.0)
+    z, u = x[:, 0].double(), x[:, 1].double()
+    want = (torch.nn.functional.gelu(z, approximate="tanh") if kind == "gelu_tanh" else z * torch.sigmoid(z)) * u
+    # one rounding to bf16; __expf is off by at most 2 + 1.173 |x| ulps, some 1.3e-5, and 1 + tanh in 64 bits by 2^-53 of a number down to 1e-9
+    assert bool(((out.double() - want[:, None]).abs() <= (2.0 ** -8 + 2e-5) * want.abs()[:, None]).all())
+    assert ops.gemm_status() == 0
+
+
 @pytest.mark.parametrize("form", ["gated_clamp", "relu2", "table"])
 def test_experts_of_a_captured_step_keep_their_outputs_in_32_bits(form):
     """64 rows an expert, from where on the outputs of a step that is launched kernel by kernel are rounded to bf16: in a graph, and in the run
