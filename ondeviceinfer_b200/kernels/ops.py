@@ -291,8 +291,10 @@ def gemm_f32(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, residual: Opti
 # 29.2 / 97.1, 130 / 344; but 8,192 x 512 13.4 / 10.0 for one row, and below four million weights (1,024 x 1,024 12.5 / 13.5, 15.4 / 16.1,
 # 49 / 76) the second launch costs a host that launches kernel by kernel what the GPU gains.
 F32_SPLIT_MIN_ROWS, F32_SPLIT_MIN_K, F32_SPLIT_MIN_SIZE = 512, 1024, 1 << 22
-# Rows that one pass of it takes: four tiles of 192 tokens, from where on the weights' bytes no longer count; bounds its scratch.
-F32_SPLIT_PASS = 768
+# Rows that one pass of it takes: four tiles of 192 tokens, from where on the weights' bytes no longer count; bounds its scratch (768 rows: 60 MB
+# for 2,048 x 2,048, 71 for 24,576 x 4,096, 422 for 16,384 x 4,096, whose 64 tiles are all cut along K).  A row's bits do not depend on the
+# rows of its pass, so where there is no memory for one, shorter passes serve (3,000 rows of 12,800 x 4,096: 1,734 us in passes of 768, 2,230 of 192).
+F32_SPLIT_PASSES = (768, 192, 32, 1)
 
 
 def gemm_f32_split_takes(a: torch.Tensor, w: torch.Tensor) -> bool:
@@ -304,19 +306,23 @@ def gemm_f32_split_takes(a: torch.Tensor, w: torch.Tensor) -> bool:
 def gemm_f32_split(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, residual: Optional[torch.Tensor] = None,
                    bias: Optional[torch.Tensor] = None) -> bool:
     """:func:`gemm_f32` (which checks the operands) on the tensor cores, for any sizes with K a multiple of 4 and operands on
-    16-byte boundaries; False, with nothing done, where there is no memory for its scratch."""
+    16-byte boundaries; False, with nothing done, where there is no memory for the scratch of a single row."""
     M, K = a.shape
     N = w.shape[0]
     lib = load_library("gemm_f32_split")
     lib.odi_gemm_f32_split_scratch.restype = c_long
-    need = lib.odi_gemm_f32_split_scratch(c_int(min(M, F32_SPLIT_PASS)), c_int(N), c_int(K))
-    try:
-        scratch = torch.empty(need, dtype=torch.uint8, device=w.device)
-    except torch.OutOfMemoryError:
+    for longest in F32_SPLIT_PASSES:
+        need = lib.odi_gemm_f32_split_scratch(c_int(min(M, longest)), c_int(N), c_int(K))
+        try:
+            scratch = torch.empty(need, dtype=torch.uint8, device=w.device)
+            break
+        except torch.OutOfMemoryError:
+            continue
+    else:
         return False
     _, _, status = _gemm_buffers(w.device, 0)
-    for first in range(0, M, F32_SPLIT_PASS):
-        rows = min(F32_SPLIT_PASS, M - first)
+    for first in range(0, M, longest):
+        rows = min(longest, M - first)
         at = lambda t, width: c_void_p(0 if t is None else t.data_ptr() + 4 * first * width)
         _check(lib.odi_gemm_f32_split(at(a, K), _ptr(w), at(out, N), at(residual, N), _ptr(bias), c_int(rows), c_int(N), c_int(K), c_int(K),
                                       c_int(K), c_int(N), c_int(N), _ptr(scratch), c_long(need), _ptr(status), _stream()),

@@ -382,6 +382,30 @@ def test_gemm_f32_routes_by_the_weight_alone():
         assert torch.equal(other, out) is not takes and torch.allclose(other, out, atol=1e-6 * K, rtol=1e-5)
 
 
+def test_gemm_f32_in_shorter_passes_where_memory_is_short(monkeypatch):
+    """A row's bits do not depend on the memory that is left either, down to the scratch of a single row; without that the
+    multiply-adds serve."""
+    torch.manual_seed(9)
+    a, w, bias = torch.randn(401, 2048, device=DEV), torch.randn(2048, 2048, device=DEV), torch.randn(2048, device=DEV)
+    out, plain = torch.empty(401, 2048, device=DEV), torch.empty(401, 2048, device=DEV)
+    ops.gemm_f32(a, w, out, out.zero_(), bias)
+    ops.gemm_f32(a, w, plain, plain.zero_(), bias, form=0)
+    lib, real = ops.load_library("gemm_f32_split"), torch.empty
+    need = [int(lib.odi_gemm_f32_split_scratch(rows, 2048, 2048)) for rows in (401, 192, 32, 1)] + [0]
+    assert need == sorted(need, reverse=True) and need[1] < need[0]
+    for room in need:
+        def empty(*size, **kw):
+            if kw.get("dtype") == torch.uint8 and size[0] > room - (room == need[-1]):
+                raise torch.OutOfMemoryError("no room")
+            return real(*size, **kw)
+        got = torch.zeros(401, 2048, device=DEV)
+        monkeypatch.setattr(torch, "empty", empty)
+        ops.gemm_f32(a, w, got, got, bias)
+        monkeypatch.setattr(torch, "empty", real)
+        assert torch.equal(got, plain if room == need[-1] else out)
+    assert not torch.equal(out, plain) and ops.gemm_status() == 0
+
+
 def test_gemm_f32_split_of_infinities_nan_and_numbers_near_the_ends():
     torch.manual_seed(3)
     M, N, K = 9, 300, 512
