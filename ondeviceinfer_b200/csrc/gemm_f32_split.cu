@@ -650,7 +650,7 @@ static F32SplitPlan plan_of(int M, int N, int K) {
   return p;
 }
 
-extern "C" long odi_gemm_f32_split_scratch(int M, int N, int K) { return (long)plan_of(M, N, K).bytes; }
+extern "C" long odi_gemm_f32_split_scratch(int M, int N, int K) { return M <= 0 || N <= 0 || K <= 0 ? 0 : (long)plan_of(M, N, K).bytes; }
 
 // x [M, ldx], w [N, ldw], out [M, ldo], res null or [M, ldr] (may be out), bias null or [N], all fp32; K, ldx and ldw multiples of 4,
 // x and w on 16-byte boundaries; scratch: odi_gemm_f32_split_scratch bytes, 256-byte aligned; status: receives a code if a wait gives up.

@@ -1,6 +1,8 @@
-"""What the tcgen05 kernels' sources have to keep and no run can show for certain (no GPU)."""
+"""What the tcgen05 kernels' sources have to keep and no run can show for certain, and their host side (no GPU)."""
 
 import re
+import subprocess
+import sys
 from pathlib import Path
 
 import pytest
@@ -40,3 +42,14 @@ def test_a_warp_that_issues_waits_as_one(name):
 
 def test_the_kernels_that_issue_are_all_here():
     assert ISSUING == ["attention_tcgen05.cu", "gemm_f32_split.cu", "gemm_prefill_tcgen05.cu", "gemm_tcgen05.cu", "grouped_tcgen05.cu"]
+
+
+def test_a_product_without_rows_needs_no_scratch():
+    """The plan divides by the tiles of rows: a call without any has to come back, not end the process."""
+    script = ("from ctypes import c_long\n"
+              "from ondeviceinfer_b200.kernels.build import load_library\n"
+              "lib = load_library('gemm_f32_split')\n"
+              "lib.odi_gemm_f32_split_scratch.restype = c_long\n"
+              "print([lib.odi_gemm_f32_split_scratch(*s) for s in ((0, 2048, 2048), (3, 0, 2048), (3, 2048, 0), (-1, 2048, 2048))])\n")
+    done = subprocess.run([sys.executable, "-c", script], capture_output=True, text=True, cwd=CSRC.parents[1])
+    assert done.returncode == 0 and done.stdout.strip() == "[0, 0, 0, 0]", (done.returncode, done.stderr)
