@@ -33,7 +33,8 @@
 // tiles of multiply-adds before / this: 185 x 24,576 x 4,096 871 / 169 (221 TFLOP/s), 185 x 4,096 x 12,288 683 / 105, 185 x 151,936 x 4,096
 // 5,550 / 979, 1,024 x 24,576 x 4,096 4,735 / 902; one row: 24,576 x 4,096 143 / 89, 151,936 x 4,096 785 / 473 (5,260 GB/s).
 //
-// Every wait is bounded: after about two seconds the role records a code in `status`, all roles leave, tensor memory is freed.
+// Every wait is bounded: after two to three seconds the role whose wait ran out records its code in `status`, all roles leave, tensor memory is
+// freed.
 #include <cuda.h>
 #include <float.h>
 
@@ -54,7 +55,14 @@
 #define REGS_CONVERT 104
 #define REGS_EPILOGUE 176
 #define PAIRS 74                  // pairs that the cut along K is made for (148 multiprocessors): part of the order of the sums
-#define WAIT_CYCLES 4000000000ll
+#ifndef ODI_WAIT_CYCLES
+#define ODI_WAIT_CYCLES 4000000000ll   // about two seconds of SM clock; a self-test build makes it milliseconds
+#endif
+// How long a role waits for a copy, for the role that waits for that copy, and for those that wait for it in turn: a copy that never comes is
+// reported by the role that missed it, in either CTA.
+#define WAIT_CYCLES ((long long)ODI_WAIT_CYCLES)
+#define WAIT_CYCLES_2 (WAIT_CYCLES + WAIT_CYCLES / 4)
+#define WAIT_CYCLES_3 (WAIT_CYCLES + WAIT_CYCLES / 2)
 
 #define ERR_WEIGHTS 41
 #define ERR_MMA 42
@@ -77,6 +85,7 @@ struct F32SplitArgs {
   int full, rest, splits;  // feature tiles in one piece, those behind them, and their parts along K
   int raw_stages, tok_stages;
   int ring;                // slots in tensor memory (at most MAX_RING): ring * (bn + A_COLS) <= 512
+  int withheld;            // self-test of the bounded waits: 1, the weights' producers request nothing; 2, the activations'
 };
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -92,23 +101,25 @@ __device__ __forceinline__ bool mbar_test(uint32_t bar, uint32_t parity) {
       : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
   return ok != 0;
 }
-// Bounded wait.  False when it gave up or when another role of the CTA did.
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
+// Bounded wait.  False when it gave up or when another role of the CTA did.  The role whose own wait ran out records its code before it raises
+// the flag, so that `status` names it and not one that merely left after it.
+__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag, int* status, int code, long long limit) {
   if (mbar_test(bar, parity)) return true;
   const long long start = clock64();
   for (uint32_t i = 0;; ++i) {
     if (mbar_test(bar, parity)) return true;
     if ((i & 0xf) == 0xf) {
       if (*abort_flag) return false;
-      if (clock64() - start > WAIT_CYCLES) break;
+      if (clock64() - start > limit) break;
     }
   }
+  atomicCAS(status, 0, code);
   *abort_flag = 1;
   return false;
 }
 // The same by a whole warp, with one answer for all of its lanes.
-__device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
-  return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag));
+__device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag, int* status, int code, long long limit) {
+  return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag, status, code, limit));
 }
 // After a role gave up: the copies that are still on their way to the stages of the last `stages` uses before `issued` (bounded).
 __device__ __forceinline__ void drain(uint32_t full, int stages, int issued) {
@@ -339,20 +350,17 @@ gemm_f32_split_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
   if (warp < 4) {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(REGS_ISSUE));
     if (warp == 0 && lane == 0) {
-      bool ok = true;
+      bool ok = a.withheld != 1;
       int it = 0, s = 0;
       uint32_t phase = 1;
       for (int u = pair; ok && unit_of(a, u, t); u += n_pairs)
         for (int st = 0; st < t.steps; ++st, ++it) {
-          if (it >= a.raw_stages && !mbar_wait(raw_empty + 8 * s, phase, abort_ptr)) { ok = false; break; }
+          if (it >= a.raw_stages && !mbar_wait(raw_empty + 8 * s, phase, abort_ptr, a.status, ERR_WEIGHTS, WAIT_CYCLES_3)) { ok = false; break; }
           mbar_expect_tx(raw_full + 8 * s, RAW_BYTES);
           tma_load_2d(raw0 + s * RAW_BYTES, &map_w, t.k0 + st * KC, t.n0 + (int)rank * BF, raw_full + 8 * s);
           if (++s == a.raw_stages) { s = 0; phase ^= 1u; }
         }
-      if (!ok) {
-        atomicCAS(a.status, 0, ERR_WEIGHTS);
-        drain(raw_full, a.raw_stages, it);
-      }
+      if (!ok) drain(raw_full, a.raw_stages, it);
     } else if (warp == 1 && rank == 0) {
       // the whole warp goes through the loop (see elect_one)
       const bool issues = elect_one();
@@ -365,10 +373,10 @@ gemm_f32_split_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
       for (int u = pair; ok && unit_of(a, u, t); u += n_pairs)
         for (int st = 0; st < t.steps; ++st) {
           if ((st & 1) == 0) {
-            if (!warp_wait(tok_full + 8 * s, tok_phase, abort_ptr)) { ok = false; break; }
+            if (!warp_wait(tok_full + 8 * s, tok_phase, abort_ptr, a.status, ERR_MMA, WAIT_CYCLES)) { ok = false; break; }
             db = smem_desc_k_sw128(tok0 + s * tok_bytes);
           }
-          if (!warp_wait(ready + 8 * slot, phase, abort_ptr)) { ok = false; break; }
+          if (!warp_wait(ready + 8 * slot, phase, abort_ptr, a.status, ERR_MMA, WAIT_CYCLES_2)) { ok = false; break; }
           tc_fence_after();
           const uint32_t d = tmem + slot * a.bn, wa = tmem_a + slot * A_COLS;
           const uint64_t b = db + (st & 1) * 4;
@@ -388,25 +396,21 @@ gemm_f32_split_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
             if (++s == a.tok_stages) { s = 0; tok_phase ^= 1u; }
           }
         }
-      if (!ok && issues) atomicCAS(a.status, 0, ERR_MMA);
     } else if (warp == 2 && lane == 0) {
       pdl_wait();                     // the pieces come from the kernel before
       const uint32_t leader_full = map_to_rank(tok_full, 0);
-      bool ok = true;
+      bool ok = a.withheld != 2;
       int it = 0, s = 0;
       uint32_t phase = 1;
       for (int u = pair; ok && unit_of(a, u, t); u += n_pairs)
         for (int b = 0; 2 * b < t.steps; ++b, ++it) {
-          if (it >= a.tok_stages && !mbar_wait(tok_empty + 8 * s, phase, abort_ptr)) { ok = false; break; }
+          if (it >= a.tok_stages && !mbar_wait(tok_empty + 8 * s, phase, abort_ptr, a.status, ERR_TOKENS, WAIT_CYCLES_3)) { ok = false; break; }
           mbar_expect_tx_cluster(leader_full + 8 * s, tok_bytes);
           for (int p = 0; p < 3; ++p)
             tma_load_2d_pair(tok0 + s * tok_bytes + p * half * 128, &map_x, t.k0 + b * KB, p * a.M + t.t0 + (int)rank * half, leader_full + 8 * s);
           if (++s == a.tok_stages) { s = 0; phase ^= 1u; }
         }
-      if (!ok) {
-        atomicCAS(a.status, 0, ERR_TOKENS);
-        if (rank == 0) drain(tok_full, a.tok_stages, it);
-      }
+      if (!ok && rank == 0) drain(tok_full, a.tok_stages, it);
     }
   } else if (warp < 8) {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(REGS_CONVERT));
@@ -418,7 +422,7 @@ gemm_f32_split_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
     uint32_t raw_phase = 0, phase = 1;
     for (int u = pair; ok && unit_of(a, u, t); u += n_pairs)
       for (int st = 0; st < t.steps; ++st) {
-        if (!warp_wait(raw_full + 8 * s, raw_phase, abort_ptr)) { ok = false; break; }
+        if (!warp_wait(raw_full + 8 * s, raw_phase, abort_ptr, a.status, ERR_CONVERT, WAIT_CYCLES)) { ok = false; break; }
         const uint8_t* mine = smem + s * RAW_BYTES + row * 128;
         float v[32];
 #pragma unroll
@@ -435,7 +439,7 @@ gemm_f32_split_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
         if (lane == 0) mbar_arrive(raw_empty + 8 * s);
         if (++s == a.raw_stages) { s = 0; raw_phase ^= 1u; }
         // the products that read the slot's weights a round ago
-        if (!first && !warp_wait(done + 8 * slot, phase, abort_ptr)) { ok = false; break; }
+        if (!first && !warp_wait(done + 8 * slot, phase, abort_ptr, a.status, ERR_CONVERT, WAIT_CYCLES_3)) { ok = false; break; }
         tc_fence_after();
         const uint32_t dst = tmem_a + lanes + slot * A_COLS;
 #pragma unroll
@@ -446,7 +450,6 @@ gemm_f32_split_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
         if (lane == 0) mbar_arrive_cluster(leader_ready + 8 * slot);
         if (++slot == a.ring) { slot = 0; phase ^= 1u; first = false; }
       }
-    if (!ok && lane == 0) atomicCAS(a.status, 0, ERR_CONVERT);
   } else {
     asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(REGS_EPILOGUE));
     pdl_wait();                       // the residual, the scales and the tickets
@@ -465,7 +468,7 @@ gemm_f32_split_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
       for (int c = 0; c < MAX_BN / 2; ++c) acc[c] = 0.f;
       // a warp whose wait gave up still walks its units: the others count on it at the barriers below
       for (int st = 0; ok && st < t.steps; ++st) {
-        if (!warp_wait(done + 8 * slot, phase, abort_ptr)) { ok = false; break; }
+        if (!warp_wait(done + 8 * slot, phase, abort_ptr, a.status, ERR_EPILOGUE, WAIT_CYCLES_3)) { ok = false; break; }
         tc_fence_after();
         const uint32_t from = src + slot * a.bn;
 #pragma unroll
@@ -584,7 +587,6 @@ gemm_f32_split_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
         }
       }
     }
-    if (!ok && lane == 0) atomicCAS(a.status, 0, ERR_EPILOGUE);
     tc_fence_before();
   }
   __syncthreads();
@@ -654,9 +656,10 @@ extern "C" long odi_gemm_f32_split_scratch(int M, int N, int K) { return M <= 0 
 
 // x [M, ldx], w [N, ldw], out [M, ldo], res null or [M, ldr] (may be out), bias null or [N], all fp32; K, ldx and ldw multiples of 4,
 // x and w on 16-byte boundaries; scratch: odi_gemm_f32_split_scratch bytes, 256-byte aligned; status: receives a code if a wait gives up.
+// withheld: 0, or a self-test of that (F32SplitArgs).
 extern "C" int odi_gemm_f32_split(const float* x, const float* w, float* out, const float* res, const float* bias, int M, int N,
                                   int K, int ldx, int ldw, int ldo, int ldr, void* scratch, long scratch_bytes, int* status,
-                                  cudaStream_t stream) {
+                                  int withheld, cudaStream_t stream) {
   if (M <= 0 || N <= 0) return 0;
   if (K <= 0 || status == nullptr) return ODI_ERR_ARGUMENT;
   if (K % 4 || ldx % 4 || ldw % 4 || ((uintptr_t)x & 15) || ((uintptr_t)w & 15) || ((uintptr_t)scratch & 255)) return ODI_ERR_UNSUPPORTED;
@@ -674,7 +677,7 @@ extern "C" int odi_gemm_f32_split(const float* x, const float* w, float* out, co
   }
   uint8_t* base = (uint8_t*)scratch;
   F32SplitArgs a;
-  a.x = x; a.w = w; a.out = out; a.res = res; a.bias = bias; a.status = status;
+  a.x = x; a.w = w; a.out = out; a.res = res; a.bias = bias; a.status = status; a.withheld = withheld;
   a.row_scale = (float*)(base + p.scale_at); a.tickets = (int*)(base + p.ticket_at); a.partial = (float*)(base + p.partial_at);
   a.M = M; a.N = N; a.K = K; a.ldx = ldx; a.ldw = ldw; a.ldo = ldo; a.ldr = ldr;
   a.bn = p.bn; a.m_tiles = p.m_tiles; a.full = p.full; a.rest = p.rest; a.splits = p.splits;

@@ -39,7 +39,13 @@
 #define STAGES 6
 #define THREADS 384
 #define MAX_GROUPS 2048
-#define WAIT_CYCLES 4000000000ll
+#ifndef ODI_WAIT_CYCLES
+#define ODI_WAIT_CYCLES 4000000000ll   // about two seconds of SM clock; a self-test build makes it milliseconds
+#endif
+// How long a role waits for a copy, and the longer wait for the role that waits for it: a copy that never comes is reported by the role that
+// missed it.
+#define WAIT_CYCLES ((long long)ODI_WAIT_CYCLES)
+#define WAIT_CYCLES_2 (WAIT_CYCLES + WAIT_CYCLES / 4)
 
 #define ERR_PRODUCER 51
 #define ERR_MMA 52
@@ -53,6 +59,7 @@ struct ExpertsArgs {
   int w_rows, groups;      // weight rows an expert
   int n_tiles;             // feature tiles
   float limit, alpha, shift;
+  int withheld;            // self-test of the bounded waits: the producers request nothing
 };
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -68,23 +75,25 @@ __device__ __forceinline__ bool mbar_test(uint32_t bar, uint32_t parity) {
       : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
   return ok != 0;
 }
-// Bounded wait.  False when it gave up or when another role of the CTA did.
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
+// Bounded wait.  False when it gave up or when another role of the CTA did.  The role whose own wait ran out records its code before it raises
+// the flag, so that `status` names it and not one that merely left after it.
+__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag, int* status, int code, long long limit) {
   if (mbar_test(bar, parity)) return true;
   const long long start = clock64();
   for (uint32_t i = 0;; ++i) {
     if (mbar_test(bar, parity)) return true;
     if ((i & 0xf) == 0xf) {
       if (*abort_flag) return false;
-      if (clock64() - start > WAIT_CYCLES) break;
+      if (clock64() - start > limit) break;
     }
   }
+  atomicCAS(status, 0, code);
   *abort_flag = 1;
   return false;
 }
 // The same by a whole warp, with one answer for all of its lanes.
-__device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
-  return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag));
+__device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag, int* status, int code, long long limit) {
+  return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag, status, code, limit));
 }
 // After a role gave up: the copies that are still on their way to the stages of the last `stages` uses before `issued` (bounded).
 __device__ __forceinline__ void drain(uint32_t full, int stages, int issued) {
@@ -255,14 +264,14 @@ grouped_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_c
   if (warp == 0) {
     if (lane == 0) {
       const uint32_t leader_full = map_to_rank(full, 0);
-      bool ok = true;
+      bool ok = !a.withheld;
       int it = 0, s = 0;
       uint32_t phase = 1;
       for (int u = pair; ok && unit_of<GATE>(a, first, u, group, t); u += n_pairs) {
         const int row = t.w0 + (int)rank * (GATE ? BF / 2 : BF), row2 = GATE ? row + a.N : row + BF / 2;
         const int tok0 = t.t0 + (int)rank * (t.bn / 2), boxes = (t.bn / 2 + BOX - 1) / BOX;
         for (int kb = 0; kb < blocks; ++kb, ++it) {
-          if (it >= STAGES && !mbar_wait(empty + 8 * s, phase, abort_ptr)) { ok = false; break; }
+          if (it >= STAGES && !mbar_wait(empty + 8 * s, phase, abort_ptr, a.status, ERR_PRODUCER, WAIT_CYCLES_2)) { ok = false; break; }
           const uint32_t dst = ring + s * STAGE_BYTES, bar = leader_full + 8 * s;
           mbar_expect_tx_cluster(bar, A_BYTES + boxes * BOX * 128);
           tma_load_2d_pair(dst, &map_w, kb * BK, row, bar);
@@ -271,10 +280,7 @@ grouped_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_c
           if (++s == STAGES) { s = 0; phase ^= 1u; }
         }
       }
-      if (!ok) {
-        atomicCAS(a.status, 0, ERR_PRODUCER);
-        if (rank == 0) drain(full, STAGES, it);
-      }
+      if (!ok && rank == 0) drain(full, STAGES, it);
     }
   } else if (warp == 1) {
     if (rank == 0) {
@@ -285,9 +291,9 @@ grouped_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_c
       for (int u = pair; ok && unit_of<GATE>(a, first, u, group, t); u += n_pairs, ++local) {
         const int buf = local & 1;
         const uint32_t idesc = instr_desc_bf16(2 * BF, t.bn), d = tmem + buf * MAX_BN;
-        if (local >= 2 && !warp_wait(acc_empty + 8 * buf, ((uint32_t)(local >> 1) & 1u) ^ 1u, abort_ptr)) { ok = false; break; }
+        if (local >= 2 && !warp_wait(acc_empty + 8 * buf, ((uint32_t)(local >> 1) & 1u) ^ 1u, abort_ptr, a.status, ERR_MMA, WAIT_CYCLES)) { ok = false; break; }
         for (int kb = 0; kb < blocks; ++kb) {
-          if (!warp_wait(full + 8 * s, phase, abort_ptr)) { ok = false; break; }
+          if (!warp_wait(full + 8 * s, phase, abort_ptr, a.status, ERR_MMA, WAIT_CYCLES)) { ok = false; break; }
           tc_fence_after();
           const uint64_t dw = smem_desc_k_sw128(ring + s * STAGE_BYTES), dx = smem_desc_k_sw128(ring + s * STAGE_BYTES + A_BYTES);
           if (issues) {
@@ -299,7 +305,6 @@ grouped_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_c
         }
         if (ok && issues) umma_commit_pair(acc_full + 8 * buf);
       }
-      if (!ok && issues) atomicCAS(a.status, 0, ERR_MMA);
     }
   } else if (warp >= 4) {
     const int lane_group = warp & 3, side = (warp - 4) >> 2;          // which half of the tile's rows
@@ -312,7 +317,7 @@ grouped_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_c
       // a warp whose wait gave up still walks its units: the others count on it at the barriers below
       const int buf = local & 1, half = t.bn / 2, c0 = side * half;
       const int n = GATE ? t.n0 + (int)rank * (BF / 2) + (row & 63) : t.n0 + (int)rank * BF + row;
-      if (ok && !warp_wait(acc_full + 8 * buf, (uint32_t)(local >> 1) & 1u, abort_ptr)) ok = false;
+      if (ok && !warp_wait(acc_full + 8 * buf, (uint32_t)(local >> 1) & 1u, abort_ptr, a.status, ERR_EPILOGUE, WAIT_CYCLES_2)) ok = false;
       tc_fence_after();
       const uint32_t src = tmem + ((uint32_t)(lane_group * 32) << 16) + buf * MAX_BN + c0;
       // columns that hold rows: no more are loaded than are waited for, so that no load lands in registers that have another use by then
@@ -383,7 +388,6 @@ grouped_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_c
       __syncwarp();
       if (lane == 0) mbar_arrive_cluster(leader_empty + 8 * buf);
     }
-    if (!ok && lane == 0) atomicCAS(a.status, 0, ERR_EPILOGUE);
     tc_fence_before();
   }
   __syncthreads();
@@ -453,9 +457,9 @@ static int launch(const CUtensorMap& mx, const CUtensorMap& mw, const ExpertsArg
 
 // x [rows, K] bf16, w [groups, w_rows, K] bf16 (EPI_GATED_CLAMP: the gate rows, then the up rows; n_out = w_rows / 2), out [rows, n_out] in bf16, or fp32 for EPI_STORE_F32,
 // offsets [groups + 1] ints on the device, rising from 0 to at most `rows`; rows beyond the last are not touched.  K a multiple of 8, x and w on
-// 16-byte boundaries.
+// 16-byte boundaries.  status: receives a code if a wait gives up; withheld: 0, or 1 for a self-test of that.
 extern "C" int odi_grouped_tcgen05(const void* x, const void* w, void* out, const int* offsets, int rows, int groups, int n_out, int K,
-                                   int w_rows, int epi, float limit, float alpha, float shift, int* status, cudaStream_t stream) {
+                                   int w_rows, int epi, float limit, float alpha, float shift, int* status, int withheld, cudaStream_t stream) {
   if (rows <= 0 || n_out <= 0) return 0;
   const bool gate = epi == EPI_GATED_CLAMP;
   if (K <= 0 || status == nullptr || offsets == nullptr || groups < 1 || (gate ? w_rows != 2 * n_out : w_rows != n_out)) return ODI_ERR_ARGUMENT;
@@ -466,7 +470,7 @@ extern "C" int odi_grouped_tcgen05(const void* x, const void* w, void* out, cons
   ExpertsArgs a = {};
   a.out = out; a.status = status; a.offsets = offsets; a.N = n_out; a.K = K; a.w_rows = w_rows; a.groups = groups;
   a.n_tiles = (n_out + (gate ? BF : 2 * BF) - 1) / (gate ? BF : 2 * BF);
-  a.limit = limit; a.alpha = alpha; a.shift = shift;
+  a.limit = limit; a.alpha = alpha; a.shift = shift; a.withheld = withheld;
   if ((long)groups * w_rows > 0x7fffffffL || ((long)rows / MAX_BN + groups) * a.n_tiles > 0x3fffffffL) return ODI_ERR_UNSUPPORTED;
   CUtensorMap mx, mw;
   rc = make_map(&mx, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, x, rows, K, K, BOX);

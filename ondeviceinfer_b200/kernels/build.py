@@ -157,9 +157,9 @@ _HEAD_SIZES_MMA = (16, 32, 48, 64, 80, 96, 112, 128, 192, 256)
 ALL_SOURCES = {
     "elementwise": [{}],
     "gemm_f32": [{}],
-    "gemm_f32_split": [{}],
+    "gemm_f32_split": [{}, {"ODI_WAIT_CYCLES": 20_000_000}],      # the second, here and below: ops.selftest_bounded_wait
     "sampling": [{}],
-    "gemm_tcgen05": [{}, {"ODI_WAIT_CYCLES": 20_000_000}],      # the second: ops.selftest_bounded_wait
+    "gemm_tcgen05": [{}, {"ODI_WAIT_CYCLES": 20_000_000}],
     "gemm_prefill_tcgen05": [{}],
     "attention_simt": [{"ODI_HEAD_DIM": d} for d in _HEAD_SIZES_MMA + (512,)]
                       + [{"ODI_HEAD_DIM": 576, "ODI_VALUE_DIM": 512, "ODI_SHARED_KV": 1}],      # a latent cache
@@ -176,7 +176,7 @@ ALL_SOURCES = {
     "attention_capped_mma": [{"ODI_HEAD_DIM": 128, "ODI_VALUE_DIM": 128}],
     "attention_latent_mma": [{"ODI_HEAD_DIM": 576, "ODI_VALUE_DIM": 512}],      # a latent cache, on the tensor cores
     "grouped_gemm": [{}],
-    "grouped_tcgen05": [{}],
+    "grouped_tcgen05": [{}, {"ODI_WAIT_CYCLES": 20_000_000}],
     "moe": [{}],
     "delta": [{"ODI_DELTA_DIM": d} for d in (64, 128)],
     "attention_mma": [{"ODI_HEAD_DIM": d} for d in _HEAD_SIZES_MMA],

@@ -325,7 +325,7 @@ def gemm_f32_split(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, residual
         rows = min(longest, M - first)
         at = lambda t, width: c_void_p(0 if t is None else t.data_ptr() + 4 * first * width)
         _check(lib.odi_gemm_f32_split(at(a, K), _ptr(w), at(out, N), at(residual, N), _ptr(bias), c_int(rows), c_int(N), c_int(K), c_int(K),
-                                      c_int(K), c_int(N), c_int(N), _ptr(scratch), c_long(need), _ptr(status), _stream()),
+                                      c_int(K), c_int(N), c_int(N), _ptr(scratch), c_long(need), _ptr(status), c_int(0), _stream()),
                "gemm_f32_split", 2)
     return True
 
@@ -569,26 +569,44 @@ def gemm_bf16(x: Optional[torch.Tensor], w: torch.Tensor, out: Optional[torch.Te
 SELFTEST_WAIT_CYCLES = 20_000_000        # about ten milliseconds of SM clock
 
 
-def selftest_bounded_wait(device="cuda:0") -> int:
-    """Make one wait of the tensor-core GEMM run out, safely, and return the code the kernel recorded.
+def selftest_bounded_wait(device="cuda:0", of: str = "gemm_tcgen05") -> int:
+    """Make one wait of a tensor-core product run out, safely, and return the code the kernel recorded.
 
-    One tile is launched from a build of ``gemm_tcgen05.cu`` whose waits last about ten milliseconds
-    (``ODI_WAIT_CYCLES``) with a producer that requests no copy at all, so nothing is in flight: the MMA role
-    gives up on its first wait, every role leaves its loop, tensor memory is freed and the kernel returns.
-    The error word then holds the MMA role's code (2) and :func:`raise_on_kernel_fault` raises naming it.
-    The product's own build and its two-second limit are not involved."""
+    One tile is launched from a build whose waits last about ten milliseconds (``ODI_WAIT_CYCLES``) with producers that
+    request no copy of one operand, so that nothing is in flight when they run out: the role that consumes the copies gives up
+    on its first wait, every role leaves its loop, tensor memory is freed and the kernel returns.  The error word then holds that
+    role's code and :func:`raise_on_kernel_fault` raises naming it.  ``of``: "gemm_tcgen05" (the MMA role, 2),
+    "gemm_f32_split weights" (the converting warps, 44), "gemm_f32_split tokens" (the MMA role, 42) or "grouped_tcgen05" (the MMA role, 52).
+    The product's own build and its limit of seconds are not involved."""
     device = torch.device(device)
-    x = torch.zeros((16, 256), dtype=torch.bfloat16, device=device)
-    w = torch.zeros((128, 256), dtype=torch.bfloat16, device=device)
-    out = torch.zeros((16, 128), dtype=torch.float32, device=device)
+    name = of.split()[0]
     scratch, tickets, status = _gemm_buffers(device, 0)
-    lib = load_library("gemm_tcgen05", {"ODI_WAIT_CYCLES": SELFTEST_WAIT_CYCLES})
-    none = _ptr(None)
+    lib = load_library(name, {"ODI_WAIT_CYCLES": SELFTEST_WAIT_CYCLES})
+    none, label = _ptr(None), f"{name} (bounded-wait self-test)"
     with torch.cuda.device(device):
-        _check(lib.odi_gemm_bf16(_ptr(x), _ptr(w), _ptr(out), c_int(16), c_int(128), c_int(256), c_int(128), c_int(128),
-                                 c_int(EPI_STORE_F32), c_int(16), c_int(1), c_int(0), _ptr(scratch), _ptr(tickets),
-                                 _ptr(status), none, none, none, c_int(0), c_float(0.0), none, none, none, c_int(1),
-                                 none, _stream()), "gemm_tcgen05 (bounded-wait self-test)")
+        if of == "gemm_tcgen05":
+            x = torch.zeros((16, 256), dtype=torch.bfloat16, device=device)
+            w = torch.zeros((128, 256), dtype=torch.bfloat16, device=device)
+            out = torch.zeros((16, 128), dtype=torch.float32, device=device)
+            _check(lib.odi_gemm_bf16(_ptr(x), _ptr(w), _ptr(out), c_int(16), c_int(128), c_int(256), c_int(128), c_int(128),
+                                     c_int(EPI_STORE_F32), c_int(16), c_int(1), c_int(0), _ptr(scratch), _ptr(tickets),
+                                     _ptr(status), none, none, none, c_int(0), c_float(0.0), none, none, none, c_int(1),
+                                     none, _stream()), label)
+        elif of in ("gemm_f32_split weights", "gemm_f32_split tokens"):
+            x, w, out = (torch.zeros(shape, device=device) for shape in ((32, 64), (256, 64), (32, 256)))
+            lib.odi_gemm_f32_split_scratch.restype = c_long
+            need = lib.odi_gemm_f32_split_scratch(c_int(32), c_int(256), c_int(64))
+            pieces = torch.empty(need, dtype=torch.uint8, device=device)
+            _check(lib.odi_gemm_f32_split(_ptr(x), _ptr(w), _ptr(out), none, none, c_int(32), c_int(256), c_int(64), c_int(64), c_int(64),
+                                          c_int(256), c_int(256), _ptr(pieces), c_long(need), _ptr(status),
+                                          c_int(1 if of.endswith("weights") else 2), _stream()), label, 2)
+        elif of == "grouped_tcgen05":
+            x, w, out = (torch.zeros(shape, dtype=torch.bfloat16, device=device) for shape in ((32, 64), (1, 256, 64), (32, 256)))
+            offsets = torch.tensor([0, 32], dtype=torch.int32, device=device)
+            _check(lib.odi_grouped_tcgen05(_ptr(x), _ptr(w), _ptr(out), _ptr(offsets), c_int(32), c_int(1), c_int(256), c_int(64), c_int(256),
+                                           c_int(0), c_float(0.0), c_float(1.0), c_float(1.0), _ptr(status), c_int(1), _stream()), label)
+        else:
+            raise KernelError(f"no bounded-wait self-test of {of!r}")
         torch.cuda.synchronize(device)
     return int(status[0].item())
 
@@ -1343,7 +1361,7 @@ def grouped_gemm_sorted(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, off
     lib = load_library("grouped_tcgen05")
     _check(lib.odi_grouped_tcgen05(_ptr(x), _ptr(w), _ptr(out), _ptr(offsets), c_int(x.shape[0]), c_int(groups), c_int(n_out), c_int(K),
                                    c_int(w_rows), c_int(6 if round_sums else _GROUPED_TCGEN05_EPILOGUES[epi]), c_float(limit), c_float(alpha),
-                                   c_float(up_shift), _ptr(status), _stream()), "grouped_tcgen05")
+                                   c_float(up_shift), _ptr(status), c_int(0), _stream()), "grouped_tcgen05")
 
 
 def moe_route(logits: torch.Tensor, correction: Optional[torch.Tensor], ids: torch.Tensor, weights: torch.Tensor, *,

@@ -1329,6 +1329,27 @@ def test_a_wait_that_runs_out_is_reported_and_leaves_the_gpu_usable():
     assert torch.allclose(out.cpu(), (x.float() @ w.float().t()).cpu(), atol=1e-4, rtol=1e-4)
 
 
+@pytest.mark.parametrize("of,code,role", [("gemm_f32_split weights", 44, "gemm_f32_split: the converting warps"),
+                                          ("gemm_f32_split tokens", 42, "gemm_f32_split: the MMA issuer"),
+                                          ("grouped_tcgen05", 52, "grouped_tcgen05: the MMA issuer")])
+def test_the_role_that_missed_a_copy_is_the_one_reported(of, code, role):
+    """As above, of the products whose tiles two CTAs share: the word names the role that waited for the copy, not one that waited for that role
+    or left after it."""
+    ops.raise_on_kernel_fault()
+    assert ops.selftest_bounded_wait(DEV, of) == code
+    with pytest.raises(ops.KernelError, match=role):
+        ops.raise_on_kernel_fault()
+    ops.raise_on_kernel_fault()
+    x, w = torch.randn(70, 72, device=DEV).bfloat16(), torch.randn(1, 40, 72, device=DEV).bfloat16()
+    out, wide = torch.empty(70, 40, device=DEV), torch.empty(70, 40, device=DEV)
+    ops.grouped_gemm_sorted(x, w, out, torch.tensor([0, 70], dtype=torch.int32, device=DEV), epi=ops.GROUPED_STORE_F32)
+    assert ops.gemm_f32_split(x.float(), w[0].float(), wide)
+    want = x.double() @ w[0].double().t()
+    for got in (out, wide):
+        assert bool(((got.double() - want).abs() <= 1e-3).all())      # sums of 72 products of normal numbers
+    assert ops.gemm_status() == 0
+
+
 @pytest.mark.parametrize("tokens,N,K", [(2048, 4096, 4096), (2048, 4096, 12288), (5000, 1024, 136), (2100, 5120, 1000),
                                         (4500, 776, 72), (19000, 256, 64)])
 def test_gemm_prefill_tcgen05_adds_a_tile_in_ordered_parts(tokens, N, K):
