@@ -331,8 +331,10 @@ extern "C" int odi_moe_group(const GroupingArgs* args, cudaStream_t stream) {
 // The routing alone: ids and weights [n_pairs] from `table` [vocab, top] for `tokens` [n_pairs / top].
 extern "C" int odi_moe_table_route(const int* table, const int* tokens, int* ids, float* weights, int n_tokens, int top, int vocab,
                                    int n_experts, float weight, cudaStream_t stream) {
-  const int n_pairs = n_tokens * top;
   if (n_tokens <= 0 || top <= 0) return 0;
+  if (vocab <= 0 || n_experts <= 0) return ODI_ERR_ARGUMENT;
+  if ((long)n_tokens * top > 0x7fffffffL) return ODI_ERR_UNSUPPORTED;
+  const int n_pairs = n_tokens * top;
   odi_rc = launch_pdl(moe_table_route_kernel, dim3((n_pairs + 127) / 128), dim3(128), 0, stream, TableRoute{table, tokens, ids, weights, top, vocab, weight},
                       n_pairs, n_experts);
   return launch_status();

@@ -586,6 +586,14 @@ def test_pairs_of_a_table_are_routed_and_sorted_at_once(tokens, top, experts):
     assert all(torch.equal(a, b) for a, b in zip(*made)) and int(counts.abs().sum()) == 0
 
 
+def test_routing_by_a_table_refuses_no_experts_and_no_rows():
+    ids, weights = torch.zeros(2, 1, dtype=torch.int32, device=DEV), torch.zeros(2, 1, device=DEV)
+    tokens, route = torch.zeros(2, dtype=torch.int32, device=DEV), torch.zeros(4, 1, dtype=torch.int32, device=DEV)
+    for table, experts in ((route, 0), (route[:0], 3)):
+        with pytest.raises(ops.KernelError):
+            ops.moe_table_route(table, tokens, ids, weights, n_experts=experts, weight=1.0)
+
+
 @pytest.mark.parametrize("tokens,H,wide", [(1, 64, True), (7, 2048, True), (600, 1032, False)])
 def test_combine_takes_a_gated_shared_expert_along(tokens, H, wide):
     torch.manual_seed(H)
