@@ -213,7 +213,10 @@ __global__ void moe_plan_kernel(GroupingArgs a) {
 // Up to THREADS x PER pairs: count, plan and scatter by one block in one launch, the counts in shared memory
 // (the global `counts` stay zero; they and the plan take 3 * n_experts ints).  A thread asks for all of its pairs before it counts one.
 #define SMALL_PAIRS 2048       // single-token steps: 256 threads
-#define ONE_BLOCK_PAIRS 16384  // prompts: 1,024 threads.  8,192 pairs of 30 experts 8.3 us; in three launches 8.2 and two gaps
+// Prompts: 1,024 threads.  In a graph, us, one block / three launches: 4,096 pairs evenly on 30 experts 4.6 / 4.7, on four of them 4.0 / 6.3; 8,192
+// pairs 6.9 / 6.2 and 5.9 / 9.2, evenly on 128 experts 9.2 / 7.4; 16,384 pairs 12.1 / 8.7, 10.1 / 14.6 and 15.3 / 9.5.  Launched one by one the
+// other two cost the host some 30 us, which a step of so many tokens waits for up to about 8,192 pairs.
+#define ONE_BLOCK_PAIRS 8192
 // TABLE: the pairs' outputs come from a routing table and are written down as well, which saves a launch of its own.
 template <int THREADS, int PER, bool TABLE>
 __global__ void __launch_bounds__(THREADS)

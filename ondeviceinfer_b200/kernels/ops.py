@@ -1407,6 +1407,9 @@ class RoutingTable:
          self.n_tiles) = torch.split(ints, cuts)
 
 
+MOE_ONE_BLOCK_PAIRS = 8192      # ONE_BLOCK_PAIRS of csrc/moe.cu
+
+
 def moe_group(ids: torch.Tensor, counts: torch.Tensor, table: RoutingTable) -> None:
     """Fill ``table`` from the chosen outputs ``ids`` [tokens, top]; outputs >= ``table.n_experts`` (identity
     outputs) and -1 take no place.  ``counts`` [experts] int32 must be zero and is zero again afterwards."""
@@ -1416,7 +1419,7 @@ def moe_group(ids: torch.Tensor, counts: torch.Tensor, table: RoutingTable) -> N
         raise KernelError("the routing table was made for other sizes")
     lib = load_library("moe")
     _check(lib.odi_moe_group(byref(_grouping(ids, counts, table)), _stream()), "moe_group",
-           1 if table.n_pairs <= 16384 and table.n_experts <= 4096 else 3)
+           1 if table.n_pairs <= MOE_ONE_BLOCK_PAIRS and table.n_experts <= 4096 else 3)
 
 
 def _grouping(ids: Optional[torch.Tensor], counts: torch.Tensor, table: RoutingTable) -> "_GroupingArgs":
@@ -1442,7 +1445,7 @@ def moe_table_group(route: torch.Tensor, token_ids: torch.Tensor, ids: torch.Ten
     lib = load_library("moe")
     _check(lib.odi_moe_table_group(byref(_grouping(ids, counts, table)), _ptr(route), _ptr(token_ids), _ptr(ids), _ptr(weights), c_int(top),
                                    c_int(route.shape[0]), c_float(weight), _stream()), "moe_table_group",
-           1 if table.n_pairs <= 16384 and table.n_experts <= 4096 else 4)
+           1 if table.n_pairs <= MOE_ONE_BLOCK_PAIRS and table.n_experts <= 4096 else 4)
 
 
 def moe_gather(x: torch.Tensor, table: RoutingTable, out: torch.Tensor, weights: Optional[torch.Tensor] = None) -> None:

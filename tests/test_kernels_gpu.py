@@ -3,6 +3,7 @@ other than the tiny models': widths and vocabularies that are no power of two, h
 16..256, any number of heads and groups, ragged batches."""
 
 import math
+from pathlib import Path
 
 import pytest
 import torch
@@ -546,7 +547,7 @@ def test_gemm_prefill_clamps_and_gates_in_its_epilogue(tokens, I, K, biased):
     assert ops.gemm_status() == 0
 
 
-# one block of 256 threads up to 2,048 pairs, of 1,024 up to 16,384, three launches beyond
+# one block of 256 threads up to 2,048 pairs, of 1,024 up to 8,192, three launches beyond
 @pytest.mark.parametrize("tokens,top,experts", [(512, 4, 30), (683, 3, 7), (2731, 3, 300), (4096, 4, 32), (16385, 1, 5)])
 def test_pairs_are_sorted_by_expert(tokens, top, experts):
     torch.manual_seed(tokens)
@@ -564,6 +565,21 @@ def test_pairs_are_sorted_by_expert(tokens, top, experts):
     assert torch.equal(table.pos[perm].long(), torch.arange(n, device=DEV))
     tiles = int(table.n_tiles)
     assert tiles == int(((want + table.tm - 1) // table.tm).sum()) and int(table.tile_rows[:tiles].sum()) == n
+
+
+@pytest.mark.parametrize("pairs,launches", [(2049, 1), (8192, 1), (8193, 3)])
+def test_pairs_at_the_edges_of_one_block(pairs, launches):
+    torch.manual_seed(pairs)
+    ids = torch.randint(0, 300, (pairs, 1), dtype=torch.int32, device=DEV)
+    table = ops.RoutingTable(pairs, 1, 300, torch.device(DEV), tensor=True)
+    counts = torch.zeros(300, dtype=torch.int32, device=DEV)
+    before = ops.LAUNCHES["own"]
+    ops.moe_group(ids, counts, table)
+    assert ops.LAUNCHES["own"] - before == launches
+    assert f"#define ONE_BLOCK_PAIRS {ops.MOE_ONE_BLOCK_PAIRS}\n" in (Path(ops.__file__).parents[1] / "csrc" / "moe.cu").read_text()
+    flat = ids.flatten().long()
+    assert torch.equal(table.offsets.long(), torch.cat([flat.new_zeros(1), torch.bincount(flat, minlength=300).cumsum(0)]))
+    assert torch.equal(flat[table.perm.long()], flat.sort().values) and int(counts.abs().sum()) == 0
 
 
 @pytest.mark.parametrize("tokens,top,experts", [(3, 2, 5), (512, 4, 30), (4096, 4, 32), (16385, 1, 5)])
