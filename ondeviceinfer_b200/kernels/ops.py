@@ -1471,9 +1471,10 @@ class _CombineArgs(Structure):
                 ("n_experts", c_int), ("out_is_t", c_int), ("assign", c_int), ("shared", c_void_p), ("gate", c_void_p)]
 
 
-def moe_combine_gates(x: torch.Tensor, gate: torch.Tensor) -> bool:
-    """Whether :func:`moe_combine` takes a gated shared expert along for rows like ``x``."""
-    return x.dtype == torch.bfloat16 and x.shape[1] % 8 == 0 and x.data_ptr() % 16 == 0 and gate.data_ptr() % 16 == 0
+def moe_combine_gates(x: torch.Tensor, gate: torch.Tensor, *others: torch.Tensor) -> bool:
+    """Whether :func:`moe_combine` takes a gated shared expert along for rows like ``x``; ``others``: its residual, the experts' rows and
+    the shared expert's."""
+    return x.dtype == torch.bfloat16 and x.shape[1] % 8 == 0 and all(t.data_ptr() % 16 == 0 for t in (x, gate, *others))
 
 
 def moe_combine(residual: torch.Tensor, expert_out: torch.Tensor, x: torch.Tensor, ids: torch.Tensor,

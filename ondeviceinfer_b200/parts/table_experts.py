@@ -99,13 +99,13 @@ class TableExperts(Part):
         gated = s.shared_size > 0 and self.w_shared_gate is not None
         if s.shared_size > 0:
             shared = activated_linear(x, self.w_shared_up, s.activation)
-        if gated and ops.moe_combine_gates(x, self.w_shared_gate):
-            y = linear(shared, self.w_shared_down, out_dtype=torch.float32)
+        y = linear(shared, self.w_shared_down, out_dtype=torch.float32) if gated else None
+        if gated and ops.moe_combine_gates(x, self.w_shared_gate, residual, expert_out, y):
             ops.moe_combine(residual, expert_out, x, ids, weights, table, assign=assign, shared=(y, self.w_shared_gate))
         else:
             ops.moe_combine(residual, expert_out, x, ids, weights, table, assign=assign)
             if gated:
-                ops.gated_row_add(residual, linear(shared, self.w_shared_down, out_dtype=torch.float32), x, self.w_shared_gate)
+                ops.gated_row_add(residual, y, x, self.w_shared_gate)
             elif s.shared_size > 0:
                 linear(shared, self.w_shared_down, residual=residual)
         if ctx is not None:
