@@ -629,6 +629,28 @@ def test_combine_takes_a_gated_shared_expert_along(tokens, H, wide):
         torch.testing.assert_close(one, two, atol=2e-6, rtol=2e-6)      # the gate's sum of H products in another order
 
 
+def test_a_gated_shared_expert_joins_a_residual_off_16_byte_borders():
+    from ondeviceinfer_b200.config.specs import TableExpertsSpec
+    from ondeviceinfer_b200.engine.step import StepDescription
+    from ondeviceinfer_b200.parts import Runtime, build_part
+    gen = torch.Generator().manual_seed(6)
+    n, H = 9, 64
+    part = build_part(TableExpertsSpec(hidden_size=H, expert_size=32, num_experts=3, top_k=2, vocab_size=3, prefix="", shared_size=48))
+    w = {d.name: torch.tensor([[0, 1], [1, 2], [2, 0]], dtype=torch.int32, device=DEV) if "distinct" in d.init else
+         (torch.randn(*d.shape, generator=gen) / math.sqrt(d.shape[-1])).bfloat16().to(DEV) for d in part.tensor_decls()}
+    part.load(type("Fetch", (), {name: staticmethod(w.__getitem__) for name in ("matrix", "vector", "integer")}),
+              Runtime(dtype=torch.bfloat16, device=torch.device(DEV)))
+    x, start = torch.randn(n, H, generator=gen).bfloat16().to(DEV), torch.randn(n, H, generator=gen).to(DEV)
+    sums = []
+    for offset in (0, 1):
+        residual = torch.empty(n * H + 1, device=DEV)[offset:offset + n * H].view(n, H).copy_(start)
+        ctx = StepDescription()
+        ctx.token_ids = (torch.arange(n, device=DEV) % 3).int()
+        part.forward(x, ctx, residual)
+        sums.append(residual.clone())
+    torch.testing.assert_close(sums[0], sums[1], atol=4e-6, rtol=4e-6)      # sums of two experts and of the gate's products in another order
+
+
 @pytest.mark.parametrize("H", [64, 2056, 20])
 def test_gathered_rows_times_their_weights(H):
     torch.manual_seed(H)
