@@ -52,6 +52,17 @@ __device__ __forceinline__ bool elect_one() {
 }
 __device__ __forceinline__ int warp_index() { return __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0); }      // the same for the whole warp, and known to be
 
+// n / d of the gates, d from 1 to infinity: the product with an approximate reciprocal and one step of Newton's iteration on the quotient
+// (Markstein, Computation of elementary functions on the IBM RISC System/6000 processor, 1990), which gave the bits of / for all of 2^25 gates
+// from -88.7 to 88.3; the product itself where the step has no number to go by (an infinite n or d).  Written out, / branches for its rare
+// operands; __fdividef is off by two ulps and gives 0 for d beyond 2^126 (SiLU of -87.4 to -88.7).
+__device__ __forceinline__ float quotient(float n, float d) {
+  float r;
+  asm("rcp.approx.f32 %0, %1;" : "=f"(r) : "f"(d));
+  const float q = n * r, better = fmaf(fmaf(-q, d, n), r, q);
+  return better == better ? better : q;
+}
+
 // Sum over a block of up to 1024 threads; every thread gets the result.  `scratch` is
 // 33 floats of shared memory.  The order of additions is fixed by the thread layout.
 __device__ __forceinline__ float block_sum(float v, float* scratch) {

@@ -158,24 +158,8 @@ __device__ __forceinline__ uint64_t smem_desc_k_sw128(uint32_t addr) {
 __host__ __device__ constexpr uint32_t instr_desc_bf16(int m, int n) {
   return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(m >> 4) << 24);
 }
-// n / d of the gates, d from 1 to infinity: the product with an approximate reciprocal and one step of Newton's iteration on the quotient
-// (Markstein, Computation of elementary functions on the IBM RISC System/6000 processor, 1990), which gave the bits of / for all of 2^25 gates
-// from -88.7 to 88.3; the product itself where the step has no number to go by (an infinite n or d).  Written out, / branches for its rare
-// operands and kept the four epilogue warps behind the MMAs; __fdividef is off by two ulps and gives 0 for d beyond 2^126 (SiLU of -87.4
-// to -88.7).  Prompts of 700 to 3,001 tokens, eight layers of 2 x 12,288 x 4,096 with SiLU, whole pass, us: / 18,627, __fdividef 17,975
-// to 18,075, this 18,159.
-__device__ __forceinline__ float quotient(float n, float d) {
-  float r;
-  asm("rcp.approx.f32 %0, %1;" : "=f"(r) : "f"(d));
-  const float q = n * r, better = fmaf(fmaf(-q, d, n), r, q);
-  return better == better ? better : q;
-}
-// The clamped gate's, whose sums were rounded to bf16 before they were gated until its epilogue took it: __fdividef as far as it goes.
-__device__ __forceinline__ float quick_quotient(float n, float d) {
-  float r;
-  asm("rcp.approx.f32 %0, %1;" : "=f"(r) : "f"(d));
-  return d > 8.5070592e37f ? n * r : __fdividef(n, d);      // 2^126
-}
+// The gates' quotients (common.cuh) written with / kept the four epilogue warps behind the MMAs.  Prompts of 700 to 3,001 tokens, eight layers of
+// 2 x 12,288 x 4,096 with SiLU, whole pass, us: / 18,627, __fdividef 17,975 to 18,075, this 18,159.
 __device__ __forceinline__ float silu_f(float g) { return quotient(g, 1.f + __expf(-g)); }
 // 0.5 g (1 + tanh y) = g sigmoid(2 y), y = sqrt(2/pi) (g + 0.044715 g^3)
 __device__ __forceinline__ float gelu_tanh_f(float g) {
@@ -187,7 +171,7 @@ __device__ __forceinline__ float gated_f(const PrefillGemmArgs& a, float g, floa
   if (EPI == EPI_GEGLU) return gelu_tanh_f(g) * u;
   g = fminf(g, a.limit);
   u = fminf(fmaxf(u, -a.limit), a.limit);
-  return quick_quotient(g, 1.f + __expf(-a.alpha * g)) * (u + a.shift);
+  return quotient(g, 1.f + expf(-a.alpha * g)) * (u + a.shift);
 }
 __device__ __forceinline__ float relu2_f(float z) { const float r = fmaxf(z, 0.f); return r * r; }
 __device__ __forceinline__ float gelu_erf_f(float z) { return 0.5f * z * (1.0f + erff(z * 0.70710678118654752440f)); }

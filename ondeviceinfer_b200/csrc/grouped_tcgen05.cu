@@ -171,15 +171,12 @@ __device__ __forceinline__ uint32_t instr_desc_bf16(int m, int n) {
 }
 
 // 0.5 g (1 + tanh y) = g sigmoid(2 y), y = sqrt(2/pi) (g + 0.044715 g^3)
-__device__ __forceinline__ float gelu_tanh_f(float g) { return __fdividef(g, 1.f + __expf(-1.5957691216057308f * fmaf(0.044715f * g * g, g, g))); }
+__device__ __forceinline__ float gelu_tanh_f(float g) { return quotient(g, 1.f + expf(-1.5957691216057308f * fmaf(0.044715f * g * g, g, g))); }
 __device__ __forceinline__ float gelu_erf_f(float z) { return 0.5f * z * (1.0f + erff(z * 0.70710678118654752440f)); }
 __device__ __forceinline__ float gated(const ExpertsArgs& a, float g, float u) {
   g = fminf(g, a.limit);
   u = fminf(fmaxf(u, -a.limit), a.limit);
-  const float d = 1.f + __expf(-a.alpha * g);
-  float r;
-  asm("rcp.approx.f32 %0, %1;" : "=f"(r) : "f"(d));
-  return (d > 8.5070592e37f ? g * r : __fdividef(g, d)) * (u + a.shift);      // __fdividef gives 0 for d beyond 2^126
+  return quotient(g, 1.f + expf(-a.alpha * g)) * (u + a.shift);
 }
 template <int EPI>
 __device__ __forceinline__ float plain(float v) {

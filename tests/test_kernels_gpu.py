@@ -486,6 +486,32 @@ def test_gates_over_the_whole_range_of_their_quotient(kind):
     assert ops.gemm_status() == 0
 
 
+@pytest.mark.parametrize("alpha", [1.0, 1.702])
+@pytest.mark.parametrize("kind", ["clamp", "experts"])
+def test_clamped_gates_are_rounded_once_behind_fp32(kind, alpha):
+    """32,768 gates from -80 to 7 with ups around 1: an exponent off by a hundred units in fp32's last place would take dozens of them across a
+    rounding border of bf16."""
+    gen = torch.Generator().manual_seed(7)
+    N, n, K, shift = 4096, 8, 64, 0.375
+    w = torch.zeros(2 * N, K)
+    w[:N, :n], w[N:, :n] = torch.rand(N, n, generator=gen) * 87.0 - 80.0, torch.randn(N, n, generator=gen)
+    w = w.bfloat16().to(DEV)
+    x = torch.eye(n, K).bfloat16().to(DEV)      # a sum is one number of w
+    out = torch.empty(n, N, dtype=torch.bfloat16, device=DEV)
+    if kind == "experts":
+        ops.grouped_gemm_sorted(x, w[None], out, torch.tensor([0, n], dtype=torch.int32, device=DEV), epi=ops.GROUPED_GATED_CLAMP, limit=6.0,
+                                alpha=alpha, up_shift=shift)
+    else:
+        ops.gemm_prefill_bf16(x, w, out, ops.EPI_GATED_CLAMP, limit=6.0, alpha=alpha, up_shift=shift)
+    g, u = w[:N, :n].t().float().clamp(max=6.0), w[N:, :n].t().float().clamp(-6.0, 6.0)
+    e = torch.exp(-(alpha * g).double())
+    want = torch.where(e < 2.0 ** 128, g.double() / (1.0 + e), 0.0) * (u + shift).double()      # beyond that fp32 holds an infinity
+    # half a unit of bf16, and fp32's: expf 4 x 2^-24, the sum below the quotient, the quotient and the product 2^-24 each
+    half = torch.exp2(want.abs().log2().floor().clamp(min=-126) - 8)
+    assert bool(((out.double() - want).abs() <= half + 8 * 2.0 ** -24 * want.abs())[want != 0].all())
+    assert ops.gemm_status() == 0
+
+
 @pytest.mark.parametrize("form", ["gated_clamp", "relu2", "table"])
 def test_experts_of_a_captured_step_keep_their_outputs_in_32_bits(form):
     """64 rows an expert, from where on the outputs of a step that is launched kernel by kernel are rounded to bf16: in a graph, and in the run
