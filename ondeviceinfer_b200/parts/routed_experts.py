@@ -6,9 +6,9 @@ Steps of ``forward`` (no step waits for the host):
    choice only, the best groups, the top-k outputs and their scores as weights;
 2. ``ops.moe_group``: the (token, choice) pairs that go to real experts, sorted by expert on the device;
 3. two grouped products over that order (``csrc/grouped_gemm.cu``): gate and up with the clamped activation,
-   then down into fp32 rows; in bfloat16, when the experts get some rows each (prompts), the rows are gathered
-   side by side instead and the two products go to tcgen05 (``csrc/grouped_tcgen05.cu``) over the experts' row ranges; of many rows
-   where that kernel refuses the sizes every expert's products go through ``linear``, for which the
+   then down into fp32 rows; in bfloat16, when the experts get many rows each (prompts), the rows are gathered
+   side by side instead and the two products go to tcgen05 (``csrc/grouped_tcgen05.cu``) over the experts' row ranges, or,
+   where that kernel refuses the sizes, every expert's products go through ``linear``, for which the
    host reads the experts' offsets once (the only wait of the part, and never inside a graph capture);
 4. ``ops.moe_combine``: each token adds its weighted rows, in the order of its choices, and its own input for
    an identity output;
@@ -34,15 +34,17 @@ from .base import Part, register_part
 from .linear import clamped_gated_linear, gated_linear, linear
 
 
-# From this many rows per expert on (on average) the experts of a bfloat16 step go to tcgen05 over gathered rows.  Measured, gather and both
-# products against the form that gathers in its loads (mma.sync), us, 30 experts of 2,048 and 1,024: 4 rows 77 / 71, 8 77 / 79, 16 78 / 121,
-# 32 80 / 187; 128 experts of 1,024 and 512: 4 77 / 77, 8 78 / 96, 15 79 / 142.
-# Ungated experts go there only with ROWS_PER_EXPERT_ROUNDED rows, and their sums, like the shared expert's, are rounded before the squared
-# ReLU (max(z, 0)^2 of a bfloat16 product, as an activation behind it gives): their layers weigh the experts' inputs by a router's
-# scores, and rounded once, after the activation, they moved the logits by 0.027 of their norm where two scores nearly tied.
-ROWS_PER_EXPERT_FOR_TCGEN05 = 8
-# From this many on the experts' outputs are rounded to the compute dtype (half the bytes of many rows), and experts that tcgen05 refuses run
-# one by one through linear(), which waits for the host: neither in a step of a graph, whose outputs stay fp32 at any number of rows.
+# From this many rows per expert on (on average) the experts' outputs are rounded to the compute dtype (half the bytes of many rows), and the
+# products go to tcgen05 over gathered rows (experts that it refuses one by one through linear(), which waits for the host): neither in a
+# step of a graph, whose outputs stay fp32 at any number of rows.  fp32 outputs come from the form that gathers in its loads
+# (mma.sync), which sums 16 k inside the tensor core and joins those sums in fp32, where tcgen05 keeps all of K in one sum that cuts off: down
+# products of 512 / 1,024 / 2,048 k are 7.1e-8 / 7.6e-8 / 8.2e-8 of their norm from 64 bits, on tcgen05 6.0e-7 / 1.2e-6 / 2.4e-6 (rounded to
+# bfloat16 both are 1.7e-3).  What that costs, gather and both products with the weights from memory, us, mma.sync / tcgen05, experts of 2,048 and 1,024:
+# 30 of 8 rows 80 / 95, of 16 108 / 95, of 31 170 / 97, four of 30 with all rows 62 / 33, 92 / 37, 157 / 43; 8 experts of 1,024 and 512, 8 rows 18 / 23,
+# 31 rows 29 / 24.  tcgen05 for gate and up alone gains nothing (30 x 16 rows 128, 31 rows 168).
+# Ungated experts' sums, like the shared expert's, are rounded before the squared ReLU (max(z, 0)^2 of a bfloat16 product, as an activation
+# behind it gives): their layers weigh the experts' inputs by a router's scores, and rounded once, after the activation, they moved the logits by
+# 0.027 of their norm where two scores nearly tied.
 ROWS_PER_EXPERT_ROUNDED = 32
 
 
@@ -132,15 +134,13 @@ class RoutedExperts(Part):
             act = torch.empty((table.n_pairs, s.expert_size), dtype=x.dtype, device=dev)
             first_epi = ops.GROUPED_GATED_CLAMP if self.gated else ops.GROUPED_RELU2
             many = rounds_outputs(x.dtype, table, ctx)
-            tcgen05 = table.n_pairs >= ROWS_PER_EXPERT_FOR_TCGEN05 * s.num_experts if self.gated else many
-            if tcgen05 and ops.grouped_tcgen05_ok(x.dtype, self.w_gate_up, self.w_down):
+            if many and ops.grouped_tcgen05_ok(x.dtype, self.w_gate_up, self.w_down):
                 rows = torch.empty((table.n_pairs, s.hidden_size), dtype=x.dtype, device=dev)
                 ops.moe_gather(x, table, rows, weights if s.weight_on_input else None)
                 ops.grouped_gemm_sorted(rows, self.w_gate_up, act, table.offsets, epi=first_epi, limit=self.limit, alpha=self.gate_alpha,
                                         up_shift=self.up_shift, round_sums=not self.gated)
-                # the gathered rows were read by the first product: of many rows the outputs, of the same size, take their place
-                expert_out = rows if many else wide_out()
-                ops.grouped_gemm_sorted(act, self.w_down, expert_out, table.offsets, epi=ops.GROUPED_STORE if many else ops.GROUPED_STORE_F32)
+                expert_out = rows           # read by the first product: the outputs, of the same size, take their place
+                ops.grouped_gemm_sorted(act, self.w_down, expert_out, table.offsets, epi=ops.GROUPED_STORE)
             elif many:
                 expert_out = wide_out()
                 self._experts_one_by_one(x, table, act, expert_out, weights)

@@ -6,7 +6,7 @@ Steps of ``forward`` (no step waits for the host):
 1. the token's experts are row ``token id`` of the table, each weighted 1 / top;
 2. the (token, choice) pairs sorted by expert on the device, with 1 in ``ops.moe_table_group``, once a step;
 3. two grouped products over that order (``csrc/grouped_gemm.cu``): up with the activation in its epilogue, then
-   down into fp32 rows; in bfloat16, when the experts get some rows each (prompts), the rows are gathered side by
+   down into fp32 rows; in bfloat16, when the experts get many rows each (prompts), the rows are gathered side by
    side and the products go to tcgen05 (``csrc/grouped_tcgen05.cu``) over the experts' row ranges;
 4. ``ops.moe_combine``: each token adds its weighted rows in the order of its choices;
 5. the shared expert, if any: up, activation, down, added times sigmoid(sg . x): by the kernel of 4, which it then comes before, or by
@@ -22,7 +22,7 @@ from ..kernels import ops
 from ..weights.tensors import TensorDecl
 from .base import Part, register_part
 from .linear import activated_linear, linear
-from .routed_experts import ROWS_PER_EXPERT_FOR_TCGEN05, rounds_outputs
+from .routed_experts import rounds_outputs
 
 GROUPED_EPILOGUE = {"gelu_erf": ops.GROUPED_GELU_ERF, "gelu_tanh": ops.GROUPED_GELU_TANH}
 
@@ -80,15 +80,12 @@ class TableExperts(Part):
         # the tokens alone decide: a layer that a step runs twice is routed once
         ids, weights, table = ctx.memo(("table_routing", self, tensor), route)
         act = torch.empty((table.n_pairs, s.expert_size), dtype=x.dtype, device=dev)
-        if (x.dtype == torch.bfloat16 and table.n_pairs >= ROWS_PER_EXPERT_FOR_TCGEN05 * s.num_experts
-                and ops.grouped_tcgen05_ok(x.dtype, self.w_up, self.w_down)):
+        if rounds_outputs(x.dtype, table, ctx) and ops.grouped_tcgen05_ok(x.dtype, self.w_up, self.w_down):
             rows = torch.empty((table.n_pairs, s.hidden_size), dtype=x.dtype, device=dev)
             ops.moe_gather(x, table, rows)
             ops.grouped_gemm_sorted(rows, self.w_up, act, table.offsets, epi=GROUPED_EPILOGUE[s.activation])
-            many = rounds_outputs(x.dtype, table, ctx)
-            # the gathered rows were read by the first product: of many rows the outputs, of the same size, take their place
-            expert_out = rows if many else torch.empty((table.n_pairs, s.hidden_size), dtype=torch.float32, device=dev)
-            ops.grouped_gemm_sorted(act, self.w_down, expert_out, table.offsets, epi=ops.GROUPED_STORE if many else ops.GROUPED_STORE_F32)
+            expert_out = rows               # read by the first product: the outputs, of the same size, take their place
+            ops.grouped_gemm_sorted(act, self.w_down, expert_out, table.offsets, epi=ops.GROUPED_STORE)
         else:
             expert_out = torch.empty((table.n_pairs, s.hidden_size), dtype=torch.float32, device=dev)
             ops.grouped_gemm_routed(x, self.w_up, act, table, gather=True, epi=GROUPED_EPILOGUE[s.activation])

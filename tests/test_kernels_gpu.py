@@ -486,6 +486,46 @@ def test_gates_over_the_whole_range_of_their_quotient(kind):
     assert ops.gemm_status() == 0
 
 
+@pytest.mark.parametrize("form", ["gated_clamp", "relu2", "table"])
+def test_experts_whose_outputs_stay_in_32_bits_join_short_sums_in_fp32(form):
+    """16 rows an expert: down products over 2,048 k of numbers as bfloat16 holds them, against 64 bits.  Sums of 16 k inside the tensor core cut off
+    at most 2^-22 of their size, and the seven joins above them round at 2^-24 each; one sum of all 2,048 k in there is some 2.4e-6 off."""
+    from ondeviceinfer_b200.config.specs import RoutedExpertsSpec, TableExpertsSpec
+    from ondeviceinfer_b200.engine.step import StepDescription
+    from ondeviceinfer_b200.parts import Runtime, build_part
+    gen = torch.Generator().manual_seed(8)
+    n, H, F, E = 16, 128, 2048, 2
+    if form == "table":
+        part = build_part(TableExpertsSpec(hidden_size=H, expert_size=F, num_experts=E, top_k=E, vocab_size=3, prefix=""))
+    else:
+        part = build_part(RoutedExpertsSpec(hidden_size=H, expert_size=F, num_experts=E, num_identity=0, top_k=E, num_groups=1, keep_groups=1,
+                                            limit=1.5, prefix="", has_correction=False, expert_form=form))
+    w = {d.name: torch.tensor([[0, 1]] * 3, dtype=torch.int32, device=DEV) if "distinct" in d.init else
+         (torch.randn(*d.shape, generator=gen) / math.sqrt(d.shape[-1])).bfloat16().to(DEV) for d in part.tensor_decls()}
+    part.load(type("Fetch", (), {name: staticmethod(w.__getitem__) for name in ("matrix", "vector", "integer")}),
+              Runtime(dtype=torch.bfloat16, device=torch.device(DEV)))
+    ctx = StepDescription()
+    ctx.token_ids = torch.zeros(n, dtype=torch.int32, device=DEV)
+    seen, real = [], (ops.grouped_gemm_routed, ops.grouped_gemm_sorted, ops.moe_combine)
+    def watched(product):
+        def call(x, *args, **kw):
+            seen.append(x)
+            return product(x, *args, **kw)
+        return call
+    def combine(residual, expert_out, x, ids, weights, table, **kw):
+        seen.extend((expert_out.clone(), ids, table))
+        return real[2](residual, expert_out, x, ids, weights, table, **kw)
+    ops.grouped_gemm_routed, ops.grouped_gemm_sorted, ops.moe_combine = watched(real[0]), watched(real[1]), combine
+    try:
+        part.forward(torch.randn(n, H, generator=gen).bfloat16().to(DEV), ctx, None)
+    finally:
+        ops.grouped_gemm_routed, ops.grouped_gemm_sorted, ops.moe_combine = real
+    _, act, out, ids, table = seen
+    expert = ids.flatten()[table.perm[:n * E].long()].long()
+    want = torch.einsum("rf,rhf->rh", act.double(), part.w_down.double()[expert])
+    assert out.dtype == torch.float32 and float((out.double() - want).norm() / want.norm()) < 2.0 ** -22 + 7 * 2.0 ** -24
+
+
 @pytest.mark.parametrize("alpha", [1.0, 1.702])
 @pytest.mark.parametrize("kind", ["clamp", "experts"])
 def test_clamped_gates_are_rounded_once_behind_fp32(kind, alpha):
