@@ -54,7 +54,8 @@
 #define EPI_GEGLU 6        // bf16 out = gelu(acc_gate) * acc_up, the tanh form of GELU; weight rows as for EPI_SWIGLU
 #define EPI_RELU2 7        // out_bf16[token, n] = max(acc, 0)^2
 #define EPI_GATED_CLAMP 8  // bf16 out = g sigmoid(alpha g) (u + shift) of g = min(acc_gate, limit), u = acc_up within +-limit
-#define EPI_IS_GATED(e) ((e) == EPI_SWIGLU || (e) == EPI_GEGLU || (e) == EPI_GATED_CLAMP)
+#define EPI_GATED_CLAMP_ROUNDED 9      // the same of the sums as bf16 holds them: the bits of EPI_STORE_BF16 and gated_clamp_kernel behind it
+#define EPI_IS_GATED(e) ((e) == EPI_SWIGLU || (e) == EPI_GEGLU || (e) == EPI_GATED_CLAMP || (e) == EPI_GATED_CLAMP_ROUNDED)
 
 #define BM 128             // token rows per CTA (the lanes of its tensor memory); a tile has 2 * BM
 #define BN 256             // accumulator columns per tile
@@ -78,7 +79,7 @@ struct PrefillGemmArgs {
   // other (see segment_of); flags: two counters per tile, zero on entry and left zero.
   int parts;
   int* flags;
-  float limit, alpha, shift;      // EPI_GATED_CLAMP
+  float limit, alpha, shift;      // of the clamped gates
   HeadPrepArgs hp;         // EPI_HEAD_PREP
 };
 
@@ -169,6 +170,7 @@ template <int EPI>
 __device__ __forceinline__ float gated_f(const PrefillGemmArgs& a, float g, float u) {
   if (EPI == EPI_SWIGLU) return silu_f(g) * u;
   if (EPI == EPI_GEGLU) return gelu_tanh_f(g) * u;
+  if (EPI == EPI_GATED_CLAMP_ROUNDED) { g = __bfloat162float(__float2bfloat16_rn(g)); u = __bfloat162float(__float2bfloat16_rn(u)); }
   g = fminf(g, a.limit);
   u = fminf(fmaxf(u, -a.limit), a.limit);
   return quotient(g, 1.f + expf(-a.alpha * g)) * (u + a.shift);
@@ -607,7 +609,7 @@ static int launch(const CUtensorMap& mx, const CUtensorMap& mw, const CUtensorMa
 // receives an error code if a wait gives up.
 // EPI_HEAD_PREP: out is not used; head_prep describes where the heads go (heads of 128, whole-head rotation or
 // none, keys and values written).
-// limit, alpha, shift: of EPI_GATED_CLAMP.
+// limit, alpha, shift: of the clamped gates.
 // bias: null, or fp32 [w_rows] (16-byte aligned), added to the product.
 // flags: n_flags ints, zero on entry and left zero (two per tile are used when the work is balanced).
 extern "C" int odi_gemm_prefill_bf16(const void* x, const void* w, void* out, int tokens, int n_out, int K, int w_rows,
@@ -690,6 +692,7 @@ extern "C" int odi_gemm_prefill_bf16(const void* x, const void* w, void* out, in
     case EPI_SWIGLU: return launch<EPI_SWIGLU>(mx, mw, mo, a, sms, stream);
     case EPI_GEGLU: return launch<EPI_GEGLU>(mx, mw, mo, a, sms, stream);
     case EPI_GATED_CLAMP: return launch<EPI_GATED_CLAMP>(mx, mw, mo, a, sms, stream);
+    case EPI_GATED_CLAMP_ROUNDED: return launch<EPI_GATED_CLAMP_ROUNDED>(mx, mw, mo, a, sms, stream);
     case EPI_HEAD_PREP: return launch<EPI_HEAD_PREP>(mx, mw, mo, a, sms, stream);
   }
   return ODI_ERR_ARGUMENT;

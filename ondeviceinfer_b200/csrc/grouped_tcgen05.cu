@@ -28,7 +28,12 @@
 #define EPI_RELU2 3
 #define EPI_STORE_F32 5
 #define EPI_GATED_CLAMP 4  // g sigmoid(alpha g) (u + shift) of g <= limit, |u| <= limit
-#define EPI_RELU2_ROUNDED 6      // max(z, 0)^2 of the sum as bf16 holds it: what a product that stores bf16 and an activation behind it give
+// The same of the sums as bf16 holds them: the bits of a product that stores bf16 and the activation's kernel behind it
+#define EPI_RELU2_ROUNDED 6
+#define EPI_GATED_CLAMP_ROUNDED 7
+#define EPI_GELU_ROUNDED 8
+#define EPI_GELU_TANH_ROUNDED 9
+#define EPI_IS_GATED(e) ((e) == EPI_GATED_CLAMP || (e) == EPI_GATED_CLAMP_ROUNDED)
 
 #define BF 128             // weight rows per CTA
 #define BK 64              // k per stage
@@ -173,7 +178,12 @@ __device__ __forceinline__ uint32_t instr_desc_bf16(int m, int n) {
 // 0.5 g (1 + tanh y) = g sigmoid(2 y), y = sqrt(2/pi) (g + 0.044715 g^3)
 __device__ __forceinline__ float gelu_tanh_f(float g) { return quotient(g, 1.f + expf(-1.5957691216057308f * fmaf(0.044715f * g * g, g, g))); }
 __device__ __forceinline__ float gelu_erf_f(float z) { return 0.5f * z * (1.0f + erff(z * 0.70710678118654752440f)); }
+// In the activation kernel's form.
+__device__ __forceinline__ float gelu_tanh_kernel_f(float z) { return 0.5f * z * (1.0f + tanhf(0.79788456080286535588f * (z + 0.044715f * z * z * z))); }
+__device__ __forceinline__ float rounded(float v) { return __bfloat162float(__float2bfloat16_rn(v)); }
+template <int EPI>
 __device__ __forceinline__ float gated(const ExpertsArgs& a, float g, float u) {
+  if (EPI == EPI_GATED_CLAMP_ROUNDED) { g = rounded(g); u = rounded(u); }
   g = fminf(g, a.limit);
   u = fminf(fmaxf(u, -a.limit), a.limit);
   return quotient(g, 1.f + expf(-a.alpha * g)) * (u + a.shift);
@@ -183,7 +193,9 @@ __device__ __forceinline__ float plain(float v) {
   if (EPI == EPI_GELU) return gelu_erf_f(v);
   if (EPI == EPI_GELU_TANH) return gelu_tanh_f(v);
   if (EPI == EPI_RELU2) { const float r = fmaxf(v, 0.f); return r * r; }
-  if (EPI == EPI_RELU2_ROUNDED) { const float r = fmaxf(__bfloat162float(__float2bfloat16_rn(v)), 0.f); return r * r; }
+  if (EPI == EPI_RELU2_ROUNDED) { const float r = fmaxf(rounded(v), 0.f); return r * r; }
+  if (EPI == EPI_GELU_ROUNDED) return gelu_erf_f(rounded(v));
+  if (EPI == EPI_GELU_TANH_ROUNDED) return gelu_tanh_kernel_f(rounded(v));
   return v;
 }
 
@@ -206,7 +218,7 @@ __device__ __forceinline__ bool unit_of(const ExpertsArgs& a, const int* first, 
 template <int EPI>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
 grouped_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w, const ExpertsArgs a) {
-  constexpr bool GATE = EPI == EPI_GATED_CLAMP;
+  constexpr bool GATE = EPI_IS_GATED(EPI);
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   // full (leader's), empty (each CTA's), acc_full (each CTA's), acc_empty (leader's)
@@ -354,11 +366,11 @@ grouped_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_c
           asm volatile("bar.sync %0, 64;" ::"r"(2 + exchange) : "memory");
           if (lane_group < 2) {
 #pragma unroll
-            for (int i = 0; i < 8; ++i) v[i] = gated(a, v[i], take[32 * i]);
+            for (int i = 0; i < 8; ++i) v[i] = gated<EPI>(a, v[i], take[32 * i]);
           } else {
             from = 8;
 #pragma unroll
-            for (int i = 0; i < 8; ++i) v[i] = gated(a, take[32 * i], v[8 + i]);
+            for (int i = 0; i < 8; ++i) v[i] = gated<EPI>(a, take[32 * i], v[8 + i]);
           }
         } else {
 #pragma unroll
@@ -452,13 +464,13 @@ static int launch(const CUtensorMap& mx, const CUtensorMap& mw, const ExpertsArg
   return launch_status();
 }
 
-// x [rows, K] bf16, w [groups, w_rows, K] bf16 (EPI_GATED_CLAMP: the gate rows, then the up rows; n_out = w_rows / 2), out [rows, n_out] in bf16, or fp32 for EPI_STORE_F32,
+// x [rows, K] bf16, w [groups, w_rows, K] bf16 (gated: the gate rows, then the up rows; n_out = w_rows / 2), out [rows, n_out] in bf16, or fp32 for EPI_STORE_F32,
 // offsets [groups + 1] ints on the device, rising from 0 to at most `rows`; rows beyond the last are not touched.  K a multiple of 8, x and w on
 // 16-byte boundaries.  status: receives a code if a wait gives up; withheld: 0, or 1 for a self-test of that.
 extern "C" int odi_grouped_tcgen05(const void* x, const void* w, void* out, const int* offsets, int rows, int groups, int n_out, int K,
                                    int w_rows, int epi, float limit, float alpha, float shift, int* status, int withheld, cudaStream_t stream) {
   if (rows <= 0 || n_out <= 0) return 0;
-  const bool gate = epi == EPI_GATED_CLAMP;
+  const bool gate = EPI_IS_GATED(epi);
   if (K <= 0 || status == nullptr || offsets == nullptr || groups < 1 || (gate ? w_rows != 2 * n_out : w_rows != n_out)) return ODI_ERR_ARGUMENT;
   if (K % 8 || ((uintptr_t)x & 15) || ((uintptr_t)w & 15) || ((uintptr_t)out & 3) || groups > MAX_GROUPS) return ODI_ERR_UNSUPPORTED;
   int pairs = 0;
@@ -479,6 +491,9 @@ extern "C" int odi_grouped_tcgen05(const void* x, const void* w, void* out, cons
     case EPI_GELU_TANH: return launch<EPI_GELU_TANH>(mx, mw, a, pairs, stream);
     case EPI_RELU2: return launch<EPI_RELU2>(mx, mw, a, pairs, stream);
     case EPI_RELU2_ROUNDED: return launch<EPI_RELU2_ROUNDED>(mx, mw, a, pairs, stream);
+    case EPI_GATED_CLAMP_ROUNDED: return launch<EPI_GATED_CLAMP_ROUNDED>(mx, mw, a, pairs, stream);
+    case EPI_GELU_ROUNDED: return launch<EPI_GELU_ROUNDED>(mx, mw, a, pairs, stream);
+    case EPI_GELU_TANH_ROUNDED: return launch<EPI_GELU_TANH_ROUNDED>(mx, mw, a, pairs, stream);
     case EPI_STORE_F32: return launch<EPI_STORE_F32>(mx, mw, a, pairs, stream);
     case EPI_GATED_CLAMP: return launch<EPI_GATED_CLAMP>(mx, mw, a, pairs, stream);
   }

@@ -450,7 +450,8 @@ extern "C" int odi_moe_combine(const CombineArgs* args, int dtype, cudaStream_t 
   const bool vec = dtype == 1 && a.H % 8 == 0 && ((uintptr_t)a.residual | (uintptr_t)a.expert_out | (uintptr_t)a.input) % 16 == 0;
   if (a.shared != nullptr && (!vec || ((uintptr_t)a.shared | (uintptr_t)a.gate) % 16 != 0)) return ODI_ERR_UNSUPPORTED;
   if (vec) {
-    const int vthreads = a.H >= 2048 ? 256 : (a.H >= 1024 ? 128 : 64);
+    // with a shared expert as many as gated_row_add takes, whose sum of the gate's products this is
+    const int vthreads = a.H >= 2048 ? 256 : (a.H >= 1024 || a.shared != nullptr ? 128 : 64);
     const int vpieces = a.n_tokens >= 512 ? 1 : min(8, (a.H / 8 + vthreads - 1) / vthreads);
     odi_rc = launch_pdl(moe_combine_vec_kernel, dim3(a.n_tokens, vpieces), dim3(vthreads), 0, stream, a);
     return launch_status();

@@ -333,7 +333,8 @@ def gemm_f32_split(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, residual
 EPI_STORE_BF16, EPI_STORE_F32, EPI_RESIDUAL, EPI_SWIGLU, EPI_HEAD_PREP, EPI_GELU, EPI_GEGLU, EPI_RELU2 = 0, 1, 2, 3, 4, 5, 6, 7
 EPI_GATED = (EPI_SWIGLU, EPI_GEGLU)      # two weight rows a feature: the gate rows, then the up rows
 EPI_GATED_CLAMP = 8                      # of gemm_prefill_bf16 alone: what gated_clamp makes of such a product
-EPI_GATED_MANY = EPI_GATED + (EPI_GATED_CLAMP,)
+EPI_GATED_CLAMP_ROUNDED = 9              # the same of the sums as bfloat16 holds them
+EPI_GATED_MANY = EPI_GATED + (EPI_GATED_CLAMP, EPI_GATED_CLAMP_ROUNDED)
 
 _gemm_state = {}
 
@@ -627,7 +628,8 @@ def gemm_prefill_bf16(x: torch.Tensor, w: torch.Tensor, out: Optional[torch.Tens
     """The persistent two-CTA tensor-core product for many tokens (``csrc/gemm_prefill_tcgen05.cu``): clusters
     of two CTAs own tiles of 256 tokens x 256 features (tcgen05.mma.cta_group::2), two accumulators in tensor
     memory so that a tile's epilogue runs under the next tile's MMAs, output by TMA store or fp32 reduce-add.
-    ``EPI_GATED_CLAMP``: :func:`gated_clamp` of the fp32 sums with ``limit``, ``alpha`` and ``up_shift``.
+    ``EPI_GATED_CLAMP``: :func:`gated_clamp` of the fp32 sums with ``limit``, ``alpha`` and ``up_shift``; ``EPI_GATED_CLAMP_ROUNDED``: of the sums
+    rounded to bfloat16, the bits that ``EPI_STORE_BF16`` and :func:`gated_clamp` behind it give.
     ``balance`` (default ``ODI_PREFILL_BALANCE``, 1): with ``EPI_RESIDUAL``, cut every tile's k-blocks into up to four
     parts that different CTA pairs add into the residual, in a fixed order, when that shortens the walk (128 tiles
     on 74 pairs: two rounds whole, 1.75 in quarters); 0 whole tiles always, 2..4 that many parts.
@@ -644,7 +646,7 @@ def gemm_prefill_bf16(x: torch.Tensor, w: torch.Tensor, out: Optional[torch.Tens
         if not gemm_bf16_supported(x, w):
             raise KernelError(f"gemm_prefill_tcgen05 needs K a multiple of 8 and 16-byte aligned operands (K={K})")
     else:
-        if epi not in (EPI_STORE_BF16, EPI_STORE_F32, EPI_RESIDUAL, EPI_SWIGLU, EPI_GELU, EPI_GEGLU, EPI_RELU2, EPI_GATED_CLAMP):
+        if epi not in (EPI_STORE_BF16, EPI_STORE_F32, EPI_RESIDUAL, EPI_GELU, EPI_RELU2) + EPI_GATED_MANY:
             raise KernelError(f"gemm_prefill_bf16 has no epilogue {epi}")
         _require(out, "out", torch.float32 if epi in (EPI_STORE_F32, EPI_RESIDUAL) else torch.bfloat16, 2)
         if w.shape[1] != K or out.shape != (tokens, n_out) or (epi in EPI_GATED_MANY and w_rows % 2):
@@ -1333,6 +1335,7 @@ class _RouteArgs(Structure):
 
 
 _GROUPED_TCGEN05_EPILOGUES = {GROUPED_STORE: 0, GROUPED_GELU_ERF: 1, GROUPED_GELU_TANH: 2, GROUPED_RELU2: 3, GROUPED_GATED_CLAMP: 4, GROUPED_STORE_F32: 5}
+_GROUPED_TCGEN05_ROUNDED = {GROUPED_RELU2: 6, GROUPED_GATED_CLAMP: 7, GROUPED_GELU_ERF: 8, GROUPED_GELU_TANH: 9}
 
 
 def grouped_tcgen05_ok(dtype: torch.dtype, *weights: torch.Tensor) -> bool:
@@ -1346,7 +1349,8 @@ def grouped_gemm_sorted(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, off
     """Rows offsets[e] .. offsets[e + 1] - 1 of ``x`` (bf16, sorted by expert) through ``w[e]`` on the tcgen05 tensor cores, for steps
     whose experts get some dozens of rows and more (:func:`grouped_tcgen05_ok`); out [rows, features] bf16 (fp32 for ``GROUPED_STORE_F32``),
     epilogues of :func:`grouped_gemm_routed`.  ``offsets``: int32 [experts + 1] on the device; rows of ``out`` beyond the last are
-    left as they are.  ``round_sums`` (``GROUPED_RELU2``): the activation of the sums as bfloat16 holds them."""
+    left as they are.  ``round_sums``: the activation of the sums as bfloat16 holds them, with the bits of a product that stores bfloat16
+    and :func:`activation` or :func:`gated_clamp` behind it."""
     _require(x, "x", torch.bfloat16, 2)
     _require(w, "w", torch.bfloat16, 3)
     _require(out, "out", torch.float32 if epi == GROUPED_STORE_F32 else torch.bfloat16, 2)
@@ -1354,13 +1358,13 @@ def grouped_gemm_sorted(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, off
     groups, w_rows, K = w.shape
     n_out = w_rows // 2 if epi == GROUPED_GATED_CLAMP else w_rows
     if (epi not in _GROUPED_TCGEN05_EPILOGUES or x.shape[1] != K or out.shape != (x.shape[0], n_out) or offsets.numel() != groups + 1
-            or (epi == GROUPED_GATED_CLAMP and w_rows % 2) or (round_sums and epi != GROUPED_RELU2)):
+            or (epi == GROUPED_GATED_CLAMP and w_rows % 2) or (round_sums and epi not in _GROUPED_TCGEN05_ROUNDED)):
         raise KernelError(f"grouped product: epilogue {epi}, x {tuple(x.shape)}, w {tuple(w.shape)}, out {tuple(out.shape)}, "
                           f"{offsets.numel()} offsets do not fit")
     _, _, status = _gemm_buffers(w.device, 0)
     lib = load_library("grouped_tcgen05")
     _check(lib.odi_grouped_tcgen05(_ptr(x), _ptr(w), _ptr(out), _ptr(offsets), c_int(x.shape[0]), c_int(groups), c_int(n_out), c_int(K),
-                                   c_int(w_rows), c_int(6 if round_sums else _GROUPED_TCGEN05_EPILOGUES[epi]), c_float(limit), c_float(alpha),
+                                   c_int(w_rows), c_int((_GROUPED_TCGEN05_ROUNDED if round_sums else _GROUPED_TCGEN05_EPILOGUES)[epi]), c_float(limit), c_float(alpha),
                                    c_float(up_shift), _ptr(status), c_int(0), _stream()), "grouped_tcgen05")
 
 

@@ -44,13 +44,13 @@ PERSISTENT_MIN_TOKENS_FUSED, PERSISTENT_MIN_TOKENS_PLAIN = 1024, 2048
 
 
 def _persistent(tokens: int, weight: torch.Tensor, x: torch.Tensor, epi: int, biased: bool = False) -> bool:
-    n_out = weight.shape[0] // 2 if epi in ops.EPI_GATED_MANY else weight.shape[0]
+    n_out = weight.shape[0] // 2 if epi in ops.EPI_GATED else weight.shape[0]
     out_dtype = torch.float32 if epi in (ops.EPI_STORE_F32, ops.EPI_RESIDUAL) else torch.bfloat16
     if PREFILL_GEMM == "library" or not ops.gemm_prefill_supported(x, weight, n_out, out_dtype):
         return False
     if PREFILL_GEMM == "own":
         return True
-    fused = biased or epi in (ops.EPI_SWIGLU, ops.EPI_GEGLU, ops.EPI_GATED_CLAMP, ops.EPI_RESIDUAL, ops.EPI_GELU, ops.EPI_RELU2)      # a bias is a fused epilogue too
+    fused = biased or epi in (ops.EPI_SWIGLU, ops.EPI_GEGLU, ops.EPI_RESIDUAL, ops.EPI_GELU, ops.EPI_RELU2)      # a bias is a fused epilogue too
     return tokens >= (PERSISTENT_MIN_TOKENS_FUSED if fused else PERSISTENT_MIN_TOKENS_PLAIN)
 
 
@@ -355,13 +355,14 @@ def activated_linear(x: torch.Tensor, weight: torch.Tensor, kind: str) -> torch.
 
 def clamped_gated_linear(x: torch.Tensor, weight_gate_up: torch.Tensor, limit: float, alpha: float, up_shift: float = 1.0, *,
                          bias: Optional[torch.Tensor] = None) -> torch.Tensor:
-    """:func:`ops.gated_clamp` of x [Wg; Wu]^T (+ bias), in the dtype of ``x``: in the epilogue of the many-token kernel, on the fp32
-    sums and with one rounding, else by a kernel behind the product."""
+    """:func:`ops.gated_clamp` of x [Wg; Wu]^T (+ bias), in the dtype of ``x``: in the epilogue of the many-token kernel where :func:`linear`
+    takes that kernel for the product, else by a kernel behind it, with the same bits: the gate is of the product as bfloat16 holds it."""
     n, I = x.shape[0], weight_gate_up.shape[0] // 2
     act = x.new_empty((n, I))
     biased = bias is not None
-    if x.dtype == torch.bfloat16 and not _own(x, weight_gate_up, biased) and _persistent(n, weight_gate_up, x, ops.EPI_GATED_CLAMP, biased):
-        ops.gemm_prefill_bf16(x, weight_gate_up, act, ops.EPI_GATED_CLAMP, bias=bias, limit=limit, alpha=alpha, up_shift=up_shift)
+    if x.dtype == torch.bfloat16 and not _own(x, weight_gate_up, biased) and _persistent(n, weight_gate_up, x, ops.EPI_STORE_BF16, biased) \
+            and ops.gemm_prefill_supported(x, weight_gate_up, I, torch.bfloat16):
+        ops.gemm_prefill_bf16(x, weight_gate_up, act, ops.EPI_GATED_CLAMP_ROUNDED, bias=bias, limit=limit, alpha=alpha, up_shift=up_shift)
     else:
         ops.gated_clamp(linear(x, weight_gate_up, bias=bias), act, limit, alpha, up_shift)
     return act

@@ -16,7 +16,7 @@ Steps of ``forward`` (no step waits for the host):
 
 Options of the spec: experts (and the shared one) that are SiLU gates without limits, the same kernels with other
 constants; weights divided by their sum and multiplied by a constant (in the routing kernel); sigmoid scores instead of the softmax (a flag of the routing kernel); ungated experts with the
-squared ReLU (one up matrix per expert, the activation in the grouped product's epilogue, of many rows on the sums as bfloat16 holds them); weights that multiply the experts' inputs (the rows are gathered in the
+squared ReLU (one up matrix per expert); the activation in the grouped product's epilogue, of many rows on the sums as bfloat16 holds them; weights that multiply the experts' inputs (the rows are gathered in the
 sorted order and multiplied by their pair's weight in fp32 on the way, ``ops.moe_gather``; the combine then adds
 the chosen rows unweighted).
 """
@@ -42,9 +42,9 @@ from .linear import clamped_gated_linear, gated_linear, linear
 # bfloat16 both are 1.7e-3).  What that costs, gather and both products with the weights from memory, us, mma.sync / tcgen05, experts of 2,048 and 1,024:
 # 30 of 8 rows 80 / 95, of 16 108 / 95, of 31 170 / 97, four of 30 with all rows 62 / 33, 92 / 37, 157 / 43; 8 experts of 1,024 and 512, 8 rows 18 / 23,
 # 31 rows 29 / 24.  tcgen05 for gate and up alone gains nothing (30 x 16 rows 128, 31 rows 168).
-# Ungated experts' sums, like the shared expert's, are rounded before the squared ReLU (max(z, 0)^2 of a bfloat16 product, as an activation
-# behind it gives): their layers weigh the experts' inputs by a router's scores, and rounded once, after the activation, they moved the logits by
-# 0.027 of their norm where two scores nearly tied.
+# Their first product's sums, like the shared expert's, are rounded before the activation (the bits of a bfloat16 product and an activation
+# behind it): layers route by what such rows leave, and sums rounded once, after the activation, moved logits by 0.027 of their norm where two
+# scores nearly tied.
 ROWS_PER_EXPERT_ROUNDED = 32
 
 
@@ -138,7 +138,7 @@ class RoutedExperts(Part):
                 rows = torch.empty((table.n_pairs, s.hidden_size), dtype=x.dtype, device=dev)
                 ops.moe_gather(x, table, rows, weights if s.weight_on_input else None)
                 ops.grouped_gemm_sorted(rows, self.w_gate_up, act, table.offsets, epi=first_epi, limit=self.limit, alpha=self.gate_alpha,
-                                        up_shift=self.up_shift, round_sums=not self.gated)
+                                        up_shift=self.up_shift, round_sums=True)
                 expert_out = rows           # read by the first product: the outputs, of the same size, take their place
                 ops.grouped_gemm_sorted(act, self.w_down, expert_out, table.offsets, epi=ops.GROUPED_STORE)
             elif many:

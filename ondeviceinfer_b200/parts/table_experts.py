@@ -83,7 +83,7 @@ class TableExperts(Part):
         if rounds_outputs(x.dtype, table, ctx) and ops.grouped_tcgen05_ok(x.dtype, self.w_up, self.w_down):
             rows = torch.empty((table.n_pairs, s.hidden_size), dtype=x.dtype, device=dev)
             ops.moe_gather(x, table, rows)
-            ops.grouped_gemm_sorted(rows, self.w_up, act, table.offsets, epi=GROUPED_EPILOGUE[s.activation])
+            ops.grouped_gemm_sorted(rows, self.w_up, act, table.offsets, epi=GROUPED_EPILOGUE[s.activation], round_sums=True)
             expert_out = rows               # read by the first product: the outputs, of the same size, take their place
             ops.grouped_gemm_sorted(act, self.w_down, expert_out, table.offsets, epi=ops.GROUPED_STORE)
         else:

@@ -613,6 +613,57 @@ def test_gemm_prefill_clamps_and_gates_in_its_epilogue(tokens, I, K, biased):
     assert ops.gemm_status() == 0
 
 
+def every_bf16(seed):
+    """The finite bfloat16 numbers, shuffled."""
+    bits = torch.arange(1 << 16, dtype=torch.int32)
+    values = (bits << 16).view(torch.float32)
+    values = torch.where(torch.isfinite(values), values, torch.ones(()))
+    return values[torch.randperm(1 << 16, generator=torch.Generator().manual_seed(seed))].bfloat16()
+
+
+@pytest.mark.parametrize("epi", ["gelu_erf", "gelu_tanh", "relu2", "clamp", "silu"])
+def test_rounded_sums_give_the_bits_of_the_kernel_behind_the_product(epi):
+    """Every finite bfloat16 number as a sum, and sums of 520 products."""
+    limit, alpha, shift = (6.0, 1.702, 1.0) if epi == "clamp" else (math.inf, 1.0, 0.0)
+    gated = epi in ("clamp", "silu")
+    code = ops.GROUPED_GATED_CLAMP if gated else {"gelu_erf": ops.GROUPED_GELU_ERF, "gelu_tanh": ops.GROUPED_GELU_TANH, "relu2": ops.GROUPED_RELU2}[epi]
+    torch.manual_seed(9)
+    for n, N, K in ((64, 1024, 64), (300, 257, 520)):
+        if K == 64:
+            x = torch.eye(n, K, device=DEV).bfloat16()
+            w = torch.cat([every_bf16(1).view(N, n)] + ([torch.randn(N, n).bfloat16()] if gated else [])).to(DEV)
+        else:
+            x = torch.randn(n, K, device=DEV).bfloat16()
+            w = (torch.randn(2 * N if gated else N, K, device=DEV) * 2 / math.sqrt(K)).bfloat16()
+        offsets = torch.tensor([0, n], dtype=torch.int32, device=DEV)
+        product, got = (torch.empty(n, rows, dtype=torch.bfloat16, device=DEV) for rows in (w.shape[0], N))
+        want = torch.empty_like(got)
+        ops.grouped_gemm_sorted(x, w[None], product, offsets, epi=ops.GROUPED_STORE)
+        ops.grouped_gemm_sorted(x, w[None], got, offsets, epi=code, limit=limit, alpha=alpha, up_shift=shift, round_sums=True)
+        if gated:
+            ops.gated_clamp(product, want, limit, alpha, shift)
+        else:
+            ops.activation(product, want, epi)
+        assert torch.equal(got.view(torch.int16), want.view(torch.int16)), int((got.view(torch.int16) != want.view(torch.int16)).sum())
+    assert ops.gemm_status() == 0
+
+
+@pytest.mark.parametrize("tokens,I,K,biased", [(64, 1024, 64, False), (257, 136, 72, True), (700, 256, 520, False)])
+def test_gemm_prefill_gates_rounded_sums_with_the_bits_of_the_kernel_behind_it(tokens, I, K, biased):
+    torch.manual_seed(tokens)
+    if tokens == K:
+        x, w = torch.eye(K, device=DEV).bfloat16(), torch.cat([every_bf16(2).view(I, K), torch.randn(I, K).bfloat16()]).to(DEV)
+    else:
+        x, w = torch.randn(tokens, K, device=DEV).bfloat16(), (torch.randn(2 * I, K, device=DEV) * 2 / math.sqrt(K)).bfloat16()
+    bias = torch.randn(2 * I, device=DEV) if biased else None
+    product, got = (torch.empty(tokens, rows, dtype=torch.bfloat16, device=DEV) for rows in (2 * I, I))
+    want = torch.empty_like(got)
+    ops.gemm_prefill_bf16(x, w, product, ops.EPI_STORE_BF16, bias=bias)
+    ops.gated_clamp(product, want, 6.0, 1.702, 1.0)
+    ops.gemm_prefill_bf16(x, w, got, ops.EPI_GATED_CLAMP_ROUNDED, bias=bias, limit=6.0, alpha=1.702, up_shift=1.0)
+    assert torch.equal(got.view(torch.int16), want.view(torch.int16)) and ops.gemm_status() == 0
+
+
 # one block of 256 threads up to 2,048 pairs, of 1,024 up to 8,192, three launches beyond
 @pytest.mark.parametrize("tokens,top,experts", [(512, 4, 30), (683, 3, 7), (2731, 3, 300), (4096, 4, 32), (16385, 1, 5)])
 def test_pairs_are_sorted_by_expert(tokens, top, experts):
@@ -715,6 +766,23 @@ def test_a_gated_shared_expert_joins_a_residual_off_16_byte_borders():
         part.forward(x, ctx, residual)
         sums.append(residual.clone())
     torch.testing.assert_close(sums[0], sums[1], atol=4e-6, rtol=4e-6)      # sums of two experts and of the gate's products in another order
+
+
+@pytest.mark.parametrize("H", [64, 520, 1024, 2048])
+def test_combine_with_a_shared_expert_gives_the_bits_of_the_kernel_behind_it(H):
+    torch.manual_seed(H)
+    tokens, top, experts = 5, 2, 3
+    ids = torch.randint(0, experts, (tokens, top), dtype=torch.int32, device=DEV)
+    table = ops.RoutingTable(tokens, top, experts, torch.device(DEV))
+    ops.moe_group(ids, torch.zeros(experts, dtype=torch.int32, device=DEV), table)
+    x, gate = torch.randn(tokens, H, device=DEV).bfloat16(), (torch.randn(H, device=DEV) / math.sqrt(H)).bfloat16()
+    rows, weights, y = torch.randn(tokens * top, H, device=DEV), torch.rand(tokens, top, device=DEV), torch.randn(tokens, H, device=DEV)
+    for assign in (True, False):
+        one, two = (torch.ones(tokens, H, device=DEV) for _ in range(2))
+        ops.moe_combine(one, rows, x, ids, weights, table, assign=assign, shared=(y, gate))
+        ops.moe_combine(two, rows, x, ids, weights, table, assign=assign)
+        ops.gated_row_add(two, y, x, gate)
+        assert torch.equal(one, two)
 
 
 @pytest.mark.parametrize("H", [64, 2056, 20])
