@@ -13,7 +13,7 @@
 //  parts  (every chunk and head at once) leaves wk, q' = G q - B wk, k^ = D_15 k, G_15, wv and B wv;
 //  scan   (a block per sequence, head and COLS value columns) goes through a sequence's chunks in order:
 //             u = wv - wk S;   o = B wv + q' S;   S <- diag(G_15) S + k^T u
-//         the 32 sums of a column over D rows lie on 16 or 32 lanes and are halved side by side, so that a chunk costs one
+//         the 32 sums of a column over D rows lie on 16 lanes and are halved side by side, so that a chunk costs one
 //         chain of shuffles where token by token costs 32.
 // Everything is fp32, as token by token.  A last chunk of fewer tokens is filled with tokens that do nothing (k, q, v
 // and beta 0, g 1).
@@ -147,7 +147,7 @@ __device__ __forceinline__ void dc_cp16(uint32_t dst, const float* src, bool ok)
 
 // The sequence of a block: the blockIdx.z-th longest, so that the blocks of the longest run, which the kernel waits for, are placed
 // first, a multiprocessor each, and the others beside them.  Runs of 333, 769 and 1,777 tokens with 16 heads of 128 in the batch's order,
-// the longest last: its blocks lay two and three to a multiprocessor and took 371 us, 184 by themselves; longest first, with the wider form below, 318.
+// the longest last: its blocks lay two and three to a multiprocessor and took 371 us, 184 by themselves; longest first 354.
 // Beyond 64 sequences in the batch's order: the chip is full either way.
 __device__ __forceinline__ int dc_longest_first(const int* cu_q, int n_seqs, int* chosen) {
   if (n_seqs == 1 || n_seqs > 64) return blockIdx.z;
@@ -164,19 +164,19 @@ __device__ __forceinline__ int dc_longest_first(const int* cu_q, int n_seqs, int
   return *chosen;
 }
 
-// COLS columns of one head's state: CPT of them per group of 16 or 32 lanes, a lane holding rows 4 (lane + LANES j) .. + 3.  dv a
+// COLS columns of one head's state: CPT of them per group of 16 lanes, a lane holding rows 4 (lane + 16 j) .. + 3.  dv a
 // multiple of 4 (16-byte copies of COLS columns).
-template <int D, int COLS, int CPT, int LANES>
-__global__ void __launch_bounds__(COLS / CPT * LANES, 2)
+template <int D, int COLS, int CPT>
+__global__ void __launch_bounds__(COLS / CPT * 16, 2)
 dc_scan_kernel(DeltaChunkArgs a) {
   pdl_wait();
-  constexpr int NTH = COLS / CPT * LANES, NJ = D / (4 * LANES), R = D / LANES;
+  constexpr int NTH = COLS / CPT * 16, NJ = D / 64, R = D / 16;
   constexpr size_t STAGE = DC_STAGE(D, COLS);
-  static_assert(D % (4 * LANES) == 0 && COLS % 4 == 0 && COLS % CPT == 0 && NTH % 32 == 0, "sizes of a block");
+  static_assert(D % 64 == 0 && COLS % 4 == 0 && COLS % CPT == 0 && NTH % 32 == 0, "sizes of a block");
   extern __shared__ __align__(16) float dc_smem[];
   __shared__ int chosen;
   const int seq = dc_longest_first(a.cu_q, a.n_seqs, &chosen), h = blockIdx.y, c0 = blockIdx.x * COLS;
-  const int tid = threadIdx.x, rl = tid & (LANES - 1), rt = tid & 15, col = tid / LANES * CPT;
+  const int tid = threadIdx.x, rl = tid & 15, col = (tid >> 4) * CPT;
   const int q_begin = a.cu_q[seq], q_len = a.cu_q[seq + 1] - q_begin;
   if (q_len <= 0) return;
   const int dv = a.dv, chunks = (q_len + DC - 1) / DC;
@@ -211,7 +211,7 @@ dc_scan_kernel(DeltaChunkArgs a) {
   for (int cc = 0; cc < CPT; ++cc)
 #pragma unroll
     for (int r = 0; r < R; ++r)
-      S[cc][r] = c0 + col + cc < dv ? S_g[(size_t)(4 * (rl + LANES * (r >> 2)) + (r & 3)) * dv + c0 + col + cc] : 0.f;
+      S[cc][r] = c0 + col + cc < dv ? S_g[(size_t)(4 * (rl + 16 * (r >> 2)) + (r & 3)) * dv + c0 + col + cc] : 0.f;
 
   for (int c = 0; c < chunks; ++c) {
     asm volatile("cp.async.wait_group %0;" ::"n"(DC_STAGES(D) - 2) : "memory");
@@ -227,7 +227,7 @@ dc_scan_kernel(DeltaChunkArgs a) {
         for (int cc = 0; cc < CPT; ++cc) sum[cc][t] = 0.f;
 #pragma unroll
         for (int j = 0; j < NJ; ++j) {
-          const float4 x = *(const float4*)(buf + (half * DC + t) * D + 4 * (rl + LANES * j));
+          const float4 x = *(const float4*)(buf + (half * DC + t) * D + 4 * (rl + 16 * j));
 #pragma unroll
           for (int cc = 0; cc < CPT; ++cc)
             sum[cc][t] = fmaf(x.x, S[cc][4 * j], fmaf(x.y, S[cc][4 * j + 1], fmaf(x.z, S[cc][4 * j + 2], fmaf(x.w, S[cc][4 * j + 3], sum[cc][t]))));
@@ -247,10 +247,6 @@ dc_scan_kernel(DeltaChunkArgs a) {
             sum[cc][i] = keep + __shfl_xor_sync(0xffffffffu, give, m);
           }
         }
-      if (LANES == 32) {
-#pragma unroll
-        for (int cc = 0; cc < CPT; ++cc) sum[cc][0] += __shfl_xor_sync(0xffffffffu, sum[cc][0], 16);
-      }
     };
     float wks[CPT][DC], qs[CPT][DC];
     rows_of(0, wks);
@@ -259,17 +255,14 @@ dc_scan_kernel(DeltaChunkArgs a) {
     float4 ahead[DC];      // the first rows' k^ for the state: requested before anything waits for u
 #pragma unroll
     for (int t = 0; t < DC; ++t) ahead[t] = *(const float4*)(buf + (2 * DC + t) * D + 4 * rl);
-    // with 32 lanes the two halves hold the same: one writes the first columns, the other the rest
-    constexpr int MINE = LANES == 32 ? CPT / 2 : CPT;
-    const int first = LANES == 32 ? (rl >> 4) * MINE : 0;
 #pragma unroll
-    for (int cc = 0; cc < MINE; ++cc) xs[(first + cc) * DC + rt] = vs[rt * COLS + col + first + cc] - (first ? wks[(LANES == 32 ? MINE : 0) + cc][0] : wks[cc][0]);
+    for (int cc = 0; cc < CPT; ++cc) xs[cc * DC + rl] = vs[rl * COLS + col + cc] - wks[cc][0];
     over_lanes(qs);
-    if (c * DC + rt < q_len) {
-      float* to = a.o + ((size_t)(q_begin + c * DC + rt) * a.heads + h) * dv + c0 + col + first;
+    if (c * DC + rl < q_len) {
+      float* to = a.o + ((size_t)(q_begin + c * DC + rl) * a.heads + h) * dv + c0 + col;
 #pragma unroll
-      for (int cc = 0; cc < MINE; ++cc)
-        if (c0 + col + first + cc < dv) to[cc] = vs[(DC + rt) * COLS + col + first + cc] + (first ? qs[(LANES == 32 ? MINE : 0) + cc][0] : qs[cc][0]);
+      for (int cc = 0; cc < CPT; ++cc)
+        if (c0 + col + cc < dv) to[cc] = vs[(DC + rl) * COLS + col + cc] + qs[cc][0];
     }
     __syncwarp();
     float u[CPT][DC];
@@ -282,14 +275,14 @@ dc_scan_kernel(DeltaChunkArgs a) {
       }
 #pragma unroll
     for (int j = 0; j < NJ; ++j) {
-      const float4 g = *(const float4*)(buf + 3 * DC * D + 4 * (rl + LANES * j));
+      const float4 g = *(const float4*)(buf + 3 * DC * D + 4 * (rl + 16 * j));
       // the chunk's writes are summed before they join the state: one rounding of the larger number instead of sixteen
       float4 add[CPT];
 #pragma unroll
       for (int cc = 0; cc < CPT; ++cc) add[cc] = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
       for (int t = 0; t < DC; ++t) {
-        const float4 x = j == 0 ? ahead[t] : *(const float4*)(buf + (2 * DC + t) * D + 4 * (rl + LANES * j));
+        const float4 x = j == 0 ? ahead[t] : *(const float4*)(buf + (2 * DC + t) * D + 4 * (rl + 16 * j));
 #pragma unroll
         for (int cc = 0; cc < CPT; ++cc) {
           add[cc].x = fmaf(x.x, u[cc][t], add[cc].x); add[cc].y = fmaf(x.y, u[cc][t], add[cc].y);
@@ -309,29 +302,29 @@ dc_scan_kernel(DeltaChunkArgs a) {
   for (int cc = 0; cc < CPT; ++cc)
 #pragma unroll
     for (int r = 0; r < R; ++r)
-      if (c0 + col + cc < dv) S_g[(size_t)(4 * (rl + LANES * (r >> 2)) + (r & 3)) * dv + c0 + col + cc] = S[cc][r];
+      if (c0 + col + cc < dv) S_g[(size_t)(4 * (rl + 16 * (r >> 2)) + (r & 3)) * dv + c0 + col + cc] = S[cc][r];
 }
 
-// Columns a block and a thread, lanes a column.  The scan is bound by the pipe of shared memory: a 16-byte read of a warp takes it four
-// clocks also where half of its lanes read the same, a shuffle about three.  More columns a thread read the chunk's rows fewer times, but
-// the chain of one chunk gets longer; so the narrow form serves as long as its blocks have a multiprocessor (heads of 64: two blocks share
-// one) to themselves.  Measured, us, 16 heads, narrow / wide: heads of 64, 2,048 tokens 106 / 167, 1,024 + 2,048 122 / 167, 4 x 2,048
-// 233 / 207 (before, with fewer requests ahead of their use: 169, 180, 245); heads of 128, 1,777 tokens 180 / 188, 333 + 769 + 1,777
-// 354 / 318, 2 x 1,777 340 / 325 (before 184, 371, 319).
-template <int D, int COLS, int CPT, int LANES>
+// Columns a block and a thread.  The scan is bound by the pipe of shared memory: a 16-byte read of a warp takes it four clocks also where half
+// of its lanes read the same, a shuffle about three.  More columns a thread read the chunk's rows fewer times, but the chain of one chunk gets
+// longer; so heads of 64 take the narrow form as long as two of its blocks a multiprocessor hold all.  A column's sums have the same order in
+// either form: they depend neither on it nor on the batch.  Measured, us, 16 heads, narrow / wide: heads of 64, 2,048 tokens 106 / 167, 1,024 + 2,048
+// 122 / 167, 4 x 2,048 233 / 207 (before, with fewer requests ahead of their use: 169, 180, 245); heads of 128, narrow: 1,777 tokens 180, 333 + 769
+// + 1,777 354, 2 x 1,777 340 (before 184, 371, 319; the pass of four layers 1,714 -> 1,630, 2,825 -> 2,641, 3,011 -> 2,911).  A form with 32 lanes a
+// column for heads of 128 took 318 and 325 of the last two, 3 and 1 % of the pass, but summed in another order.
+template <int D, int COLS, int CPT>
 static int dc_launch_form(const DeltaChunkArgs& a, cudaStream_t stream) {
   constexpr size_t smem = sizeof(float) * (DC_STAGES(D) * DC_STAGE(D, COLS) + COLS * DC);
-  auto kernel = dc_scan_kernel<D, COLS, CPT, LANES>;
+  auto kernel = dc_scan_kernel<D, COLS, CPT>;
   const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return (int)e;
   // an ordinary launch: started early, while the kernel before still holds multiprocessors, the few long blocks of a
   // single sequence would be packed several to one and stay there
-  kernel<<<dim3((a.dv + COLS - 1) / COLS, a.heads, a.n_seqs), dim3(COLS / CPT * LANES), smem, stream>>>(a);
+  kernel<<<dim3((a.dv + COLS - 1) / COLS, a.heads, a.n_seqs), dim3(COLS / CPT * 16), smem, stream>>>(a);
   return (int)cudaPeekAtLastError();
 }
 template <int D>
 static int dc_launch(const DeltaChunkArgs& a, cudaStream_t stream) {
-  constexpr int COLS = D == 64 ? 8 : 16, BLOCKS = D == 64 ? 296 : 148;
-  if ((long)((a.dv + COLS - 1) / COLS) * a.heads * a.n_seqs <= BLOCKS) return dc_launch_form<D, COLS, 2, 16>(a, stream);
-  return dc_launch_form<D, 16, 4, D == 64 ? 16 : 32>(a, stream);
+  if (D == 64 && (long)((a.dv + 7) / 8) * a.heads * a.n_seqs <= 296) return dc_launch_form<D, 8, 2>(a, stream);
+  return dc_launch_form<D, 16, D == 64 ? 4 : 2>(a, stream);
 }

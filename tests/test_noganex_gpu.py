@@ -451,6 +451,37 @@ def test_delta_rule_in_chunks_of_tokens(dtype, heads, kv_heads, d, dv, taps):
 
 
 @pytest.mark.parametrize("d", [64, 128])
+def test_chunks_of_a_run_have_the_same_bits_beside_others(d):
+    """16 heads: a run by itself has a multiprocessor for each block of the scan, four runs have not."""
+    gen = torch.Generator().manual_seed(d)
+    heads, lens, taps = 16, [301, 64, 517, 130], 4
+    C, v = 3 * heads * d, heads * d
+    proj, ab = (torch.randn(sum(lens), n, generator=gen).cuda() for n in (C + v, 2 * heads))
+    proj = proj.bfloat16()
+    weights = (torch.randn(taps, C, generator=gen) * 0.5, torch.log(0.03 + torch.rand(heads, generator=gen)),
+               torch.randn(heads, generator=gen) * 0.5 - 1, 1 + 0.1 * torch.randn(d, generator=gen))
+    weights = [w.cuda() for w in weights]
+
+    def run(first, lens):
+        cu = [0]
+        for n in lens:
+            cu.append(cu[-1] + n)
+        state, conv_state = torch.zeros(4, heads, d, d, device="cuda"), torch.zeros(4, taps - 1, C, device="cuda")
+        out = torch.empty(cu[-1], v, dtype=torch.bfloat16, device="cuda")
+        ops.head_delta(proj[first:first + cu[-1]], ab[first:first + cu[-1]], *weights, conv_state, state, out, ints(*cu),
+                       ints(*[s for s, n in enumerate(lens) for _ in range(n)]), ints(*range(len(lens))), n_seqs=len(lens), max_q_len=max(lens),
+                       heads=heads, kv_heads=heads, d=d, dv=d, eps=1e-5, unit_eps=1e-6, in_chunks=True)
+        return out, state
+
+    out, state = run(0, lens)
+    at = 0
+    for i, n in enumerate(lens):
+        alone, alone_state = run(at, [n])
+        assert torch.equal(alone, out[at:at + n]) and torch.equal(alone_state[0], state[i])
+        at += n
+
+
+@pytest.mark.parametrize("d", [64, 128])
 def test_chunks_are_no_further_off_than_four_tokens_at_a_time(d):
     """Read-outs of runs with memories of a few to a thousand tokens, against the recurrence in 64 bits, three seeds together."""
     heads, T, off = 8, 300, {True: 0.0, False: 0.0}
