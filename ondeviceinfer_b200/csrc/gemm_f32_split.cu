@@ -667,14 +667,16 @@ extern "C" int odi_gemm_f32_split(const float* x, const float* w, float* out, co
   if (scratch == nullptr || (size_t)scratch_bytes < p.bytes) return ODI_ERR_ARGUMENT;
   const long units = (long)p.full * p.m_tiles + (long)p.rest * p.splits * p.m_tiles;
   if (units > 0x3fffffffL || 3L * M > 0x7fffffffL) return ODI_ERR_UNSUPPORTED;
-  static thread_local int sms = 0;
-  if (sms == 0) {
-    int device = 0;
-    cudaError_t e = cudaGetDevice(&device);
-    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+  static thread_local int sms = 0, known = -1;      // of the device that this thread launched on last: the attribute is the device's
+  int device = 0;
+  cudaError_t e = cudaGetDevice(&device);
+  if (e == cudaSuccess && device != known) {
+    known = -1;
+    e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(gemm_f32_split_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024 - 1024);
-    if (e != cudaSuccess) { sms = 0; return (int)e; }
+    if (e == cudaSuccess) known = device;
   }
+  if (e != cudaSuccess) return (int)e;
   uint8_t* base = (uint8_t*)scratch;
   F32SplitArgs a;
   a.x = x; a.w = w; a.out = out; a.res = res; a.bias = bias; a.status = status; a.withheld = withheld;

@@ -436,29 +436,28 @@ static int make_map(CUtensorMap* map, CUtensorMapDataType type, int elem_bytes, 
   return r == CUDA_SUCCESS ? 0 : ODI_ERR_ARGUMENT;
 }
 
-
-static int device_pairs(int* pairs) {
-  static thread_local int known = 0;
-  if (known == 0) {
-    int device = 0, sms = 0;
-    cudaError_t e = cudaGetDevice(&device);
-    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
-    if (e != cudaSuccess) return (int)e;
-    known = sms / 2;
+// Of the current device; what is known is of the device that this thread asked for last.
+static int device_pairs(int* device, int* pairs) {
+  static thread_local int known = -1, sms = 0;
+  cudaError_t e = cudaGetDevice(device);
+  if (e == cudaSuccess && *device != known) {
+    known = -1;
+    e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, *device);
+    if (e == cudaSuccess) known = *device;
   }
-  *pairs = known;
-  return 0;
+  *pairs = sms / 2;
+  return (int)e;
 }
 
 template <int EPI>
-static int launch(const CUtensorMap& mx, const CUtensorMap& mw, const ExpertsArgs& a, int pairs, cudaStream_t stream) {
+static int launch(const CUtensorMap& mx, const CUtensorMap& mw, const ExpertsArgs& a, int device, int pairs, cudaStream_t stream) {
   auto kernel = grouped_tcgen05_kernel<EPI>;
   constexpr int SMEM = STAGES * STAGE_BYTES + 1024;
-  static thread_local bool configured = false;
-  if (!configured) {
+  static thread_local int configured = -1;      // the attribute is the device's
+  if (device != configured) {
     const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
     if (e != cudaSuccess) return (int)e;
-    configured = true;
+    configured = device;
   }
   odi_rc = launch_pdl(kernel, dim3(2 * pairs), dim3(THREADS), SMEM, stream, mx, mw, a);
   return launch_status();
@@ -473,8 +472,8 @@ extern "C" int odi_grouped_tcgen05(const void* x, const void* w, void* out, cons
   const bool gate = EPI_IS_GATED(epi);
   if (K <= 0 || status == nullptr || offsets == nullptr || groups < 1 || (gate ? w_rows != 2 * n_out : w_rows != n_out)) return ODI_ERR_ARGUMENT;
   if (K % 8 || ((uintptr_t)x & 15) || ((uintptr_t)w & 15) || ((uintptr_t)out & 3) || groups > MAX_GROUPS) return ODI_ERR_UNSUPPORTED;
-  int pairs = 0;
-  int rc = device_pairs(&pairs);
+  int device = 0, pairs = 0;
+  int rc = device_pairs(&device, &pairs);
   if (rc != 0) return rc;
   ExpertsArgs a = {};
   a.out = out; a.status = status; a.offsets = offsets; a.N = n_out; a.K = K; a.w_rows = w_rows; a.groups = groups;
@@ -486,16 +485,16 @@ extern "C" int odi_grouped_tcgen05(const void* x, const void* w, void* out, cons
   if (rc == 0) rc = make_map(&mw, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, w, (long)groups * w_rows, K, K, BF / 2);
   if (rc != 0) return rc;
   switch (epi) {
-    case EPI_STORE_BF16: return launch<EPI_STORE_BF16>(mx, mw, a, pairs, stream);
-    case EPI_GELU: return launch<EPI_GELU>(mx, mw, a, pairs, stream);
-    case EPI_GELU_TANH: return launch<EPI_GELU_TANH>(mx, mw, a, pairs, stream);
-    case EPI_RELU2: return launch<EPI_RELU2>(mx, mw, a, pairs, stream);
-    case EPI_RELU2_ROUNDED: return launch<EPI_RELU2_ROUNDED>(mx, mw, a, pairs, stream);
-    case EPI_GATED_CLAMP_ROUNDED: return launch<EPI_GATED_CLAMP_ROUNDED>(mx, mw, a, pairs, stream);
-    case EPI_GELU_ROUNDED: return launch<EPI_GELU_ROUNDED>(mx, mw, a, pairs, stream);
-    case EPI_GELU_TANH_ROUNDED: return launch<EPI_GELU_TANH_ROUNDED>(mx, mw, a, pairs, stream);
-    case EPI_STORE_F32: return launch<EPI_STORE_F32>(mx, mw, a, pairs, stream);
-    case EPI_GATED_CLAMP: return launch<EPI_GATED_CLAMP>(mx, mw, a, pairs, stream);
+    case EPI_STORE_BF16: return launch<EPI_STORE_BF16>(mx, mw, a, device, pairs, stream);
+    case EPI_GELU: return launch<EPI_GELU>(mx, mw, a, device, pairs, stream);
+    case EPI_GELU_TANH: return launch<EPI_GELU_TANH>(mx, mw, a, device, pairs, stream);
+    case EPI_RELU2: return launch<EPI_RELU2>(mx, mw, a, device, pairs, stream);
+    case EPI_RELU2_ROUNDED: return launch<EPI_RELU2_ROUNDED>(mx, mw, a, device, pairs, stream);
+    case EPI_GATED_CLAMP_ROUNDED: return launch<EPI_GATED_CLAMP_ROUNDED>(mx, mw, a, device, pairs, stream);
+    case EPI_GELU_ROUNDED: return launch<EPI_GELU_ROUNDED>(mx, mw, a, device, pairs, stream);
+    case EPI_GELU_TANH_ROUNDED: return launch<EPI_GELU_TANH_ROUNDED>(mx, mw, a, device, pairs, stream);
+    case EPI_STORE_F32: return launch<EPI_STORE_F32>(mx, mw, a, device, pairs, stream);
+    case EPI_GATED_CLAMP: return launch<EPI_GATED_CLAMP>(mx, mw, a, device, pairs, stream);
   }
   return ODI_ERR_ARGUMENT;
 }

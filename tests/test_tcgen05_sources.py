@@ -44,6 +44,15 @@ def test_the_kernels_that_issue_are_all_here():
     assert ISSUING == ["attention_tcgen05.cu", "gemm_f32_split.cu", "gemm_prefill_tcgen05.cu", "gemm_tcgen05.cu", "grouped_tcgen05.cu"]
 
 
+@pytest.mark.parametrize("name", ["gemm_f32_split.cu", "grouped_tcgen05.cu"])
+def test_shared_memory_is_asked_for_on_every_device(name):
+    """The limit of a kernel's shared memory is the device's: a thread that goes on to another one has to set it there too."""
+    text = _code(name)
+    assert text.count("cudaFuncSetAttribute(") == 1
+    condition = re.findall(r"if \(([^{]*)\) \{", text[:text.index("cudaFuncSetAttribute(")])[-1]
+    assert re.search(r"\bdevice != \w+", condition) and "cudaGetDevice(" in text
+
+
 def test_a_product_without_rows_needs_no_scratch():
     """The plan divides by the tiles of rows: a call without any has to come back, not end the process."""
     script = ("from ctypes import c_long\n"
