@@ -12,12 +12,10 @@
 //               their columns through shared memory, so that each finishes half
 // The tiles are dealt out in turn, an expert's together: those that run side by side share its weights and rows in L2.
 //
-// What bounds it: few rows an expert, the weights' bytes; many, its way from L2 (a stage of 256 rows moves 64 KB per 512 clocks of math).
-// Measured, us, 30 experts of 2,048 -> 2 x 1,024 gated and 1,024 -> 2,048, this against the vendor library's grouped product (and the gate's
-// kernel behind it), rows an expert 16: 48 + 27 / 69 + 39 (mma.sync form: 121 for both), 64: 55 + 31 / 75 + 39, 256: 67 + 40 / 95 + 43,
-// 533: 140 + 70 / 164 + 71.  With the gate's division in IEEE form and each 16 columns waited for before they were worked on, 256 rows took
-// 102 + 43.
-//
+// What bounds it: few rows an expert, the weights' bytes (64 rows 0.72 of the copy bandwidth); many, no one pipe: 41 % of the tensor pipe and
+// 34 % of L2 at 273 rows.  Measured, us, operands from memory, 30 experts of 2,048 -> 2 x 1,024 gated (sums rounded first) and 1,024 -> 2,048, this against
+// the vendor library's grouped product and the gate's kernel behind it, rows an expert 64: 68 + 40 / 85 + 51, 256: 84 + 47 / 91 + 50, 533:
+// 147 + 78 / 153 + 76.  Without a gate the first product of 533 rows takes 137, with the rounded GELU 158.
 #include <cuda.h>
 
 #include "common.cuh"
