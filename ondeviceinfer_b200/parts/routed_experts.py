@@ -42,7 +42,7 @@ from .linear import clamped_gated_linear, gated_linear, linear
 # bfloat16 both are 1.7e-3).  What that costs, gather and both products with the weights from memory, us, mma.sync / tcgen05, experts of 2,048 and 1,024:
 # 30 of 8 rows 80 / 95, of 16 108 / 95, of 31 170 / 97, four of 30 with all rows 62 / 33, 92 / 37, 157 / 43; 8 experts of 1,024 and 512, 8 rows 18 / 23,
 # 31 rows 29 / 24.  tcgen05 for gate and up alone gains nothing (30 x 16 rows 128, 31 rows 168).
-# Their first product's sums, like the shared expert's, are rounded before the activation (the bits of a bfloat16 product and an activation
+# On tcgen05 the first product's sums, like the shared expert's, are rounded before the activation (the bits of a bfloat16 product and an activation
 # behind it): layers route by what such rows leave, and sums rounded once, after the activation, moved logits by 0.027 of their norm where two
 # scores nearly tied.
 ROWS_PER_EXPERT_ROUNDED = 32
