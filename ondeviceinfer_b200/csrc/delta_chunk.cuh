@@ -147,7 +147,7 @@ __device__ __forceinline__ void dc_cp16(uint32_t dst, const float* src, bool ok)
 
 // The sequence of a block: the blockIdx.z-th longest, so that the blocks of the longest run, which the kernel waits for, are placed
 // first, a multiprocessor each, and the others beside them.  Runs of 333, 769 and 1,777 tokens with 16 heads of 128 in the batch's order,
-// the longest last: its blocks lay two and three to a multiprocessor and took 371 us, 184 by themselves; longest first 354.
+// the longest last: its blocks lay two and three to a multiprocessor and took 371 us, 184 by themselves.
 // Beyond 64 sequences in the batch's order: the chip is full either way.
 __device__ __forceinline__ int dc_longest_first(const int* cu_q, int n_seqs, int* chosen) {
   if (n_seqs == 1 || n_seqs > 64) return blockIdx.z;
@@ -174,8 +174,10 @@ dc_scan_kernel(DeltaChunkArgs a) {
   constexpr size_t STAGE = DC_STAGE(D, COLS);
   static_assert(D % 64 == 0 && COLS % 4 == 0 && COLS % CPT == 0 && NTH % 32 == 0, "sizes of a block");
   extern __shared__ __align__(16) float dc_smem[];
-  __shared__ int chosen;
-  const int seq = dc_longest_first(a.cu_q, a.n_seqs, &chosen), h = blockIdx.y, c0 = blockIdx.x * COLS;
+  // behind the chunks, not a variable of its own: 16 static bytes put every row of the chunks across one more 128-byte line of shared memory
+  // (the mixer of two runs of 1,777 tokens, heads of 128: 601 us against 549)
+  int* chosen = (int*)(dc_smem + DC_STAGES(D) * STAGE + COLS * DC);
+  const int seq = dc_longest_first(a.cu_q, a.n_seqs, chosen), h = blockIdx.y, c0 = blockIdx.x * COLS;
   const int tid = threadIdx.x, rl = tid & 15, col = (tid >> 4) * CPT;
   const int q_begin = a.cu_q[seq], q_len = a.cu_q[seq + 1] - q_begin;
   if (q_len <= 0) return;
@@ -252,9 +254,6 @@ dc_scan_kernel(DeltaChunkArgs a) {
     rows_of(0, wks);
     rows_of(1, qs);
     over_lanes(wks);
-    float4 ahead[DC];      // the first rows' k^ for the state: requested before anything waits for u
-#pragma unroll
-    for (int t = 0; t < DC; ++t) ahead[t] = *(const float4*)(buf + (2 * DC + t) * D + 4 * rl);
 #pragma unroll
     for (int cc = 0; cc < CPT; ++cc) xs[cc * DC + rl] = vs[rl * COLS + col + cc] - wks[cc][0];
     over_lanes(qs);
@@ -282,7 +281,7 @@ dc_scan_kernel(DeltaChunkArgs a) {
       for (int cc = 0; cc < CPT; ++cc) add[cc] = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
       for (int t = 0; t < DC; ++t) {
-        const float4 x = j == 0 ? ahead[t] : *(const float4*)(buf + (2 * DC + t) * D + 4 * (rl + 16 * j));
+        const float4 x = *(const float4*)(buf + (2 * DC + t) * D + 4 * (rl + 16 * j));
 #pragma unroll
         for (int cc = 0; cc < CPT; ++cc) {
           add[cc].x = fmaf(x.x, u[cc][t], add[cc].x); add[cc].y = fmaf(x.y, u[cc][t], add[cc].y);
@@ -308,13 +307,13 @@ dc_scan_kernel(DeltaChunkArgs a) {
 // Columns a block and a thread.  The scan is bound by the pipe of shared memory: a 16-byte read of a warp takes it four clocks also where half
 // of its lanes read the same, a shuffle about three.  More columns a thread read the chunk's rows fewer times, but the chain of one chunk gets
 // longer; so heads of 64 take the narrow form as long as two of its blocks a multiprocessor hold all.  A column's sums have the same order in
-// either form: they depend neither on it nor on the batch.  Measured, us, 16 heads, narrow / wide: heads of 64, 2,048 tokens 106 / 167, 1,024 + 2,048
-// 122 / 167, 4 x 2,048 233 / 207 (before, with fewer requests ahead of their use: 169, 180, 245); heads of 128, narrow: 1,777 tokens 180, 333 + 769
-// + 1,777 354, 2 x 1,777 340 (before 184, 371, 319; the pass of four layers 1,714 -> 1,630, 2,825 -> 2,641, 3,011 -> 2,911).  A form with 32 lanes a
-// column for heads of 128 took 318 and 325 of the last two, 3 and 1 % of the pass, but summed in another order.
+// either form: they depend neither on it nor on the batch.  Measured, us, the scan, 16 heads of 64, narrow / wide: 2,048 tokens 106 / 167,
+// 1,024 + 2,048 122 / 167, 4 x 2,048 233 / 207.  The whole mixer, with the copies' loops rolled and runs in the batch's order / now: heads of 64, 2,048
+// tokens 264 / 194, 1,024 + 2,048 318 / 246, 4 x 1,500 430 / 386; heads of 128, 1,777 tokens 322 / 299, 2 x 1,777 576 / 549, 333 + 769 + 1,777
+// 584 / 511, 3 x 1,000 475 / 455, 4 x 512 327 / 315.  32 lanes a column for many heads of 128 gained less than that and summed in another order.
 template <int D, int COLS, int CPT>
 static int dc_launch_form(const DeltaChunkArgs& a, cudaStream_t stream) {
-  constexpr size_t smem = sizeof(float) * (DC_STAGES(D) * DC_STAGE(D, COLS) + COLS * DC);
+  constexpr size_t smem = sizeof(float) * (DC_STAGES(D) * DC_STAGE(D, COLS) + COLS * DC + 4);
   auto kernel = dc_scan_kernel<D, COLS, CPT>;
   const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return (int)e;
@@ -325,6 +324,7 @@ static int dc_launch_form(const DeltaChunkArgs& a, cudaStream_t stream) {
 }
 template <int D>
 static int dc_launch(const DeltaChunkArgs& a, cudaStream_t stream) {
-  if (D == 64 && (long)((a.dv + 7) / 8) * a.heads * a.n_seqs <= 296) return dc_launch_form<D, 8, 2>(a, stream);
+  if constexpr (D == 64)
+    if ((long)((a.dv + 7) / 8) * a.heads * a.n_seqs <= 296) return dc_launch_form<D, 8, 2>(a, stream);
   return dc_launch_form<D, 16, D == 64 ? 4 : 2>(a, stream);
 }
