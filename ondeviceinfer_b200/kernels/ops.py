@@ -1767,8 +1767,8 @@ class _DeltaArgs(Structure):
 
 
 # Delta rules over runs of tokens go 16 tokens at a time (csrc/delta_chunk.cuh) when a sequence brings this many on average
-# (24 tokens: 37 us in chunks, 35 token by token; 8 x 24: 56 and 42; 64: 46 and 62; times of the scan before its requests went ahead of
-# their use, which made it up to 1.6 times as fast: the line may lie lower now).
+# (24 tokens: 37 us in chunks, 35 token by token; 8 x 24: 56 and 42; 64: 46 and 62; times of the scan before its copies' loops were
+# unrolled, which made the mixer up to 1.36 times as fast: the line may lie lower now).
 DELTA_CHUNK, DELTA_CHUNK_MIN_RUN, DELTA_CHUNK_MAX_SCRATCH = 16, 40, 1 << 30
 
 
@@ -1858,8 +1858,8 @@ HEAD_DELTA_MAX_DIM, HEAD_DELTA_MAX_TAPS = 512, 16
 # 1,000 + 500 529 and 493, 800 285 and 285).  Measured against four tokens at a time, the mixer, us: 16 heads of 128 x 128, one
 # sequence of 2,048 tokens 338 and 431, 800 140 and 178, 192 49 and 53 (4 heads 46 and 45); 333 + 769 + 1,777 tokens 553 and 598; 8 x
 # 512 543 and 428; heads of 64 x 64: 2,048 247 and 368, 333 + 769 + 1,777 283 and 492, 8 x 512 261 and 229.  All times of chunks here are
-# of the scan before its requests went ahead and the longest run came first (of 333 + 769 + 1,777 tokens 371 us, 354 since): the lines may lie
-# higher now.
+# of the scan before its copies' loops were unrolled and the longest run came first (the mixer of 333 + 769 + 1,777 tokens by itself 584 us then,
+# 517 now, of 2,048 tokens with heads of 64 264 and 194): the lines may lie higher now.
 HEAD_DELTA_CHUNK_MAX_HEADS, HEAD_DELTA_CHUNK_MIN_RUN, HEAD_DELTA_CHUNK_MAX_LONGEST = 64, 224, 32
 
 
